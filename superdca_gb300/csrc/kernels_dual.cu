@@ -25,7 +25,6 @@
 #include "df.cuh"
 #include "engine.h"
 #include "kernels_common.cuh"
-#include "lbfgs_host.h"
 #include "linesearch.h"
 
 namespace sdca {
@@ -1030,8 +1029,57 @@ __device__ void write_summary(const DualCtl &S, DualSum &o)
     for (int a = 0; a < Q; ++a) o.eta_x[a] = S.eta_x[a];
 }
 
+// The compact-form coefficients of lbfgs_host.h by one warp: lane a holds
+// row a of the small systems, so a substitution step is one multiply-add on
+// every lane and one broadcast instead of a chain over the row.  A thread
+// working alone waits for the FP64 pipe's latency some 200 times at k = 10:
+// the control kernel took 42 us whatever the number of slots (64 slots of
+// 1000 x 4001, 512 of 3000 x 94,000), most of it here; with the warp's lanes
+// the kernel takes 21 us.  Divisions by the diagonal are a multiplication by
+// its reciprocal and one residual correction (the quotient to the last bit
+// or two).  R, YY, sg, yg: shared memory, as there.  False (on every lane)
+// if R is singular; else lane a < k holds coefS[a], coefY[a].
+__device__ __forceinline__ bool warp_compact_coeffs(int k, const double *R, const double *YY, const double *sg,
+                                                    const double *yg, double gamma, double &coefS, double &coefY)
+{
+    const int lane = threadIdx.x & 31, a = lane < k ? lane : 0;
+    const double diag = R[a * k + a];
+    if (__any_sync(0xffffffffu, !(diag != 0.0))) return false;
+    const double inv = 1.0 / diag;
+    auto quotient = [&](double v) {
+        const double q = v * inv;
+        return fma(fma(-q, diag, v), inv, q);
+    };
+    // t = R^-1 sg (back substitution)
+    double v = sg[a], t = 0.0;
+    for (int j = k - 1; j >= 0; --j) {
+        const double tj = __shfl_sync(0xffffffffu, quotient(v), j);
+        if (lane == j) t = tj;
+        if (lane < j) v = fma(-R[a * k + j], tj, v);
+    }
+    // w = (D + gamma YY) t - gamma yg
+    double w0 = 0.0, w1 = 0.0;
+    int j = 0;
+    for (; j + 1 < k; j += 2) {
+        w0 = fma(YY[a * k + j], __shfl_sync(0xffffffffu, t, j), w0);
+        w1 = fma(YY[a * k + j + 1], __shfl_sync(0xffffffffu, t, j + 1), w1);
+    }
+    if (j < k) w0 = fma(YY[a * k + j], __shfl_sync(0xffffffffu, t, j), w0);
+    v = fma(diag, t, gamma * ((w0 + w1) - yg[a]));
+    // p = R^-T w (forward substitution)
+    double p = 0.0;
+    for (j = 0; j < k; ++j) {
+        const double pj = __shfl_sync(0xffffffffu, quotient(v), j);
+        if (lane == j) p = pj;
+        if (lane > j && lane < k) v = fma(-R[j * k + a], pj, v);
+    }
+    coefS = -p;
+    coefY = gamma * t;
+    return true;
+}
+
 // After the gradient pass: the L-BFGS bookkeeping of one slot per warp, in
-// FP64 by lane 0 on a shared-memory copy of the slot's state (SuperDCA's
+// FP64 on a shared-memory copy of the slot's state (SuperDCA's
 // LbfgsSolver iteration, driven from plmDCA.hpp:298-304; stop on max|g| <
 // threshold or the iteration limit, plmDCA.hpp:218-221):
 //   h gradient from the residual sums, the (s, y) pair kept when
@@ -1049,108 +1097,140 @@ k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32
     const int b = list[blockIdx.x];
     __shared__ DualCtl S;
     __shared__ double s_eg[Q], s_dt[2 * MAXHIST], s_R[MAXHIST * MAXHIST], s_YY[MAXHIST * MAXHIST];
+    __shared__ double s_dots[4 * MAXHIST];
     __shared__ int s_go;
+    const int lane = threadIdx.x;
     {
+        // every load of the slot in flight at once
         const unsigned long long *src = reinterpret_cast<const unsigned long long *>(ctl + b);
         unsigned long long *dst = reinterpret_cast<unsigned long long *>(&S);
-        for (int k = threadIdx.x; k < CTL_WORDS; k += 32) dst[k] = src[k];
+        const double *dp = dots + (int64_t)b * 4 * MAXHIST;
+#pragma unroll
+        for (int k = lane; k < CTL_WORDS; k += 32) dst[k] = src[k];
+#pragma unroll
+        for (int k = lane; k < 4 * MAXHIST; k += 32) s_dots[k] = dp[k];
     }
-    if (threadIdx.x == 0) s_go = 0;
+    const double *ac = acc + (int64_t)b * NACC;
+    const double a_rs = lane < Q ? ac[ACC_RS0 + lane] : 0.0;
+    const double a_f = ac[ACC_F], a_g2 = ac[ACC_G2], a_x2J = ac[ACC_X2J], a_sy = ac[ACC_SY], a_yy = ac[ACC_YY],
+                 a_ss = ac[ACC_SS], mg = amax[2 * b], mx = amax[2 * b + 1];
+    if (lane == 0) s_go = 0;
     __syncwarp();
     int &go = s_go;
-    if (threadIdx.x == 0 && S.phase != DC_STOP) {
-        const double *ac = acc + (int64_t)b * NACC;
+    if (S.phase != DC_STOP) {
         const bool init = S.phase == DC_EVAL0;
-        if (!init) {
-            // the accepted step's h part: x_h += stp d_h, s_h
-            for (int a = 0; a < Q; ++a) {
-                const double xn = S.eta_x[a] + S.stp * S.eta_d[a];
-                if (S.push && S.ring_new >= 0) S.eta_s[S.ring_new][a] = xn - S.eta_x[a];
-                S.eta_x[a] = xn;
-            }
-        }
-        const int gn = 1 - S.gcur;
-        double eg[Q];
-        for (int a = 0; a < Q; ++a) eg[a] = ac[ACC_RS0 + a] + 2.0 * lambda_h * S.eta_x[a];
         const bool pushed = S.push && S.ring_new >= 0;
-        if (pushed)
-            for (int a = 0; a < Q; ++a) S.eta_y[S.ring_new][a] = eg[a] - S.eta_g[S.gcur][a];
-        for (int a = 0; a < Q; ++a) S.eta_g[gn][a] = eg[a];
-        S.gcur = gn;
-        S.g2J = ac[ACC_G2];
-        S.g2 = S.g2J + dot4d(eg, eg);
-        S.x2J = ac[ACC_X2J];
-        const double x2H = dot4d(S.eta_x, S.eta_x);
-        S.amax_g = amax[2 * b];
-        S.amax_x = amax[2 * b + 1];
-        const double gnorm = sqrt(fmax(S.g2, 0.0));
-        S.gmax = S.chk_ratio > 0.0 ? S.chk_ratio * gnorm : gnorm;   // estimate until checked
-        bool st = false;
-        if (init) {
-            S.f = ac[ACC_F] + lambda_J * S.x2J + lambda_h * x2H;
-            S.nfeval = 1;
-        } else {
-            S.iterations++;
-            S.nfeval += 2 + S.trials;
-            const int pr = S.ring_new >= 0 ? S.ring_new : 0;
-            const double sy = ac[ACC_SY] + (pushed ? dot4d(S.eta_s[pr], S.eta_y[pr]) : 0.0);
-            const double yy = ac[ACC_YY] + (pushed ? dot4d(S.eta_y[pr], S.eta_y[pr]) : 0.0);
-            const double ss = ac[ACC_SS] + (pushed ? dot4d(S.eta_s[pr], S.eta_s[pr]) : 0.0);
-            if (pushed && sy > 1e-3 * sqrt(ss * yy) && yy > 0.0 && isfinite(sy) && isfinite(yy)) {
-                if (S.nhist == m) {
-                    for (int j = 1; j < m; ++j) S.hist[j - 1] = S.hist[j];
-                    S.nhist--;
-                }
-                S.hist[S.nhist++] = S.ring_new;
-                S.gamma = sy / yy;
-                S.sy_new = sy;
-                S.yy_new = yy;
-                S.iter++;
+        const int gn = 1 - S.gcur, pr = S.ring_new >= 0 ? S.ring_new : 0;
+        // the h parts on lanes 0..3: x_h += stp d_h (not at a start), the h
+        // gradient, s_h and y_h, and their five dot products
+        double eg = 0.0, xh = 0.0, es = 0.0, ey = 0.0;
+        if (lane < Q) {
+            const double x0 = S.eta_x[lane];
+            xh = init ? x0 : fma(S.stp, S.eta_d[lane], x0);
+            es = xh - x0;
+            eg = a_rs + 2.0 * lambda_h * xh;
+            ey = eg - S.eta_g[S.gcur][lane];
+            S.eta_x[lane] = xh;
+            S.eta_g[gn][lane] = eg;
+            s_eg[lane] = eg;
+            if (pushed) {
+                if (!init) S.eta_s[pr][lane] = es;
+                S.eta_y[pr][lane] = ey;
+            }
+        }
+        double d[5] = {eg * eg, xh * xh, es * ey, ey * ey, es * es};
+#pragma unroll
+        for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < 5; ++q) d[q] += __shfl_xor_sync(0xffffffffu, d[q], o);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) d[q] = __shfl_sync(0xffffffffu, d[q], 0);
+        const double g2 = a_g2 + d[0], x2H = d[1];
+        const double sy = pushed ? a_sy + d[2] : a_sy, yy = pushed ? a_yy + d[3] : a_yy, ss = pushed ? a_ss + d[4] : a_ss;
+        // the three roots at once, one per lane
+        const double root = sqrt(lane == 0 ? fmax(g2, 0.0) : lane == 1 ? ss * yy : a_x2J + x2H);
+        const double gnorm = __shfl_sync(0xffffffffu, root, 0), rss = __shfl_sync(0xffffffffu, root, 1),
+                     xnorm = __shfl_sync(0xffffffffu, root, 2);
+        const double gamma = sy / yy;
+        const bool keep = !init && pushed && sy > 1e-3 * rss && yy > 0.0 && isfinite(sy) && isfinite(yy);
+        // the history, oldest first on lanes 0.., with the new pair if it is kept
+        int nh = S.nhist, hj = lane < MAXHIST ? S.hist[lane] : 0;
+        const int rn = S.ring_new;
+        __syncwarp();
+        if (keep) {
+            const int next = __shfl_down_sync(0xffffffffu, hj, 1);
+            if (nh == m) {
+                hj = next;
+                --nh;
+            }
+            if (lane == nh) hj = rn;
+            ++nh;
+            if (lane < nh) S.hist[lane] = hj;
+        }
+        if (lane == 0) {
+            S.gcur = gn;
+            S.g2J = a_g2;
+            S.g2 = g2;
+            S.x2J = a_x2J;
+            S.amax_g = mg;
+            S.amax_x = mx;
+            S.gmax = S.chk_ratio > 0.0 ? S.chk_ratio * gnorm : gnorm;   // estimate until checked
+            bool st = false;
+            if (init) {
+                S.f = a_f + lambda_J * a_x2J + lambda_h * x2H;
+                S.nfeval = 1;
             } else {
-                S.ring_new = -1;
-                S.skipped++;
+                S.iterations++;
+                S.nfeval += 2 + S.trials;
+                if (keep) {
+                    S.nhist = nh;
+                    S.gamma = gamma;
+                    S.sy_new = sy;
+                    S.yy_new = yy;
+                    S.iter++;
+                } else {
+                    S.ring_new = -1;
+                    S.skipped++;
+                }
+                if (S.iterations > max_iterations) {
+                    S.status = 1;
+                    st = true;
+                } else if (S.stalled) {
+                    S.status = 2;
+                    st = true;
+                }
             }
-            if (S.iterations > max_iterations) {
-                S.status = 1;
-                st = true;
-            } else if (S.stalled) {
-                S.status = 2;
+            if (!isfinite(S.f) || !isfinite(S.g2)) {
+                S.status = -1;
                 st = true;
             }
-        }
-        if (!isfinite(S.f) || !isfinite(S.g2)) {
-            S.status = -1;
-            st = true;
-        }
-        if (st) {
-            S.phase = DC_STOP;
-            S.want_check = 0;
-        } else {
-            // the relative-norm stop is decided after the max-norm test (by the host's check pass)
-            const double releps = 1e-4 * fmax(1.0, sqrt(S.x2J + x2H));
-            S.releps_stop = gnorm < releps;
-            // the max-norm test needs J = Phi^T a_g: wanted when the last check's
-            // ratio max|g| / ||g|| predicts a pass, and every 15 iterations
-            const bool due = S.iterations - S.last_check >= 15 && (S.chk_ratio > 0.0 || gnorm < 150.0 * gtol);
-            const bool near = S.chk_ratio > 0.0 && S.chk_ratio * gnorm < 1.1 * gtol;
-            S.want_check = (due || near || gnorm < gtol || S.releps_stop) ? 1 : 0;
-            S.chk_wait = S.want_check ? S.chk_wait + 1 : 0;
-            S.coef_g = -1.0;
-            for (int a = 0; a < Q; ++a) s_eg[a] = eg[a];
-            go = 1;
+            if (st) {
+                S.phase = DC_STOP;
+                S.want_check = 0;
+            } else {
+                // the relative-norm stop is decided after the max-norm test (by the host's check pass)
+                const double releps = 1e-4 * fmax(1.0, xnorm);
+                S.releps_stop = gnorm < releps;
+                // the max-norm test needs J = Phi^T a_g: wanted when the last check's
+                // ratio max|g| / ||g|| predicts a pass, and every 15 iterations
+                const bool due = S.iterations - S.last_check >= 15 && (S.chk_ratio > 0.0 || gnorm < 150.0 * gtol);
+                const bool near = S.chk_ratio > 0.0 && S.chk_ratio * gnorm < 1.1 * gtol;
+                S.want_check = (due || near || gnorm < gtol || S.releps_stop) ? 1 : 0;
+                S.chk_wait = S.want_check ? S.chk_wait + 1 : 0;
+                S.coef_g = -1.0;
+                go = 1;
+            }
         }
     }
     __syncwarp();
-    // compact-form coefficients of the next direction: the per-pair work on
-    // the warp's lanes (lane j: history pair j), the small triangular solve
-    // on one thread
+    // compact-form coefficients of the next direction, on the warp's lanes
+    // (lane j: history pair j)
     if (go) {
-        const int lane = threadIdx.x, k = S.nhist;
-        const double *dp = dots + (int64_t)b * 4 * MAXHIST;
+        const int k = S.nhist;
         if (lane < k) {
             const int pj = S.hist[lane];
-            s_dt[lane] = dp[pj] + dot4d(S.eta_s[pj], s_eg);
-            s_dt[MAXHIST + lane] = dp[DOT_Y + pj] + dot4d(S.eta_y[pj], s_eg);
+            s_dt[lane] = s_dots[pj] + dot4d(S.eta_s[pj], s_eg);
+            s_dt[MAXHIST + lane] = s_dots[DOT_Y + pj] + dot4d(S.eta_y[pj], s_eg);
         }
         __syncwarp();
         if (lane < k) {
@@ -1177,25 +1257,31 @@ k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32
             s_YY[e] = S.YY[S.hist[ra]][S.hist[rc]];
         }
         __syncwarp();
-        if (lane == 0 && k > 0) {
-            double cg, cS[MAXHIST], cY[MAXHIST];
-            if (lbfgs_compact_coeffs(k, s_R, s_YY, s_dt, s_dt + MAXHIST, S.gamma, &cg, cS, cY)) {
-                S.coef_g = cg;
-                for (int a = 0; a < k; ++a) {
-                    S.coefS[a] = cS[a];
-                    S.coefY[a] = cY[a];
+        if (k > 0) {   // (the same on every lane)
+            double cS, cY;
+            const bool ok = warp_compact_coeffs(k, s_R, s_YY, s_dt, s_dt + MAXHIST, S.gamma, cS, cY);
+            if (ok && lane < k) {
+                S.coefS[lane] = cS;
+                S.coefY[lane] = cY;
+            }
+            if (lane == 0) {
+                if (ok) {
+                    S.coef_g = -S.gamma;
+                } else {
+                    S.nhist = 0;
+                    S.iter = 0;
                 }
-            } else {
-                S.nhist = 0;
-                S.iter = 0;
             }
         }
         __syncwarp();
         const int kk = S.nhist;
         if (lane < Q) {
-            double v = S.coef_g * s_eg[lane];
-            for (int j = 0; j < kk; ++j)
-                v += S.coefS[j] * S.eta_s[S.hist[j]][lane] + S.coefY[j] * S.eta_y[S.hist[j]][lane];
+            double v = S.coef_g * s_eg[lane], u = 0.0;
+            for (int j = 0; j < kk; ++j) {
+                v = fma(S.coefS[j], S.eta_s[S.hist[j]][lane], v);
+                u = fma(S.coefY[j], S.eta_y[S.hist[j]][lane], u);
+            }
+            v += u;
             S.eta_d[lane] = v;
             S.cdf[2 * MAXHIST + 1 + lane] = df_from_d(v);
         }
@@ -1203,16 +1289,11 @@ k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32
             S.cdf[lane] = df_from_d(S.coefS[lane]);
             S.cdf[MAXHIST + lane] = df_from_d(S.coefY[lane]);
         }
+        // the next accepted step fills the first ring position outside the live history
+        const unsigned used = __reduce_or_sync(0xffffffffu, lane < kk ? 1u << S.hist[lane] : 0u);
         if (lane == 0) {
             S.cdf[2 * MAXHIST] = df_from_d(S.coef_g);
-            // the next accepted step fills a ring position outside the live history
-            int pos = 0;
-            for (bool used = true; used;) {
-                used = false;
-                for (int j = 0; j < kk; ++j) used = used || S.hist[j] == pos;
-                if (used) ++pos;
-            }
-            S.ring_new = pos;
+            S.ring_new = __ffs(~used) - 1;
             S.push = 1;
             S.phase = DC_STEP;
         }
@@ -1221,6 +1302,7 @@ k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32
     {
         unsigned long long *dst = reinterpret_cast<unsigned long long *>(ctl + b);
         const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&S);
+#pragma unroll
         for (int k = threadIdx.x; k < CTL_WORDS; k += 32) dst[k] = src[k];
     }
     if (threadIdx.x == 0) write_summary(S, sum[b]);

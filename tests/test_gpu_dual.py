@@ -53,6 +53,24 @@ def test_dual_matches_oracle(oracle_mod, shape, seed):
         assert np.abs(g).max() < 1.05e-3, (r, np.abs(g).max())
 
 
+@pytest.mark.parametrize("history", [1, 2, 3, 10])
+def test_dual_history_lengths(oracle_mod, history):
+    """Every history length (the warp solves k x k systems, the ring wraps
+    after history + 1 pairs) reaches the oracle's optimum."""
+    from superdca_gb300 import _lib, synthetic
+    states, _, _ = synthetic.workload("tree-3000x10000", seed=9, N=130, L=700)
+    N, L = states.shape
+    loci = np.random.default_rng(5).choice(L, 12, replace=False)
+    w = np.ones(N)
+    res, (lh, lJ, _) = _solve(states, w, loci, _lib.FORM_DUAL, batch=8, history=history)
+    assert np.all(res.status == 0), res.status
+    P = oracle_mod.Problem(states, w, lh, lJ)
+    _, st = P.solve(loci, threads=4, gtol=1e-5)
+    np.testing.assert_allclose(res.f, [s["f"] for s in st], rtol=1e-6)
+    for k, r in enumerate(loci):
+        assert np.abs(P.objective(int(r), res.x[k])[1]).max() < 1.05e-3
+
+
 def test_dual_iterations_match_other_forms():
     from superdca_gb300 import _lib, synthetic
     states, _, _ = synthetic.workload("tree-3000x10000", seed=4, N=600, L=2500)

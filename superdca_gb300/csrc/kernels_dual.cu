@@ -290,14 +290,21 @@ k_dual_grad(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
 // iteration's: S^T y = S^T g - S^T g_old.)
 // A block takes DOT_CHUNK entries of one slot: k_g staged in shared memory;
 // the work is cut into (history vector, quarter of the chunk) units, taken
-// by the warps in turn, so every warp gets the same number of units whatever
-// the history length (8k units for 8 warps); 16-byte loads, eight in flight
-// per lane, one accumulator per lane.
+// by the warps of the slot's gridDim.z blocks in turn, so every warp gets the
+// same number of units whatever the history length (8k units for 8 warps at
+// gridDim.z = 1).  A lane's eight 16-byte loads of a unit are all issued
+// before its multiply-adds: with the loads left to the compiler (32
+// registers, two or three in flight) and few blocks on the chip the kernel
+// waited for memory unit after unit: 50 us a launch at 64 slots of
+// 1000 x 4001 (now 12) and 191 at 512 slots of 3000 x 94,000 (now 177, 5.8 TB/s).
+constexpr int DOT_THREADS = 256;
 constexpr int DOT_CHUNK = 2048;
 constexpr int DOT_SUBS = 4;                       // units per vector and chunk
 constexpr int DOT_SUB_Q = DOT_CHUNK / 2 / DOT_SUBS;   // float4 pairs per unit (256)
+constexpr int DOT_LOADS = DOT_SUB_Q / 32;         // float4 loads per lane and unit
+constexpr int DOT_MAX_K = MAXHIST + 1;            // the live history and the pushed pair
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(DOT_THREADS, 4)
 k_dual_dots(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, int64_t Nx, int NV, int ring,
             int newg, const float2 *__restrict__ dv, double *__restrict__ dots, const int *__restrict__ cnt)
 {
@@ -307,30 +314,36 @@ k_dual_dots(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
     if (S.phase == DC_STOP) return;
     // the live history and the pair the last accept pushed
     const bool pushed = S.push && S.ring_new >= 0;
-    const int k = S.nhist + (pushed ? 1 : 0);
+    const int nh = S.nhist, k = nh + (pushed ? 1 : 0);
     const int64_t E = Nx * 4, e0 = (int64_t)blockIdx.x * DOT_CHUNK;
     const int ne = E - e0 < DOT_CHUNK ? (int)(E - e0) : DOT_CHUNK;   // a multiple of 4 (Nx is of 64)
     const int nq = ne / 2;                                            // float4 pairs
+    const int subs = (nq + DOT_SUB_Q - 1) / DOT_SUB_Q;                // units per vector that hold entries
     __shared__ float4 g[DOT_CHUNK / 2];
+    __shared__ int s_pos[DOT_MAX_K];
     const float2 *kg = dv + dvo(b, DV_G + (newg ? 1 - S.gcur : S.gcur), 1, NV, Nx) + e0;   // (gcur flips in the control kernel)
-    for (int t = threadIdx.x; t < nq; t += blockDim.x) g[t] = reinterpret_cast<const float4 *>(kg)[t];
+    if (threadIdx.x < k) s_pos[threadIdx.x] = (int)threadIdx.x < nh ? S.hist[threadIdx.x] : S.ring_new;
+    for (int t = threadIdx.x; t < subs * DOT_SUB_Q; t += DOT_THREADS)
+        g[t] = t < nq ? reinterpret_cast<const float4 *>(kg)[t] : make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int u = warp; u < 2 * k * DOT_SUBS; u += nw) {
-        const int qv = u / DOT_SUBS, t0 = (u % DOT_SUBS) * DOT_SUB_Q;
+    const int lane = threadIdx.x & 31, nw = (DOT_THREADS >> 5) * gridDim.z;
+    for (int u = (threadIdx.x >> 5) + (DOT_THREADS >> 5) * blockIdx.z; u < 2 * k * subs; u += nw) {
+        const int qv = u / subs, t0 = (u - qv * subs) * DOT_SUB_Q + lane;
         const bool isy = qv >= k;
-        const int j = isy ? qv - k : qv;
-        const int pos = j < S.nhist ? S.hist[j] : S.ring_new;
+        const int pos = s_pos[isy ? qv - k : qv];
         const float4 *v = reinterpret_cast<const float4 *>(dv + dvo(b, DV_S + (isy ? ring : 0) + pos, 0, NV, Nx) + e0);
-        const int t1 = min(nq, t0 + DOT_SUB_Q);
-        float2 acc = df_zero();
-#pragma unroll 8
-        for (int t = t0 + lane; t < t1; t += 32) {
-            const float4 x = v[t], y = g[t];
-            acc = df_fma(make_float2(x.x, x.y), make_float2(y.x, y.y), acc);
-            acc = df_fma(make_float2(x.z, x.w), make_float2(y.z, y.w), acc);
+        // (past the end: the last pair again, against a zero of g)
+        float4 x[DOT_LOADS];
+#pragma unroll
+        for (int i = 0; i < DOT_LOADS; ++i) x[i] = v[min(t0 + 32 * i, nq - 1)];
+        float2 a0 = df_zero(), a1 = df_zero();
+#pragma unroll
+        for (int i = 0; i < DOT_LOADS; ++i) {
+            const float4 y = g[t0 + 32 * i];
+            a0 = df_fma(make_float2(x[i].x, x[i].y), make_float2(y.x, y.y), a0);
+            a1 = df_fma(make_float2(x[i].z, x[i].w), make_float2(y.z, y.w), a1);
         }
-        const float2 sum = df_warp_sum(acc);
+        const float2 sum = df_warp_sum(df_add(a0, a1));
         if (lane == 0 && (sum.x != 0.f || sum.y != 0.f))
             atomicAdd(dots + (int64_t)b * 4 * MAXHIST + (isy ? DOT_Y : 0) + pos, df_to_d(sum));
     }
@@ -1459,8 +1472,12 @@ void launch_dual_dots(const Problem &P, const DualCtl *ctl, const int32_t *list,
                       double *dots, cudaStream_t st, const int *cnt)
 {
     if (n <= 0) return;
-    dim3 g((unsigned)((P.Nx * 4 + DOT_CHUNK - 1) / DOT_CHUNK), n);
-    k_dual_dots<<<g, 256, 0, st>>>(ctl, list, P.Nx, DV_S + 2 * P.ring, P.ring, newg, dv, dots, cnt);
+    // few slots of few sequences leave the chip idle: share a slot's units out
+    // over more blocks until every SM has its eight (each stages k_g again, 16 KB)
+    const int64_t blocks = (P.Nx * 4 + DOT_CHUNK - 1) / DOT_CHUNK * n;
+    const unsigned z = (unsigned)std::max<int64_t>(1, std::min<int64_t>(10, 8 * 152 / blocks));
+    dim3 g((unsigned)((P.Nx * 4 + DOT_CHUNK - 1) / DOT_CHUNK), n, z);
+    k_dual_dots<<<g, DOT_THREADS, 0, st>>>(ctl, list, P.Nx, DV_S + 2 * P.ring, P.ring, newg, dv, dots, cnt);
 }
 
 void launch_dual_direction(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, float2 *dv,

@@ -19,6 +19,7 @@
 // are taken in 64-bit integers; QB keeps them below 2^62.  K = K_all minus
 // the agreement at r itself, a class sum per state of r.
 #include <cstdint>
+#include <algorithm>
 #include <cstdlib>
 #include <new>
 
@@ -787,17 +788,24 @@ __device__ __forceinline__ double dot4d(const double *a, const double *b)
     return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3];
 }
 
-// Threads per search block (LS_THREADS, 128 by default): the search is
-// latency-bound (short passes over the slot's sequences between block
-// reductions and the FP64 state machine of one thread), so smaller blocks
-// let more searches share an SM.
+// Threads per search block: LS_THREADS for the trials and one warp for the
+// state machine.  The search is latency-bound (short passes over the slot's
+// sequences between block reductions and the FP64 state machine of one
+// thread), so with many slots small blocks (128) let more searches share an
+// SM, and with few slots larger ones shorten the passes (the launcher's rule).
+// The state machine's warp works out what a trial's verdict needs besides
+// its sums (the L2 part, 1 / (stp - stx)) while the others evaluate it, and
+// takes the sums over the warps itself: two barriers a trial.  A launch at 512
+// slots of 3000 x 94,000 went from 154 to 141 us, at 233 slots of 200 x 500 from
+// 52 to 42, at 64 slots of 1000 x 4001 from 44 to 36.
 
 // The whole line search of one slot in one thread block (SuperDCA: the
 // More-Thuente search of CppNumericalSolvers' LbfgsSolver, one
 // value_and_gradient per trial, LBFGS_interface_CppNumericalSolvers.hpp:
-// 111-117).  Thread 0 holds the More-Thuente state machine (FP64, in shared
-// memory); all threads evaluate each trial over the slot's sequences and
-// reduce it (FP32 per thread and warp, FP64 across warps).
+// 111-117).  The last warp's first lane holds the More-Thuente state machine
+// (FP64, in shared memory); the other warps evaluate each trial over the
+// slot's sequences and reduce it (FP32 per thread and warp; FP64 across
+// warps, on the last warp).
 //   1. Restart test: a direction that is not downhill in angle
 //      (cos(g, d) >= -1e-10), or one the last search asked to restart,
 //      becomes steepest descent: d = -g, its logit direction, differences
@@ -811,7 +819,7 @@ __device__ __forceinline__ double dot4d(const double *a, const double *b)
 //      trial, so R holds its residual rows, acc[ACC_RS*] their sums and the
 //      slot's f, stp the point's objective and step.
 template <int LS_THREADS>
-__global__ void __launch_bounds__(LS_THREADS, 768 / LS_THREADS)
+__global__ void __launch_bounds__(LS_THREADS + 32, 800 / (LS_THREADS + 32))
 k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, int N, int64_t Nx, int NV,
                   double lambda_J, double lambda_h, const double *__restrict__ dacc, float2 *__restrict__ dv,
                   float4 *__restrict__ ud,
@@ -823,22 +831,24 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
     DualCtl &S = ctl[b];
     if (S.phase != DC_STEP) return;   // (the same for the whole block)
     __shared__ __align__(16) unsigned char mt_raw[sizeof(MoreThuente)];
-    __shared__ double red[LS_THREADS / 32][8];
+    __shared__ double red[LS_THREADS / 32 + 1][8];
     __shared__ double s_stp;
     __shared__ float2 s_stp_df;
     __shared__ double s_tot[8];
+    constexpr int NW = LS_THREADS / 32;   // trial warps; warp NW runs the state machine
     __shared__ int s_restart, s_done;
     __shared__ float2 s_ex[Q], s_ed[Q];   // eta_x, eta_d as double-float (the h parts of the logits and of u)
     MoreThuente &mt = *reinterpret_cast<MoreThuente *>(mt_raw);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const bool lead = tid == LS_THREADS;
     const double *da = dacc + (int64_t)b * NDACC;
-    // FP64 scalars of the search, thread 0's (in shared memory, so that they
+    // FP64 scalars of the search, the lead thread's (in shared memory, so that they
     // hold no registers of the other threads through the trial loop)
     __shared__ double sc[9];
     double &xdJ = sc[0], &xdH = sc[1], &ddJ = sc[2], &ddH = sc[3], &dg0 = sc[4], &f0d = sc[5], &dg0d = sc[6],
            &x2H = sc[7];
     __shared__ int s_mode;   // 0 searching, 1 evaluating the current point (start not downhill)
-    if (tid == 0) {
+    if (lead) {
         const double *eg = S.eta_g[S.gcur];
         const double gd = da[DA_GD] + dot4d(eg, S.eta_d);
         ddJ = da[DA_DDJ];
@@ -861,7 +871,7 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
         const float2 *ax = dv + dvo(b, DV_X, 0, NV, Nx);
         float2 *ad = dv + dvo(b, DV_D, 0, NV, Nx), *kd = dv + dvo(b, DV_D, 1, NV, Nx);
         float2 xd = df_zero(), d0 = df_zero();
-        for (int64_t i = tid; i < Nx; i += LS_THREADS) {
+        for (int64_t i = tid; i < Nx; i += LS_THREADS + 32) {
             const int64_t o = (int64_t)b * Nx + i;
             float2 uu[4];
 #pragma unroll
@@ -894,9 +904,9 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
             red[wid][1] = df_to_d(s0);
         }
         __syncthreads();
-        if (tid == 0) {
+        if (lead) {
             double t0 = 0, t1 = 0;
-            for (int k = 0; k < LS_THREADS / 32; ++k) {
+            for (int k = 0; k <= NW; ++k) {
                 t0 += red[k][0];
                 t1 += red[k][1];
             }
@@ -916,7 +926,7 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
         }
         __syncthreads();
     }
-    if (tid == 0) {
+    if (lead) {
         for (int c = 0; c < Q; ++c) {
             s_ex[c] = df_from_d(S.eta_x[c]);
             s_ed[c] = df_from_d(S.eta_d[c]);
@@ -945,52 +955,67 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
     }
     // More-Thuente stops within 20 trials; the bound only guards the loop
     for (int it = 0; it < 64; ++it) {
-        __syncthreads();
+        __syncthreads();   // the step (or the end) is published
+        if (s_done) break;
         const double stp = s_stp;
         const float2 stpd = s_stp_df;
-        const float stpf = stpd.x + stpd.y;
-        float f = 0.f, dg = 0.f, rs[4] = {0.f, 0.f, 0.f, 0.f};
-        float2 fbig = df_zero(), dgbig = df_zero();
-        const float2 *kxs = dv + dvo(b, DV_X, 1, NV, Nx), *kds = dv + dvo(b, DV_D, 1, NV, Nx);
-        // two sequences per pass, both sequences' loads in flight before
-        // either is computed (the search has few warps per SM to hide
-        // latency with)
+        double l2 = 0.0, dl2 = 0.0;
+        if (wid < NW) {
+            const float stpf = stpd.x + stpd.y;
+            float f = 0.f, dg = 0.f, rs[4] = {0.f, 0.f, 0.f, 0.f};
+            float2 fbig = df_zero(), dgbig = df_zero();
+            const float2 *kxs = dv + dvo(b, DV_X, 1, NV, Nx), *kds = dv + dvo(b, DV_D, 1, NV, Nx);
+            // two sequences per pass, both sequences' loads in flight before
+            // either is computed (the search has few warps per SM to hide
+            // latency with)
 #pragma unroll 1
-        for (int i0 = tid; i0 < N; i0 += 2 * LS_THREADS) {
-            const int i1 = i0 + LS_THREADS;
-            const bool two = i1 < N;
-            const int64_t o0 = (int64_t)b * Nx + i0, o1 = (int64_t)b * Nx + (two ? i1 : i0);
-            const TrialIn t0 = trial_load(o0, i0, ud, rstate, w, P0);
-            const TrialIn t1 = trial_load(o1, two ? i1 : i0, ud, rstate, w, P0);
-            trial_seq(o0, i0, t0, stpd, stpf, kxs, kds, s_ex, s_ed, R, f, dg, rs, fbig, dgbig);
-            if (two) trial_seq(o1, i1, t1, stpd, stpf, kxs, kds, s_ex, s_ed, R, f, dg, rs, fbig, dgbig);
-        }
-        // FP32 sums per warp (each lane's value is an FP32 partial over a few
-        // sequences), double-float for the large-step terms, FP64 across warps
-        const float v[6] = {warp_sum_f(f), warp_sum_f(dg), warp_sum_f(rs[0]), warp_sum_f(rs[1]), warp_sum_f(rs[2]),
-                            warp_sum_f(rs[3])};
-        fbig = df_warp_sum(fbig);
-        dgbig = df_warp_sum(dgbig);
-        if (lane == 0) {
+            for (int i0 = tid; i0 < N; i0 += 2 * LS_THREADS) {
+                const int i1 = i0 + LS_THREADS;
+                const bool two = i1 < N;
+                const int64_t o0 = (int64_t)b * Nx + i0, o1 = (int64_t)b * Nx + (two ? i1 : i0);
+                const TrialIn t0 = trial_load(o0, i0, ud, rstate, w, P0);
+                const TrialIn t1 = trial_load(o1, two ? i1 : i0, ud, rstate, w, P0);
+                trial_seq(o0, i0, t0, stpd, stpf, kxs, kds, s_ex, s_ed, R, f, dg, rs, fbig, dgbig);
+                if (two) trial_seq(o1, i1, t1, stpd, stpf, kxs, kds, s_ex, s_ed, R, f, dg, rs, fbig, dgbig);
+            }
+            // FP32 sums per warp (each lane's value is an FP32 partial over a few
+            // sequences), double-float for the large-step terms (most trials
+            // have none), FP64 across warps
+            const float v[6] = {warp_sum_f(f), warp_sum_f(dg), warp_sum_f(rs[0]), warp_sum_f(rs[1]), warp_sum_f(rs[2]),
+                                warp_sum_f(rs[3])};
+            const bool any_big =
+                __any_sync(0xffffffffu, fbig.x != 0.f || fbig.y != 0.f || dgbig.x != 0.f || dgbig.y != 0.f);
+            if (any_big) {
+                fbig = df_warp_sum(fbig);
+                dgbig = df_warp_sum(dgbig);
+            }
+            if (lane == 0) {
 #pragma unroll
-            for (int k = 0; k < 6; ++k) red[wid][k] = (double)v[k];
-            red[wid][6] = df_to_d(fbig);
-            red[wid][7] = df_to_d(dgbig);
+                for (int k = 0; k < 6; ++k) red[wid][k] = (double)v[k];
+                red[wid][6] = df_to_d(fbig);
+                red[wid][7] = df_to_d(dgbig);
+            }
+        } else if (lane == 0) {
+            l2 = lambda_J * (S.x2J + 2.0 * stp * xdJ + stp * stp * ddJ) +
+                 lambda_h * (x2H + 2.0 * stp * xdH + stp * stp * ddH);
+            dl2 = 2.0 * lambda_J * (xdJ + stp * ddJ) + 2.0 * lambda_h * (xdH + stp * ddH);
+            l2 += f0d;
+            dl2 += dg0d;
+            mt.ahead();
         }
         __syncthreads();
-        if (tid < 8) {
+        if (wid < NW) continue;
+        if (lane < 8) {
             double t = 0.0;
-            for (int k = 0; k < LS_THREADS / 32; ++k) t += red[k][tid];
-            s_tot[tid] = t;
+#pragma unroll
+            for (int k = 0; k < NW; ++k) t += red[k][lane];
+            s_tot[lane] = t;
         }
-        __syncthreads();
-        if (tid == 0) {
+        __syncwarp();
+        if (lane == 0) {
             const double *tot = s_tot;
-            const double l2 = lambda_J * (S.x2J + 2.0 * stp * xdJ + stp * stp * ddJ) +
-                              lambda_h * (x2H + 2.0 * stp * xdH + stp * stp * ddH);
-            const double dl2 = 2.0 * lambda_J * (xdJ + stp * ddJ) + 2.0 * lambda_h * (xdH + stp * ddH);
-            const double ff = f0d + (tot[0] + tot[6]) + l2;
-            const double dd = dg0d + (tot[1] + tot[7]) + dl2;
+            const double ff = (tot[0] + tot[6]) + l2;
+            const double dd = (tot[1] + tot[7]) + dl2;
             S.trials++;
             bool done = s_mode == 1 || it == 63;
             if (!done && (!isfinite(ff) || !isfinite(dd))) done = true;
@@ -1013,8 +1038,6 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
                 s_done = 1;
             }
         }
-        __syncthreads();
-        if (s_done) break;
     }
 }
 
@@ -1564,13 +1587,18 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
                             const float *w, const float *P0, float *R, double *acc, cudaStream_t st, const int *cnt)
 {
     if (n <= 0) return;
-    static const int threads = [] {
+    // Few slots: larger blocks, while every SM still holds its slots' blocks
+    // at once.  64 slots of 1000 x 4001: 51, 39 and 36 us
+    // with 64, 128 and 256 threads; 233 slots of 200 x 500: 44, 42 and 43.
+    // SDCA_LS_THREADS overrides the rule.
+    static const int forced = [] {
         const char *e = std::getenv("SDCA_LS_THREADS");
-        const int v = e ? std::atoi(e) : 128;
-        return (v == 64 || v == 256) ? v : 128;
+        const int v = e ? std::atoi(e) : 0;
+        return (v == 64 || v == 128 || v == 256) ? v : 0;
     }();
+    const int threads = forced ? forced : (n <= 152 ? 256 : 128);
 #define SDCA_LS_LAUNCH(T)                                                                                          \
-    k_dual_linesearch<T><<<n, T, 0, st>>>(ctl, list, (int)P.N, P.Nx, DV_S + 2 * P.ring, P.lambda_J, P.lambda_h,   \
+    k_dual_linesearch<T><<<n, T + 32, 0, st>>>(ctl, list, (int)P.N, P.Nx, DV_S + 2 * P.ring, P.lambda_J, P.lambda_h,   \
                                           dacc, dv, reinterpret_cast<float4 *>(ud), rstate, w,                    \
                                           reinterpret_cast<const float4 *>(P0), reinterpret_cast<float4 *>(R), acc, \
                                           cnt)

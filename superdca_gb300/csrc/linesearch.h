@@ -17,6 +17,8 @@
 #pragma once
 
 #include <math.h>
+#include <stdint.h>
+#include <string.h>
 
 #ifdef __CUDACC__
 #define SDCA_HD __host__ __device__
@@ -30,6 +32,31 @@ namespace sdca {
 // comparisons), usable in device code
 SDCA_HD inline double mt_min(double a, double b) { return (b < a) ? b : a; }
 SDCA_HD inline double mt_max(double a, double b) { return (a < b) ? b : a; }
+
+// The power of two at or below s (s >= 0), and its reciprocal: scaling by it
+// is exact and needs no division (GB300's FP64 divisions are long serial
+// chains, and one thread runs this search between two trials).
+SDCA_HD inline double mt_pow2(double s, double &inv)
+{
+    uint64_t b;
+    memcpy(&b, &s, sizeof(b));
+    b &= 0x7ff0000000000000ull;
+    const uint64_t i = b >= 0x7fe0000000000000ull ? 0ull : 0x7fe0000000000000ull - b;
+    double p;
+    memcpy(&p, &b, sizeof(p));
+    memcpy(&inv, &i, sizeof(inv));
+    return p;
+}
+
+// s sqrt((theta / s)^2 - (a / s)(b / s)) (not below zero if `clip`), with s the
+// power of two of the largest magnitude, so that no square overflows
+SDCA_HD inline double mt_gamma(double theta, double a, double b, bool clip)
+{
+    double inv;
+    const double s = mt_pow2(mt_max(fabs(theta), mt_max(fabs(a), fabs(b))), inv);
+    const double t = theta * inv, r = t * t - (a * inv) * (b * inv);
+    return s * sqrt(clip ? mt_max(0.0, r) : r);
+}
 
 class MoreThuente {
 public:
@@ -45,6 +72,7 @@ public:
         nfev = 0;
         info = 0;
         infoc = 1;
+        have_rinv = false;
         if (!(dg0 < 0.0)) return NO_DESCENT;
         brackt = false;
         stage1 = true;
@@ -59,8 +87,19 @@ public:
         return NEED_EVAL;
     }
 
+    // The part of the next feed() that does not need its trial's values
+    // (1 / (stp - stx)), for a caller that has time while the trial runs;
+    // feed() does it otherwise.
+    SDCA_HD void ahead()
+    {
+        rinv = 1.0 / (stp - stx);
+        have_rinv = true;
+    }
+
     SDCA_HD Result feed(double f, double dg)
     {
+        if (!have_rinv) ahead();
+        have_rinv = false;
         nfev++;
         const double ftest1 = finit + stp * dgtest;
         if ((brackt && ((stp <= stmin) || (stp >= stmax))) || (infoc == 0)) info = 6;
@@ -99,8 +138,9 @@ private:
     static constexpr double kStpmin = 1e-15, kStpmax = 1e15, kXtrapf = 4.0;
     static constexpr int kMaxfev = 20;
 
-    bool brackt = false, stage1 = true;
+    bool brackt = false, stage1 = true, have_rinv = false;
     int infoc = 1;
+    double rinv = 0;   // 1 / (stp - stx) of the trial in flight
     double finit = 0, dginit = 0, dgtest = 0, width = 0, width1 = 0;
     double stx = 0, fx = 0, dgx = 0, sty = 0, fy = 0, dgy = 0, stmin = 0, stmax = 0;
 
@@ -130,25 +170,24 @@ private:
             (dx * (st - sx) >= 0.0) || (stmax < stmin))
             return;
         bool bound = false;
-        const double sgnd = dp * (dx / fabs(dx));
+        const double sgnd = dx > 0.0 ? dp : -dp;   // (dx is not zero here)
+        const double slope = (fxv - fp) * rinv;     // (fx - f) / (st - sx)
         double stpf, stpc, stpq;
         if (fp > fxv) {
             infoc = 1;
             bound = true;
-            const double theta = 3.0 * (fxv - fp) / (st - sx) + dx + dp;
-            const double s = mt_max(fabs(theta), mt_max(fabs(dx), fabs(dp)));
-            double gamma = s * sqrt((theta / s) * (theta / s) - (dx / s) * (dp / s));
+            const double theta = 3.0 * slope + dx + dp;
+            double gamma = mt_gamma(theta, dx, dp, false);
             if (st < sx) gamma = -gamma;
             const double p = (gamma - dx) + theta, q = ((gamma - dx) + gamma) + dp;
             stpc = sx + (p / q) * (st - sx);
-            stpq = sx + ((dx / ((fxv - fp) / (st - sx) + dx)) / 2.0) * (st - sx);
+            stpq = sx + ((dx / (slope + dx)) / 2.0) * (st - sx);
             stpf = (fabs(stpc - sx) < fabs(stpq - sx)) ? stpc : stpc + (stpq - stpc) / 2.0;
             brackt = true;
         } else if (sgnd < 0.0) {
             infoc = 2;
-            const double theta = 3.0 * (fxv - fp) / (st - sx) + dx + dp;
-            const double s = mt_max(fabs(theta), mt_max(fabs(dx), fabs(dp)));
-            double gamma = s * sqrt((theta / s) * (theta / s) - (dx / s) * (dp / s));
+            const double theta = 3.0 * slope + dx + dp;
+            double gamma = mt_gamma(theta, dx, dp, false);
             if (st > sx) gamma = -gamma;
             const double p = (gamma - dp) + theta, q = ((gamma - dp) + gamma) + dx;
             stpc = st + (p / q) * (sx - st);
@@ -158,9 +197,8 @@ private:
         } else if (fabs(dp) < fabs(dx)) {
             infoc = 3;
             bound = true;
-            const double theta = 3.0 * (fxv - fp) / (st - sx) + dx + dp;
-            const double s = mt_max(fabs(theta), mt_max(fabs(dx), fabs(dp)));
-            double gamma = s * sqrt(mt_max(0.0, (theta / s) * (theta / s) - (dx / s) * (dp / s)));
+            const double theta = 3.0 * slope + dx + dp;
+            double gamma = mt_gamma(theta, dx, dp, true);
             if (st > sx) gamma = -gamma;
             const double p = (gamma - dp) + theta, q = (gamma + (dx - dp)) + gamma;
             const double r = p / q;
@@ -174,8 +212,7 @@ private:
             infoc = 4;
             if (brackt) {
                 const double theta = 3.0 * (fp - fyv) / (sy - st) + dy + dp;
-                const double s = mt_max(fabs(theta), mt_max(fabs(dy), fabs(dp)));
-                double gamma = s * sqrt((theta / s) * (theta / s) - (dy / s) * (dp / s));
+                double gamma = mt_gamma(theta, dy, dp, false);
                 if (st > sy) gamma = -gamma;
                 const double p = (gamma - dp) + theta, q = ((gamma - dp) + gamma) + dy;
                 stpc = st + (p / q) * (sy - st);

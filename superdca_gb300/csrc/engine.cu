@@ -1534,7 +1534,7 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
         return rc;
     CKL();
     if (dev || n[DC_GW] > 0) {
-        CK(cudaMemsetAsync(h->csum, 0, sizeof(long long) * 16 * P.Bmax, h->stream));
+        CK(cudaMemsetAsync(h->csum, 0, sizeof(long long) * CSUM * P.Bmax, h->stream));
         CK(cudaMemsetAsync(h->amax, 0, sizeof(double) * 2 * P.Bmax, h->stream));
         CK(cudaMemsetAsync(h->dots, 0, sizeof(double) * 4 * MAXHIST * P.Bmax, h->stream));
     }
@@ -2115,13 +2115,13 @@ static int create_lane(const sdca_config *cfg, const sdca_handle *owner, sdca_ha
                   (rc = dalloc(h, &h->dacc, B * NDACC)) || (rc = dalloc(h, &h->dlist, 4 * B + DC_N)) ||
                   (rc = dalloc(h, &h->dv, B * NV * 2 * P.Nx * 4)) ||
                   (rc = dalloc(h, &h->KR, B * P.Nx * 4)) || (rc = dalloc(h, &h->amax, 2 * B)) ||
-                  (rc = dalloc(h, &h->rq, B * P.Nx * 4)) || (rc = dalloc(h, &h->csum, 16 * B)) ||
+                  (rc = dalloc(h, &h->rq, B * P.Nx * 4)) || (rc = dalloc(h, &h->csum, CSUM * B)) ||
                   (rc = dalloc(h, &h->Rchk, B * P.Nx * 4)) || (dual_small && (rc = dalloc(h, &h->J64, B * P.Dp))) ||
                   (rc = dalloc(h, &h->P0, B * P.Nx * 4)) || (rc = dalloc(h, &h->ud, B * P.Nx * 4)) ||
                   (!shared && (rc = dalloc(h, &h->Kmat, (size_t)P.Nx * P.Nx))) ||
                   (P.N <= 4000 && P.L < (1 << 18) &&
                    ((!shared && (rc = dalloc(h, &h->Kd, (size_t)3 * kd_nk_rows(P) * P.Nx))) ||
-                    (rc = dalloc(h, &h->Rd, (size_t)4 * kd_nr_rows(P) * P.Nx)))))) ||
+                    (rc = dalloc(h, &h->Rd, (size_t)kd_nr_rows(P) * P.Nx)))))) ||
         (tcres &&
          ((!dual && (rc = dalloc(h, &h->Dhi, 4 * B * (size_t)round_up(4 * P.L, 64)))) ||
           (!dual && (rc = dalloc(h, &h->Dlo, 4 * B * (size_t)round_up(4 * P.L, 64)))) ||
@@ -2241,7 +2241,7 @@ int sdca_set_alignment(sdca_handle *h, const uint8_t *states, const double *weig
         }
         double wmax = 0.0;
         for (int64_t i = 0; i < P.N; ++i) wmax = std::max(wmax, weights[i]);
-        // the tensor-core product's four base-128 digit planes hold |rho_q| <= 2^27
+        // the tensor-core product's three base-640 digit planes hold |rho_q| <= 2^27
         const int qb = std::min(h->kd ? 27 : 30, 62 - (int)std::ceil(std::log2((double)P.N * (double)P.L + 1.0)));
         h->qscale = wmax > 0.0 ? std::ldexp(1.0, qb) / wmax : 1.0;
     }

@@ -155,6 +155,11 @@ enum DualAcc {
     NDACC = 4
 };
 
+// class sums of rho_q per slot: [a * 4 + c] the sum of column c over the
+// sequences with state a at the slot's locus (0 in scan mode), then the sums
+// of columns 0..2 over all sequences
+constexpr int CSUM = 20, CSUM_ALL = 16;
+
 enum SlotFlags {
     SLOT_F_USE_U = 1,       // trial logits use lbase + stp u (else lbase)
     SLOT_F_PUSH = 2,        // accept pushes an (s, y) pair into the history

@@ -44,7 +44,7 @@ __global__ void k_dual_kmat(const int32_t *__restrict__ dist, int N, int64_t Nx,
 // entry at the sequence's own state set to minus the sum of the other three,
 // so that every row sums to zero exactly (a residual w (p - onehot) does; the
 // K rho product then needs three columns); class sums csum[b][a][c] = sum
-// over i with s_i(r) = a
+// over i with s_i(r) = a, and the sums over all i (CSUM_ALL)
 __global__ void __launch_bounds__(256)
 k_dual_quant(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N, int64_t Nx,
              const float4 *__restrict__ R, const uint8_t *__restrict__ rstate, float qscale, int4 *__restrict__ rq,
@@ -53,10 +53,10 @@ k_dual_quant(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, i
     if (cnt && (int)blockIdx.y >= *cnt) return;
     const int b = list[blockIdx.y];
     const bool own = sd[b].locus >= 0;   // scan mode: no own-agreement correction
-    __shared__ unsigned long long red[16];
-    if (threadIdx.x < 16) red[threadIdx.x] = 0ull;
+    __shared__ unsigned long long red[CSUM];
+    if (threadIdx.x < CSUM) red[threadIdx.x] = 0ull;
     __syncthreads();
-    long long cs[4][4] = {};
+    long long cs[5][4] = {};   // by state; [4]: all
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < Nx; i += (int64_t)gridDim.x * blockDim.x) {
         int4 q = make_int4(0, 0, 0, 0);
         if (i < N) {
@@ -74,11 +74,12 @@ k_dual_quant(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, i
                 if (a != y) continue;
                 cs[a][0] += q.x; cs[a][1] += q.y; cs[a][2] += q.z; cs[a][3] += q.w;
             }
+            cs[4][0] += q.x; cs[4][1] += q.y; cs[4][2] += q.z;
         }
         rq[(int64_t)b * Nx + i] = q;
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 5; ++a)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             long long v = cs[a][c];
@@ -86,7 +87,8 @@ k_dual_quant(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, i
             if ((threadIdx.x & 31) == 0 && v != 0) atomicAdd(&red[a * 4 + c], (unsigned long long)v);
         }
     __syncthreads();
-    if (threadIdx.x < 16 && red[threadIdx.x] != 0ull) atomicAdd(csum + (int64_t)b * 16 + threadIdx.x, red[threadIdx.x]);
+    if (threadIdx.x < CSUM && red[threadIdx.x] != 0ull)
+        atomicAdd(csum + (int64_t)b * CSUM + threadIdx.x, red[threadIdx.x]);
 }
 
 constexpr int KP_M = 64;   // rows (sequences i) per CTA
@@ -145,7 +147,7 @@ k_dual_kprod(const int32_t *__restrict__ K, int64_t Nx, int N, const int32_t *__
             continue;
         }
         const int y = rstate[(int64_t)b * Nx + i] & 3;
-        const long long *cs = csum + (int64_t)b * 16 + y * 4;
+        const long long *cs = csum + (int64_t)b * CSUM + y * 4;
 #pragma unroll
         for (int c = 0; c < 4; ++c) o[c] = df_mul(df_from_ll(acc[a][c] - cs[c]), iq);
     }

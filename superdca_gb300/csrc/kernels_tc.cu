@@ -448,257 +448,342 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
 // ---------------------------------------------------------------------------
 // Exact K rho for the dual form on the tensor cores.
 //
-// K (agreement counts, < 2^18) is held as three fp16 planes of base-64
-// digits (0..63), rho_q (integers, |rho_q| <= 2^27) as four fp16 planes of
-// balanced base-128 digits (|digit| <= 64, the top one <= 65).  Every product
-// of two digits is an integer below 4096 and the sum over at most 4000
-// sequences stays below 2^24, so each of the 12 digit-pair GEMMs is exact in
-// its FP32 TMEM accumulator; the epilogue combines them with their weights
-// 2^(6k + 7p) in 64-bit integers (modulo 2^64: the total is below 2^62).
+// K (agreement counts, 0..L, L < 2^18) less its middle c = (L + 1) / 2 is held
+// as three fp16 planes of balanced base-64 digits (|digit| <= 32), rho_q
+// (integers, |rho_q| <= 2^27) as three fp16 planes of balanced base-640 digits
+// (|digit| <= 320, the top one <= 328).  A product of two digits is an integer
+// of at most 32 x 328 = 10,496, so sums over up to 1598 sequences stay below
+// 2^24 and are exact in the FP32 TMEM accumulators: the sequences are taken in
+// segments of 1536, and after each the epilogue warps add the nine
+// accumulators, weighted 64^k 640^p, to 64-bit integers (modulo 2^64: the
+// total is below 2^62).  K rho is that plus c times the column's sum of rho_q.
+// (Twelve products of unsigned base-64 and base-128 digits, which need no
+// second drain, issue a third more MMAs and hold four planes of rho.)
 //
 // Every row of rho_q sums to zero (k_dual_quant makes it so exactly), so the
 // fourth column of K rho is minus the sum of the other three: only three
-// columns per slot enter the product.  A CTA takes 128 rows of K and 13
-// slots (39 columns; with one unused row, 40 rows per rho digit plane), the
-// most that the 12 accumulators leave room for in TMEM (3 K digits x 4 planes
-// x 40 columns = 480 of 512), so each K tile staged from L2 serves 13 slots.
-// The B operand of one MMA stacks the four planes' first 32 rows (4 x 4 KB)
-// and then their last 8 rows (4 x 1 KB): every plane's accumulator columns
-// start 32-aligned (x32 loads) and its tail 8-aligned (x8 loads).
+// columns per slot enter the product.
+//
+// A pair of CTAs (cta_group::2) takes 256 rows of K, 128 each, and 17 slots:
+// 51 columns x 3 planes = 153 of the MMA's N = 160, 3 K digits x 160 = 480 of
+// the 512 TMEM columns.  An M128 N160 MMA of one CTA reads 9 KB of shared
+// memory per K16 step in the 80 cycles it computes, and the TMA writes about
+// as much: shared memory was the bound (0.8 us per 64 sequences against 0.46
+// of MMA work).  In the pair each CTA holds half of the rho rows, so an SM
+// reads 6.5 KB and receives 4.8 KB per MMA.
+// The kernel is persistent over the (row pair, slot group) tiles: the TMA
+// loads of the next tile run on while the epilogue warps, which keep their
+// sums in registers, store the last one; the MMAs wait only for the
+// accumulators to be read.
+// 186 us a launch at 512 slots of 3000 x 94,000 (303 with twelve products on
+// single CTAs of 13 slots), tensor pipe 63 % active; 64 slots of 1000 x 4001:
+// 23 us (26).
 
 constexpr int KD_BM = 128, KD_BK = 64;
-constexpr int KD_KDIG = 3, KD_RDIG = 4;
-constexpr int KD_S = 13;                     // slots per CTA
+constexpr int KD_KDIG = 3, KD_RDIG = 3;
+constexpr int KD_S = 17;                     // slots per tile
 constexpr int KD_C = 3;                      // product columns per slot (the fourth follows)
-constexpr int KD_COLS = KD_S * KD_C;         // 39 live columns per plane
-constexpr int KD_BN = 40;                    // rows per rho digit plane in a B tile
-constexpr int KD_HEAD = 32, KD_TAIL = KD_BN - KD_HEAD;
-constexpr int KD_A_BYTES = KD_BM * KD_BK * 2;          // one K digit plane tile, 16 KB
-constexpr int KD_HEAD_BYTES = KD_HEAD * KD_BK * 2;     // 4 KB
-constexpr int KD_TAIL_BYTES = KD_TAIL * KD_BK * 2;     // 1 KB
-constexpr int KD_STAGE = KD_KDIG * KD_A_BYTES + KD_RDIG * (KD_HEAD_BYTES + KD_TAIL_BYTES);
+constexpr int KD_COLS = KD_S * KD_C;         // 51 live columns per plane
+constexpr int KD_PS = 52;                    // rows (accumulator columns) from one plane to the next
+constexpr int KD_NB = 160;                   // rho rows of a tile: accumulator columns per K digit
+constexpr int KD_SEG = 24;                   // k-steps per segment: 1536 sequences
+constexpr int KD_RBASE = 640, KD_RHALF = 320;
+constexpr int KD_A_BYTES = KD_BM * KD_BK * 2;             // one K digit plane tile, 16 KB
+constexpr int KD_B_BYTES = KD_NB / 2 * KD_BK * 2;         // this CTA's half of the rho rows, 10 KB
+constexpr int KD_STAGE = KD_KDIG * KD_A_BYTES + KD_B_BYTES;
 constexpr int KD_STG = 3;
 constexpr int KD_SMEM = KD_STG * KD_STAGE + 1024 + 256;
+constexpr int KD_THREADS = 64 + 512, KD_READERS = 32;    // TMA, MMA and 16 epilogue warps
 constexpr uint32_t KD_TMEM_COLS = 512;
-constexpr int KD_NB = KD_RDIG * KD_BN;                 // 160 accumulator columns per K digit
-constexpr uint32_t IDESC_KD = (1u << 4) | ((uint32_t)(KD_NB >> 3) << 17) | ((uint32_t)(KD_BM >> 4) << 24);
-static_assert(KD_STAGE % 1024 == 0, "stage must keep 1024-byte alignment");
-static_assert(KD_HEAD_BYTES % 1024 == 0 && KD_TAIL_BYTES % 1024 == 0, "TMA destinations 1024-aligned");
-static_assert(KD_TAIL == 0 || KD_TAIL == 8, "plane tails of 8 rows (or none)");
+// kind::f16, D = F32, A = B = F16, K-major, M = 256 over the CTA pair
+constexpr uint32_t IDESC_KD = (1u << 4) | ((uint32_t)(KD_NB >> 3) << 17) | ((uint32_t)(2 * KD_BM >> 4) << 24);
+static_assert(KD_STAGE % 1024 == 0 && KD_B_BYTES % 1024 == 0, "tiles keep 1024-byte alignment");
 static_assert(KD_KDIG * KD_NB <= (int)KD_TMEM_COLS, "accumulators fit TMEM");
-static_assert(KD_NB % 16 == 0 && KD_NB <= 256, "MMA N for M = 128");
-static_assert(KD_COLS < KD_BN, "one unused row per plane");
+static_assert(KD_NB % 16 == 0 && KD_NB <= 256, "MMA N for M = 256");
+static_assert((KD_RDIG - 1) * KD_PS + KD_COLS <= KD_NB && KD_COLS <= KD_PS && KD_PS % 4 == 0, "planes of a tile");
+static_assert(32ll * 328 * KD_SEG * KD_BK < (1ll << 24), "a segment's sums are exact in FP32");
 
-__device__ __forceinline__ void mma_f16_kd(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
+// one MMA of the CTA pair, issued by the leader: each CTA's A rows and half
+// of the B rows at the same shared-memory offsets
+__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
         "l"(adesc), "l"(bdesc), "r"(IDESC_KD), "r"(accumulate)
         : "memory");
 }
 
 struct KdArgs {
     int kt_total;        // Nx / 64
-    int nk_rows;         // rows per K digit plane (multiple of 128)
-    int nr_rows;         // rows per rho digit plane (>= 3 x slots + 1)
+    int nk_rows;         // rows per K digit plane (multiple of 256)
     int N;
     int64_t Nx;
     int nlist;
     const int32_t *list;
     const uint8_t *rstate;
-    const long long *csum;
+    const long long *csum;       // class sums and column sums of rho_q (CSUM per slot)
+    long long center;            // c: K = K' + c
     double inv_qscale;
     float2 *KR;                  // K rho / qscale in double-float
     int *err;
     const int *ncount;           // list length in device memory (the grid covers the most slots), or null
 };
 
-__global__ void __launch_bounds__(THREADS, 1)
-k_kdig(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmRh,
-       const __grid_constant__ CUtensorMap tmRt, const KdArgs args)
+struct KdEpilogue {
+    uint32_t tmem_base, acc_full, lead_read;   // lead_read: the leader's barrier (shared::cluster address)
+    int rank, m_pairs, tiles, tile0, tstep, nkt, nlist;
+};
+
+// Slots S0 .. S0 + NS - 1 of this CTA pair's tiles: the warp's 32 rows of K.
+// The digit products' sums are integers below 2^24 (exact in the FP32
+// accumulators): each is converted with a 32-bit conversion; the K digits of
+// a plane are combined by shifts and the planes by Horner's rule in 64-bit
+// integers (no 64-bit conversion, which runs on GB300's narrow FP64 pipe).
+// False when a wait gave up.
+template <int S0, int NS>
+__device__ __forceinline__ bool kd_epilogue(const KdArgs &args, const KdEpilogue &e, int q, int lane)
+{
+    constexpr int C0 = S0 * KD_C, NC = NS * KD_C;
+    static_assert(C0 % 4 == 0, "columns are read in groups of four");
+    const uint32_t tm = e.tmem_base + ((uint32_t)(q * 32) << 16);
+    const float2 iq = df_from_d(args.inv_qscale);
+    int dr = 0;
+    for (int tile = e.tile0; tile < e.tiles; tile += e.tstep) {
+        const int row = (tile % e.m_pairs) * 2 * KD_BM + e.rank * KD_BM + q * 32 + lane;
+        const int P0 = (tile / e.m_pairs) * KD_S + S0;
+        // start from what the products lack: c times the column sums, less the
+        // agreement at the slot's own locus (read while the MMAs run)
+        long long acc[NC];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const bool live = P0 + s < e.nlist && row < args.N;
+            const int b = live ? args.list[P0 + s] : 0;
+            const int y = live ? args.rstate[(int64_t)b * args.Nx + row] & 3 : 0;
+            const long long *cs = args.csum + (int64_t)b * CSUM;
+#pragma unroll
+            for (int c = 0; c < KD_C; ++c)
+                acc[KD_C * s + c] = live ? args.center * cs[CSUM_ALL + c] - cs[y * 4 + c] : 0ll;
+        }
+        for (int j0 = 0; j0 < e.nkt; j0 += KD_SEG, ++dr) {
+            if (!mbar_wait(e.acc_full, (uint32_t)(dr & 1))) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int c0 = 0; c0 < NC; c0 += 4) {
+                long long h[4] = {0ll, 0ll, 0ll, 0ll};
+#pragma unroll
+                for (int p = KD_RDIG - 1; p >= 0; --p) {
+                    float v[KD_KDIG][4];
+#pragma unroll
+                    for (int k = 0; k < KD_KDIG; ++k)
+                        tmem_ld4(tm + (uint32_t)(k * KD_NB + p * KD_PS + C0 + c0), v[k]);
+                    tmem_ld_wait<KD_KDIG * 4>(&v[0][0]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const int low = __float2int_rn(v[0][c]) + (__float2int_rn(v[1][c]) << 6);   // below 2^31
+                        h[c] = h[c] * KD_RBASE + ((long long)__float2int_rn(v[2][c]) * 4096 + low);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 4 && c0 + c < NC; ++c) acc[c0 + c] += h[c];
+            }
+            // this warp has read its accumulators
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(e.lead_read);
+        }
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const int P = P0 + s;
+            if (P >= e.nlist || row >= args.Nx) continue;
+            const int b = args.list[P];
+            float2 val[4] = {df_zero(), df_zero(), df_zero(), df_zero()};
+            if (row < args.N) {
+                long long tot[4];
+#pragma unroll
+                for (int c = 0; c < KD_C; ++c) tot[c] = acc[KD_C * s + c];
+                tot[3] = -(tot[0] + tot[1] + tot[2]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) val[c] = df_mul(df_from_ll_fast(tot[c]), iq);
+            }
+            float4 *o = reinterpret_cast<float4 *>(args.KR + ((int64_t)b * args.Nx + row) * 4);
+            o[0] = make_float4(val[0].x, val[0].y, val[1].x, val[1].y);
+            o[1] = make_float4(val[2].x, val[2].y, val[3].x, val[3].y);
+        }
+    }
+    return true;
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(KD_THREADS, 1)
+k_kdig(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmR, const KdArgs args)
 {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase0 = smem_u32(smem_raw);
     const uint32_t sbase = (sbase0 + 1023u) & ~1023u;
     uint8_t *const sgen = smem_raw + (sbase - sbase0);
     const uint32_t bars = sbase + KD_STG * KD_STAGE;
+    // full (the leader's: both CTAs' loads), empty (in each CTA: the MMAs have
+    // read the stage), accumulators complete (in each CTA), accumulators read
+    // (the leader's: both CTAs' epilogue warps), TMEM address
     auto full = [&](int s) { return bars + 8u * s; };
     auto empty = [&](int s) { return bars + 8u * (KD_STG + s); };
-    const uint32_t tmem_full = bars + 8u * (2 * KD_STG);
-    const uint32_t tmem_slot = bars + 8u * (2 * KD_STG + 1);
-    uint32_t *tmem_slot_gen = reinterpret_cast<uint32_t *>(sgen + KD_STG * KD_STAGE + 8 * (2 * KD_STG + 1));
-    constexpr uint32_t BOFF = KD_KDIG * KD_A_BYTES;                      // plane heads
-    constexpr uint32_t TOFF = BOFF + KD_RDIG * KD_HEAD_BYTES;            // plane tails
+    const uint32_t acc_full = bars + 8u * (2 * KD_STG), acc_read = bars + 8u * (2 * KD_STG + 1);
+    const uint32_t tmem_slot = bars + 8u * (2 * KD_STG + 2);
+    uint32_t *tmem_slot_gen = reinterpret_cast<uint32_t *>(sgen + KD_STG * KD_STAGE + 8 * (2 * KD_STG + 2));
+    constexpr uint32_t BOFF = KD_KDIG * KD_A_BYTES;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m_tile = blockIdx.x, n_tile = blockIdx.y;
+    const uint32_t rank = cluster_rank();
     const int nkt = args.kt_total;
     const int nlist = args.ncount ? *args.ncount : args.nlist;
-    if (n_tile * KD_S >= nlist) return;   // (the whole CTA, before any barrier or TMEM allocation)
+    const int m_pairs = args.nk_rows / (2 * KD_BM);
+    const int tiles = m_pairs * ((nlist + KD_S - 1) / KD_S);
+    const int tile0 = blockIdx.x >> 1, tstep = gridDim.x >> 1;
+    if (tile0 >= tiles) return;   // (both CTAs of the pair, before any barrier or TMEM allocation)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < KD_STG; ++s) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
         }
-        mbar_init(tmem_full, 1);
+        mbar_init(acc_full, 1);
+        mbar_init(acc_read, KD_READERS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot),
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot),
                      "r"(KD_TMEM_COLS)
                      : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    cluster_sync();               // the peer's barriers are initialised
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot_gen;
     bool failed = false;
 
     if (warp == 0) {
         if (lane == 0) {
-            const int r0 = n_tile * KD_COLS;   // this CTA's first rho row in each plane
-            for (int j = 0; j < nkt; ++j) {
-                const int s = j % KD_STG;
-                const uint32_t ph = (uint32_t)((j / KD_STG) & 1);
-                if (!mbar_wait(empty(s), ph ^ 1u)) { failed = true; break; }
-                const uint32_t st = sbase + (uint32_t)s * KD_STAGE;
-                mbar_expect_tx(full(s), KD_STAGE);
+            const uint32_t lead_bars = map_to_rank(bars, 0);
+            int it = 0;
+            for (int tile = tile0; tile < tiles && !failed; tile += tstep) {
+                const int m0 = (tile % m_pairs) * 2 * KD_BM + (int)rank * KD_BM;
+                const int r0 = (tile / m_pairs) * KD_NB + (int)rank * (KD_NB / 2);
+                for (int j = 0; j < nkt; ++j, ++it) {
+                    const int s = it % KD_STG;
+                    if (!mbar_wait(empty(s), (uint32_t)((it / KD_STG) & 1) ^ 1u)) { failed = true; break; }
+                    const uint32_t st = sbase + (uint32_t)s * KD_STAGE;
+                    if (rank == 0) mbar_expect_tx(full(s), 2 * KD_STAGE);   // the pair's bytes
 #pragma unroll
-                for (int k = 0; k < KD_KDIG; ++k)
-                    tma_load_2d(st + k * KD_A_BYTES, &tmK, j * KD_BK, k * args.nk_rows + m_tile * KD_BM, full(s));
-#pragma unroll
-                for (int p = 0; p < KD_RDIG; ++p) {
-                    tma_load_2d(st + BOFF + p * KD_HEAD_BYTES, &tmRh, j * KD_BK, p * args.nr_rows + r0, full(s));
-                    if (KD_TAIL > 0)
-                        tma_load_2d(st + TOFF + p * KD_TAIL_BYTES, &tmRt, j * KD_BK, p * args.nr_rows + r0 + KD_HEAD,
-                                    full(s));
+                    for (int k = 0; k < KD_KDIG; ++k)
+                        tma_load_2d_pair(st + k * KD_A_BYTES, &tmK, j * KD_BK, k * args.nk_rows + m0, lead_bars + 8u * s);
+                    tma_load_2d_pair(st + BOFF, &tmR, j * KD_BK, r0, lead_bars + 8u * s);
                 }
             }
-            for (int j = max(0, nkt - KD_STG); j < nkt; ++j)
-                if (!mbar_wait(full(j % KD_STG), (uint32_t)((j / KD_STG) & 1))) failed = true;
+            // loads still in flight (both CTAs') land before the pair leaves
+            // its last cluster barrier
+            if (rank == 0)
+                for (int i = max(0, it - KD_STG); i < it; ++i)
+                    if (!mbar_wait(full(i % KD_STG), (uint32_t)((i / KD_STG) & 1))) failed = true;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            for (int j = 0; j < nkt; ++j) {
-                const int s = j % KD_STG;
-                const uint32_t ph = (uint32_t)((j / KD_STG) & 1);
-                if (!mbar_wait(full(s), ph)) { failed = true; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t st = sbase + (uint32_t)s * KD_STAGE;
+        if (lane == 0 && rank == 0) {
+            int it = 0, dr = 0;
+            for (int tile = tile0; tile < tiles && !failed; tile += tstep) {
+                for (int j0 = 0; j0 < nkt && !failed; j0 += KD_SEG, ++dr) {
+                    const int j1 = min(nkt, j0 + KD_SEG);
+                    // (the accumulators of the segment before have been read)
+                    if (!mbar_wait(acc_read, (uint32_t)(dr & 1) ^ 1u)) { failed = true; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int j = j0; j < j1; ++j, ++it) {
+                        const int s = it % KD_STG;
+                        if (!mbar_wait(full(s), (uint32_t)((it / KD_STG) & 1))) { failed = true; break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t st = sbase + (uint32_t)s * KD_STAGE;
 #pragma unroll
-                for (int kk = 0; kk < KD_BK / 16; ++kk) {
-                    const uint64_t bd = smem_desc_sw128(st + BOFF + kk * 32);
+                        for (int kk = 0; kk < KD_BK / 16; ++kk) {
+                            const uint64_t bd = smem_desc_sw128(st + BOFF + kk * 32);
 #pragma unroll
-                    for (int k = 0; k < KD_KDIG; ++k) {
-                        const uint64_t ad = smem_desc_sw128(st + k * KD_A_BYTES + kk * 32);
-                        mma_f16_kd(tmem_base + (uint32_t)(k * KD_NB), ad, bd, (j > 0 || kk > 0) ? 1u : 0u);
+                            for (int k = 0; k < KD_KDIG; ++k) {
+                                const uint64_t ad = smem_desc_sw128(st + k * KD_A_BYTES + kk * 32);
+                                mma_f16_pair(tmem_base + (uint32_t)(k * KD_NB), ad, bd, (j > j0 || kk > 0) ? 1u : 0u);
+                            }
+                        }
+                        mma_commit_pair(empty(s));
                     }
+                    mma_commit_pair(acc_full);
                 }
-                mma_commit(empty(s));
             }
-            mma_commit(tmem_full);
         }
     } else {
-        const bool ok = nkt > 0 && mbar_wait(tmem_full, 0u);
-        if (!ok && nkt > 0) failed = true;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int q = warp & 3;
-        const int row = m_tile * KD_BM + q * 32 + lane;
-        const float2 iq = df_from_d(args.inv_qscale);
-        // The 12 digit products are integers below 2^24 in magnitude (exact
-        // in the FP32 accumulators): each is converted with a 32-bit
-        // conversion and shifted into place in 64-bit integers (no 64-bit
-        // conversion or multiply, which run on GB300's narrow FP64 pipe).
-        long long acc[KD_COLS];
-#pragma unroll
-        for (int c = 0; c < KD_COLS; ++c) acc[c] = 0ll;
-        if (ok) {
-            const uint32_t lanes = (uint32_t)(q * 32) << 16;
-#pragma unroll 1
-            for (int k = 0; k < KD_KDIG; ++k)
-#pragma unroll 1
-                for (int p = 0; p < KD_RDIG; ++p) {
-                    const int sh = 6 * k + 7 * p;
-                    float v[32], t[8] = {};
-                    tmem_ld32(tmem_base + lanes + (uint32_t)(k * KD_NB + p * KD_HEAD), v);
-                    if (KD_TAIL > 0)
-                        tmem_ld8(tmem_base + lanes + (uint32_t)(k * KD_NB + KD_RDIG * KD_HEAD + p * KD_TAIL), t);
-#pragma unroll
-                    for (int c = 0; c < (KD_HEAD < KD_COLS ? KD_HEAD : KD_COLS); ++c)
-                        acc[c] += (long long)__float2int_rn(v[c]) << sh;
-#pragma unroll
-                    for (int c = KD_HEAD; c < KD_COLS; ++c) acc[c] += (long long)__float2int_rn(t[c - KD_HEAD]) << sh;
-                }
-#pragma unroll
-            for (int s = 0; s < KD_S; ++s) {
-                const int P = n_tile * KD_S + s;
-                if (P >= nlist || row >= args.Nx) continue;
-                const int b = args.list[P];
-                float2 val[4] = {df_zero(), df_zero(), df_zero(), df_zero()};
-                if (row < args.N) {
-                    const int y = args.rstate[(int64_t)b * args.Nx + row] & 3;
-                    const long long *cs = args.csum + (int64_t)b * 16 + y * 4;
-                    long long tot[4];
-#pragma unroll
-                    for (int c = 0; c < KD_C; ++c) tot[c] = acc[KD_C * s + c] - cs[c];
-                    tot[3] = -(tot[0] + tot[1] + tot[2]);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) val[c] = df_mul(df_from_ll_fast(tot[c]), iq);
-                }
-                float4 *o = reinterpret_cast<float4 *>(args.KR + ((int64_t)b * args.Nx + row) * 4);
-                o[0] = make_float4(val[0].x, val[0].y, val[1].x, val[1].y);
-                o[1] = make_float4(val[2].x, val[2].y, val[3].x, val[3].y);
-            }
-        }
+        // four warps per TMEM lane quadrant: slots 0..3, 4..7, 8..11 and 12..16 of the tile
+        const KdEpilogue e{tmem_base, acc_full, map_to_rank(acc_read, 0), (int)rank, m_pairs, tiles, tile0, tstep,
+                           nkt, nlist};
+        const int part = (warp - 2) >> 2, q = warp & 3;
+        failed = part == 0   ? !kd_epilogue<0, 4>(args, e, q, lane)
+                 : part == 1 ? !kd_epilogue<4, 4>(args, e, q, lane)
+                 : part == 2 ? !kd_epilogue<8, 4>(args, e, q, lane)
+                             : !kd_epilogue<12, 5>(args, e, q, lane);
     }
+    __syncwarp();
     if (failed) atomicExch(args.err, 1);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    cluster_sync();   // no MMA, load or remote arrival of the pair is left
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(KD_TMEM_COLS)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(KD_TMEM_COLS)
                      : "memory");
     }
 }
 
-// K (int32, Nx x Nx) -> three fp16 planes of base-64 digits, rows padded to nk_rows
-__global__ void k_kdig_split_k(const int32_t *__restrict__ K, int64_t Nx, int nk_rows, __half *__restrict__ Kd)
+// K (int32, Nx x Nx) less c -> three fp16 planes of balanced base-64 digits,
+// rows padded to nk_rows (padding sequences hold 0: their rho is 0)
+__global__ void k_kdig_split_k(const int32_t *__restrict__ K, int64_t Nx, int N, int center, int nk_rows,
+                               __half *__restrict__ Kd)
 {
     const int64_t total = (int64_t)nk_rows * Nx;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / Nx;
-        const int v = i < Nx ? K[t] : 0;
-        Kd[t] = __int2half_rn(v & 63);
-        Kd[(int64_t)nk_rows * Nx + t] = __int2half_rn((v >> 6) & 63);
-        Kd[2 * (int64_t)nk_rows * Nx + t] = __int2half_rn(v >> 12);
+        const int64_t i = t / Nx, j = t - i * Nx;
+        int v = i < N && j < N ? K[t] - center : 0;
+        const int d0 = ((v + 32) & 63) - 32;
+        v = (v - d0) >> 6;
+        const int d1 = ((v + 32) & 63) - 32;
+        Kd[t] = __int2half_rn(d0);
+        Kd[(int64_t)nk_rows * Nx + t] = __int2half_rn(d1);
+        Kd[2 * (int64_t)nk_rows * Nx + t] = __int2half_rn((v - d1) >> 6);
     }
 }
 
-// rho_q of list position P (slot list[P]), its first three columns -> four
-// fp16 planes of balanced base-128 digits, rows P*3+c
-__global__ void k_kdig_split_r(const int32_t *__restrict__ list, int64_t Nx, int nr_rows,
-                               const int4 *__restrict__ rq, __half *__restrict__ Rd, const int *__restrict__ cnt)
+// rho_q of list position P (slot list[P]), its first three columns -> fp16
+// balanced base-640 digits: plane p of column c in row 52 p + 3 (P % 17) + c
+// of tile P / 17
+__global__ void k_kdig_split_r(const int32_t *__restrict__ list, int64_t Nx, const int4 *__restrict__ rq,
+                               __half *__restrict__ Rd, const int *__restrict__ cnt)
 {
     if (cnt && (int)blockIdx.y >= *cnt) return;
     const int P = blockIdx.y, b = list[P];
+    const int64_t row0 = (int64_t)(P / KD_S) * KD_NB + (P % KD_S) * KD_C;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < Nx; j += (int64_t)gridDim.x * blockDim.x) {
         const int4 q = rq[(int64_t)b * Nx + j];
         const int qq[KD_C] = {q.x, q.y, q.z};
 #pragma unroll
         for (int c = 0; c < KD_C; ++c) {
-            long long v = qq[c];
+            int v = qq[c];
 #pragma unroll
             for (int p = 0; p < KD_RDIG; ++p) {
-                long long d = v;
+                int d = v;
                 if (p < KD_RDIG - 1) {
-                    d = ((v + 64) & 127) - 64;   // balanced digit, v - d divisible by 128
-                    v = (v - d) / 128;
+                    // |v| < 2^28: shifted by a multiple of the base to be positive
+                    constexpr int UP = (1 << 28) / KD_RBASE;
+                    const unsigned t = (unsigned)(v + KD_RHALF) + (unsigned)(UP * KD_RBASE);
+                    const unsigned qt = t / KD_RBASE;
+                    d = (int)(t - qt * KD_RBASE) - KD_RHALF;
+                    v = (int)qt - UP;
                 }
-                Rd[((int64_t)p * nr_rows + (int64_t)P * KD_C + c) * Nx + j] = __int2half_rn((int)d);
+                Rd[(row0 + p * KD_PS + c) * Nx + j] = __int2half_rn(d);
             }
         }
     }
@@ -911,31 +996,26 @@ TcPlan *tc_plan_create(const Problem &P, const uint8_t *X, const uint8_t *XT, __
 void tc_plan_destroy(TcPlan *p) { delete p; }
 
 struct KdPlan {
-    CUtensorMap mK, mRh, mRt;   // K digits; rho digit plane heads (32 rows) and tails (8 rows)
-    int nk_rows = 0, nr_rows = 0;
+    CUtensorMap mK, mR;   // K digit planes; the tiles' rho digit rows
+    int nk_rows = 0;
 };
 
-int kd_nk_rows(const Problem &P) { return (int)(((P.Nx + tc::KD_BM - 1) / tc::KD_BM) * tc::KD_BM); }
-// rows per rho digit plane: 3 per slot for whole CTAs of 13 slots, one more
-// for the last CTA's unused row, rounded to 8
-int kd_nr_rows(const Problem &P)
-{
-    const int64_t slots = (P.Bmax + tc::KD_S - 1) / tc::KD_S * tc::KD_S;
-    return (int)((tc::KD_C * slots + 1 + 7) / 8 * 8);
-}
+int kd_nk_rows(const Problem &P) { return (int)((P.Nx + 2 * tc::KD_BM - 1) / (2 * tc::KD_BM) * (2 * tc::KD_BM)); }
+// rho digit rows: whole tiles of 17 slots
+int kd_nr_rows(const Problem &P) { return (int)((P.Bmax + tc::KD_S - 1) / tc::KD_S * tc::KD_NB); }
+
+namespace {
+int kd_center(const Problem &P) { return (int)((P.L + 1) / 2); }
+} // namespace
 
 KdPlan *tc_kdig_plan_create(const Problem &P, __half *Kd, __half *Rd)
 {
     KdPlan *p = new KdPlan();
     p->nk_rows = kd_nk_rows(P);
-    p->nr_rows = kd_nr_rows(P);
     bool ok = make_map(&p->mK, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Kd, (uint64_t)P.Nx, (uint64_t)tc::KD_KDIG * p->nk_rows,
                        (uint64_t)P.Nx * 2, tc::KD_BK, tc::KD_BM, CU_TENSOR_MAP_SWIZZLE_128B);
-    ok &= make_map(&p->mRh, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Rd, (uint64_t)P.Nx, (uint64_t)tc::KD_RDIG * p->nr_rows,
-                   (uint64_t)P.Nx * 2, tc::KD_BK, tc::KD_HEAD, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (tc::KD_TAIL > 0)
-        ok &= make_map(&p->mRt, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Rd, (uint64_t)P.Nx, (uint64_t)tc::KD_RDIG * p->nr_rows,
-                       (uint64_t)P.Nx * 2, tc::KD_BK, tc::KD_TAIL > 0 ? tc::KD_TAIL : 8, CU_TENSOR_MAP_SWIZZLE_128B);
+    ok &= make_map(&p->mR, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Rd, (uint64_t)P.Nx, (uint64_t)kd_nr_rows(P),
+                   (uint64_t)P.Nx * 2, tc::KD_BK, tc::KD_NB / 2, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!ok) {
         delete p;
         return nullptr;
@@ -948,8 +1028,8 @@ void tc_kdig_plan_destroy(KdPlan *p) { delete p; }
 void tc_kdig_fill_k(const KdPlan *pl, const Problem &P, const int32_t *K, __half *Kd, cudaStream_t st)
 {
     const int64_t total = (int64_t)pl->nk_rows * P.Nx;
-    tc::k_kdig_split_k<<<(unsigned)std::min<int64_t>((total + 255) / 256, 8192), 256, 0, st>>>(K, P.Nx, pl->nk_rows,
-                                                                                          Kd);
+    tc::k_kdig_split_k<<<(unsigned)std::min<int64_t>((total + 255) / 256, 8192), 256, 0, st>>>(
+        K, P.Nx, (int)P.N, kd_center(P), pl->nk_rows, Kd);
 }
 
 cudaError_t tc_launch_kdig(const KdPlan *pl, const Problem &P, const int32_t *list, int n, const int32_t *rq,
@@ -959,24 +1039,26 @@ cudaError_t tc_launch_kdig(const KdPlan *pl, const Problem &P, const int32_t *li
     if (n <= 0) return cudaSuccess;
     {
         dim3 g((unsigned)std::min<int64_t>((P.Nx + 255) / 256, 64), (unsigned)n);
-        tc::k_kdig_split_r<<<g, 256, 0, st>>>(list, P.Nx, pl->nr_rows, reinterpret_cast<const int4 *>(rq), Rd, cnt);
+        tc::k_kdig_split_r<<<g, 256, 0, st>>>(list, P.Nx, reinterpret_cast<const int4 *>(rq), Rd, cnt);
     }
     tc::KdArgs a{};
     a.kt_total = (int)(P.Nx / tc::KD_BK);
     a.nk_rows = pl->nk_rows;
-    a.nr_rows = pl->nr_rows;
     a.N = (int)P.N;
     a.Nx = P.Nx;
     a.nlist = n;
     a.list = list;
     a.rstate = rstate;
     a.csum = csum;
+    a.center = kd_center(P);
     a.inv_qscale = inv_qscale;
     a.KR = KR;
     a.err = err;
     a.ncount = cnt;
-    dim3 grid((unsigned)(pl->nk_rows / tc::KD_BM), (unsigned)((n + tc::KD_S - 1) / tc::KD_S));
-    tc::k_kdig<<<grid, tc::THREADS, tc::KD_SMEM, st>>>(pl->mK, pl->mRh, pl->mRt, a);
+    // persistent: at most one CTA pair per two of the 152 SMs
+    const int64_t tiles = (int64_t)(pl->nk_rows / (2 * tc::KD_BM)) * ((n + tc::KD_S - 1) / tc::KD_S);
+    const unsigned pairs = (unsigned)std::min<int64_t>(tiles, 76);
+    tc::k_kdig<<<2 * pairs, tc::KD_THREADS, tc::KD_SMEM, st>>>(pl->mK, pl->mR, a);
     return cudaGetLastError();
 }
 

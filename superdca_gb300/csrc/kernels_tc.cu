@@ -10,9 +10,9 @@
 // scatter (plmDCA_objective.hpp:153-190) for a batch of target loci.
 //
 // Data path per CTA (128 x 128 output tile, K in steps of 64):
-//   * warp 0, one thread: TMA loads of the u8 state tile (2 KB) and of the
-//     fp16 hi and lo tiles of B (128 B swizzle), completing on full_raw[s];
-//   * warps 2-5: expand the u8 tile to the fp16 one-hot A tile directly in the
+//   * warps 0 and 2, one thread each: TMA loads of the u8 state tiles (2 KB
+//     per 128 rows) and of the fp16 hi and lo tiles of B (128 B swizzle);
+//   * warps 3-10: expand the u8 tile to the fp16 one-hot A tile directly in the
 //     128-byte-swizzled K-major layout the MMA reads (the one-hot matrix never
 //     exists in HBM: 1 byte per locus is read instead of 8), fence to the async
 //     proxy, arrive on full_a[s];
@@ -20,7 +20,7 @@
 //     accumulators in TMEM): A x B_hi and then A x B_lo into the same
 //     accumulator (or, with exact fp16 operands, a second N tile in the lo
 //     slot); tcgen05.commit frees the stage;
-//   * warps 2-5 again: tcgen05.ld the accumulator and store it, scaled back
+//   * warps 3-10 again: tcgen05.ld the accumulator and store it, scaled back
 //     by the per-slot power of two.
 // With hi + lo operands the backward keeps the expanded A tiles in TMEM
 // instead (tcgen05.st by the expansion warps, MMAs reading A from TMEM; see
@@ -49,7 +49,8 @@ constexpr int BM = 128, BN = 128, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;   // one 128-row one-hot subtile
 constexpr int B_BYTES = BN * BK * 2;   // one fp16 half (hi or lo) of the slot operand
 constexpr int RAW_BYTES = 2048;        // u8 states behind one subtile
-constexpr int THREADS = 192;
+constexpr int B_BOX = 32;              // slot-operand rows per TMA box: a tile loads its live rows only
+constexpr int THREADS = 96 + 256;      // two TMA, one MMA and eight expansion (then epilogue) warps
 
 // A CTA owns MSUB consecutive 128-row subtiles and reuses each staged B tile
 // for all of them: the slot operand is the traffic that the L2 has to carry,
@@ -68,13 +69,21 @@ constexpr int THREADS = 192;
 // cycle shared memory delivers.  TMEM then holds the accumulators
 // (MSUB x NT x 128 columns) and STG stages of MSUB A subtiles (32 columns
 // each: 64 sequences).
+// The state tiles have a ring of their own, deeper than the stages of A and
+// B: they come from HBM, and a stage that waited for its state tile only
+// after the MMAs had released it spent most of its time on that latency (a
+// check pass of 8 slots: 24k of 39k cycles a CTA waiting for state tiles).
 template <int MSUB, int STG, int NT = 1, bool AT = false> struct Cfg {
-    static constexpr int STAGE_BYTES = (AT ? 0 : MSUB * A_BYTES) + 2 * B_BYTES + MSUB * RAW_BYTES;
-    static constexpr int SMEM_BYTES = STG * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+    static constexpr int STAGE_BYTES = (AT ? 0 : MSUB * A_BYTES) + 2 * B_BYTES;
+    static constexpr int RAW_STG = AT ? 16 : 16 / MSUB;          // state-tile stages
+    static constexpr int RAW_STAGE = MSUB * RAW_BYTES;
+    static constexpr int BARS = 2 * RAW_STG + 3 * STG + 2;       // barriers and the TMEM address
+    static constexpr int SMEM_BYTES = STG * STAGE_BYTES + RAW_STG * RAW_STAGE + 1024 /*align*/ + 8 * BARS + 64;
     static constexpr uint32_t ACC_COLS = MSUB * BN * NT;
     static constexpr uint32_t A_COLS = AT ? MSUB * (BK / 2) * STG : 0;
     static constexpr uint32_t TMEM_COLS = AT ? 512 : ACC_COLS;
     static_assert(STAGE_BYTES % 1024 == 0, "stage must keep 1024-byte alignment");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
     static_assert(ACC_COLS + A_COLS <= 512, "TMEM holds 512 columns");
     static_assert(NT == 1 || NT == 2, "one or two N tiles per CTA");
 };
@@ -85,27 +94,31 @@ enum { MODE_FWD = 0, MODE_BWD = 1 };
 constexpr uint32_t IDESC = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(BN >> 3) << 17) |
                            ((uint32_t)(BM >> 4) << 24);
 
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+// (the elected lane's; descriptors by their low words)
+__device__ __forceinline__ void mma_f16(uint32_t lead, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
                                         uint32_t accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(accumulate)
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 e, %6, 0;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(tmem_d),
+        "r"(a_lo), "r"(b_lo), "r"(SMEM_DESC_HI), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
 
-// the same MMA with A read from TMEM (column tmem_a, lanes 0-127) and the
-// instruction descriptor given (its N fitted to the tile's live columns)
-__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                           uint32_t accumulate)
+// the same MMA with A read from TMEM (column tmem_a, lanes 0-127)
+__device__ __forceinline__ void mma_f16_ts(uint32_t lead, uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo,
+                                           uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t"
+        "setp.ne.b32 e, %6, 0;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "r"(b_lo), "r"(SMEM_DESC_HI), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
 
@@ -152,13 +165,14 @@ __device__ __forceinline__ void expand_fwd(const uint8_t *raw, uint32_t a_base, 
     }
 }
 
-// four bytes -> four fp16 lanes holding 1.0 where the byte equals s
+// four bytes (states 0..3) -> four fp16 lanes holding 1.0 where the byte
+// equals s: the byte's two bits against s, 0x3C per equal byte, and each byte
+// moved to the high half of its fp16 lane
 __device__ __forceinline__ uint2 eq_halves(uint32_t bytes, uint32_t s4)
 {
-    const uint32_t m = __vcmpeq4(bytes, s4);  // 0xFF per equal byte
-    const uint32_t a = __byte_perm(m, 0u, 0x1404) & 0x3C003C00u;
-    const uint32_t b = __byte_perm(m, 0u, 0x3424) & 0x3C003C00u;
-    return make_uint2(a, b);
+    const uint32_t t = bytes ^ s4;
+    const uint32_t m = (~(t | (t >> 1)) & 0x01010101u) * 0x3Cu;
+    return make_uint2(__byte_perm(m, 0u, 0x1404), __byte_perm(m, 0u, 0x3424));
 }
 
 // backward, A in TMEM: row t's 64 one-hot values as 32 sequence pairs
@@ -236,33 +250,39 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
        const __grid_constant__ CUtensorMap tmBlo, const GemmArgs args)
 {
     using C = Cfg<MSUB, STG, NT, AT>;
-    constexpr int SB = C::STAGE_BYTES;
+    constexpr int SB = C::STAGE_BYTES, RST = C::RAW_STG;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase0 = smem_u32(smem_raw);
     const uint32_t sbase = (sbase0 + 1023u) & ~1023u;
     uint8_t *const sgen = smem_raw + (sbase - sbase0);
-    const uint32_t bars = sbase + STG * SB;
-    // stage layout: [A subtiles (not with AT) | B hi | B lo | raw u8 tiles]
-    auto a_off = [](int ms) { return (uint32_t)(ms * A_BYTES); };
-    constexpr uint32_t BHI = AT ? 0 : MSUB * A_BYTES, BLO = BHI + B_BYTES, RAW = BLO + B_BYTES;
-    // barrier layout: full_raw[STG], full_a[STG], empty[STG], tmem_full, tmem addr
-    auto full_raw = [&](int s) { return bars + 8u * s; };
-    auto full_a = [&](int s) { return bars + 8u * (STG + s); };
-    auto empty = [&](int s) { return bars + 8u * (2 * STG + s); };
-    const uint32_t tmem_full = bars + 8u * (3 * STG);
-    const uint32_t tmem_slot = bars + 8u * (3 * STG + 1);
-    uint32_t *tmem_slot_gen = reinterpret_cast<uint32_t *>(sgen + STG * SB + 8 * (3 * STG + 1));
+    const uint32_t raws = sbase + STG * SB, bars = raws + RST * C::RAW_STAGE;
+    // stage layout: [A subtiles (not with AT) | B hi | B lo]; then the state-tile ring
+    constexpr uint32_t BHI = AT ? 0 : MSUB * A_BYTES, BLO = BHI + B_BYTES;
+    // barriers: state tile landed / read, slot operand landed, A expanded,
+    // stage free (its MMAs are done), accumulators complete; TMEM address
+    auto full_raw = [&](int r) { return bars + 8u * r; };
+    auto free_raw = [&](int r) { return bars + 8u * (RST + r); };
+    auto full_b = [&](int s) { return bars + 8u * (2 * RST + s); };
+    auto full_a = [&](int s) { return bars + 8u * (2 * RST + STG + s); };
+    auto empty = [&](int s) { return bars + 8u * (2 * RST + 2 * STG + s); };
+    const uint32_t tmem_full = bars + 8u * (2 * RST + 3 * STG);
+    const uint32_t tmem_slot = tmem_full + 8u;
+    uint32_t *tmem_slot_gen = reinterpret_cast<uint32_t *>(sgen + (tmem_slot - sbase));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp: uniform)
     const int m_group = blockIdx.x, n_tile = blockIdx.y * NT, split = blockIdx.z;   // first N tile
     const int kt0 = split * args.kt_begin_stride;
     const int kt1 = min(args.kt_total, kt0 + args.kt_begin_stride);
     const int nkt = max(0, kt1 - kt0);
 
     if (threadIdx.x == 0) {
+        for (int r = 0; r < RST; ++r) {
+            mbar_init(full_raw(r), 1);
+            mbar_init(free_raw(r), 8);
+        }
         for (int s = 0; s < STG; ++s) {
-            mbar_init(full_raw(s), 1);
-            mbar_init(full_a(s), 128);
+            mbar_init(full_b(s), 1);
+            mbar_init(full_a(s), 256);
             mbar_init(empty(s), 1);
         }
         mbar_init(tmem_full, 1);
@@ -277,93 +297,113 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_slot_gen;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot_gen, 0);   // (uniform)
     bool failed = false;
+    // live columns of this CTA's N tiles (4 per list position) and the TMA
+    // boxes that hold them: a check pass of 8 slots (32 columns) loads a
+    // quarter of what a full tile takes
+    constexpr int BOX_BYTES = B_BOX * BK * 2;
+    const int cols0 = min(BN, 4 * args.nlist - n_tile * BN), cols1 = min(BN, 4 * args.nlist - (n_tile + 1) * BN);
+    const int boxes0 = max(0, (cols0 + B_BOX - 1) / B_BOX), boxes1 = max(0, (cols1 + B_BOX - 1) / B_BOX);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (lane == 0) {   // state tiles
             for (int j = 0; j < nkt; ++j) {
-                const int s = j % STG;
-                const uint32_t ph = (uint32_t)((j / STG) & 1);
-                if (!mbar_wait(empty(s), ph ^ 1u)) { failed = true; break; }
-                const uint32_t st = sbase + (uint32_t)s * SB;
-                mbar_expect_tx(full_raw(s), MSUB * RAW_BYTES + (NT == 2 || !args.hi_only ? 2 : 1) * B_BYTES);
-                const int kt = kt0 + j;
+                const int r = j % RST, kt = kt0 + j;
+                if (!mbar_wait(free_raw(r), (uint32_t)((j / RST) & 1) ^ 1u)) { failed = true; break; }
+                mbar_expect_tx(full_raw(r), C::RAW_STAGE);
 #pragma unroll
                 for (int ms = 0; ms < MSUB; ++ms) {
                     const int mt = m_group * MSUB + ms;
-                    if (args.mode == MODE_FWD)
-                        tma_load_2d(st + RAW + ms * RAW_BYTES, &tmRaw, kt * 16, mt * BM, full_raw(s));
-                    else
-                        tma_load_2d(st + RAW + ms * RAW_BYTES, &tmRaw, kt * BK, mt * 32, full_raw(s));
+                    const uint32_t dst = raws + (uint32_t)(r * C::RAW_STAGE + ms * RAW_BYTES);
+                    if (args.mode == MODE_FWD) tma_load_2d(dst, &tmRaw, kt * 16, mt * BM, full_raw(r));
+                    else tma_load_2d(dst, &tmRaw, kt * BK, mt * 32, full_raw(r));
                 }
-                tma_load_2d(st + BHI, &tmBhi, kt * BK, n_tile * BN, full_raw(s));
-                if (NT == 2)   // the second N tile (rows past the operand's end read as zero)
-                    tma_load_2d(st + BLO, &tmBhi, kt * BK, (n_tile + 1) * BN, full_raw(s));
-                else if (!args.hi_only)
-                    tma_load_2d(st + BLO, &tmBlo, kt * BK, n_tile * BN, full_raw(s));
             }
             // loads still in flight land before the block retires
+            for (int j = max(0, nkt - RST); j < nkt; ++j)
+                if (!mbar_wait(full_raw(j % RST), (uint32_t)((j / RST) & 1))) failed = true;
+        }
+    } else if (warp == 2) {
+        if (lane == 0) {   // the slot operand
+            const int lo_boxes = NT == 2 ? boxes1 : args.hi_only ? 0 : boxes0;
+            for (int j = 0; j < nkt; ++j) {
+                const int s = j % STG, kt = kt0 + j;
+                if (!mbar_wait(empty(s), (uint32_t)((j / STG) & 1) ^ 1u)) { failed = true; break; }
+                const uint32_t st = sbase + (uint32_t)s * SB;
+                mbar_expect_tx(full_b(s), (boxes0 + lo_boxes) * BOX_BYTES);
+                for (int x = 0; x < boxes0; ++x)
+                    tma_load_2d(st + BHI + x * BOX_BYTES, &tmBhi, kt * BK, n_tile * BN + x * B_BOX, full_b(s));
+                // the lo half, or the second N tile
+                for (int x = 0; x < lo_boxes; ++x)
+                    tma_load_2d(st + BLO + x * BOX_BYTES, NT == 2 ? &tmBhi : &tmBlo, kt * BK,
+                                (n_tile + (NT == 2 ? 1 : 0)) * BN + x * B_BOX, full_b(s));
+            }
             for (int j = max(0, nkt - STG); j < nkt; ++j)
-                if (!mbar_wait(full_raw(j % STG), (uint32_t)((j / STG) & 1))) failed = true;
+                if (!mbar_wait(full_b(j % STG), (uint32_t)((j / STG) & 1))) failed = true;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // live columns of this CTA's N tiles (4 per list position)
-            const int cols0 = 4 * args.nlist - n_tile * BN, cols1 = cols0 - BN;
-            const uint32_t id0 = idesc_fit(cols0), id1 = idesc_fit(cols1);
-            for (int j = 0; j < nkt; ++j) {
-                const int s = j % STG;
-                const uint32_t ph = (uint32_t)((j / STG) & 1);
-                if (!mbar_wait(full_a(s), ph)) { failed = true; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t st = sbase + (uint32_t)s * SB;
-#pragma unroll
-                for (int kk = 0; kk < BK / 16; ++kk) {
-                    const uint64_t bh = smem_desc_sw128(st + BHI + kk * 32);
-                    const uint64_t bl = smem_desc_sw128(st + BLO + kk * 32);
-#pragma unroll
-                    for (int ms = 0; ms < MSUB; ++ms) {
-                        const uint32_t td = tmem_base + (uint32_t)(ms * BN);
-                        if (AT) {
-                            // K16 step kk: 8 of the subtile's 32 A columns
-                            const uint32_t ta =
-                                tmem_base + C::ACC_COLS + (uint32_t)((s * MSUB + ms) * (BK / 2) + kk * 8);
-                            mma_f16_ts(td, ta, bh, id0, (j > 0 || kk > 0) ? 1u : 0u);
-                            if (NT == 2) {
-                                if (cols1 > 0)   // (a second tile with no live column is not computed)
-                                    mma_f16_ts(td + (uint32_t)(MSUB * BN), ta, bl, id1, (j > 0 || kk > 0) ? 1u : 0u);
-                            } else if (!args.hi_only) {
-                                mma_f16_ts(td, ta, bl, id0, 1u);
-                            }
-                        } else {
-                            const uint64_t ad = smem_desc_sw128(st + a_off(ms) + kk * 32);
-                            mma_f16(td, ad, bh, (j > 0 || kk > 0) ? 1u : 0u);
-                            if (NT == 2)
-                                mma_f16(td + (uint32_t)(MSUB * BN), ad, bl, (j > 0 || kk > 0) ? 1u : 0u);
-                            else if (!args.hi_only)
-                                mma_f16(td, ad, bl, 1u);
-                        }
-                    }
-                }
-                mma_commit(empty(s));
-            }
-            // the accumulators are complete (or abandoned) once every issued MMA retired
-            mma_commit(tmem_full);
-        }
-    } else {
-        // with AT a warp writes only its TMEM lane quadrant: row = 32 (warp % 4) + lane
-        const int t = AT ? 32 * (warp & 3) + lane : threadIdx.x - 64;  // 0..127
+        const uint32_t lead = elect_lane();
+        const uint32_t id0 = idesc_fit(cols0), id1 = idesc_fit(cols1);
         for (int j = 0; j < nkt; ++j) {
             const int s = j % STG;
             const uint32_t ph = (uint32_t)((j / STG) & 1);
-            // (full_raw(s) completes only after the producer saw empty(s): the
-            // MMAs that read this stage's A before have retired)
-            if (!mbar_wait(full_raw(s), ph)) { failed = true; break; }
+            if (!mbar_wait_warp(full_b(s), ph) || !mbar_wait_warp(full_a(s), ph)) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t st = smem_desc_lo(sbase + (uint32_t)s * SB);
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; ++kk) {
+                const uint32_t bh = st + (BHI + kk * 32) / 16, bl = st + (BLO + kk * 32) / 16;
+                const uint32_t more = (j > 0 || kk > 0) ? 1u : 0u;
+#pragma unroll
+                for (int ms = 0; ms < MSUB; ++ms) {
+                    const uint32_t td = tmem_base + (uint32_t)(ms * BN);
+                    if (AT) {
+                        // K16 step kk: 8 of the subtile's 32 A columns
+                        const uint32_t ta =
+                            tmem_base + C::ACC_COLS + (uint32_t)((s * MSUB + ms) * (BK / 2) + kk * 8);
+                        mma_f16_ts(lead, td, ta, bh, id0, more);
+                        if (NT == 2) {
+                            if (cols1 > 0)   // (a second tile with no live column is not computed)
+                                mma_f16_ts(lead, td + (uint32_t)(MSUB * BN), ta, bl, id1, more);
+                        } else if (!args.hi_only) {
+                            mma_f16_ts(lead, td, ta, bl, id0, 1u);
+                        }
+                    } else {
+                        const uint32_t ad = st + (uint32_t)(ms * A_BYTES + kk * 32) / 16;
+                        mma_f16(lead, td, ad, bh, id0, more);
+                        if (NT == 2) {
+                            if (cols1 > 0) mma_f16(lead, td + (uint32_t)(MSUB * BN), ad, bl, id1, more);
+                        } else if (!args.hi_only) {
+                            mma_f16(lead, td, ad, bl, id0, 1u);
+                        }
+                    }
+                }
+            }
+            mma_commit_if(lead, empty(s));
+        }
+        // the accumulators are complete (or abandoned) once every issued MMA retired
+        mma_commit_if(lead, tmem_full);
+    } else {
+        // two groups of four warps, each taking every other subtile (with one
+        // warp per scheduler the expansion waited on its own latencies and
+        // set the pace); a warp writes only its TMEM lane quadrant: row =
+        // 32 (warp % 4) + lane
+        const int t = 32 * (warp & 3) + lane, group = (warp - 3) >> 2;
+        for (int j = 0; j < nkt; ++j) {
+            const int s = j % STG, r = j % RST;
+            // the state tile is here, and the MMAs that read this stage's A before are done
+            if (!mbar_wait(full_raw(r), (uint32_t)((j / RST) & 1)) ||
+                !mbar_wait(empty(s), (uint32_t)((j / STG) & 1) ^ 1u)) {
+                failed = true;
+                break;
+            }
             const uint32_t st = sbase + (uint32_t)s * SB;
 #pragma unroll
-            for (int ms = 0; ms < MSUB; ++ms) {
-                const uint8_t *raw = sgen + s * SB + RAW + ms * RAW_BYTES;
+            for (int ms2 = 0; ms2 < MSUB; ms2 += 2) {
+                const int ms = ms2 + group;
+                if (ms >= MSUB) break;
+                const uint8_t *raw = sgen + (raws - sbase) + r * C::RAW_STAGE + ms * RAW_BYTES;
                 if (AT) {
                     uint32_t o[32];
                     expand_bwd_regs(raw, t, o);
@@ -371,9 +411,9 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
                                   (uint32_t)((s * MSUB + ms) * (BK / 2)),
                               o);
                 } else if (args.mode == MODE_FWD) {
-                    expand_fwd(raw, st + a_off(ms), t);
+                    expand_fwd(raw, st + (uint32_t)(ms * A_BYTES), t);
                 } else {
-                    expand_bwd(raw, st + a_off(ms), t);
+                    expand_bwd(raw, st + (uint32_t)(ms * A_BYTES), t);
                 }
             }
             if (AT) {
@@ -383,6 +423,8 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             mbar_arrive(full_a(s));
+            __syncwarp();
+            if (lane == 0) mbar_arrive(free_raw(r));
         }
         // epilogue
         const bool ok = nkt > 0 && mbar_wait(tmem_full, 0u);
@@ -396,7 +438,8 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
             const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(nm * BN);
             const int row = (m_group * MSUB + ms) * BM + r;
 #pragma unroll 1
-            for (int cj = 0; cj < BN / 32; ++cj) {
+            for (int cj = group; cj < BN / 32; cj += 2) {   // (the groups share the columns out)
+                if (cj * 32 >= (nt == 0 ? cols0 : cols1)) break;
                 float v[32];
                 if (ok) tmem_ld32(tbase + (uint32_t)(cj * 32), v);
                 if (!ok) continue;
@@ -503,15 +546,18 @@ static_assert(KD_NB % 16 == 0 && KD_NB <= 256, "MMA N for M = 256");
 static_assert((KD_RDIG - 1) * KD_PS + KD_COLS <= KD_NB && KD_COLS <= KD_PS && KD_PS % 4 == 0, "planes of a tile");
 static_assert(32ll * 328 * KD_SEG * KD_BK < (1ll << 24), "a segment's sums are exact in FP32");
 
-// one MMA of the CTA pair, issued by the leader: each CTA's A rows and half
-// of the B rows at the same shared-memory offsets
-__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate)
+// one MMA of the CTA pair, issued by the leader's elected lane: each CTA's A
+// rows and half of the B rows at the same shared-memory offsets
+__device__ __forceinline__ void mma_f16_pair(uint32_t lead, uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo,
+                                             uint32_t accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(IDESC_KD), "r"(accumulate)
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 e, %6, 0;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(tmem_d),
+        "r"(a_lo), "r"(b_lo), "r"(SMEM_DESC_HI), "r"(IDESC_KD), "r"(accumulate), "r"(lead)
         : "memory");
 }
 
@@ -633,7 +679,7 @@ k_kdig(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensor
     uint32_t *tmem_slot_gen = reinterpret_cast<uint32_t *>(sgen + KD_STG * KD_STAGE + 8 * (2 * KD_STG + 2));
     constexpr uint32_t BOFF = KD_KDIG * KD_A_BYTES;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp: uniform)
     const uint32_t rank = cluster_rank();
     const int nkt = args.kt_total;
     const int nlist = args.ncount ? *args.ncount : args.nlist;
@@ -661,7 +707,7 @@ k_kdig(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensor
     __syncthreads();
     cluster_sync();               // the peer's barriers are initialised
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_slot_gen;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot_gen, 0);   // (uniform)
     bool failed = false;
 
     if (warp == 0) {
@@ -689,31 +735,29 @@ k_kdig(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensor
                     if (!mbar_wait(full(i % KD_STG), (uint32_t)((i / KD_STG) & 1))) failed = true;
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const uint32_t lead = elect_lane();
             int it = 0, dr = 0;
             for (int tile = tile0; tile < tiles && !failed; tile += tstep) {
                 for (int j0 = 0; j0 < nkt && !failed; j0 += KD_SEG, ++dr) {
                     const int j1 = min(nkt, j0 + KD_SEG);
                     // (the accumulators of the segment before have been read)
-                    if (!mbar_wait(acc_read, (uint32_t)(dr & 1) ^ 1u)) { failed = true; break; }
+                    if (!mbar_wait_warp(acc_read, (uint32_t)(dr & 1) ^ 1u)) { failed = true; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     for (int j = j0; j < j1; ++j, ++it) {
                         const int s = it % KD_STG;
-                        if (!mbar_wait(full(s), (uint32_t)((it / KD_STG) & 1))) { failed = true; break; }
+                        if (!mbar_wait_warp(full(s), (uint32_t)((it / KD_STG) & 1))) { failed = true; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint32_t st = sbase + (uint32_t)s * KD_STAGE;
+                        const uint32_t st = smem_desc_lo(sbase + (uint32_t)s * KD_STAGE);
 #pragma unroll
-                        for (int kk = 0; kk < KD_BK / 16; ++kk) {
-                            const uint64_t bd = smem_desc_sw128(st + BOFF + kk * 32);
+                        for (int kk = 0; kk < KD_BK / 16; ++kk)
 #pragma unroll
-                            for (int k = 0; k < KD_KDIG; ++k) {
-                                const uint64_t ad = smem_desc_sw128(st + k * KD_A_BYTES + kk * 32);
-                                mma_f16_pair(tmem_base + (uint32_t)(k * KD_NB), ad, bd, (j > j0 || kk > 0) ? 1u : 0u);
-                            }
-                        }
-                        mma_commit_pair(empty(s));
+                            for (int k = 0; k < KD_KDIG; ++k)
+                                mma_f16_pair(lead, tmem_base + (uint32_t)(k * KD_NB), st + (k * KD_A_BYTES + kk * 32) / 16,
+                                             st + (BOFF + kk * 32) / 16, (j > j0 || kk > 0) ? 1u : 0u);
+                        mma_commit_pair_if(lead, empty(s));
                     }
-                    mma_commit_pair(acc_full);
+                    mma_commit_pair_if(lead, acc_full);
                 }
             }
         }
@@ -904,13 +948,14 @@ void launch_gemm(dim3 grid, const CUtensorMap &a, const CUtensorMap &bh, const C
 
 // The backward with hi + lo operands (the tensor-core form's gradient, the
 // dual form's max-norm checks) keeps its one-hot A in TMEM: two subtiles,
-// four stages of 36 KB, the MMAs' N fitted to the live columns.  Measured
-// with ncu on the 3000 x 94,000 workload (192-slot check launches): 337-375
-// against 426-439 us for A in shared memory.  Exact (hi-only) operands -- the
-// dual form's solution digit planes, two N tiles per CTA -- stay with A in
-// shared memory: the TMEM form with one subtile and six stages took 689
-// against 607 us there.  SDCA_TC_BWD_SMEM_A=1 keeps A in shared memory
-// everywhere.
+// four stages, the MMAs' N fitted to the live columns.  On the 3000 x 94,000
+// workload (ncu, check launches of about 8 slots) it takes 234 us; A in shared
+// memory took 426-439 against 337-375 when both fed the MMAs from one lane
+// and the state tiles from the same ring.  Exact (hi-only) operands -- the
+// dual form's solution digit planes, two N tiles per CTA, 455 us for 21 slots
+// -- stay with A in shared memory: the TMEM form with one subtile and six
+// stages took 689 against 607 us there.  SDCA_TC_BWD_SMEM_A=1 keeps A in
+// shared memory everywhere.
 bool bwd_tmem_a()
 {
     static const bool v = [] {
@@ -978,14 +1023,14 @@ TcPlan *tc_plan_create(const Problem &P, const uint8_t *X, const uint8_t *XT, __
     p->has_fwd = Dhi && Dlo;
     if (p->has_fwd) {
         ok &= make_map(&p->mDhi, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Dhi, (uint64_t)Kp, (uint64_t)4 * P.Bmax,
-                       (uint64_t)Kp * 2, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+                       (uint64_t)Kp * 2, 64, tc::B_BOX, CU_TENSOR_MAP_SWIZZLE_128B);
         ok &= make_map(&p->mDlo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Dlo, (uint64_t)Kp, (uint64_t)4 * P.Bmax,
-                       (uint64_t)Kp * 2, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+                       (uint64_t)Kp * 2, 64, tc::B_BOX, CU_TENSOR_MAP_SWIZZLE_128B);
     }
     ok &= make_map(&p->mRhi, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Rhi, (uint64_t)P.Nx, (uint64_t)4 * P.Bmax,
-                   (uint64_t)P.Nx * 2, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+                   (uint64_t)P.Nx * 2, 64, tc::B_BOX, CU_TENSOR_MAP_SWIZZLE_128B);
     ok &= make_map(&p->mRlo, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, Rlo, (uint64_t)P.Nx, (uint64_t)4 * P.Bmax,
-                   (uint64_t)P.Nx * 2, 64, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+                   (uint64_t)P.Nx * 2, 64, tc::B_BOX, CU_TENSOR_MAP_SWIZZLE_128B);
     if (!ok) {
         delete p;
         return nullptr;

@@ -61,6 +61,28 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
+// ---- warp-uniform issue
+// The instructions that feed the tensor core take their descriptors from
+// uniform registers.  Issued by one lane of a divergent branch, each costs a
+// string of moves there (about 70 cycles an MMA, more than a small MMA's own
+// time); issued by a whole warp whose control flow is uniform, under the
+// predicate of its elected lane, the descriptors are formed in uniform
+// registers to begin with.
+
+// 1 in the warp's elected lane (the same lane every time), else 0
+__device__ __forceinline__ uint32_t elect_lane()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
+}
+
+// bounded wait by a whole warp; the verdict is uniform
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *tm, int x, int y,
                                             uint32_t bar)
 {
@@ -82,6 +104,20 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr)
     d |= (uint64_t)1 << 46;                          // version
     d |= (uint64_t)2 << 61;                          // SWIZZLE_128B
     return d;
+}
+
+// the descriptor's low word (its address field) and its constant high word
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t addr) { return (addr >> 4) & 0x3FFF; }
+constexpr uint32_t SMEM_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+
+// tcgen05.commit by the elected lane
+__device__ __forceinline__ void mma_commit_if(uint32_t lead, uint32_t bar)
+{
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(lead)
+        : "memory");
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t bar)
@@ -146,12 +182,15 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         : "memory");
 }
 
-// completion of the pair's MMAs issued so far, at the same barrier offset in both CTAs
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar)
+// completion of the pair's MMAs issued so far, at the same barrier offset in
+// both CTAs, by the elected lane
+__device__ __forceinline__ void mma_commit_pair_if(uint32_t lead, uint32_t bar)
 {
     asm volatile(
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-        "h"((uint16_t)3)
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(
+            bar),
+        "h"((uint16_t)3), "r"(lead)
         : "memory");
 }
 

@@ -20,7 +20,7 @@
 //     accumulators in TMEM): A x B_hi and then A x B_lo into the same
 //     accumulator (or, with exact fp16 operands, a second N tile in the lo
 //     slot); tcgen05.commit frees the stage;
-//   * warps 3-10 again: tcgen05.ld the accumulator and store it, scaled back
+//   * warps 11-14: tcgen05.ld the accumulator and store it, scaled back
 //     by the per-slot power of two.
 // With hi + lo operands the backward keeps the expanded A tiles in TMEM
 // instead (tcgen05.st by the expansion warps, MMAs reading A from TMEM; see
@@ -50,7 +50,7 @@ constexpr int A_BYTES = BM * BK * 2;   // one 128-row one-hot subtile
 constexpr int B_BYTES = BN * BK * 2;   // one fp16 half (hi or lo) of the slot operand
 constexpr int RAW_BYTES = 2048;        // u8 states behind one subtile
 constexpr int B_BOX = 32;              // slot-operand rows per TMA box: a tile loads its live rows only
-constexpr int THREADS = 96 + 256;      // two TMA, one MMA and eight expansion (then epilogue) warps
+constexpr int THREADS = 96 + 256 + 128;   // two TMA, one MMA, eight expansion and four epilogue warps
 
 // A CTA owns MSUB consecutive 128-row subtiles and reuses each staged B tile
 // for all of them: the slot operand is the traffic that the L2 has to carry,
@@ -77,7 +77,7 @@ template <int MSUB, int STG, int NT = 1, bool AT = false> struct Cfg {
     static constexpr int STAGE_BYTES = (AT ? 0 : MSUB * A_BYTES) + 2 * B_BYTES;
     static constexpr int RAW_STG = AT ? 16 : 16 / MSUB;          // state-tile stages
     static constexpr int RAW_STAGE = MSUB * RAW_BYTES;
-    static constexpr int BARS = 2 * RAW_STG + 3 * STG + 2;       // barriers and the TMEM address
+    static constexpr int BARS = 2 * RAW_STG + 3 * STG + 5;       // barriers and the TMEM address
     static constexpr int SMEM_BYTES = STG * STAGE_BYTES + RAW_STG * RAW_STAGE + 1024 /*align*/ + 8 * BARS + 64;
     static constexpr uint32_t ACC_COLS = MSUB * BN * NT;
     static constexpr uint32_t A_COLS = AT ? MSUB * (BK / 2) * STG : 0;
@@ -218,6 +218,7 @@ struct GemmArgs {
     int mode;
     int kt_begin_stride;  // k-tiles per split
     int kt_total;
+    int m_groups, n_groups, splits;   // tiles: groups of MSUB subtiles x groups of NT N tiles x K splits
     int m_rows;           // valid output rows (N for forward, 4L for backward)
     int nlist;
     const int32_t *list;  // list position -> slot
@@ -259,21 +260,48 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
     // stage layout: [A subtiles (not with AT) | B hi | B lo]; then the state-tile ring
     constexpr uint32_t BHI = AT ? 0 : MSUB * A_BYTES, BLO = BHI + B_BYTES;
     // barriers: state tile landed / read, slot operand landed, A expanded,
-    // stage free (its MMAs are done), accumulators complete; TMEM address
+    // stage free (its MMAs are done), accumulators complete / read; TMEM address
     auto full_raw = [&](int r) { return bars + 8u * r; };
     auto free_raw = [&](int r) { return bars + 8u * (RST + r); };
     auto full_b = [&](int s) { return bars + 8u * (2 * RST + s); };
     auto full_a = [&](int s) { return bars + 8u * (2 * RST + STG + s); };
     auto empty = [&](int s) { return bars + 8u * (2 * RST + 2 * STG + s); };
-    const uint32_t tmem_full = bars + 8u * (2 * RST + 3 * STG);
-    const uint32_t tmem_slot = tmem_full + 8u;
+    auto acc_full = [&](int u) { return bars + 8u * (2 * RST + 3 * STG + u); };
+    auto acc_free = [&](int u) { return bars + 8u * (2 * RST + 3 * STG + 2 + u); };
+    const uint32_t tmem_slot = bars + 8u * (2 * RST + 3 * STG + 4);
     uint32_t *tmem_slot_gen = reinterpret_cast<uint32_t *>(sgen + (tmem_slot - sbase));
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (warp: uniform)
-    const int m_group = blockIdx.x, n_tile = blockIdx.y * NT, split = blockIdx.z;   // first N tile
-    const int kt0 = split * args.kt_begin_stride;
-    const int kt1 = min(args.kt_total, kt0 + args.kt_begin_stride);
-    const int nkt = max(0, kt1 - kt0);
+    // The CTA's share of the tiles (output subtile group, N tile, K split), in
+    // turn.  Every role walks them with its own counters through the rings, so
+    // the state tiles of the next tile load and expand while the last one is
+    // in its epilogue: with one tile per CTA, 10 us of launch, set-up, first
+    // loads and epilogue stood beside each tile's 4 us of work at 616 sequences.
+    const int tiles = args.m_groups * args.n_groups * args.splits;
+    // live columns of a tile's N tiles (4 per list position) and the TMA
+    // boxes that hold them: a check pass of 8 slots (32 columns) loads a
+    // quarter of what a full tile takes
+    struct Tile {
+        int m_group, n_tile, split, kt0, nkt, cols0, cols1, boxes0, boxes1;
+    };
+    auto tile_at = [&](int i) {
+        Tile T;
+        T.m_group = i % args.m_groups;
+        const int rest = i / args.m_groups;
+        T.n_tile = rest % args.n_groups * NT;
+        T.split = rest / args.n_groups;
+        T.kt0 = T.split * args.kt_begin_stride;
+        T.nkt = max(0, min(args.kt_total, T.kt0 + args.kt_begin_stride) - T.kt0);
+        T.cols0 = min(BN, 4 * args.nlist - T.n_tile * BN);
+        T.cols1 = min(BN, 4 * args.nlist - (T.n_tile + 1) * BN);
+        T.boxes0 = max(0, (T.cols0 + B_BOX - 1) / B_BOX);
+        T.boxes1 = max(0, (T.cols1 + B_BOX - 1) / B_BOX);
+        return T;
+    };
+    constexpr int BOX_BYTES = B_BOX * BK * 2;
+    // with at most 64 live columns a subtile's 128 accumulator columns hold
+    // two tiles' sums: the MMAs of one run during the epilogue of the other
+    const int nbuf = NT == 1 && 4 * args.nlist <= BN / 2 ? 2 : 1;
 
     if (threadIdx.x == 0) {
         for (int r = 0; r < RST; ++r) {
@@ -285,7 +313,10 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
             mbar_init(full_a(s), 256);
             mbar_init(empty(s), 1);
         }
-        mbar_init(tmem_full, 1);
+        for (int u = 0; u < 2; ++u) {
+            mbar_init(acc_full(u), 1);
+            mbar_init(acc_free(u), 4);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -299,185 +330,243 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot_gen, 0);   // (uniform)
     bool failed = false;
-    // live columns of this CTA's N tiles (4 per list position) and the TMA
-    // boxes that hold them: a check pass of 8 slots (32 columns) loads a
-    // quarter of what a full tile takes
-    constexpr int BOX_BYTES = B_BOX * BK * 2;
-    const int cols0 = min(BN, 4 * args.nlist - n_tile * BN), cols1 = min(BN, 4 * args.nlist - (n_tile + 1) * BN);
-    const int boxes0 = max(0, (cols0 + B_BOX - 1) / B_BOX), boxes1 = max(0, (cols1 + B_BOX - 1) / B_BOX);
 
     if (warp == 0) {
         if (lane == 0) {   // state tiles
-            for (int j = 0; j < nkt; ++j) {
-                const int r = j % RST, kt = kt0 + j;
-                if (!mbar_wait(free_raw(r), (uint32_t)((j / RST) & 1) ^ 1u)) { failed = true; break; }
-                mbar_expect_tx(full_raw(r), C::RAW_STAGE);
+            int it = 0;
+            for (int i = blockIdx.x; i < tiles && !failed; i += gridDim.x) {
+                const Tile T = tile_at(i);
+                for (int j = 0; j < T.nkt; ++j, ++it) {
+                    const int r = it % RST, kt = T.kt0 + j;
+                    if (!mbar_wait(free_raw(r), (uint32_t)((it / RST) & 1) ^ 1u)) { failed = true; break; }
+                    mbar_expect_tx(full_raw(r), C::RAW_STAGE);
 #pragma unroll
-                for (int ms = 0; ms < MSUB; ++ms) {
-                    const int mt = m_group * MSUB + ms;
-                    const uint32_t dst = raws + (uint32_t)(r * C::RAW_STAGE + ms * RAW_BYTES);
-                    if (args.mode == MODE_FWD) tma_load_2d(dst, &tmRaw, kt * 16, mt * BM, full_raw(r));
-                    else tma_load_2d(dst, &tmRaw, kt * BK, mt * 32, full_raw(r));
-                }
-            }
-            // loads still in flight land before the block retires
-            for (int j = max(0, nkt - RST); j < nkt; ++j)
-                if (!mbar_wait(full_raw(j % RST), (uint32_t)((j / RST) & 1))) failed = true;
-        }
-    } else if (warp == 2) {
-        if (lane == 0) {   // the slot operand
-            const int lo_boxes = NT == 2 ? boxes1 : args.hi_only ? 0 : boxes0;
-            for (int j = 0; j < nkt; ++j) {
-                const int s = j % STG, kt = kt0 + j;
-                if (!mbar_wait(empty(s), (uint32_t)((j / STG) & 1) ^ 1u)) { failed = true; break; }
-                const uint32_t st = sbase + (uint32_t)s * SB;
-                mbar_expect_tx(full_b(s), (boxes0 + lo_boxes) * BOX_BYTES);
-                for (int x = 0; x < boxes0; ++x)
-                    tma_load_2d(st + BHI + x * BOX_BYTES, &tmBhi, kt * BK, n_tile * BN + x * B_BOX, full_b(s));
-                // the lo half, or the second N tile
-                for (int x = 0; x < lo_boxes; ++x)
-                    tma_load_2d(st + BLO + x * BOX_BYTES, NT == 2 ? &tmBhi : &tmBlo, kt * BK,
-                                (n_tile + (NT == 2 ? 1 : 0)) * BN + x * B_BOX, full_b(s));
-            }
-            for (int j = max(0, nkt - STG); j < nkt; ++j)
-                if (!mbar_wait(full_b(j % STG), (uint32_t)((j / STG) & 1))) failed = true;
-        }
-    } else if (warp == 1) {
-        const uint32_t lead = elect_lane();
-        const uint32_t id0 = idesc_fit(cols0), id1 = idesc_fit(cols1);
-        for (int j = 0; j < nkt; ++j) {
-            const int s = j % STG;
-            const uint32_t ph = (uint32_t)((j / STG) & 1);
-            if (!mbar_wait_warp(full_b(s), ph) || !mbar_wait_warp(full_a(s), ph)) { failed = true; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t st = smem_desc_lo(sbase + (uint32_t)s * SB);
-#pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-                const uint32_t bh = st + (BHI + kk * 32) / 16, bl = st + (BLO + kk * 32) / 16;
-                const uint32_t more = (j > 0 || kk > 0) ? 1u : 0u;
-#pragma unroll
-                for (int ms = 0; ms < MSUB; ++ms) {
-                    const uint32_t td = tmem_base + (uint32_t)(ms * BN);
-                    if (AT) {
-                        // K16 step kk: 8 of the subtile's 32 A columns
-                        const uint32_t ta =
-                            tmem_base + C::ACC_COLS + (uint32_t)((s * MSUB + ms) * (BK / 2) + kk * 8);
-                        mma_f16_ts(lead, td, ta, bh, id0, more);
-                        if (NT == 2) {
-                            if (cols1 > 0)   // (a second tile with no live column is not computed)
-                                mma_f16_ts(lead, td + (uint32_t)(MSUB * BN), ta, bl, id1, more);
-                        } else if (!args.hi_only) {
-                            mma_f16_ts(lead, td, ta, bl, id0, 1u);
-                        }
-                    } else {
-                        const uint32_t ad = st + (uint32_t)(ms * A_BYTES + kk * 32) / 16;
-                        mma_f16(lead, td, ad, bh, id0, more);
-                        if (NT == 2) {
-                            if (cols1 > 0) mma_f16(lead, td + (uint32_t)(MSUB * BN), ad, bl, id1, more);
-                        } else if (!args.hi_only) {
-                            mma_f16(lead, td, ad, bl, id0, 1u);
-                        }
+                    for (int ms = 0; ms < MSUB; ++ms) {
+                        const int mt = T.m_group * MSUB + ms;
+                        const uint32_t dst = raws + (uint32_t)(r * C::RAW_STAGE + ms * RAW_BYTES);
+                        if (args.mode == MODE_FWD) tma_load_2d(dst, &tmRaw, kt * 16, mt * BM, full_raw(r));
+                        else tma_load_2d(dst, &tmRaw, kt * BK, mt * 32, full_raw(r));
                     }
                 }
             }
-            mma_commit_if(lead, empty(s));
+            // loads still in flight land before the block retires
+            for (int k = max(0, it - RST); k < it; ++k)
+                if (!mbar_wait(full_raw(k % RST), (uint32_t)((k / RST) & 1))) failed = true;
         }
-        // the accumulators are complete (or abandoned) once every issued MMA retired
-        mma_commit_if(lead, tmem_full);
-    } else {
+    } else if (warp == 2) {
+        if (lane == 0) {   // the slot operand
+            int it = 0;
+            for (int i = blockIdx.x; i < tiles && !failed; i += gridDim.x) {
+                const Tile T = tile_at(i);
+                const int lo_boxes = NT == 2 ? T.boxes1 : args.hi_only ? 0 : T.boxes0;
+                for (int j = 0; j < T.nkt; ++j, ++it) {
+                    const int s = it % STG, kt = T.kt0 + j;
+                    if (!mbar_wait(empty(s), (uint32_t)((it / STG) & 1) ^ 1u)) { failed = true; break; }
+                    const uint32_t st = sbase + (uint32_t)s * SB;
+                    mbar_expect_tx(full_b(s), (T.boxes0 + lo_boxes) * BOX_BYTES);
+                    for (int x = 0; x < T.boxes0; ++x)
+                        tma_load_2d(st + BHI + x * BOX_BYTES, &tmBhi, kt * BK, T.n_tile * BN + x * B_BOX, full_b(s));
+                    // the lo half, or the second N tile
+                    for (int x = 0; x < lo_boxes; ++x)
+                        tma_load_2d(st + BLO + x * BOX_BYTES, NT == 2 ? &tmBhi : &tmBlo, kt * BK,
+                                    (T.n_tile + (NT == 2 ? 1 : 0)) * BN + x * B_BOX, full_b(s));
+                }
+            }
+            for (int k = max(0, it - STG); k < it; ++k)
+                if (!mbar_wait(full_b(k % STG), (uint32_t)((k / STG) & 1))) failed = true;
+        }
+    } else if (warp == 1) {
+        const uint32_t lead = elect_lane();
+        int it = 0, dr = 0;
+        for (int i = blockIdx.x; i < tiles && !failed; i += gridDim.x, ++dr) {
+            const Tile T = tile_at(i);
+            const uint32_t id0 = idesc_fit(T.cols0), id1 = idesc_fit(T.cols1);
+            const int u = nbuf == 2 ? dr & 1 : 0, use = nbuf == 2 ? dr >> 1 : dr;
+            const uint32_t acc0 = tmem_base + (uint32_t)(u * (BN / 2));
+            // (the sums of the tile before in this buffer have been read)
+            if (!mbar_wait_warp(acc_free(u), (uint32_t)(use & 1) ^ 1u)) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int j = 0; j < T.nkt; ++j, ++it) {
+                const int s = it % STG;
+                const uint32_t ph = (uint32_t)((it / STG) & 1);
+                if (!mbar_wait_warp(full_b(s), ph) || !mbar_wait_warp(full_a(s), ph)) { failed = true; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t st = smem_desc_lo(sbase + (uint32_t)s * SB);
+#pragma unroll
+                for (int kk = 0; kk < BK / 16; ++kk) {
+                    const uint32_t bh = st + (BHI + kk * 32) / 16, bl = st + (BLO + kk * 32) / 16;
+                    const uint32_t more = (j > 0 || kk > 0) ? 1u : 0u;
+#pragma unroll
+                    for (int ms = 0; ms < MSUB; ++ms) {
+                        const uint32_t td = acc0 + (uint32_t)(ms * BN);
+                        if (AT) {
+                            // K16 step kk: 8 of the subtile's 32 A columns
+                            const uint32_t ta =
+                                tmem_base + C::ACC_COLS + (uint32_t)((s * MSUB + ms) * (BK / 2) + kk * 8);
+                            mma_f16_ts(lead, td, ta, bh, id0, more);
+                            if (NT == 2) {
+                                if (T.cols1 > 0)   // (a second tile with no live column is not computed)
+                                    mma_f16_ts(lead, td + (uint32_t)(MSUB * BN), ta, bl, id1, more);
+                            } else if (!args.hi_only) {
+                                mma_f16_ts(lead, td, ta, bl, id0, 1u);
+                            }
+                        } else {
+                            const uint32_t ad = st + (uint32_t)(ms * A_BYTES + kk * 32) / 16;
+                            mma_f16(lead, td, ad, bh, id0, more);
+                            if (NT == 2) {
+                                if (T.cols1 > 0) mma_f16(lead, td + (uint32_t)(MSUB * BN), ad, bl, id1, more);
+                            } else if (!args.hi_only) {
+                                mma_f16(lead, td, ad, bl, id0, 1u);
+                            }
+                        }
+                    }
+                }
+                mma_commit_if(lead, empty(s));
+            }
+            // the accumulators are complete (or abandoned) once every issued MMA retired
+            mma_commit_if(lead, acc_full(u));
+        }
+    } else if (warp < 11) {
         // two groups of four warps, each taking every other subtile (with one
         // warp per scheduler the expansion waited on its own latencies and
         // set the pace); a warp writes only its TMEM lane quadrant: row =
         // 32 (warp % 4) + lane
         const int t = 32 * (warp & 3) + lane, group = (warp - 3) >> 2;
-        for (int j = 0; j < nkt; ++j) {
-            const int s = j % STG, r = j % RST;
-            // the state tile is here, and the MMAs that read this stage's A before are done
-            if (!mbar_wait(full_raw(r), (uint32_t)((j / RST) & 1)) ||
-                !mbar_wait(empty(s), (uint32_t)((j / STG) & 1) ^ 1u)) {
-                failed = true;
-                break;
-            }
-            const uint32_t st = sbase + (uint32_t)s * SB;
-#pragma unroll
-            for (int ms2 = 0; ms2 < MSUB; ms2 += 2) {
-                const int ms = ms2 + group;
-                if (ms >= MSUB) break;
-                const uint8_t *raw = sgen + (raws - sbase) + r * C::RAW_STAGE + ms * RAW_BYTES;
-                if (AT) {
-                    uint32_t o[32];
-                    expand_bwd_regs(raw, t, o);
-                    tmem_st32(tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + C::ACC_COLS +
-                                  (uint32_t)((s * MSUB + ms) * (BK / 2)),
-                              o);
-                } else if (args.mode == MODE_FWD) {
-                    expand_fwd(raw, st + (uint32_t)(ms * A_BYTES), t);
-                } else {
-                    expand_bwd(raw, st + (uint32_t)(ms * A_BYTES), t);
+        int it = 0;
+        for (int i = blockIdx.x; i < tiles && !failed; i += gridDim.x) {
+            const Tile T = tile_at(i);
+            for (int j = 0; j < T.nkt; ++j, ++it) {
+                const int s = it % STG, r = it % RST;
+                // the state tile is here, and the MMAs that read this stage's A before are done
+                if (!mbar_wait(full_raw(r), (uint32_t)((it / RST) & 1)) ||
+                    !mbar_wait(empty(s), (uint32_t)((it / STG) & 1) ^ 1u)) {
+                    failed = true;
+                    break;
                 }
-            }
-            if (AT) {
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            } else {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            }
-            mbar_arrive(full_a(s));
-            __syncwarp();
-            if (lane == 0) mbar_arrive(free_raw(r));
-        }
-        // epilogue
-        const bool ok = nkt > 0 && mbar_wait(tmem_full, 0u);
-        if (!ok && nkt > 0) failed = true;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int q = warp & 3;  // TMEM lane quadrant of this warp
-        const int r = q * 32 + lane;
-#pragma unroll 1
-        for (int nm = 0; nm < NT * MSUB; ++nm) {
-            const int nt = nm / MSUB, ms = nm % MSUB;
-            const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(nm * BN);
-            const int row = (m_group * MSUB + ms) * BM + r;
-#pragma unroll 1
-            for (int cj = group; cj < BN / 32; cj += 2) {   // (the groups share the columns out)
-                if (cj * 32 >= (nt == 0 ? cols0 : cols1)) break;
-                float v[32];
-                if (ok) tmem_ld32(tbase + (uint32_t)(cj * 32), v);
-                if (!ok) continue;
+                const uint32_t st = sbase + (uint32_t)s * SB;
 #pragma unroll
-                for (int tt = 0; tt < 8; ++tt) {
-                    const int P = ((n_tile + nt) * BN + cj * 32) / 4 + tt;
+                for (int ms2 = 0; ms2 < MSUB; ms2 += 2) {
+                    const int ms = ms2 + group;
+                    if (ms >= MSUB) break;
+                    const uint8_t *raw = sgen + (raws - sbase) + r * C::RAW_STAGE + ms * RAW_BYTES;
+                    if (AT) {
+                        uint32_t o[32];
+                        expand_bwd_regs(raw, t, o);
+                        tmem_st32(tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + C::ACC_COLS +
+                                      (uint32_t)((s * MSUB + ms) * (BK / 2)),
+                                  o);
+                    } else if (args.mode == MODE_FWD) {
+                        expand_fwd(raw, st + (uint32_t)(ms * A_BYTES), t);
+                    } else {
+                        expand_bwd(raw, st + (uint32_t)(ms * A_BYTES), t);
+                    }
+                }
+                if (AT) {
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                } else {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
+                mbar_arrive(full_a(s));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(free_raw(r));
+            }
+        }
+    } else {
+        // epilogue: warp = TMEM lane quadrant
+        const int q = warp & 3;
+        const int r = q * 32 + lane;
+        // What a store needs of its slot, one slot of the N tile per lane
+        // (lane p: list position 32 n_tile + p), read when the N tile changes
+        // and passed round by shuffles: with the slot's list entry and state
+        // read at every use, their latency was most of a tile's epilogue.
+        int loc[NT], cur = -1;
+        int64_t off[NT];
+        float sc[NT];
+        unsigned top[NT];   // max-only: the slot's largest |g| so far (float bits)
+        auto flush = [&]() {   // one atomic per warp and slot
+            if (args.gmax_acc)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+                    if (cur >= 0 && top[nt] != 0u)
+                        atomicMax(reinterpret_cast<unsigned long long *>(args.gmax_acc + off[nt]),
+                                  (unsigned long long)__double_as_longlong((double)__uint_as_float(top[nt])));
+        };
+        int dr = 0;
+        for (int i = blockIdx.x; i < tiles; i += gridDim.x, ++dr) {
+            const Tile T = tile_at(i);
+            if (T.n_tile != cur) {
+                flush();
+                cur = T.n_tile;
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    const int P = (cur + nt) * (BN / 4) + lane;
+                    loc[nt] = -1;
+                    off[nt] = 0;
+                    sc[nt] = args.inv_scale_bwd;
+                    top[nt] = 0u;
                     if (P >= args.nlist) continue;
                     const int b = args.planes > 1 ? args.list[P % args.nslot] : args.list[P];
                     if (args.mode == MODE_FWD) {
-                        if (row < args.Nx) {
-                            const float sc = (float)args.sd[b].tc_inv_scale;
-                            args.partial[((int64_t)split * args.Bmax + b) * args.Nx + row] =
-                                make_float4(v[4 * tt] * sc, v[4 * tt + 1] * sc, v[4 * tt + 2] * sc,
-                                            v[4 * tt + 3] * sc);
-                        }
+                        sc[nt] = (float)args.sd[b].tc_inv_scale;
+                        off[nt] = (int64_t)b * args.Nx;
                     } else if (args.gmax_acc) {
-                        // (the list position P is the same in every lane of the warp)
-                        float mv = 0.f;
-                        if (row < args.m_rows && (row >> 2) != args.sd[b].locus)
-                            mv = fmaxf(fmaxf(fabsf(v[4 * tt]), fabsf(v[4 * tt + 1])),
-                                       fmaxf(fabsf(v[4 * tt + 2]), fabsf(v[4 * tt + 3]))) * args.inv_scale_bwd;
-                        const unsigned mask = __activemask();
-                        const unsigned mb = __reduce_max_sync(mask, __float_as_uint(mv));
-                        if (lane == __ffs(mask) - 1 && mb != 0u)
-                            atomicMax(reinterpret_cast<unsigned long long *>(args.gmax_acc +
-                                                                             (int64_t)b * args.gmax_stride),
-                                      (unsigned long long)__double_as_longlong((double)__uint_as_float(mb)));
-                    } else if (row < args.m_rows) {
-                        const float sc = args.inv_scale_bwd;
-                        const int64_t buf = args.planes > 1 ? (int64_t)P : (int64_t)(2 * b + 1 - args.sd[b].gcur);
-                        float *gn = args.gpool + buf * args.Dp + (int64_t)(row >> 2) * QQ + (row & 3) * Q;
-                        *reinterpret_cast<float4 *>(gn) = make_float4(v[4 * tt] * sc, v[4 * tt + 1] * sc,
-                                                                      v[4 * tt + 2] * sc, v[4 * tt + 3] * sc);
+                        loc[nt] = args.sd[b].locus;
+                        off[nt] = (int64_t)b * args.gmax_stride;
+                    } else {
+                        off[nt] = (args.planes > 1 ? (int64_t)P : (int64_t)(2 * b + 1 - args.sd[b].gcur)) * args.Dp;
                     }
                 }
             }
+            const int u = nbuf == 2 ? dr & 1 : 0, use = nbuf == 2 ? dr >> 1 : dr;
+            if (!mbar_wait_warp(acc_full(u), (uint32_t)(use & 1))) { failed = true; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const int cols = nt == 0 ? T.cols0 : T.cols1;
+#pragma unroll 1
+                for (int ms = 0; ms < MSUB && T.nkt > 0; ++ms) {
+                    const uint32_t tbase =
+                        tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(u * (BN / 2) + (nt * MSUB + ms) * BN);
+                    const int row = (T.m_group * MSUB + ms) * BM + r;
+#pragma unroll 1
+                    for (int c0 = 0; c0 < cols; c0 += 32) {
+                        float v[32];
+                        tmem_ld32(tbase + (uint32_t)c0, v);
+#pragma unroll
+                        for (int tt = 0; tt < 8; ++tt) {
+                            const int p = c0 / 4 + tt;   // the slot's place in the N tile: its lane
+                            if (4 * p >= cols) break;
+                            if (args.gmax_acc) {
+                                const int locus = __shfl_sync(0xffffffffu, loc[nt], p);
+                                float mv = 0.f;
+                                if (row < args.m_rows && (row >> 2) != locus)
+                                    mv = fmaxf(fmaxf(fabsf(v[4 * tt]), fabsf(v[4 * tt + 1])),
+                                               fmaxf(fabsf(v[4 * tt + 2]), fabsf(v[4 * tt + 3]))) * args.inv_scale_bwd;
+                                const unsigned mb = __reduce_max_sync(0xffffffffu, __float_as_uint(mv));
+                                if (lane == p) top[nt] = max(top[nt], mb);
+                                continue;
+                            }
+                            const int64_t o = __shfl_sync(0xffffffffu, off[nt], p);
+                            const float f = __shfl_sync(0xffffffffu, sc[nt], p);
+                            const float4 w = make_float4(v[4 * tt] * f, v[4 * tt + 1] * f, v[4 * tt + 2] * f, v[4 * tt + 3] * f);
+                            if (args.mode == MODE_FWD) {
+                                if (row < args.Nx) args.partial[(int64_t)T.split * args.Bmax * args.Nx + o + row] = w;
+                            } else if (row < args.m_rows) {
+                                *reinterpret_cast<float4 *>(args.gpool + o + (int64_t)row * Q) = w;
+                            }
+                        }
+                    }
+                }
+            }
+            // this warp has read the buffer
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_free(u));
         }
+        flush();
     }
+    __syncwarp();
     if (failed) atomicExch(args.err, 1);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -939,21 +1028,28 @@ int msub_choice()
 }
 
 template <int MSUB, int STG, int NT = 1, bool AT = false>
-void launch_gemm(dim3 grid, const CUtensorMap &a, const CUtensorMap &bh, const CUtensorMap &bl,
-                 const tc::GemmArgs &args, cudaStream_t st)
+void launch_gemm(int m_tiles, int n_tiles, int splits, const CUtensorMap &a, const CUtensorMap &bh,
+                 const CUtensorMap &bl, tc::GemmArgs args, cudaStream_t st)
 {
+    args.m_groups = (m_tiles + MSUB - 1) / MSUB;
+    args.n_groups = (n_tiles + NT - 1) / NT;
+    args.splits = splits;
+    // persistent: one CTA per SM (its shared memory allows no second)
+    const int64_t tiles = (int64_t)args.m_groups * args.n_groups * splits;
     tc::k_gemm<MSUB, STG, NT, AT>
-        <<<grid, tc::THREADS, tc::Cfg<MSUB, STG, NT, AT>::SMEM_BYTES, st>>>(a, bh, bl, args);
+        <<<(unsigned)std::min<int64_t>(tiles, 152), tc::THREADS, tc::Cfg<MSUB, STG, NT, AT>::SMEM_BYTES, st>>>(a, bh, bl,
+                                                                                                        args);
 }
 
 // The backward with hi + lo operands (the tensor-core form's gradient, the
 // dual form's max-norm checks) keeps its one-hot A in TMEM: two subtiles,
 // four stages, the MMAs' N fitted to the live columns.  On the 3000 x 94,000
-// workload (ncu, check launches of about 8 slots) it takes 234 us; A in shared
-// memory took 426-439 against 337-375 when both fed the MMAs from one lane
-// and the state tiles from the same ring.  Exact (hi-only) operands -- the
-// dual form's solution digit planes, two N tiles per CTA, 455 us for 21 slots
-// -- stay with A in shared memory: the TMEM form with one subtile and six
+// workload (ncu, check launches of about 8 slots) it takes 204 us (234 with a
+// CTA per tile; 65 against 95 at 616 x 65,563); A in shared memory took
+// 426-439 against 337-375 when both fed the MMAs from one lane and the state
+// tiles from the same ring.  Exact (hi-only) operands -- the dual form's
+// solution digit planes, two N tiles per CTA, 392 us for 21 slots (455 with a
+// CTA per tile; 120 against 164 at 616 x 65,563) -- stay with A in shared memory: the TMEM form with one subtile and six
 // stages took 689 against 607 us there.  SDCA_TC_BWD_SMEM_A=1 keeps A in
 // shared memory everywhere.
 bool bwd_tmem_a()
@@ -968,21 +1064,17 @@ bool bwd_tmem_a()
 void launch_gemm_any(int msub, int m_tiles, int n_tiles, int splits, const CUtensorMap &a, const CUtensorMap &bh,
                      const CUtensorMap &bl, const tc::GemmArgs &args, cudaStream_t st)
 {
-    if (args.mode == tc::MODE_BWD && !args.hi_only && bwd_tmem_a()) {
-        const dim3 grid((unsigned)((m_tiles + 1) / 2), (unsigned)n_tiles, (unsigned)splits);
-        launch_gemm<2, 4, 1, true>(grid, a, bh, bl, args, st);
-        return;
-    }
-    if (args.hi_only && args.mode == tc::MODE_BWD) {
+    if (args.mode == tc::MODE_BWD && !args.hi_only && bwd_tmem_a())
+        launch_gemm<2, 4, 1, true>(m_tiles, n_tiles, splits, a, bh, bl, args, st);
+    else if (args.hi_only && args.mode == tc::MODE_BWD)
         // exact fp16 operands: two N tiles per CTA, two subtiles, three stages
-        const dim3 grid((unsigned)((m_tiles + 1) / 2), (unsigned)((n_tiles + 1) / 2), (unsigned)splits);
-        launch_gemm<2, 3, 2>(grid, a, bh, bl, args, st);
-        return;
-    }
-    const dim3 grid((unsigned)((m_tiles + msub - 1) / msub), (unsigned)n_tiles, (unsigned)splits);
-    if (msub == 4) launch_gemm<4, 2>(grid, a, bh, bl, args, st);
-    else if (msub == 2) launch_gemm<2, 3>(grid, a, bh, bl, args, st);
-    else launch_gemm<1, 4>(grid, a, bh, bl, args, st);
+        launch_gemm<2, 3, 2>(m_tiles, n_tiles, splits, a, bh, bl, args, st);
+    else if (msub == 4)
+        launch_gemm<4, 2>(m_tiles, n_tiles, splits, a, bh, bl, args, st);
+    else if (msub == 2)
+        launch_gemm<2, 3>(m_tiles, n_tiles, splits, a, bh, bl, args, st);
+    else
+        launch_gemm<1, 4>(m_tiles, n_tiles, splits, a, bh, bl, args, st);
 }
 
 } // namespace

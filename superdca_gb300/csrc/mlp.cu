@@ -7,10 +7,10 @@
 // Inference, and the forward pass of training, is one fused tcgen05 kernel
 // (k_mlp_tc): BF16 weights and activations, FP32 accumulators in TMEM, all
 // three layers of a 128-row tile without leaving the SM.  The backward pass
-// is tiled FP32 kernels C = op(A) op(B) on the FP32 master weights from the
-// saved FP32 activations (mixed-precision training); Adam and the loss are
-// elementwise kernels.  sdca_mlp_grad takes the FP32 forward, the exact
-// derivative the CPU oracle checks.  The parameter blob (MLP_* offsets in
+// (k_mlp_bwd) is one fused FP32 kernel on the FP32 master weights from the
+// saved FP32 activations (mixed-precision training), and one more kernel adds
+// its partial sums and takes the Adam step.  sdca_mlp_grad takes the FP32
+// forward (tiled products, k_mm), the exact derivative the CPU oracle checks.  The parameter blob (MLP_* offsets in
 // engine.h) holds the input normalisation, the FP32 weights and the output
 // scale; the BF16 weight image is made from it (k_mlp_pack).
 //
@@ -37,38 +37,24 @@ namespace {
 
 constexpr int TM = 64, TN = 64, TK = 16;
 
-// C[M x N] (=, or += with atomics when split along K) op(A)[M x K] . op(B)[K x N]
-//   op(A)(m,k) = TA ? A[k*lda + m] : A[m*lda + k]
-//   op(B)(k,n) = TB ? B[n*ldb + k] : B[k*ldb + n]
-// epilogue: + bias[n], ReLU, or * [mask(m,n) > 0]
-template <bool TA, bool TB>
+// C[M x N] = A[M x K] . B[N x K]^T + bias, with ReLU when asked
 __global__ void __launch_bounds__(256)
-k_mm(int M, int N, int K, const float *__restrict__ A, int lda, const float *__restrict__ B, int ldb,
-     float *__restrict__ C, int ldc, const float *__restrict__ bias, int relu, const float *__restrict__ mask,
-     int k_per_split)
+k_mm(int M, int N, int K, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ C,
+     const float *__restrict__ bias, int relu)
 {
     __shared__ float sA[TK][TM + 4];
     __shared__ float sB[TK][TN + 4];
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int kbeg = blockIdx.z * k_per_split, kend = min(K, kbeg + k_per_split);
     float acc[4][4] = {};
-    for (int k0 = kbeg; k0 < kend; k0 += TK) {
+    for (int k0 = 0; k0 < K; k0 += TK) {
         for (int e = threadIdx.x; e < TM * TK; e += 256) {
-            int mm, kk;
-            if (TA) { mm = e % TM; kk = e / TM; } else { kk = e % TK; mm = e / TK; }
-            const int m = m0 + mm, k = k0 + kk;
-            float v = 0.f;
-            if (m < M && k < kend) v = TA ? A[(int64_t)k * lda + m] : A[(int64_t)m * lda + k];
-            sA[kk][mm] = v;
+            const int kk = e % TK, mm = e / TK, m = m0 + mm, k = k0 + kk;
+            sA[kk][mm] = m < M && k < K ? A[(int64_t)m * K + k] : 0.f;
         }
         for (int e = threadIdx.x; e < TN * TK; e += 256) {
-            int nn, kk;
-            if (TB) { kk = e % TK; nn = e / TK; } else { nn = e % TN; kk = e / TN; }
-            const int n = n0 + nn, k = k0 + kk;
-            float v = 0.f;
-            if (n < N && k < kend) v = TB ? B[(int64_t)n * ldb + k] : B[(int64_t)k * ldb + n];
-            sB[kk][nn] = v;
+            const int kk = e % TK, nn = e / TK, n = n0 + nn, k = k0 + kk;
+            sB[kk][nn] = n < N && k < K ? B[(int64_t)n * K + k] : 0.f;
         }
         __syncthreads();
 #pragma unroll
@@ -85,7 +71,6 @@ k_mm(int M, int N, int K, const float *__restrict__ A, int lda, const float *__r
         }
         __syncthreads();
     }
-    const bool split = gridDim.z > 1;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int m = m0 + ty + 16 * i;
@@ -94,34 +79,20 @@ k_mm(int M, int N, int K, const float *__restrict__ A, int lda, const float *__r
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx + 16 * j;
             if (n >= N) continue;
-            float v = acc[i][j];
-            float *c = C + (int64_t)m * ldc + n;
-            if (split) {
-                atomicAdd(c, v);
-                continue;
-            }
-            if (bias) v += bias[n];
-            if (relu) v = fmaxf(v, 0.f);
-            if (mask && !(mask[(int64_t)m * ldc + n] > 0.f)) v = 0.f;
-            *c = v;
+            float v = acc[i][j] + bias[n];
+            C[(int64_t)m * N + n] = relu ? fmaxf(v, 0.f) : v;
         }
     }
 }
 
-template <bool TA, bool TB>
-void mm(cudaStream_t st, int M, int N, int K, const float *A, int lda, const float *B, int ldb, float *C, int ldc,
-        const float *bias, int relu, const float *mask, int splits = 1)
+void mm(cudaStream_t st, int M, int N, int K, const float *A, const float *B, float *C, const float *bias, int relu)
 {
-    const int kps = ((K + splits - 1) / splits + TK - 1) / TK * TK;
-    splits = (K + kps - 1) / kps;
-    // rows in pieces that keep grid.y within its limit (row-major A only)
-    const int rows = TA ? M : std::min(M, 65535 * TM);
+    // rows in pieces that keep grid.y within its limit
+    const int rows = std::min(M, 65535 * TM);
     for (int m0 = 0; m0 < M; m0 += rows) {
         const int mr = std::min(rows, M - m0);
-        dim3 grid((N + TN - 1) / TN, (mr + TM - 1) / TM, splits);
-        k_mm<TA, TB><<<grid, 256, 0, st>>>(mr, N, K, A + (TA ? 0 : (int64_t)m0 * lda), lda, B, ldb,
-                                           C + (int64_t)m0 * ldc, ldc, bias, relu,
-                                           mask ? mask + (int64_t)m0 * ldc : nullptr, kps);
+        dim3 grid((N + TN - 1) / TN, (mr + TM - 1) / TM);
+        k_mm<<<grid, 256, 0, st>>>(mr, N, K, A + (int64_t)m0 * K, B, C + (int64_t)m0 * N, bias, relu);
     }
 }
 
@@ -135,61 +106,253 @@ __global__ void k_normalise(int64_t M, const float *__restrict__ X, const float 
     Xn[t] = (X[t] - p[MLP_IN_MEAN + c]) * p[MLP_IN_SCALE + c];
 }
 
-// rows of src picked by idx -> dst
-__global__ void k_gather_rows(int64_t M, int width, const int32_t *__restrict__ idx, const float *__restrict__ src,
-                              float *__restrict__ dst)
+// ---- the fused backward (FP32)
+//
+// From the outputs, targets and saved activations of M rows to the gradient
+// of every weight: one CTA takes tiles of up to 64 rows, holds W2 and W3 and
+// the tile's h1, h2, inputs and output gradient in shared memory, and keeps
+// its sums of the three weight gradients in registers (92 per thread) over
+// all its tiles.  h2 becomes d2 = (dout W3) masked, and h1 becomes d1 = (d2
+// W2) masked, in place.  Each CTA writes its sums once; k_mlp_reduce adds the
+// CTAs' up.  FP32 multiply-adds bound it (0.7 GFLOP at 8192 rows, some 10 us
+// on all SMs).  As separate tiled products C = op(A) op(B) split along the
+// rows, the three weight gradients ran on 4 to 16 CTAs and took 617 us each at 8192
+// rows (1.9 ms of a 2 ms step); this kernel takes 32 us, the reduction and
+// Adam 8, the forward 19.
+constexpr int BW_THREADS = 256, BW_ROWS = 64;
+constexpr int MLP_NPAR = MLP_TRAIN_END - MLP_W1;                 // trained parameters, W1 .. b3
+constexpr int BW_W2 = 0, BW_W3 = BW_W2 + MLP_H * MLP_H, BW_H1 = BW_W3 + MLP_OUT * MLP_H, BW_H2 = BW_H1 + BW_ROWS * MLP_H,
+              BW_X = BW_H2 + BW_ROWS * MLP_H, BW_D = BW_X + BW_ROWS * MLP_IN, BW_FLOATS = BW_D + BW_ROWS * MLP_OUT;
+constexpr int BW_SMEM = BW_FLOATS * 4;
+static_assert(MLP_H == 128 && MLP_OUT == 16 && MLP_IN == 40, "thread tiles of k_mlp_bwd");
+
+__device__ __forceinline__ void fma4(float (&c)[4], float a, float4 b)
 {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= M * width) return;
-    const int64_t m = t / width;
-    const int c = (int)(t % width);
-    dst[t] = src[(int64_t)idx[m] * width + c];
+    c[0] = fmaf(a, b.x, c[0]);
+    c[1] = fmaf(a, b.y, c[1]);
+    c[2] = fmaf(a, b.z, c[2]);
+    c[3] = fmaf(a, b.w, c[3]);
 }
 
-// mean squared error over M x MLP_OUT; dOut = 2 (out - t) / M
-__global__ void k_mse(int64_t M, const float *__restrict__ out, const float *__restrict__ t, float *__restrict__ dout,
-                      double *__restrict__ loss)
+// idx (may be null): row m of the batch is row idx[m] of X and T.  tile_rows:
+// rows per tile (a multiple of 4, at most BW_ROWS).  part[blockIdx.x]: this
+// CTA's sums; loss += the mean squared error.
+__global__ void __launch_bounds__(BW_THREADS, 1)
+k_mlp_bwd(int64_t M, int tile_rows, const int32_t *__restrict__ idx, const float *__restrict__ X,
+          const float *__restrict__ T, const float *__restrict__ p, const float *__restrict__ out,
+          const float *__restrict__ h1, const float *__restrict__ h2, float *__restrict__ part,
+          double *__restrict__ loss)
 {
-    double s = 0.0;
+    extern __shared__ __align__(16) float sm[];
+    float4 *const s4 = reinterpret_cast<float4 *>(sm);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, tx = t & 15, ty = t >> 4;
+    static_assert(MLP_W2 % 4 == 0 && MLP_W3 % 4 == 0 && MLP_IN_MEAN % 4 == 0 && MLP_IN_SCALE % 4 == 0, "float4 loads of the blob");
+#pragma unroll 8
+    for (int e = t; e < MLP_H * MLP_H / 4; e += BW_THREADS) s4[BW_W2 / 4 + e] = reinterpret_cast<const float4 *>(p + MLP_W2)[e];
+#pragma unroll
+    for (int e = t; e < MLP_OUT * MLP_H / 4; e += BW_THREADS) s4[BW_W3 / 4 + e] = reinterpret_cast<const float4 *>(p + MLP_W3)[e];
+    float g2[8][2][4] = {};   // W2: rows 4 ty + (0..3) and 64 + .., columns 4 tx + (0..3) and 64 + ..
+    float g1[4][5] = {};      // W1: rows 4 (t / 8) + .., columns 5 (t % 8) + ..
+    float g3[2][4] = {};      // W3: rows 2 warp + .., columns 4 lane + ..
+    float gb = 0.f, gb3 = 0.f;   // b2[t] (t < 128) or b1[t - 128]; b3[t] (t < 16)
+    double ls = 0.0;
     const float inv = 2.f / (float)M;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < M * MLP_OUT;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const float r = out[e] - t[e];
-        dout[e] = inv * r;
-        s += (double)r * r;
+    const int64_t tiles = (M + tile_rows - 1) / tile_rows;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t m0 = tile * tile_rows;
+        const int R = (int)min((int64_t)tile_rows, M - m0);
+        __syncthreads();   // (the tile before is used up)
+        // (16-byte loads: a row of X is ten of them, of T and the outputs four)
+        for (int e = t; e < R * (MLP_OUT / 4); e += BW_THREADS) {
+            const int m = e >> 2, o = e & 3;
+            const int64_t row = idx ? (int64_t)idx[m0 + m] : m0 + m;
+            const float4 y = reinterpret_cast<const float4 *>(out)[(m0 + m) * (MLP_OUT / 4) + o];
+            const float4 w = reinterpret_cast<const float4 *>(T)[row * (MLP_OUT / 4) + o];
+            const float4 r = make_float4(y.x - w.x, y.y - w.y, y.z - w.z, y.w - w.w);
+            s4[BW_D / 4 + e] = make_float4(inv * r.x, inv * r.y, inv * r.z, inv * r.w);
+            ls += (double)r.x * r.x + (double)r.y * r.y + (double)r.z * r.z + (double)r.w * r.w;
+        }
+#pragma unroll 3
+        for (int e = t; e < R * (MLP_IN / 4); e += BW_THREADS) {
+            const int m = e / (MLP_IN / 4), c = e % (MLP_IN / 4);
+            const int64_t row = idx ? (int64_t)idx[m0 + m] : m0 + m;
+            const float4 x = reinterpret_cast<const float4 *>(X)[row * (MLP_IN / 4) + c];
+            const float4 mu = reinterpret_cast<const float4 *>(p + MLP_IN_MEAN)[c],
+                         sc = reinterpret_cast<const float4 *>(p + MLP_IN_SCALE)[c];
+            s4[BW_X / 4 + e] = make_float4((x.x - mu.x) * sc.x, (x.y - mu.y) * sc.y, (x.z - mu.z) * sc.z, (x.w - mu.w) * sc.w);
+        }
+#pragma unroll 4
+        for (int e = t; e < R * (MLP_H / 4); e += BW_THREADS) {
+            s4[BW_H1 / 4 + e] = reinterpret_cast<const float4 *>(h1 + m0 * MLP_H)[e];
+            s4[BW_H2 / 4 + e] = reinterpret_cast<const float4 *>(h2 + m0 * MLP_H)[e];
+        }
+        __syncthreads();
+        // W3 gradient: dout^T h2
+        for (int m = 0; m < R; ++m) {
+            const float4 h = s4[BW_H2 / 4 + m * (MLP_H / 4) + lane];
+            fma4(g3[0], sm[BW_D + m * MLP_OUT + 2 * warp], h);
+            fma4(g3[1], sm[BW_D + m * MLP_OUT + 2 * warp + 1], h);
+        }
+        if (t < MLP_OUT)
+            for (int m = 0; m < R; ++m) gb3 += sm[BW_D + m * MLP_OUT + t];
+        __syncthreads();
+        // d2 = (dout W3) where h2 > 0, in place of h2: 8 rows per warp at a time
+        for (int r0 = 8 * warp; r0 < R; r0 += 64) {
+            float d[8][4] = {};
+#pragma unroll 4
+            for (int o = 0; o < MLP_OUT; ++o) {
+                const float4 w = s4[BW_W3 / 4 + o * (MLP_H / 4) + lane];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) fma4(d[k], sm[BW_D + (r0 + k) * MLP_OUT + o], w);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                if (r0 + k >= R) break;
+                float4 &h = s4[BW_H2 / 4 + (r0 + k) * (MLP_H / 4) + lane];
+                h = make_float4(h.x > 0.f ? d[k][0] : 0.f, h.y > 0.f ? d[k][1] : 0.f, h.z > 0.f ? d[k][2] : 0.f,
+                                h.w > 0.f ? d[k][3] : 0.f);
+            }
+        }
+        __syncthreads();
+        // W2 gradient: d2^T h1
+#pragma unroll 2
+        for (int m = 0; m < R; ++m) {
+            const float4 a0 = s4[BW_H2 / 4 + m * 32 + ty], a1 = s4[BW_H2 / 4 + m * 32 + 16 + ty];
+            const float4 b0 = s4[BW_H1 / 4 + m * 32 + tx], b1 = s4[BW_H1 / 4 + m * 32 + 16 + tx];
+            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                fma4(g2[i][0], a[i], b0);
+                fma4(g2[i][1], a[i], b1);
+            }
+        }
+        if (t < MLP_H)
+            for (int m = 0; m < R; ++m) gb += sm[BW_H2 + m * MLP_H + t];
+        __syncthreads();
+        // d1 = (d2 W2) where h1 > 0, in place of h1: rows 4 ty + .., columns as above
+        if (4 * ty < R) {
+            float d[4][2][4] = {};
+#pragma unroll 2
+            for (int j = 0; j < MLP_H; j += 4) {
+                float4 a[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = s4[BW_H2 / 4 + (4 * ty + i) * 32 + j / 4];
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) {
+                    const float4 b0 = s4[BW_W2 / 4 + (j + jj) * 32 + tx], b1 = s4[BW_W2 / 4 + (j + jj) * 32 + 16 + tx];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float v = jj == 0 ? a[i].x : jj == 1 ? a[i].y : jj == 2 ? a[i].z : a[i].w;
+                        fma4(d[i][0], v, b0);
+                        fma4(d[i][1], v, b1);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    if (4 * ty + i >= R) break;
+                    float4 &h = s4[BW_H1 / 4 + (4 * ty + i) * 32 + 16 * hh + tx];
+                    h = make_float4(h.x > 0.f ? d[i][hh][0] : 0.f, h.y > 0.f ? d[i][hh][1] : 0.f,
+                                    h.z > 0.f ? d[i][hh][2] : 0.f, h.w > 0.f ? d[i][hh][3] : 0.f);
+                }
+        }
+        __syncthreads();
+        // W1 gradient: d1^T x
+        {
+            const int k4 = t >> 3, c0 = 5 * (t & 7);
+#pragma unroll 2
+            for (int m = 0; m < R; ++m) {
+                const float4 a = s4[BW_H1 / 4 + m * 32 + k4];
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    const float x = sm[BW_X + m * MLP_IN + c0 + c];
+                    g1[0][c] = fmaf(a.x, x, g1[0][c]);
+                    g1[1][c] = fmaf(a.y, x, g1[1][c]);
+                    g1[2][c] = fmaf(a.z, x, g1[2][c]);
+                    g1[3][c] = fmaf(a.w, x, g1[3][c]);
+                }
+            }
+        }
+        if (t >= MLP_H)
+            for (int m = 0; m < R; ++m) gb += sm[BW_H1 + m * MLP_H + t - MLP_H];
     }
-    s = warp_sum(s);
-    __shared__ double red[32];
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    float *o = part + (int64_t)blockIdx.x * MLP_NPAR - MLP_W1;   // (blob offsets)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int r = 4 * ty + (i & 3) + 64 * (i >> 2), c = 4 * tx + 64 * hh;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) o[MLP_W2 + r * MLP_H + c + k] = g2[i][hh][k];
+        }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 5; ++c) o[MLP_W1 + (4 * (t >> 3) + i) * MLP_IN + 5 * (t & 7) + c] = g1[i][c];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o[MLP_W3 + (2 * warp + i) * MLP_H + 4 * lane + k] = g3[i][k];
+    o[t < MLP_H ? MLP_B2 + t : MLP_B1 + t - MLP_H] = gb;
+    if (t < MLP_OUT) o[MLP_B3 + t] = gb3;
+    ls = warp_sum(ls);
+    __shared__ double red[BW_THREADS / 32];
+    if (lane == 0) red[warp] = ls;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        double v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        v = warp_sum(v);
-        if (threadIdx.x == 0) atomicAdd(loss, v / (double)M);
+    if (t == 0) {
+        double v = 0.0;
+        for (int k = 0; k < BW_THREADS / 32; ++k) v += red[k];
+        atomicAdd(loss, v / (double)M);
     }
 }
 
-// column sums of dC (M x N) into g[n]
-__global__ void k_colsum(int64_t M, int N, const float *__restrict__ dC, float *__restrict__ g)
+// The parameter's place in the BF16 weight image, -1 for a bias
+__device__ __forceinline__ int wb_place(int e)
 {
-    const int n = threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int64_t m = blockIdx.x; m < M; m += gridDim.x) s += dC[m * N + n];
-    atomicAdd(g + n, s);
+    if (e < MLP_B1) return (e - MLP_W1) / MLP_IN * 64 + (e - MLP_W1) % MLP_IN;
+    if (e >= MLP_W2 && e < MLP_B2) return MLP_H * 64 + e - MLP_W2;
+    if (e >= MLP_W3 && e < MLP_B3) return MLP_H * 64 + MLP_H * MLP_H + e - MLP_W3;
+    return -1;
 }
 
-__global__ void k_adam(int n, float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m1,
-                       float *__restrict__ m2, float lr, float b1, float b2, float eps, float c1, float c2)
+// The gradient of a parameter is the sum of the CTAs' partial sums (RD_SEG
+// threads share them out); written to g, or (g null) an Adam step on p and
+// the parameter's entry of the BF16 image.
+constexpr int RD_PAR = 32, RD_SEG = 8;
+
+__global__ void __launch_bounds__(RD_PAR * RD_SEG)
+k_mlp_reduce(int blocks, const float *__restrict__ part, float *__restrict__ g, float *__restrict__ p,
+             float *__restrict__ m1, float *__restrict__ m2, __nv_bfloat16 *__restrict__ wb, float lr, float b1,
+             float b2, float eps, float c1, float c2)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float a = b1 * m1[i] + (1.f - b1) * gi;
-    const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    p[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+    __shared__ float red[RD_SEG][RD_PAR];
+    const int k = threadIdx.x % RD_PAR, seg = threadIdx.x / RD_PAR, i = blockIdx.x * RD_PAR + k;
+    float s = 0.f;
+    if (i < MLP_NPAR) {
+#pragma unroll 8
+        for (int b = seg; b < blocks; b += RD_SEG) s += part[(int64_t)b * MLP_NPAR + i];
+    }
+    red[seg][k] = s;
+    __syncthreads();
+    if (seg != 0 || i >= MLP_NPAR) return;
+    float gi = 0.f;
+#pragma unroll
+    for (int q = 0; q < RD_SEG; ++q) gi += red[q][k];
+    const int e = MLP_W1 + i;
+    if (g) {
+        g[e] = gi;
+        return;
+    }
+    const float a = b1 * m1[e] + (1.f - b1) * gi;
+    const float b = b2 * m2[e] + (1.f - b2) * gi * gi;
+    m1[e] = a;
+    m2[e] = b;
+    const float v = p[e] - lr * (a / c1) / (sqrtf(b / c2) + eps);
+    p[e] = v;
+    const int place = wb_place(e);
+    if (place >= 0) wb[place] = __float2bfloat16_rn(v);
 }
 
 // ---- the fused tensor-core forward (BF16 weights, FP32 accumulators)
@@ -202,7 +365,8 @@ __global__ void k_adam(int n, float *__restrict__ p, const float *__restrict__ g
 // tcgen05.mma (M128, K16 steps) into TMEM and commits to an mbarrier; every
 // thread reads its row's accumulators back (tcgen05.ld, TMEM lane = row),
 // adds the bias, applies ReLU and writes the next layer's BF16 A tile.
-// Layer 3 (N = 16) writes the outputs.  h1, h2 (optional) receive the FP32
+// Layer 3 (N = 16) writes the outputs.  Row m of the input is row idx[m] of X
+// when idx is given.  h1, h2 (optional) receive the FP32
 // activations for the backward pass.
 constexpr int MT_THREADS = 128;
 constexpr int MT_K1 = 64;                                       // layer-1 K, padded
@@ -270,8 +434,8 @@ __device__ __forceinline__ void mt_hidden(const float (&v)[32], const float *__r
 }
 
 __global__ void __launch_bounds__(MT_THREADS, 2)
-k_mlp_tc(int64_t M, const float *__restrict__ X, const float *__restrict__ p, const __nv_bfloat16 *__restrict__ wb,
-         float *__restrict__ out, float *__restrict__ h1, float *__restrict__ h2, int *__restrict__ err)
+k_mlp_tc(int64_t M, const int32_t *__restrict__ idx, const float *__restrict__ X, const float *__restrict__ p,
+         const __nv_bfloat16 *__restrict__ wb, float *__restrict__ out, float *__restrict__ h1, float *__restrict__ h2, int *__restrict__ err)
 {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t s0 = tc::smem_u32(smem_raw);
@@ -332,9 +496,10 @@ k_mlp_tc(int64_t M, const float *__restrict__ X, const float *__restrict__ p, co
 #pragma unroll
             for (int k = 0; k < MT_K1; ++k) x[k] = 0.f;
             if (live) {
+                const float *xr = X + (idx ? (int64_t)idx[row] : row) * MLP_IN;
 #pragma unroll
                 for (int k = 0; k < MLP_IN; k += 4) {
-                    const float4 v = *reinterpret_cast<const float4 *>(X + row * MLP_IN + k);
+                    const float4 v = *reinterpret_cast<const float4 *>(xr + k);
                     x[k] = (v.x - p[MLP_IN_MEAN + k]) * p[MLP_IN_SCALE + k];
                     x[k + 1] = (v.y - p[MLP_IN_MEAN + k + 1]) * p[MLP_IN_SCALE + k + 1];
                     x[k + 2] = (v.z - p[MLP_IN_MEAN + k + 2]) * p[MLP_IN_SCALE + k + 2];
@@ -427,32 +592,34 @@ struct Scratch {
 // forward over M normalised rows; activations kept for the backward
 void forward(cudaStream_t st, const float *p, const float *Xn, int64_t M, const Scratch &s)
 {
-    mm<false, true>(st, (int)M, MLP_H, MLP_IN, Xn, MLP_IN, p + MLP_W1, MLP_IN, s.h1, MLP_H, p + MLP_B1, 1, nullptr);
-    mm<false, true>(st, (int)M, MLP_H, MLP_H, s.h1, MLP_H, p + MLP_W2, MLP_H, s.h2, MLP_H, p + MLP_B2, 1, nullptr);
-    mm<false, true>(st, (int)M, MLP_OUT, MLP_H, s.h2, MLP_H, p + MLP_W3, MLP_H, s.out, MLP_OUT, p + MLP_B3, 0,
-                    nullptr);
+    mm(st, (int)M, MLP_H, MLP_IN, Xn, p + MLP_W1, s.h1, p + MLP_B1, 1);
+    mm(st, (int)M, MLP_H, MLP_H, s.h1, p + MLP_W2, s.h2, p + MLP_B2, 1);
+    mm(st, (int)M, MLP_OUT, MLP_H, s.h2, p + MLP_W3, s.out, p + MLP_B3, 0);
 }
 
-// gradient of the loss whose output gradient is dout (M x MLP_OUT), into g
-// (blob layout, zeroed by the caller); d1/d2 are M x MLP_H scratch
-void backward(cudaStream_t st, const float *p, const float *Xn, int64_t M, const Scratch &s, const float *dout,
-              float *d1, float *d2, float *g)
+// CTAs of the backward over M rows and their tiles' rows: every SM one tile
+// of up to 64 rows, then further tiles
+int bwd_tile_rows(int64_t M) { return (int)std::min<int64_t>(BW_ROWS, ((M + 151) / 152 + 7) / 8 * 8); }
+int bwd_blocks(int64_t M)
 {
-    const int splits = (int)std::min<int64_t>(64, std::max<int64_t>(1, M / 2048));
-    const int cs_blocks = (int)std::min<int64_t>(256, std::max<int64_t>(1, M / 64));
-    // layer 3
-    mm<true, false>(st, MLP_OUT, MLP_H, (int)M, dout, MLP_OUT, s.h2, MLP_H, g + MLP_W3, MLP_H, nullptr, 0, nullptr,
-                    splits);
-    k_colsum<<<cs_blocks, 128, 0, st>>>(M, MLP_OUT, dout, g + MLP_B3);
-    mm<false, false>(st, (int)M, MLP_H, MLP_OUT, dout, MLP_OUT, p + MLP_W3, MLP_H, d2, MLP_H, nullptr, 0, s.h2);
-    // layer 2
-    mm<true, false>(st, MLP_H, MLP_H, (int)M, d2, MLP_H, s.h1, MLP_H, g + MLP_W2, MLP_H, nullptr, 0, nullptr, splits);
-    k_colsum<<<cs_blocks, 128, 0, st>>>(M, MLP_H, d2, g + MLP_B2);
-    mm<false, false>(st, (int)M, MLP_H, MLP_H, d2, MLP_H, p + MLP_W2, MLP_H, d1, MLP_H, nullptr, 0, s.h1);
-    // layer 1
-    mm<true, false>(st, MLP_H, MLP_IN, (int)M, d1, MLP_H, Xn, MLP_IN, g + MLP_W1, MLP_IN, nullptr, 0, nullptr,
-                    splits);
-    k_colsum<<<cs_blocks, 128, 0, st>>>(M, MLP_H, d1, g + MLP_B1);
+    const int64_t r = bwd_tile_rows(M);
+    return (int)std::min<int64_t>(152, (M + r - 1) / r);
+}
+
+cudaError_t bwd_configure()
+{
+    static std::once_flag once;
+    static cudaError_t e = cudaSuccess;
+    std::call_once(once, [] { e = cudaFuncSetAttribute(k_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, BW_SMEM); });
+    return e;
+}
+
+// the gradient's partial sums (bwd_blocks(M) x MLP_NPAR) and the loss
+void backward(cudaStream_t st, const float *p, const int32_t *idx, const float *X, const float *T, int64_t M,
+              const Scratch &s, float *part, double *loss)
+{
+    if (bwd_configure() != cudaSuccess) return;   // the caller's launch check reports it
+    k_mlp_bwd<<<bwd_blocks(M), BW_THREADS, BW_SMEM, st>>>(M, bwd_tile_rows(M), idx, X, T, p, s.out, s.h1, s.h2, part, loss);
 }
 
 thread_local std::string t_err;
@@ -496,8 +663,8 @@ cudaError_t mt_configure()
 }
 
 // the fused forward over M rows: outputs, and the FP32 activations when h1, h2 are given
-void mt_forward(const float *p_dev, const void *wb, const float *X, int64_t M, float *out, float *h1, float *h2,
-                int *err, cudaStream_t st)
+void mt_forward(const float *p_dev, const void *wb, const int32_t *idx, const float *X, int64_t M, float *out,
+                float *h1, float *h2, int *err, cudaStream_t st)
 {
     if (M <= 0) return;
     if (mt_configure() != cudaSuccess) return;   // the caller's launch check reports it
@@ -506,7 +673,7 @@ void mt_forward(const float *p_dev, const void *wb, const float *X, int64_t M, f
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 152;
     const int64_t tiles = (M + 127) / 128;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * (int64_t)sms);
-    k_mlp_tc<<<grid, MT_THREADS, MT_SMEM, st>>>(M, X, p_dev, static_cast<const __nv_bfloat16 *>(wb), out, h1, h2,
+    k_mlp_tc<<<grid, MT_THREADS, MT_SMEM, st>>>(M, idx, X, p_dev, static_cast<const __nv_bfloat16 *>(wb), out, h1, h2,
                                                   err);
 }
 
@@ -514,7 +681,7 @@ void mt_forward(const float *p_dev, const void *wb, const float *X, int64_t M, f
 
 void mlp_infer(const float *p_dev, const void *wb, const float *X, int64_t M, float *out, int *err, cudaStream_t st)
 {
-    mt_forward(p_dev, wb, X, M, out, nullptr, nullptr, err, st);
+    mt_forward(p_dev, wb, nullptr, X, M, out, nullptr, nullptr, err, st);
 }
 
 } // namespace sdca
@@ -532,8 +699,8 @@ int sdca_mlp_grad(const float *params, const float *X, const float *T, int64_t M
     Dev d;
     float *p = d.alloc<float>(MLP_BLOB_SIZE), *x = d.alloc<float>(M * MLP_IN), *xn = d.alloc<float>(M * MLP_IN);
     float *t = d.alloc<float>(M * MLP_OUT), *h1 = d.alloc<float>(M * MLP_H), *h2 = d.alloc<float>(M * MLP_H);
-    float *out = d.alloc<float>(M * MLP_OUT), *dout = d.alloc<float>(M * MLP_OUT);
-    float *d1 = d.alloc<float>(M * MLP_H), *d2 = d.alloc<float>(M * MLP_H), *g = d.alloc<float>(MLP_BLOB_SIZE);
+    float *out = d.alloc<float>(M * MLP_OUT), *g = d.alloc<float>(MLP_BLOB_SIZE);
+    float *part = d.alloc<float>((size_t)bwd_blocks(M) * MLP_NPAR);
     double *l = d.alloc<double>(1);
     if (!d.ok) return mfail("device allocation failed"), SDCA_E_NOMEM;
     MK(cudaMemcpy(p, params, sizeof(float) * MLP_BLOB_SIZE, cudaMemcpyHostToDevice));
@@ -544,8 +711,9 @@ int sdca_mlp_grad(const float *params, const float *X, const float *T, int64_t M
     k_normalise<<<(unsigned)((M * MLP_IN + 255) / 256), 256, 0, st>>>(M, x, p, xn);
     const Scratch s{h1, h2, out};
     forward(st, p, xn, M, s);
-    k_mse<<<(unsigned)std::min<int64_t>(1024, (M * MLP_OUT + 255) / 256), 256, 0, st>>>(M, out, t, dout, l);
-    backward(st, p, xn, M, s, dout, d1, d2, g);
+    backward(st, p, nullptr, x, t, M, s, part, l);
+    k_mlp_reduce<<<(MLP_NPAR + RD_PAR - 1) / RD_PAR, RD_PAR * RD_SEG, 0, st>>>(
+        bwd_blocks(M), part, g, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f);
     MK(cudaGetLastError());
     MK(cudaMemcpy(grad, g, sizeof(float) * MLP_BLOB_SIZE, cudaMemcpyDeviceToHost));
     MK(cudaMemcpy(loss, l, sizeof(double), cudaMemcpyDeviceToHost));
@@ -580,15 +748,12 @@ int sdca_mlp_train(float *params, const float *X, const float *T, int64_t M, int
     cudaStream_t st = 0;
     const int64_t Bm = std::min<int64_t>(batch, M);
     Dev d;
-    float *p = d.alloc<float>(MLP_BLOB_SIZE), *x = d.alloc<float>(M * MLP_IN), *xn = d.alloc<float>(M * MLP_IN);
-    float *t = d.alloc<float>(M * MLP_OUT);
-    float *bx = d.alloc<float>(Bm * MLP_IN), *bt = d.alloc<float>(Bm * MLP_OUT);
+    float *p = d.alloc<float>(MLP_BLOB_SIZE), *x = d.alloc<float>(M * MLP_IN), *t = d.alloc<float>(M * MLP_OUT);
     float *h1 = d.alloc<float>(Bm * MLP_H), *h2 = d.alloc<float>(Bm * MLP_H), *out = d.alloc<float>(Bm * MLP_OUT);
-    float *dout = d.alloc<float>(Bm * MLP_OUT), *d1 = d.alloc<float>(Bm * MLP_H), *d2 = d.alloc<float>(Bm * MLP_H);
-    float *g = d.alloc<float>(MLP_BLOB_SIZE), *m1 = d.alloc<float>(MLP_BLOB_SIZE), *m2 = d.alloc<float>(MLP_BLOB_SIZE);
+    float *part = d.alloc<float>((size_t)bwd_blocks(Bm) * MLP_NPAR);
+    float *m1 = d.alloc<float>(MLP_BLOB_SIZE), *m2 = d.alloc<float>(MLP_BLOB_SIZE);
     int32_t *perm_d = d.alloc<int32_t>(M);
     double *l = d.alloc<double>(1);
-    float *braw = d.alloc<float>(Bm * MLP_IN);
     __nv_bfloat16 *wb = d.alloc<__nv_bfloat16>(MT_WB_ELEMS);
     int *err = d.alloc<int>(1);
     if (!d.ok) return mfail("device allocation failed"), SDCA_E_NOMEM;
@@ -598,7 +763,7 @@ int sdca_mlp_train(float *params, const float *X, const float *T, int64_t M, int
     MK(cudaMemcpy(t, T, sizeof(float) * M * MLP_OUT, cudaMemcpyHostToDevice));
     MK(cudaMemset(m1, 0, sizeof(float) * MLP_BLOB_SIZE));
     MK(cudaMemset(m2, 0, sizeof(float) * MLP_BLOB_SIZE));
-    k_normalise<<<(unsigned)((M * MLP_IN + 255) / 256), 256, 0, st>>>(M, x, p, xn);
+    mlp_pack(p, wb, st);   // (the weights' entries follow every step; the padding stays zero)
     std::mt19937_64 rng(seed);
     std::vector<int32_t> perm((size_t)M);
     const float b1 = 0.9f, b2 = 0.999f;
@@ -612,20 +777,13 @@ int sdca_mlp_train(float *params, const float *X, const float *T, int64_t M, int
         int64_t nb = 0;
         for (int64_t b0 = 0; b0 + Bm <= M; b0 += Bm, ++nb) {
             // forward on the tensor cores (BF16 image of the current weights),
-            // backward in FP32 from its saved activations
-            k_gather_rows<<<(unsigned)((Bm * MLP_IN + 255) / 256), 256, 0, st>>>(Bm, MLP_IN, perm_d + b0, x, braw);
-            k_gather_rows<<<(unsigned)((Bm * MLP_IN + 255) / 256), 256, 0, st>>>(Bm, MLP_IN, perm_d + b0, xn, bx);
-            k_gather_rows<<<(unsigned)((Bm * MLP_OUT + 255) / 256), 256, 0, st>>>(Bm, MLP_OUT, perm_d + b0, t, bt);
-            mlp_pack(p, wb, st);
-            mt_forward(p, wb, braw, Bm, out, h1, h2, err, st);
-            k_mse<<<(unsigned)std::min<int64_t>(1024, (Bm * MLP_OUT + 255) / 256), 256, 0, st>>>(Bm, out, bt, dout, l);
-            MK(cudaMemsetAsync(g, 0, sizeof(float) * MLP_BLOB_SIZE, st));
-            backward(st, p, bx, Bm, s, dout, d1, d2, g);
+            // backward in FP32 from its saved activations, Adam
+            mt_forward(p, wb, perm_d + b0, x, Bm, out, h1, h2, err, st);
+            backward(st, p, perm_d + b0, x, t, Bm, s, part, l);
             c1 *= b1;
             c2 *= b2;
-            k_adam<<<(MLP_TRAIN_END - MLP_W1 + 255) / 256, 256, 0, st>>>(MLP_TRAIN_END - MLP_W1, p + MLP_W1,
-                                                                       g + MLP_W1, m1 + MLP_W1, m2 + MLP_W1, lr,
-                                                                       b1, b2, 1e-8f, 1.f - c1, 1.f - c2);
+            k_mlp_reduce<<<(MLP_NPAR + RD_PAR - 1) / RD_PAR, RD_PAR * RD_SEG, 0, st>>>(
+                bwd_blocks(Bm), part, nullptr, p, m1, m2, wb, lr, b1, b2, 1e-8f, 1.f - c1, 1.f - c2);
         }
         MK(cudaGetLastError());
         int e = 0;

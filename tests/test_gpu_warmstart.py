@@ -39,6 +39,24 @@ def test_mlp_gradient_matches_cpu_oracle(engine_lib):
         assert np.abs(out - ref).max() <= 3e-2 * scale
 
 
+@pytest.mark.parametrize("M", [1, 63, 64, 65, 1217, 20001])
+def test_mlp_fused_backward_row_tiles(engine_lib, M):
+    """The fused backward at the edges of its row tiles (one row; 64-row
+    tiles; more tiles than SMs) against the FP64 restatement."""
+    from oracle import mlp_oracle as MO
+    from superdca_gb300 import warmstart
+    rng = np.random.default_rng(M)
+    X = rng.normal(size=(M, 40)).astype(np.float32)
+    T = rng.normal(size=(M, 16)).astype(np.float32)
+    blob = warmstart.new_blob(rng.normal(size=(64, 40)).astype(np.float32),
+                              rng.normal(size=(64, 16)).astype(np.float32), seed=M)
+    loss, g = warmstart.grad(blob, X, T)
+    loss64, g64 = MO.loss_and_grad(blob, X, T)
+    assert abs(loss - loss64) <= 1e-5 * abs(loss64)
+    # FP32 kernels against FP64: 1e-4 of the largest gradient entry
+    assert np.abs(g - g64).max() <= 1e-4 * np.abs(g64).max()
+
+
 @pytest.mark.parametrize("M", [1, 127, 128, 129, 40000, 100003])
 def test_mlp_tensor_core_forward_ragged_rows(engine_lib, M):
     """Row counts around the 128-row tile and beyond one tile per CTA."""

@@ -137,6 +137,7 @@ struct sdca_handle {
     std::vector<void *> allocs;
     uint8_t *X = nullptr, *XT = nullptr, *rstate = nullptr;
     double *w = nullptr;
+    uint64_t *packed = nullptr;    // packed states and neighbour sums of the pair kernels, kept once allocated
     float *wf = nullptr;           // the weights in FP32 (kernels that need no more)
     float *wa = nullptr, *d = nullptr, *gpool = nullptr, *u = nullptr, *R = nullptr;
     float *partial = nullptr, *rows = nullptr;
@@ -340,6 +341,21 @@ template <typename T> int halloc(sdca_handle *h, T **p, size_t count)
     return SDCA_OK;
 }
 
+// The workspace of the pair kernels (packed states, then 2 N doubles), kept
+// for the handle's life: an allocation and a release cost each call up to 0.1
+// ms, depending on what else the process had allocated.
+int pair_workspace(sdca_handle *h, uint64_t **packed, double **sums)
+{
+    const size_t words = (size_t)h->P.N * packed_words(h->P.L);
+    if (!h->packed) {
+        const int rc = dalloc(h, &h->packed, words + 2 * (size_t)h->P.N);
+        if (rc) return rc;
+    }
+    *packed = h->packed;
+    *sums = reinterpret_cast<double *>(h->packed + words);
+    return SDCA_OK;
+}
+
 void free_all(sdca_handle *h)
 {
     for (void *p : h->allocs) cudaFree(p);
@@ -357,30 +373,62 @@ void free_all(sdca_handle *h)
     h->sd_h = nullptr; h->list_h = nullptr; h->acc_h = nullptr; h->dots_h = nullptr;
     h->rows_h = nullptr; h->flag_h = nullptr;
     h->X = h->XT = h->rstate = nullptr;
+    h->packed = nullptr;
     h->has_alignment = false;
 }
 
-// X [N][Lx] -> XT [L][Nx]; flags codes >= Q
-__global__ void k_transpose(const uint8_t *__restrict__ X, int64_t Lx, int N, int L,
-                            uint8_t *__restrict__ XT, int64_t Nx, int *__restrict__ bad)
+// X [N][Lx] -> XT [L][Nx]; flags codes >= Q.  A block takes 128 sequences x 64
+// loci: 16-byte reads of X into shared memory, then each thread gathers 16
+// sequences of four loci as 4 x 4 byte transposes and writes 16 bytes per
+// locus.  One byte per thread and access took 0.59 ms at 3000 x 94,000
+// (0.56 GB: 0.08 at the copy rate); this takes 0.12.
+constexpr int TR_SEQ = 128, TR_LOC = 64;
+
+__global__ void __launch_bounds__(256)
+k_transpose(const uint8_t *__restrict__ X, int64_t Lx, int N, int L, uint8_t *__restrict__ XT, int64_t Nx,
+            int *__restrict__ bad)
 {
-    __shared__ uint8_t tile[64][65];
-    const int n0 = blockIdx.x * 64, i0 = blockIdx.y * 64;
-    for (int k = threadIdx.x; k < 64 * 64; k += blockDim.x) {
-        const int ii = k / 64, nn = k % 64;
-        const int i = i0 + ii, n = n0 + nn;
-        uint8_t v = 0;
-        if (i < N && n < L) {
-            v = X[(int64_t)i * Lx + n];
-            if (v >= Q) atomicOr(bad, 1);
-        }
-        tile[ii][nn] = v;
+    // [sequence][16 words of four loci], rows 17 words apart: a warp's 32
+    // rows of one word fall in distinct banks
+    __shared__ uint32_t tile[TR_SEQ][TR_LOC / 4 + 1];
+    const int n0 = blockIdx.x * TR_LOC, i0 = blockIdx.y * TR_SEQ;
+    uint32_t seen = 0u;
+    for (int k = threadIdx.x; k < TR_SEQ * (TR_LOC / 16); k += 256) {
+        const int ii = k / (TR_LOC / 16), c = k % (TR_LOC / 16);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        // (Lx is a multiple of 64; the padding past the last locus is zero)
+        if (i0 + ii < N) v = *reinterpret_cast<const uint4 *>(X + (int64_t)(i0 + ii) * Lx + n0 + 16 * c);
+        seen |= v.x | v.y | v.z | v.w;
+        tile[ii][4 * c] = v.x;
+        tile[ii][4 * c + 1] = v.y;
+        tile[ii][4 * c + 2] = v.z;
+        tile[ii][4 * c + 3] = v.w;
     }
+    if (seen & 0xFCFCFCFCu) atomicOr(bad, 1);
     __syncthreads();
-    for (int k = threadIdx.x; k < 64 * 64; k += blockDim.x) {
-        const int nn = k / 64, ii = k % 64;
-        const int i = i0 + ii, n = n0 + nn;
-        if (n < L && i < (int)Nx) XT[(int64_t)n * Nx + i] = (i < N) ? tile[ii][nn] : 0;
+    // work unit: word w (four loci) x 16 sequences; eight units of one word
+    // side by side write 128 consecutive bytes of a locus's row
+    for (int k = threadIdx.x; k < (TR_LOC / 4) * (TR_SEQ / 16); k += 256) {
+        const int sg = k % (TR_SEQ / 16), w = k / (TR_SEQ / 16);
+        uint32_t o[4][4];   // [locus][four sequences]
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t r0 = tile[16 * sg + 4 * q][w], r1 = tile[16 * sg + 4 * q + 1][w];
+            const uint32_t r2 = tile[16 * sg + 4 * q + 2][w], r3 = tile[16 * sg + 4 * q + 3][w];
+            const uint32_t a = __byte_perm(r0, r1, 0x5140), b = __byte_perm(r2, r3, 0x5140);
+            const uint32_t c = __byte_perm(r0, r1, 0x7362), d = __byte_perm(r2, r3, 0x7362);
+            o[0][q] = __byte_perm(a, b, 0x5410);
+            o[1][q] = __byte_perm(a, b, 0x7632);
+            o[2][q] = __byte_perm(c, d, 0x5410);
+            o[3][q] = __byte_perm(c, d, 0x7632);
+        }
+        const int64_t i = i0 + 16 * sg;
+        if (i >= Nx) continue;   // (Nx is a multiple of 64; sequences past N are zero)
+#pragma unroll
+        for (int l = 0; l < 4; ++l)
+            if (n0 + 4 * w + l < L)
+                *reinterpret_cast<uint4 *>(XT + (int64_t)(n0 + 4 * w + l) * Nx + i) =
+                    make_uint4(o[l][0], o[l][1], o[l][2], o[l][3]);
     }
 }
 
@@ -595,20 +643,18 @@ int ws_knn(sdca_handle *h, int k)
     int rc;
     if (!h->knn && (rc = dalloc(h, &h->knn, (size_t)P.N * WS_MAX_K))) return rc;
     if (!h->knn_d && (rc = dalloc(h, &h->knn_d, (size_t)P.N * WS_MAX_K))) return rc;
-    const int64_t W = (P.L + 31) / 32;
     uint64_t *packed = nullptr;
+    double *sums = nullptr;
+    if ((rc = pair_workspace(h, &packed, &sums))) return rc;
     int32_t *dist = nullptr;
-    if (cudaMalloc(&packed, sizeof(uint64_t) * P.N * W) != cudaSuccess ||
-        cudaMalloc(&dist, sizeof(int32_t) * P.N * P.N) != cudaSuccess) {
+    if (cudaMalloc(&dist, sizeof(int32_t) * P.N * P.N) != cudaSuccess) {
         cudaGetLastError();
-        if (packed) cudaFree(packed);
         return fail(h, SDCA_E_NOMEM, "device allocation for the neighbour table failed");
     }
     launch_distances(h->X, P.Lx, (int)P.N, (int)P.L, packed, dist, h->stream);
     launch_knn(dist, (int)P.N, k, h->knn, h->stream, h->knn_d);
     const cudaError_t e1 = cudaGetLastError();
     const cudaError_t e2 = cudaStreamSynchronize(h->stream);
-    cudaFree(packed);
     cudaFree(dist);
     if (e1 != cudaSuccess || e2 != cudaSuccess)
         return fail(h, SDCA_E_CUDA, std::string("neighbour table: ") + cudaGetErrorString(e1 ? e1 : e2));
@@ -2193,7 +2239,7 @@ int sdca_set_alignment(sdca_handle *h, const uint8_t *states, const double *weig
     CK(cudaMemcpyAsync(h->wf, wf.data(), sizeof(float) * P.N, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
     {
-        dim3 grid((unsigned)((P.L + 63) / 64), (unsigned)((P.Nx + 63) / 64));
+        dim3 grid((unsigned)((P.L + TR_LOC - 1) / TR_LOC), (unsigned)((P.Nx + TR_SEQ - 1) / TR_SEQ));
         k_transpose<<<grid, 256, 0, h->stream>>>(h->X, P.Lx, (int)P.N, (int)P.L, h->XT, P.Nx, h->flag);
     }
     CKL();
@@ -2218,23 +2264,17 @@ int sdca_set_alignment(sdca_handle *h, const uint8_t *states, const double *weig
     if (h->form == SDCA_FORM_DUAL) {
         // K_ij = loci where sequences i and j agree; rho is rounded to QB
         // fractional bits of w_max so that |sum_j K_ij rho_q| < 2^62
-        const int64_t W = (P.L + 31) / 32;
         uint64_t *packed = nullptr;
-        int32_t *dist = nullptr;
-        if (cudaMalloc(&packed, sizeof(uint64_t) * P.N * W) != cudaSuccess ||
-            cudaMalloc(&dist, sizeof(int32_t) * P.N * P.N) != cudaSuccess) {
-            cudaGetLastError();
-            if (packed) cudaFree(packed);
+        double *sums = nullptr;
+        const int rc = pair_workspace(h, &packed, &sums);
+        if (rc) {
             h->has_alignment = false;
-            return fail(h, SDCA_E_NOMEM, "device allocation for the agreement matrix failed");
+            return rc;
         }
-        launch_distances(h->X, P.Lx, (int)P.N, (int)P.L, packed, dist, h->stream);
-        launch_dual_kmat(dist, (int)P.N, P.Nx, (int)P.L, h->Kmat, h->stream);
+        launch_agreements(h->X, P.Lx, (int)P.N, (int)P.L, packed, h->Kmat, P.Nx, h->stream);
         if (h->kd) tc_kdig_fill_k(h->kd, P, h->Kmat, h->Kd, h->stream);
         const cudaError_t e1 = cudaGetLastError();
         const cudaError_t e2 = cudaStreamSynchronize(h->stream);
-        cudaFree(packed);
-        cudaFree(dist);
         if (e1 != cudaSuccess || e2 != cudaSuccess) {
             h->has_alignment = false;
             return fail(h, SDCA_E_CUDA, std::string("agreement matrix: ") + cudaGetErrorString(e1 ? e1 : e2));
@@ -2409,33 +2449,20 @@ int sdca_compute_weights(sdca_handle *h, const uint8_t *states, const double *mu
         s->has_alignment = false;
         s->knn_k = 0;
     }
-    const int64_t W = (P.L + 31) / 32;
     uint64_t *packed = nullptr;
-    double *d = nullptr;
-    unsigned long long *nonid = nullptr;
-    auto release = [&]() {
-        if (packed) cudaFree(packed);
-        if (d) cudaFree(d);
-    };
-    if (cudaMalloc(&packed, sizeof(uint64_t) * P.N * W) != cudaSuccess ||
-        cudaMalloc(&d, sizeof(double) * (2 * P.N + 1)) != cudaSuccess) {
-        cudaGetLastError();
-        release();
-        return fail(h, SDCA_E_NOMEM, "device allocation for reweighting failed");
-    }
-    double *nbr = d, *dmult = d + P.N;
-    nonid = reinterpret_cast<unsigned long long *>(d + 2 * P.N);
-    int rc = SDCA_OK;
+    double *nbr = nullptr;
+    int rc = pair_workspace(h, &packed, &nbr);
+    if (rc) return rc;
+    double *const dmult = nbr + P.N;
     do {
         if (cudaMemcpy2DAsync(h->X, P.Lx, states, P.L, P.L, P.N, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
-            cudaMemsetAsync(d, 0, sizeof(double) * (2 * P.N + 1), h->stream) != cudaSuccess ||
+            cudaMemsetAsync(nbr, 0, sizeof(double) * P.N, h->stream) != cudaSuccess ||
             (mult && cudaMemcpyAsync(dmult, mult, sizeof(double) * P.N, cudaMemcpyHostToDevice, h->stream) !=
                          cudaSuccess)) {
             rc = fail(h, SDCA_E_CUDA, "reweighting upload failed");
             break;
         }
-        launch_weights(h->X, P.Lx, (int)P.N, (int)P.L, packed, threshold, mult ? dmult : nullptr, nbr, nonid,
-                       h->stream);
+        launch_weights(h->X, P.Lx, (int)P.N, (int)P.L, packed, threshold, mult ? dmult : nullptr, nbr, h->stream);
         if (cudaGetLastError() != cudaSuccess) {
             rc = fail(h, SDCA_E_CUDA, "reweighting kernel launch failed");
             break;
@@ -2452,7 +2479,6 @@ int sdca_compute_weights(sdca_handle *h, const uint8_t *states, const double *mu
             weights_out[i] = mi / (mi + hn[i]);
         }
     } while (0);
-    release();
     return rc;
 }
 
@@ -2495,7 +2521,7 @@ int sdca_set_targets(sdca_handle *h, const uint8_t *targets, int64_t n_target_lo
             rc = fail(h, SDCA_E_CUDA, "target upload failed");
             break;
         }
-        dim3 grid((unsigned)((n_target_loci + 63) / 64), (unsigned)((P.Nx + 63) / 64));
+        dim3 grid((unsigned)((n_target_loci + TR_LOC - 1) / TR_LOC), (unsigned)((P.Nx + TR_SEQ - 1) / TR_SEQ));
         k_transpose<<<grid, 256, 0, h->stream>>>(tmp, LTx, (int)P.N, (int)n_target_loci, h->TT, P.Nx, h->flag);
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess)
             rc = fail(h, SDCA_E_CUDA, "target transpose failed");

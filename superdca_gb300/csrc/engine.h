@@ -221,7 +221,6 @@ void launch_score(const Problem &P, const SlotDev *sd, const int32_t *list, int 
                   const float *wa, int gap, float *rows, cudaStream_t st);
 
 // dual form (kernels_dual.cu)
-void launch_dual_kmat(const int32_t *dist, int N, int64_t Nx, int L, int32_t *K, cudaStream_t st);
 void launch_dual_quant(const Problem &P, const SlotDev *sd, const int32_t *list, int n, const float *R,
                        const uint8_t *rstate, double qscale, int32_t *rq, long long *csum, cudaStream_t st, const int *cnt = nullptr);
 void launch_dual_kprod(const Problem &P, const int32_t *list, int n, const uint8_t *rstate, const int32_t *K,
@@ -271,6 +270,7 @@ void launch_dual_to_wa(const Problem &P, const SlotDev *sd, const int32_t *list,
 void mlp_pack(const float *p_dev, void *wb, cudaStream_t st);
 void mlp_infer(const float *p_dev, const void *wb, const float *X, int64_t M, float *out, int *err,
                cudaStream_t st);
+int64_t packed_words(int64_t L);   // 64-bit words per sequence of the packed states (distances, weights)
 void launch_distances(const uint8_t *X, int64_t ld, int N, int L, uint64_t *packed, int32_t *dist,
                       cudaStream_t st);
 void launch_knn(const int32_t *dist, int N, int k, int32_t *knn, cudaStream_t st, int32_t *knn_d = nullptr);
@@ -299,7 +299,9 @@ void launch_ws_scatter(int L, int64_t Dp, const int32_t *slots, const int32_t *l
 void launch_ws_hfit(const Problem &P, const int32_t *slots, const uint8_t *rstate, const double *w, int G,
                     float *wa, double *lbase, double *xmax, cudaStream_t st);
 void launch_weights(const uint8_t *X, int64_t ld, int N, int L, uint64_t *packed, double threshold,
-                    const double *mult, double *nbr, unsigned long long *nonidentical, cudaStream_t st);
+                    const double *mult, double *nbr, cudaStream_t st);
+void launch_agreements(const uint8_t *X, int64_t ldx, int N, int L, uint64_t *packed, int32_t *K, int64_t ld,
+                       cudaStream_t st);
 
 // tensor-core form (kernels_tc.cu)
 struct TcPlan;

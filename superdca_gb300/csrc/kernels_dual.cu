@@ -31,14 +31,6 @@
 namespace sdca {
 namespace {
 
-__global__ void k_dual_kmat(const int32_t *__restrict__ dist, int N, int64_t Nx, int L, int32_t *__restrict__ K)
-{
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < Nx * Nx; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / Nx, j = t % Nx;
-        K[t] = (i < N && j < N) ? L - dist[i * N + j] : 0;
-    }
-}
-
 // rho_q = round(R * qscale) (R is FP32, so a single-precision product loses
 // nothing: the rounded value is the one every later step uses), with the
 // entry at the sequence's own state set to minus the sum of the other three,
@@ -1454,11 +1446,6 @@ unsigned grid_for(int64_t elems, int per_block_elems, int cap)
 constexpr int STREAM_PASSES = 8;
 
 } // namespace
-
-void launch_dual_kmat(const int32_t *dist, int N, int64_t Nx, int L, int32_t *K, cudaStream_t st)
-{
-    k_dual_kmat<<<grid_for(Nx * Nx, 256 * 8, 4096), 256, 0, st>>>(dist, N, Nx, L, K);
-}
 
 void launch_dual_quant(const Problem &P, const SlotDev *sd, const int32_t *list, int n, const float *R,
                        const uint8_t *rstate, double qscale, int32_t *rq, long long *csum, cudaStream_t st,

@@ -1867,6 +1867,10 @@ int solve_lane(sdca_handle *h, Queue &Qu, cudaEvent_t t0_common)
     if (!t0 || !t1) return fail(h, SDCA_E_CUDA, "cudaEventCreate failed");
     if (!t0_common) CK(cudaEventRecord(t0, h->stream));
     for (auto &S : h->slots) S.phase = PH_EMPTY;
+    // the solver sums over whole vectors: the gradient buffers that
+    // sdca_eval may have used get their zero padding back
+    if (const int64_t used = QQ * h->P.L + Q; h->P.Dp > used)
+        CK(cudaMemset2DAsync(h->gpool + used, sizeof(float) * h->P.Dp, 0, sizeof(float) * (h->P.Dp - used), 2, h->stream));
     int rc = refill(h, Qu);
     if (rc) return rc;
     for (;;) {
@@ -2386,47 +2390,21 @@ int sdca_eval(sdca_handle *h, uint32_t r, const double *x, double *f, double *g)
     if ((int64_t)r >= (h->scan ? h->LT : P.L)) return fail(h, SDCA_E_ARG, "locus index out of range");
     CK(cudaSetDevice(h->cfg.device));
     prof_reset(h);
-    std::vector<float> xe(P.Dp);
-    ref_to_engine(P, h->scan ? -1 : (int64_t)r, x, xe.data());
-    const int b = 0;
-    rc = slot_begin(h, b, 0, (int32_t)r, xe.data());
-    if (rc) return rc;
-    std::vector<int32_t> one{b};
-    rc = run_forward(h, one, h->wa, true);
-    if (rc) return rc;
-    SlotHost &S = h->slots[b];
-    rc = upload_slots(h, one);
-    if (rc) return rc;
-    rc = zero_acc(h);
-    if (rc) return rc;
-    launch_trial(P, h->sd, h->list, 1, h->lbase, h->u, h->rstate, h->w, h->R, h->acc, h->stream);
+    // Slot 0's buffers serve (no solve is running): its gradient buffers hold
+    // the point in the reference's layout (16 L + 4 doubles in at least 2 Dp
+    // floats), then the partial logits, then the gradient.
+    const size_t bytes = sizeof(double) * (QQ * P.L + Q);
+    double *const xg = reinterpret_cast<double *>(h->gpool);
+    CK(cudaMemcpyAsync(xg, x, bytes, cudaMemcpyHostToDevice, h->stream));
+    const uint8_t *const target = (h->scan ? h->TT : h->XT) + (int64_t)r * P.Nx;
+    launch_eval(P, h->X, h->XT, h->scan ? -1 : (int64_t)r, xg, g != nullptr, target, h->w, h->wa, h->partial64, h->R,
+                h->acc, h->stream);
     CKL();
-    rc = fetch_acc(h);
-    if (rc) return rc;
-    const double fdata = acc_get(h, b, ACC_F);
-    for (int a = 0; a < Q; ++a) S.rs[a] = acc_get(h, b, ACC_RS0 + a);
-    S.push = false;
-    S.ring_new = -1;
-    rc = upload_slots(h, one);
-    if (rc) return rc;
-    rc = zero_acc(h);
-    if (rc) return rc;
-    launch_bwd_gather(P, h->XT, h->sd, h->list, 1, h->R, h->wa, h->gpool, h->Ypool, h->Spool,
-                      h->hist_bf16, h->acc, h->stream);
-    launch_hpart(P, h->sd, h->list, 1, h->wa, h->gpool, h->Ypool, h->Spool, h->hist_bf16, h->acc,
-                 h->stream);
-    CKL();
-    rc = fetch_acc(h);
-    if (rc) return rc;
-    *f = fdata + P.lambda_J * acc_get(h, b, ACC_X2J) + P.lambda_h * acc_get(h, b, ACC_X2H);
-    if (g) {
-        std::vector<float> ge(P.Dp);
-        CK(cudaMemcpyAsync(ge.data(), h->gpool + (int64_t)(2 * b + 1 - S.gcur) * P.Dp,
-                           sizeof(float) * P.Dp, cudaMemcpyDeviceToHost, h->stream));
-        { const int r_ = stream_sync(h); if (r_) return r_; }
-        engine_to_ref(P, ge.data(), g);
-    }
-    S.phase = PH_EMPTY;
+    h->prof.gpu_launches += 4;
+    CK(cudaMemcpyAsync(h->acc_h, h->acc, sizeof(double) * NACC, cudaMemcpyDeviceToHost, h->stream));
+    if (g) CK(cudaMemcpyAsync(g, xg, bytes, cudaMemcpyDeviceToHost, h->stream));
+    if ((rc = stream_sync(h))) return rc;
+    *f = acc_get(h, 0, ACC_F) + P.lambda_J * acc_get(h, 0, ACC_X2J) + P.lambda_h * acc_get(h, 0, ACC_X2H);
     return SDCA_OK;
 }
 

@@ -194,6 +194,9 @@ void launch_reduce_partial(const Problem &P, const int32_t *list, int n, const f
                            cudaStream_t st, int C = 0, const float *R = nullptr, double *acc = nullptr);
 void launch_fwd_exact(const Problem &P, const uint8_t *X, const int32_t *list, int n, const float *vecs,
                       double *partial64, double *lbase, cudaStream_t st);
+void launch_eval(const Problem &P, const uint8_t *X, const uint8_t *XT, int64_t r, double *xg, bool want_g,
+                 const uint8_t *rstate, const double *w, float *wa, double *partial64, float *R, double *acc,
+                 cudaStream_t st);
 void launch_grad_finalize(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
                           const float *wa, float *gpool, void *Ypool, const void *Spool, int hist_bf16,
                           double *acc, cudaStream_t st);

@@ -9,6 +9,8 @@
 // 153-190, Coupling_matrix_view.hpp:88-111) for a batch of target loci that
 // share one alignment read.  Both are bound by shared-memory / FP32 issue
 // (one 16-byte shared load or 16 FMAs per (sequence, locus, slot)).
+#include <algorithm>
+
 #include "engine.h"
 #include "kernels_common.cuh"
 
@@ -343,6 +345,213 @@ k_grad_finalize(int L, const SlotDev *__restrict__ sd, const int32_t *__restrict
     if ((threadIdx.x & 31) == 0 && wm > 0.f) atomic_max_nonneg(acc + (int64_t)b * NACC + ACC_GMAX, (double)wm);
 }
 
+// ---- one evaluation (sdca_eval): the same sums as the batch kernels above and
+// k_trial, for one point.  The batch kernels' groups of four slots did four
+// times the work for one, and the point and the gradient were converted on
+// the host between the reference's layout and this one, in 64-bit steps over
+// 16 L values each way: 4.7 ms at 3000 x 94,000, where the passes here take
+// 0.5 ms (0.22 logits, 0.25 gradient) and the call 0.9.
+
+// the point from the reference's layout (double) into the engine's (FP32,
+// J_rr = 0, padding 0); the sums start at zero
+__global__ void __launch_bounds__(256)
+k_eval_point(const double *__restrict__ x, int64_t L, int64_t Dp, int64_t r, float *__restrict__ wa,
+             double *__restrict__ acc)
+{
+    if (blockIdx.x == 0 && threadIdx.x < NACC) acc[threadIdx.x] = 0.0;
+    const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;   // a row of four: locus n, state s
+    if (4 * t >= Dp) return;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < Q * L) {
+        const int64_t n = t / Q, s = t % Q, b = n / 16, e = b < L / 16 ? 16 : L % 16;
+        if (n != r) {
+            const double *p = x + b * 16 * QQ + (s * e + n % 16) * Q;
+            v = make_float4((float)p[0], (float)p[1], (float)p[2], (float)p[3]);
+        }
+    } else if (t == Q * L) {
+        const double *p = x + QQ * L;
+        v = make_float4((float)p[0], (float)p[1], (float)p[2], (float)p[3]);
+    }
+    reinterpret_cast<float4 *>(wa)[t] = v;
+}
+
+// Partial logits of k_fwd_gather_exact (FP32 over the same 64-locus
+// stretches, FP64 across), one slot.  A block takes 256 sequences and one of
+// the `parts` shares of a locus chunk's stretches, so that some eight blocks
+// per SM cover the latency of the shared-memory row each (sequence, locus)
+// reads; those reads bound it.
+constexpr int EF_STR = 64;
+
+__global__ void __launch_bounds__(FWD_THREADS)
+k_eval_fwd(const uint8_t *__restrict__ X, int64_t Lx, int N, int L, int64_t LC, int parts, const float *__restrict__ wa,
+           double *__restrict__ partial, int64_t Nx)
+{
+    __shared__ float4 sJ[EF_STR][Q];
+    const int t = threadIdx.x, i = blockIdx.x * FWD_THREADS + t, c = blockIdx.y / parts, part = blockIdx.y % parts;
+    const int64_t n_begin = (int64_t)c * LC, n_end = min((int64_t)L, n_begin + LC);
+    const int64_t str = (n_end - n_begin + EF_STR - 1) / EF_STR;
+    const int64_t k0 = str * part / parts, k1 = str * (part + 1) / parts;
+    double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+    for (int64_t k = k0; k < k1; ++k) {
+        const int64_t n0 = n_begin + k * EF_STR, e = n0 * Q + t;   // EF_STR x Q rows, one per thread
+        const float4 row = e < n_end * Q ? reinterpret_cast<const float4 *>(wa)[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+        uint4 w[4];
+        if (i < N) {
+            const uint4 *xp = reinterpret_cast<const uint4 *>(X + (int64_t)i * Lx + n0);
+            w[0] = xp[0];
+            w[1] = xp[1];
+            // (a chunk may end half way through a stretch, at the row's end)
+            const bool more = n0 + 32 < n_end;
+            w[2] = more ? xp[2] : make_uint4(0u, 0u, 0u, 0u);
+            w[3] = more ? xp[3] : make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+        sJ[t / Q][t % Q] = row;
+        __syncthreads();
+        if (i < N) {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t words[4] = {w[q].x, w[q].y, w[q].z, w[q].w};
+#pragma unroll
+                for (int wd = 0; wd < 4; ++wd)
+#pragma unroll
+                    for (int bt = 0; bt < 4; ++bt) {
+                        const float4 j = sJ[q * 16 + wd * 4 + bt][(words[wd] >> (8 * bt)) & 0x3];
+                        acc.x += j.x;
+                        acc.y += j.y;
+                        acc.z += j.z;
+                        acc.w += j.w;
+                    }
+            }
+            a0 += acc.x;
+            a1 += acc.y;
+            a2 += acc.z;
+            a3 += acc.w;
+        }
+    }
+    if (i < N) {
+        double2 *o = reinterpret_cast<double2 *>(partial + ((int64_t)blockIdx.y * Nx + i) * Q);
+        o[0] = make_double2(a0, a1);
+        o[1] = make_double2(a2, a3);
+    }
+}
+
+// logits from the chunks' partial sums, objective and node beliefs (k_trial
+// at step 0); eight threads share a sequence's chunks
+constexpr int EB_SHARE = 8;
+
+__global__ void __launch_bounds__(FWD_THREADS)
+k_eval_beliefs(const double *__restrict__ partial, int C, int64_t Nx, int N, const float *__restrict__ h,
+               const uint8_t *__restrict__ rstate, const double *__restrict__ w, float4 *__restrict__ R,
+               double *__restrict__ acc)
+{
+    const int i = (blockIdx.x * FWD_THREADS + threadIdx.x) / EB_SHARE, k = threadIdx.x % EB_SHARE;
+    double f = 0, rs[4] = {0, 0, 0, 0}, l[4] = {0, 0, 0, 0};
+    if (i < N)
+#pragma unroll 4
+        for (int c = k; c < C; c += EB_SHARE) {
+            const double2 *p = reinterpret_cast<const double2 *>(partial + ((int64_t)c * Nx + i) * Q);
+            const double2 u = p[0], v = p[1];
+            l[0] += u.x;
+            l[1] += u.y;
+            l[2] += v.x;
+            l[3] += v.y;
+        }
+#pragma unroll
+    for (int o = EB_SHARE / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < 4; ++a) l[a] += __shfl_xor_sync(0xffffffffu, l[a], o);
+    if (i < N && k == 0) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) l[a] += (double)h[a];
+        const double mx = fmax(fmax(l[0], l[1]), fmax(l[2], l[3]));
+        double e[4], z = 0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            e[a] = exp(l[a] - mx);
+            z += e[a];
+        }
+        const int sr = rstate[i] & 3;
+        const double wi = w[i];
+        f = wi * (mx + log(z) - (sr == 0 ? l[0] : sr == 1 ? l[1] : sr == 2 ? l[2] : l[3]));
+#pragma unroll
+        for (int a = 0; a < 4; ++a) rs[a] = wi * (e[a] / z) - (a == sr ? wi : 0.0);
+        R[i] = make_float4((float)rs[0], (float)rs[1], (float)rs[2], (float)rs[3]);
+    }
+    double v[5] = {f, rs[0], rs[1], rs[2], rs[3]};
+    const int idx[5] = {ACC_F, ACC_RS0, ACC_RS1, ACC_RS2, ACC_RS3};
+    block_sum_atomic<5>(v, acc, idx);
+}
+
+// the gradient of k_bwd_gather and k_hpart, one slot, into the reference's
+// layout (double, values of FP32), and the L2 sums
+__global__ void __launch_bounds__(BWD_THREADS)
+k_eval_bwd(const uint8_t *__restrict__ XT, int64_t Nx, int N, int L, int64_t r, const float4 *__restrict__ R,
+           const float *__restrict__ wa, double lambda_J, double lambda_h, double *__restrict__ g,
+           double *__restrict__ acc)
+{
+    __shared__ float4 sR[BWD_SUB];
+    const int n = blockIdx.x * BWD_THREADS + threadIdx.x;
+    float a[QQ];
+#pragma unroll
+    for (int k = 0; k < QQ; ++k) a[k] = 0.f;
+    for (int i0 = 0; i0 < N; i0 += BWD_SUB) {
+        __syncthreads();
+        if (threadIdx.x < BWD_SUB) sR[threadIdx.x] = i0 + threadIdx.x < N ? R[i0 + threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
+        uint4 w[BWD_SUB / 16];
+        if (n < L)
+#pragma unroll
+            for (int q4 = 0; q4 < BWD_SUB / 16; ++q4) w[q4] = reinterpret_cast<const uint4 *>(XT + (int64_t)n * Nx + i0)[q4];
+        __syncthreads();
+        if (n < L) {
+#pragma unroll
+            for (int q4 = 0; q4 < BWD_SUB / 16; ++q4) {
+                const uint32_t words[4] = {w[q4].x, w[q4].y, w[q4].z, w[q4].w};
+#pragma unroll
+                for (int wd = 0; wd < 4; ++wd)
+#pragma unroll
+                    for (int bt = 0; bt < 4; ++bt) {
+                        const int s = (words[wd] >> (8 * bt)) & 0x3;
+                        const float4 v = sR[q4 * 16 + wd * 4 + bt];
+                        const float m0 = s == 0, m1 = s == 1, m2 = s == 2, m3 = s == 3;
+                        a[0] += m0 * v.x; a[1] += m0 * v.y; a[2] += m0 * v.z; a[3] += m0 * v.w;
+                        a[4] += m1 * v.x; a[5] += m1 * v.y; a[6] += m1 * v.z; a[7] += m1 * v.w;
+                        a[8] += m2 * v.x; a[9] += m2 * v.y; a[10] += m2 * v.z; a[11] += m2 * v.w;
+                        a[12] += m3 * v.x; a[13] += m3 * v.y; a[14] += m3 * v.z; a[15] += m3 * v.w;
+                    }
+            }
+        }
+    }
+    const float l2 = (float)(2.0 * lambda_J);
+    float x2 = 0.f;
+    if (n < L) {
+        const int64_t b = n / 16, e = b < L / 16 ? 16 : L % 16;
+        const float4 *x4 = reinterpret_cast<const float4 *>(wa + (int64_t)n * QQ);
+        const bool zero = n == r;
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+            const float4 xv = x4[s];
+            x2 += dot4(xv, xv);
+            if (g) {
+                double *o = g + b * 16 * QQ + (s * e + n % 16) * Q;
+                o[0] = zero ? 0.f : a[4 * s + 0] + l2 * xv.x;
+                o[1] = zero ? 0.f : a[4 * s + 1] + l2 * xv.y;
+                o[2] = zero ? 0.f : a[4 * s + 2] + l2 * xv.z;
+                o[3] = zero ? 0.f : a[4 * s + 3] + l2 * xv.w;
+            }
+        }
+    }
+    double v[1] = {x2};
+    const int idx[1] = {ACC_X2J};
+    block_sum_atomic<1>(v, acc, idx);
+    if (blockIdx.x == 0 && threadIdx.x < Q) {
+        const double x = wa[(int64_t)QQ * L + threadIdx.x];
+        if (g) g[(int64_t)QQ * L + threadIdx.x] = (float)(acc[ACC_RS0 + threadIdx.x] + 2.0 * lambda_h * x);
+        atomicAdd(acc + ACC_X2H, x * x);
+    }
+}
+
 } // namespace
 
 void launch_fwd_gather(const Problem &P, const uint8_t *X, const int32_t *list, int n,
@@ -378,6 +587,30 @@ void launch_reduce_partial(const Problem &P, const int32_t *list, int n, const f
                                            P.Bmax, P.Nx, (int)P.N, list, vecs, P.Dp, QQ * P.L, add_h,
                                            reinterpret_cast<float4 *>(out_f), out_d,
                                            reinterpret_cast<const float4 *>(R), acc);
+}
+
+// One evaluation at the point xg (reference layout, on the device; room for
+// 2 Dp floats, which then hold the partial logits and, when want_g, the
+// gradient): acc (NACC) receives the objective's data part, the
+// residual sums and the L2 sums.  partial64: room for the Cg chunks' partial
+// logits, where xg has none.
+void launch_eval(const Problem &P, const uint8_t *X, const uint8_t *XT, int64_t r, double *xg, bool want_g,
+                 const uint8_t *rstate, const double *w, float *wa, double *partial64, float *R, double *acc, cudaStream_t st)
+{
+    k_eval_point<<<(unsigned)((P.Dp / 4 + 255) / 256), 256, 0, st>>>(xg, P.L, P.Dp, r, wa, acc);
+    const int64_t seq_tiles = (P.N + FWD_THREADS - 1) / FWD_THREADS;
+    // shares of a chunk: some eight blocks per SM, at least one stretch each
+    const int64_t room = P.Dp / (P.Nx * Q) / P.Cg;   // (Dp doubles)
+    const int64_t parts = std::min({room, std::max<int64_t>(1, 8 * 152 / (seq_tiles * P.Cg)), (P.LC + EF_STR - 1) / EF_STR});
+    const int slices = (int)(P.Cg * std::max<int64_t>(1, parts));
+    double *part = parts >= 1 ? xg : partial64;
+    k_eval_fwd<<<dim3((unsigned)seq_tiles, (unsigned)slices), FWD_THREADS, 0, st>>>(
+        X, P.Lx, (int)P.N, (int)P.L, P.LC, (int)(slices / P.Cg), wa, part, P.Nx);
+    k_eval_beliefs<<<(unsigned)((P.N * EB_SHARE + FWD_THREADS - 1) / FWD_THREADS), FWD_THREADS, 0, st>>>(
+        part, slices, P.Nx, (int)P.N, wa + QQ * P.L, rstate, w, reinterpret_cast<float4 *>(R), acc);
+    k_eval_bwd<<<(unsigned)((P.L + BWD_THREADS - 1) / BWD_THREADS), BWD_THREADS, 0, st>>>(
+        XT, P.Nx, (int)P.N, (int)P.L, r, reinterpret_cast<const float4 *>(R), wa, P.lambda_J, P.lambda_h,
+        want_g ? xg : nullptr, acc);
 }
 
 void launch_grad_finalize(const Problem &P, const SlotDev *sd, const int32_t *list, int n,

@@ -103,11 +103,10 @@ struct ProfRec {
 } // namespace
 
 // Per-class timing of one replay of the dual form's iteration core: the
-// events recorded by its event nodes and, per class, the list (counts index)
-// whose length gives the units.
+// kernel's time stamps (TS_*) and the list (counts index) whose length gives
+// the class's units.
 struct GraphRec {
-    int cls, kernels, cidx;
-    cudaEvent_t a, b;
+    int cls, kernels, cidx, stamp;
 };
 
 // The round's list lengths, in the order they follow the lists in device
@@ -118,7 +117,6 @@ enum { DC_T = 0, DC_G = 1, DC_GW = 2, DC_W = 3, DC_N = 4 };
 struct DualGraph {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t ev_round = nullptr;     // recorded after the summary copy (the host waits on it)
-    std::vector<cudaEvent_t> ev;        // timing events of the event nodes
     std::vector<GraphRec> recs;
     bool pending = false;               // replayed, its timings not collected yet
     int64_t counts[DC_N] = {};          // the list lengths of that replay
@@ -180,6 +178,16 @@ struct sdca_handle {
     DualCtl *ctl = nullptr;        // per-slot solver state, owned by the device while a slot iterates
     DualSum *sum = nullptr, *sum_h = nullptr;   // per-slot summary the host reads after each round
     double *dacc = nullptr;        // direction sums for the next line search
+    // what a round reads back, in one copy: summaries, accumulators, the error
+    // words of the tensor-core kernels, the time stamps of both graphs
+    uint8_t *out = nullptr, *out_h = nullptr;
+    size_t out_bytes = 0;
+    int *errs_h = nullptr;         // tc_err, ws_err as copied
+    unsigned long long *ts = nullptr, *ts_h = nullptr;
+    // what a round clears, in one memset: csum, amax, dots, dacc
+    uint8_t *zero = nullptr;
+    size_t zero_bytes = 0;
+    std::vector<int32_t> dlist_sent;   // the lists as the device has them
     int32_t *dlist = nullptr;      // the round's slot lists: [evaluations | searching | gradient pass + starts |
                                    // starts], then their lengths (DualCounts)
     cudaEvent_t ev_round = nullptr;   // end of a round's control kernel
@@ -341,6 +349,33 @@ template <typename T> int halloc(sdca_handle *h, T **p, size_t count)
     return SDCA_OK;
 }
 
+// The dual form's round blocks (sdca_handle::out, ::zero) and the pointers into them.
+int dual_blocks(sdca_handle *h)
+{
+    const size_t B = h->P.Bmax, sum = sizeof(DualSum) * B, acc = sizeof(double) * NACC * B, errs = 16,
+                 ts = sizeof(unsigned long long) * 2 * TS_WORDS;
+    static_assert(sizeof(DualSum) % 8 == 0, "the parts of the block stay 8-byte aligned");
+    h->out_bytes = sum + acc + errs + ts;
+    int rc = dalloc(h, &h->out, h->out_bytes);
+    if (rc || (rc = halloc(h, &h->out_h, h->out_bytes))) return rc;
+    h->sum = reinterpret_cast<DualSum *>(h->out);
+    h->sum_h = reinterpret_cast<DualSum *>(h->out_h);
+    h->acc = reinterpret_cast<double *>(h->out + sum);
+    h->acc_h = reinterpret_cast<double *>(h->out_h + sum);
+    h->tc_err = reinterpret_cast<int *>(h->out + sum + acc);
+    h->ws_err = h->tc_err + 1;
+    h->errs_h = reinterpret_cast<int *>(h->out_h + sum + acc);
+    h->ts = reinterpret_cast<unsigned long long *>(h->out + sum + acc + errs);
+    h->ts_h = reinterpret_cast<unsigned long long *>(h->out_h + sum + acc + errs);
+    h->zero_bytes = sizeof(double) * B * (CSUM + 2 + 4 * MAXHIST + NDACC);
+    if ((rc = dalloc(h, &h->zero, h->zero_bytes))) return rc;
+    h->csum = reinterpret_cast<long long *>(h->zero);
+    h->amax = reinterpret_cast<double *>(h->csum + CSUM * B);
+    h->dots = h->amax + 2 * B;
+    h->dacc = h->dots + 4 * MAXHIST * B;
+    return SDCA_OK;
+}
+
 // The workspace of the pair kernels (packed states, then 2 N doubles), kept
 // for the handle's life: an allocation and a release cost each call up to 0.1
 // ms, depending on what else the process had allocated.
@@ -362,6 +397,12 @@ void free_all(sdca_handle *h)
     h->allocs.clear();
     if (h->sd_h) cudaFreeHost(h->sd_h);
     if (h->list_h) cudaFreeHost(h->list_h);
+    if (h->out_h) {   // (the dual form's mirrors lie in it)
+        cudaFreeHost(h->out_h);
+        h->out_h = nullptr;
+        h->acc_h = nullptr;
+        h->sum_h = nullptr;
+    }
     if (h->acc_h) cudaFreeHost(h->acc_h);
     if (h->dots_h) cudaFreeHost(h->dots_h);
     if (h->rows_h) cudaFreeHost(h->rows_h);
@@ -1537,8 +1578,9 @@ int dual_ws_rows(sdca_handle *h, int nW, const int32_t *l_W)
 // accept and gradient, history-dot and control kernels, the summary
 // copy and the event `ev`, then the directions.  dev: every grid covers
 // Bmax slots and the kernels read the list lengths from device memory -- the
-// form captured in a CUDA graph and replayed every round, its classes timed
-// by event nodes into `g`; otherwise the grids are the host's list lengths
+// form captured in a CUDA graph and replayed every round, its kernels timed
+// by their own stamps (sixteen event nodes took 46 us of a replay); otherwise
+// the grids are the host's list lengths
 // and the classes are timed as usual.
 int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev, DualGraph *g)
 {
@@ -1549,22 +1591,17 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
     const int *cnt = h->dlist + 4 * (size_t)B;
     auto len = [&](int i) { return dev ? B : (int)n[i]; };
     auto dcnt = [&](int i) -> const int * { return dev ? cnt + i : nullptr; };
-    // one profile class: Timed, or an event pair recorded by the graph
-    auto region = [&](int cls, int kernels, int cidx, auto &&fn) -> int {
+    unsigned long long *const ts = dev ? h->ts + (g - h->dgraph) * TS_WORDS : nullptr;
+    unsigned long long *const ts_other = dev ? h->ts + (1 - (g - h->dgraph)) * TS_WORDS : nullptr;
+    // one kernel of a profile class: timed by events, or by its own stamps
+    auto region = [&](int cls, int stamp, int cidx, auto &&fn) -> int {
         if (!dev) {
             if (n[cidx] <= 0) return SDCA_OK;
-            Timed t(h, cls, kernels, n[cidx]);
-            return fn();
+            Timed t(h, cls, 1, n[cidx]);
+            return fn(nullptr);
         }
-        const size_t k = 2 * g->recs.size();
-        if (k + 1 >= g->ev.size()) return fn();   // (no event pair left: untimed)
-        GraphRec r{cls, kernels, cidx, g->ev[k], g->ev[k + 1]};
-        // (external: event nodes that record the event at every replay)
-        CK(cudaEventRecordWithFlags(r.a, h->stream, cudaEventRecordExternal));
-        const int rc = fn();
-        CK(cudaEventRecordWithFlags(r.b, h->stream, cudaEventRecordExternal));
-        g->recs.push_back(r);
-        return rc;
+        g->recs.push_back(GraphRec{cls, 1, cidx, stamp});
+        return fn(ts + 2 * stamp);
     };
     int rc;
     // Profile classes of this form: "forward" is K rho (a coefficient vector's
@@ -1572,72 +1609,64 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
     // contractions X^T a (max-norm checks, final J), "accept" the iterate
     // update and gradient assembly, "other" the control kernel and the
     // learned starts.
-    if ((rc = region(SDCA_K_LINESEARCH, 1, DC_T, [&] {
+    if ((rc = region(SDCA_K_LINESEARCH, TS_LINESEARCH, DC_T, [&](unsigned long long *t) {
              launch_dual_linesearch(P, h->ctl, l_T, len(DC_T), h->dacc, h->dv, h->ud, h->rstate,
-                                    h->wf, h->P0, h->R, h->acc, h->stream, dcnt(DC_T));
+                                    h->wf, h->P0, h->R, h->acc, h->stream, dcnt(DC_T), t);
              return SDCA_OK;
          })))
         return rc;
     CKL();
-    if (dev || n[DC_GW] > 0) {
-        CK(cudaMemsetAsync(h->csum, 0, sizeof(long long) * CSUM * P.Bmax, h->stream));
-        CK(cudaMemsetAsync(h->amax, 0, sizeof(double) * 2 * P.Bmax, h->stream));
-        CK(cudaMemsetAsync(h->dots, 0, sizeof(double) * 4 * MAXHIST * P.Bmax, h->stream));
-    }
-    if ((rc = region(SDCA_K_ACCEPT, 1, DC_GW, [&] {
-             launch_dual_quant(P, h->sd, l_G, len(DC_GW), h->R, h->rstate, h->qscale, h->rq, h->csum, h->stream,
-                               dcnt(DC_GW));
+    // class sums, maxima, history dots and (read by the search above) the direction sums
+    CK(cudaMemsetAsync(h->zero, 0, h->zero_bytes, h->stream));
+    if ((rc = region(SDCA_K_ACCEPT, TS_QUANT, DC_GW, [&](unsigned long long *t) {
+             launch_dual_quant(P, h->sd, l_G, len(DC_GW), h->R, h->rstate, h->qscale, h->rq, h->csum,
+                               h->kd ? h->Rd : nullptr, h->stream, dcnt(DC_GW), t);
              return SDCA_OK;
          })))
         return rc;
-    if ((rc = region(SDCA_K_FORWARD, h->kd ? 2 : 1, DC_GW, [&] {
+    if ((rc = region(SDCA_K_FORWARD, TS_KRHO, DC_GW, [&](unsigned long long *t) {
              if (h->kd)
-                 CK(tc_launch_kdig(h->kd, P, l_G, len(DC_GW), h->rq, h->rstate, h->csum, 1.0 / h->qscale, h->Rd,
-                                   h->KR, h->tc_err, h->stream, dcnt(DC_GW)));
+                 CK(tc_launch_kdig(h->kd, P, l_G, len(DC_GW), h->rstate, h->csum, 1.0 / h->qscale, h->KR, h->tc_err,
+                                   h->stream, dcnt(DC_GW), t));
              else
                  launch_dual_kprod(P, l_G, len(DC_GW), h->rstate, h->Kmat, h->qscale, h->rq, h->csum, h->KR,
-                                   h->stream, dcnt(DC_GW));
+                                   h->stream, dcnt(DC_GW), t);
              return SDCA_OK;
          })))
         return rc;
     if (!dev || h->ws_dual) {
         // the learned start: a_x = -rho^ / (2 lambda_J), K a_x exactly from the pass above
-        if ((rc = region(SDCA_K_OTHER, 1, DC_W, [&] {
+        if ((rc = region(SDCA_K_OTHER, TS_START, DC_W, [&](unsigned long long *t) {
                  launch_dual_ws_init(P, l_W, len(DC_W), -0.5 / P.lambda_J, h->qscale, h->rq, h->KR, h->dv,
-                                     h->stream, dcnt(DC_W));
+                                     h->stream, dcnt(DC_W), t);
                  return SDCA_OK;
              })))
             return rc;
     }
-    if ((rc = region(SDCA_K_ACCEPT, 1, DC_G, [&] {
+    if ((rc = region(SDCA_K_ACCEPT, TS_GRAD, DC_G, [&](unsigned long long *t) {
              launch_dual_grad(P, h->ctl, l_G, len(DC_G), h->qscale, h->rq, h->KR, h->dv, h->acc, h->amax, h->stream,
-                              dcnt(DC_G));
+                              dcnt(DC_G), t);
              return SDCA_OK;
          })))
         return rc;
-    if ((rc = region(SDCA_K_HISTORY, 1, DC_G, [&] {
-             launch_dual_dots(P, h->ctl, l_G, len(DC_G), 1, h->dv, h->dots, h->stream, dcnt(DC_G));
+    if ((rc = region(SDCA_K_HISTORY, TS_DOTS, DC_G, [&](unsigned long long *t) {
+             launch_dual_dots(P, h->ctl, l_G, len(DC_G), 1, h->dv, h->dots, h->stream, dcnt(DC_G), t);
              return SDCA_OK;
          })))
         return rc;
-    if ((rc = region(SDCA_K_OTHER, 1, DC_G, [&] {
+    if ((rc = region(SDCA_K_OTHER, TS_CONTROL, DC_G, [&](unsigned long long *t) {
              launch_dual_control(P, h->ctl, h->sum, l_G, len(DC_G), h->cfg.max_iterations, gtol, h->acc, h->amax,
-                                 h->dots, h->stream, dcnt(DC_G));
+                                 h->dots, h->stream, dcnt(DC_G), t);
              return SDCA_OK;
          })))
         return rc;
     CKL();
-    CK(cudaMemcpyAsync(h->sum_h, h->sum, sizeof(DualSum) * P.Bmax, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(h->acc_h, h->acc, sizeof(double) * NACC * P.Bmax, cudaMemcpyDeviceToHost, h->stream));
-    if (h->tc_err) CK(cudaMemcpyAsync(h->flag_h + 1, h->tc_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    if (h->ws_err && (dev ? h->ws_dual : n[DC_W] > 0))
-        CK(cudaMemcpyAsync(h->flag_h + 2, h->ws_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaMemcpyAsync(h->out_h, h->out, h->out_bytes, cudaMemcpyDeviceToHost, h->stream));
     if (dev) CK(cudaEventRecordWithFlags(ev, h->stream, cudaEventRecordExternal));
     else CK(cudaEventRecord(ev, h->stream));
-    if (dev || n[DC_G] > 0) CK(cudaMemsetAsync(h->dacc, 0, sizeof(double) * NDACC * P.Bmax, h->stream));
-    if ((rc = region(SDCA_K_DIRECTION, 1, DC_G, [&] {
+    if ((rc = region(SDCA_K_DIRECTION, TS_DIRECTION, DC_G, [&](unsigned long long *t) {
              launch_dual_direction(P, h->ctl, l_G, len(DC_G), h->dv, h->P0, h->wf, h->rstate, h->ud, h->dacc,
-                                   h->stream, dcnt(DC_G));
+                                   h->stream, dcnt(DC_G), t, ts_other);
              return SDCA_OK;
          })))
         return rc;
@@ -1650,11 +1679,7 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
 int dual_graph_build(sdca_handle *h, DualGraph &g)
 {
     if (!g.ev_round) CK(cudaEventCreateWithFlags(&g.ev_round, cudaEventDisableTiming));
-    while (g.ev.size() < 24) {
-        cudaEvent_t e;
-        CK(cudaEventCreate(&e));
-        g.ev.push_back(e);
-    }
+    CK(cudaMemsetAsync(h->ts + (&g - h->dgraph) * TS_WORDS, 0, sizeof(unsigned long long) * TS_WORDS, h->stream));
     g.recs.clear();
     const int64_t any[DC_N] = {1, 1, 1, 1};
     cudaGraph_t graph = nullptr;
@@ -1678,17 +1703,16 @@ int dual_graph_build(sdca_handle *h, DualGraph &g)
 }
 
 // A completed replay's class timings into the profile (units: the list
-// lengths of that replay).
+// lengths of that replay), from its stamps as the host has them.
 void dual_graph_collect(sdca_handle *h, DualGraph &g)
 {
     if (!g.pending) return;
+    const unsigned long long *ts = h->ts_h + (&g - h->dgraph) * TS_WORDS;
     for (const GraphRec &r : g.recs) {
-        float ms = 0.f;
-        if (cudaEventElapsedTime(&ms, r.a, r.b) == cudaSuccess) {
-            h->prof.kernel_ms[r.cls] += ms;
-            h->prof.kernel_launches[r.cls] += r.kernels;
-            h->prof.kernel_units[r.cls] += g.counts[r.cidx];
-        }
+        const unsigned long long begin = ~ts[2 * r.stamp], end = ts[2 * r.stamp + 1];
+        if (ts[2 * r.stamp] != 0ull && end > begin) h->prof.kernel_ms[r.cls] += 1e-6 * (double)(end - begin);
+        h->prof.kernel_launches[r.cls] += r.kernels;
+        h->prof.kernel_units[r.cls] += g.counts[r.cidx];
         h->prof.gpu_launches += r.kernels;
     }
     g.pending = false;
@@ -1711,8 +1735,6 @@ void dual_graph_free(sdca_handle *h)
 {
     dual_graph_reset(h);
     for (DualGraph &g : h->dgraph) {
-        for (cudaEvent_t e : g.ev) cudaEventDestroy(e);
-        g.ev.clear();
         if (g.ev_round) cudaEventDestroy(g.ev_round);
         g.ev_round = nullptr;
     }
@@ -1758,9 +1780,13 @@ int dual_round(sdca_handle *h, Queue &Qu)
             if (h->slots[b].phase == PH_INIT)
                 for (int a = 0; a < Q; ++a) h->sd_h[b].eta[a] = 0.0;
         }
-        int rc = staged_h2d(h, h->sd, h->sd_h, sizeof(SlotDev) * P.Bmax);
-        if (rc) return rc;
-        if ((rc = staged_h2d(h, h->dlist, all.data(), sizeof(int32_t) * all.size()))) return rc;
+        // (between admissions and retirements the same slots iterate)
+        int rc;
+        if ((!ef.empty() || !W.empty()) && (rc = staged_h2d(h, h->sd, h->sd_h, sizeof(SlotDev) * P.Bmax))) return rc;
+        if (all != h->dlist_sent) {
+            if ((rc = staged_h2d(h, h->dlist, all.data(), sizeof(int32_t) * all.size()))) return rc;
+            h->dlist_sent.swap(all);
+        }
     }
     int rc;
     if (!W.empty() && (rc = dual_ws_rows(h, (int)W.size(), l_W))) return rc;
@@ -1794,9 +1820,9 @@ int dual_round(sdca_handle *h, Queue &Qu)
     if (other) dual_graph_collect(h, *other);
     // every staged host-to-device copy was queued before the event
     h->stage_off = 0;
-    if (h->tc_err && h->flag_h[1])
+    if (h->errs_h[0])
         return fail(h, SDCA_E_CUDA, "tensor-core pipeline wait timed out (kernel abandoned its tile)");
-    if (!W.empty() && h->flag_h[2])
+    if (!W.empty() && h->errs_h[1])
         return fail(h, SDCA_E_CUDA, "warm start: a tensor-core pipeline wait gave up");
     if (Qu.scores) dual_flush_rows(h, Qu);
 
@@ -1894,7 +1920,12 @@ int solve_lane(sdca_handle *h, Queue &Qu, cudaEvent_t t0_common)
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, t0, t1));
     h->prof.solve_ms = ms;
-    for (DualGraph &g : h->dgraph) dual_graph_collect(h, g);
+    if (h->dgraph[0].pending || h->dgraph[1].pending) {
+        // the last replay's stamps, the directions' included
+        CK(cudaMemcpyAsync(h->ts_h, h->ts, sizeof(unsigned long long) * 2 * TS_WORDS, cudaMemcpyDeviceToHost, h->stream));
+        { const int r_ = stream_sync(h); if (r_) return r_; }
+        for (DualGraph &g : h->dgraph) dual_graph_collect(h, g);
+    }
     prof_collect(h);
     return SDCA_OK;
 }
@@ -2151,21 +2182,20 @@ static int create_lane(const sdca_config *cfg, const sdca_handle *owner, sdca_ha
         (rc = dalloc(h, &h->R, B * P.Nx * 4)) || (rc = dalloc(h, &h->lbase, B * P.Nx * 4)) ||
         (rc = dalloc(h, &h->partial, (size_t)P.C * B * P.Nx * 4)) ||
         (rc = dalloc(h, &h->partial64, (size_t)P.Cg * B * P.Nx * 4)) ||
-        (rc = dalloc(h, &h->rows, B * P.L)) || (rc = dalloc(h, &h->acc, B * NACC)) ||
-        (rc = dalloc(h, &h->dots, B * 4 * MAXHIST)) || (rc = dalloc(h, &h->sd, B)) ||
+        (rc = dalloc(h, &h->rows, B * P.L)) || (!dual && (rc = dalloc(h, &h->acc, B * NACC))) ||
+        (!dual && (rc = dalloc(h, &h->dots, B * 4 * MAXHIST))) || (rc = dalloc(h, &h->sd, B)) ||
         (rc = dalloc(h, &h->list, B)) || (rc = dalloc(h, &h->flag, 4)) ||
         (rc = dalloc(h, reinterpret_cast<uint8_t **>(&h->Spool), hist_bytes)) ||
         (rc = dalloc(h, reinterpret_cast<uint8_t **>(&h->Ypool), hist_bytes)) ||
         (rc = halloc(h, &h->sd_h, B)) || (rc = halloc(h, &h->list_h, B)) ||
-        (rc = halloc(h, &h->acc_h, B * NACC)) || (rc = halloc(h, &h->dots_h, B * 4 * MAXHIST)) ||
+        (!dual && (rc = halloc(h, &h->acc_h, B * NACC))) || (rc = halloc(h, &h->dots_h, B * 4 * MAXHIST)) ||
         (rc = halloc(h, &h->rows_h, B * P.L)) || (rc = halloc(h, &h->flag_h, 4)) ||
         (rc = halloc(h, &h->stage, (h->stage_cap = 64 * (((sizeof(SlotDev) + 4) * B + 1024 + 255) & ~(size_t)255)))) ||
-        (dual && ((rc = halloc(h, &h->amax_h, 2 * B)) || (rc = halloc(h, &h->sum_h, B)) ||
-                  (rc = dalloc(h, &h->ctl, B)) || (rc = dalloc(h, &h->sum, B)) ||
-                  (rc = dalloc(h, &h->dacc, B * NDACC)) || (rc = dalloc(h, &h->dlist, 4 * B + DC_N)) ||
+        (dual && ((rc = halloc(h, &h->amax_h, 2 * B)) || (rc = dual_blocks(h)) ||
+                  (rc = dalloc(h, &h->ctl, B)) || (rc = dalloc(h, &h->dlist, 4 * B + DC_N)) ||
                   (rc = dalloc(h, &h->dv, B * NV * 2 * P.Nx * 4)) ||
-                  (rc = dalloc(h, &h->KR, B * P.Nx * 4)) || (rc = dalloc(h, &h->amax, 2 * B)) ||
-                  (rc = dalloc(h, &h->rq, B * P.Nx * 4)) || (rc = dalloc(h, &h->csum, CSUM * B)) ||
+                  (rc = dalloc(h, &h->KR, B * P.Nx * 4)) ||
+                  (rc = dalloc(h, &h->rq, B * P.Nx * 4)) ||
                   (rc = dalloc(h, &h->Rchk, B * P.Nx * 4)) || (dual_small && (rc = dalloc(h, &h->J64, B * P.Dp))) ||
                   (rc = dalloc(h, &h->P0, B * P.Nx * 4)) || (rc = dalloc(h, &h->ud, B * P.Nx * 4)) ||
                   (!shared && (rc = dalloc(h, &h->Kmat, (size_t)P.Nx * P.Nx))) ||
@@ -2176,7 +2206,7 @@ static int create_lane(const sdca_config *cfg, const sdca_handle *owner, sdca_ha
          ((!dual && (rc = dalloc(h, &h->Dhi, 4 * B * (size_t)round_up(4 * P.L, 64)))) ||
           (!dual && (rc = dalloc(h, &h->Dlo, 4 * B * (size_t)round_up(4 * P.L, 64)))) ||
           (rc = dalloc(h, &h->Rhi, 4 * B * (size_t)P.Nx)) || (rc = dalloc(h, &h->Rlo, 4 * B * (size_t)P.Nx)) ||
-          (rc = dalloc(h, &h->tc_err, 4))))) {
+          (!dual && (rc = dalloc(h, &h->tc_err, 4)))))) {
         std::string msg = h->err;
         free_all(h);
         if (h->own_stream) cudaStreamDestroy(h->stream);

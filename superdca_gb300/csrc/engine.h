@@ -160,6 +160,11 @@ enum DualAcc {
 // of columns 0..2 over all sequences
 constexpr int CSUM = 20, CSUM_ALL = 16;
 
+// time stamps of a replay of the dual form's iteration core: a begin and an
+// end word per kernel (stamp_begin, stamp_end)
+enum { TS_LINESEARCH = 0, TS_QUANT, TS_KRHO, TS_START, TS_GRAD, TS_DOTS, TS_CONTROL, TS_DIRECTION, TS_KERNELS };
+constexpr int TS_WORDS = 2 * TS_KERNELS;
+
 enum SlotFlags {
     SLOT_F_USE_U = 1,       // trial logits use lbase + stp u (else lbase)
     SLOT_F_PUSH = 2,        // accept pushes an (s, y) pair into the history
@@ -225,19 +230,20 @@ void launch_score(const Problem &P, const SlotDev *sd, const int32_t *list, int 
 
 // dual form (kernels_dual.cu)
 void launch_dual_quant(const Problem &P, const SlotDev *sd, const int32_t *list, int n, const float *R,
-                       const uint8_t *rstate, double qscale, int32_t *rq, long long *csum, cudaStream_t st, const int *cnt = nullptr);
+                       const uint8_t *rstate, double qscale, int32_t *rq, long long *csum, __half *Rd, cudaStream_t st,
+                       const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_kprod(const Problem &P, const int32_t *list, int n, const uint8_t *rstate, const int32_t *K,
-                       double qscale, const int32_t *rq, const long long *csum, float2 *KR, cudaStream_t st, const int *cnt = nullptr);
+                       double qscale, const int32_t *rq, const long long *csum, float2 *KR, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 // the accept (x += stp d, s push, logits += stp u) of the slots that searched
 // this round, then the gradient at the new point (y push, sums)
 void launch_dual_grad(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, double qscale,
                       const int32_t *rq, const float2 *KR, float2 *dv, double *acc, double *amax, cudaStream_t st,
-                      const int *cnt = nullptr);
+                      const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_dots(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, int newg, const float2 *dv,
-                      double *dots, cudaStream_t st, const int *cnt = nullptr);
+                      double *dots, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_direction(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, float2 *dv,
                            float *P0, const float *w, const uint8_t *rstate, float *ud, double *dacc,
-                           cudaStream_t st, const int *cnt = nullptr);
+                           cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr, unsigned long long *ts_clear = nullptr);
 // start and final evaluations of the dual form (logits k_x + eta, FP64 log-sum-exp)
 void launch_dual_eval(const Problem &P, const SlotDev *sd, const int32_t *list, int n, const float2 *dv,
                       const uint8_t *rstate, const double *w, float *R, double *acc, cudaStream_t st);
@@ -246,10 +252,10 @@ void launch_dual_to_r(const Problem &P, const DualCtl *ctl, const int32_t *list,
 // the per-iteration decisions of the dual form on the device
 void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list, int n, const double *dacc,
                             float2 *dv, float *ud, const uint8_t *rstate,
-                            const float *w, const float *P0, float *R, double *acc, cudaStream_t st, const int *cnt = nullptr);
+                            const float *w, const float *P0, float *R, double *acc, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_control(const Problem &P, DualCtl *ctl, DualSum *sum, const int32_t *list, int n,
                          int max_iterations, double gtol, const double *acc, const double *amax, const double *dots,
-                         cudaStream_t st, const int *cnt = nullptr);
+                         cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_check_apply(DualCtl *ctl, DualSum *sum, const int32_t *list, int n, double gtol, const double *acc,
                              cudaStream_t st);
 void launch_dual_digits(const Problem &P, const SlotDev *sd, const int32_t *list, int n, int d, const float2 *dv,
@@ -286,7 +292,7 @@ void launch_dual_ws_feats(const uint8_t *cols, const int32_t *idx, int n, int N,
 void launch_dual_ws_r(const int32_t *slots, int n, int N, int64_t Nx, const float *out, const float *p_dev, float alpha,
                       const float *w, float *R, cudaStream_t st);
 void launch_dual_ws_init(const Problem &P, const int32_t *list, int n, double c, double qscale, const int32_t *rq,
-                         const float2 *KR, float2 *dv, cudaStream_t st, const int *cnt = nullptr);
+                         const float2 *KR, float2 *dv, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_ws_residual(const uint8_t *XT, int64_t Nx, int N, const int32_t *loci, int G, const double *w,
                         const int32_t *knn, int k, float eps, float *Rws, cudaStream_t st);
 void launch_ws_residual_split(const uint8_t *XT, int64_t Nx, int N, const int32_t *loci, const int32_t *slots, int G,
@@ -334,8 +340,8 @@ int kd_nr_rows(const Problem &P);
 KdPlan *tc_kdig_plan_create(const Problem &P, __half *Kd, __half *Rd);
 void tc_kdig_plan_destroy(KdPlan *p);
 void tc_kdig_fill_k(const KdPlan *pl, const Problem &P, const int32_t *K, __half *Kd, cudaStream_t st);
-cudaError_t tc_launch_kdig(const KdPlan *pl, const Problem &P, const int32_t *list, int n, const int32_t *rq,
-                           const uint8_t *rstate, const long long *csum, double inv_qscale, __half *Rd, float2 *KR,
-                           int *err, cudaStream_t st, const int *cnt = nullptr);
+cudaError_t tc_launch_kdig(const KdPlan *pl, const Problem &P, const int32_t *list, int n, const uint8_t *rstate,
+                           const long long *csum, double inv_qscale, float2 *KR, int *err, cudaStream_t st,
+                           const int *cnt = nullptr, unsigned long long *ts = nullptr);
 
 } // namespace sdca

@@ -126,6 +126,27 @@ __device__ __forceinline__ float dot4(float4 a, float4 b)
     return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
 }
 
+// Time stamps of a kernel in a replayed graph (ts null: none): ts[0] the
+// complement of its earliest start, ts[1] its latest end, nanoseconds, both
+// kept by maxima over the blocks that stamp (zero before).  Event nodes do the
+// same from outside, at some 3 us of the replay each.
+__device__ __forceinline__ unsigned long long global_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ void stamp_begin(unsigned long long *ts)
+{
+    if (ts && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) atomicMax(ts, ~global_ns());
+}
+
+__device__ __forceinline__ void stamp_end(unsigned long long *ts, bool mine)
+{
+    if (ts && threadIdx.x == 0 && mine) atomicMax(ts + 1, global_ns());
+}
+
 struct GradRed {
     float gmax = 0.f, g2 = 0.f, x2 = 0.f, sy = 0.f, yy = 0.f, ss = 0.f;
 };

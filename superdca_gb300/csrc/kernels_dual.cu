@@ -25,6 +25,7 @@
 
 #include "df.cuh"
 #include "engine.h"
+#include "kdig.cuh"
 #include "kernels_common.cuh"
 #include "linesearch.h"
 
@@ -36,13 +37,16 @@ namespace {
 // entry at the sequence's own state set to minus the sum of the other three,
 // so that every row sums to zero exactly (a residual w (p - onehot) does; the
 // K rho product then needs three columns); class sums csum[b][a][c] = sum
-// over i with s_i(r) = a, and the sums over all i (CSUM_ALL)
+// over i with s_i(r) = a, and the sums over all i (CSUM_ALL); the digits of
+// the tensor-core product into Rd when given (list position blockIdx.y)
 __global__ void __launch_bounds__(256)
 k_dual_quant(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N, int64_t Nx,
              const float4 *__restrict__ R, const uint8_t *__restrict__ rstate, float qscale, int4 *__restrict__ rq,
-             unsigned long long *__restrict__ csum, const int *__restrict__ cnt)
+             unsigned long long *__restrict__ csum, __half *__restrict__ Rd, const int *__restrict__ cnt,
+             unsigned long long *__restrict__ ts)
 {
     if (cnt && (int)blockIdx.y >= *cnt) return;
+    stamp_begin(ts);
     const int b = list[blockIdx.y];
     const bool own = sd[b].locus >= 0;   // scan mode: no own-agreement correction
     __shared__ unsigned long long red[CSUM];
@@ -69,6 +73,7 @@ k_dual_quant(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, i
             cs[4][0] += q.x; cs[4][1] += q.y; cs[4][2] += q.z;
         }
         rq[(int64_t)b * Nx + i] = q;
+        if (Rd) kd_digits((int)blockIdx.y, i, Nx, q, Rd);
     }
 #pragma unroll
     for (int a = 0; a < 5; ++a)
@@ -81,6 +86,7 @@ k_dual_quant(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, i
     __syncthreads();
     if (threadIdx.x < CSUM && red[threadIdx.x] != 0ull)
         atomicAdd(csum + (int64_t)b * CSUM + threadIdx.x, red[threadIdx.x]);
+    stamp_end(ts, blockIdx.x == gridDim.x - 1);
 }
 
 constexpr int KP_M = 64;   // rows (sequences i) per CTA
@@ -91,8 +97,9 @@ constexpr int KP_J = 16;   // sequences j per shared-memory stage
 __global__ void __launch_bounds__(256)
 k_dual_kprod(const int32_t *__restrict__ K, int64_t Nx, int N, const int32_t *__restrict__ list, int nlist,
              const int4 *__restrict__ rq, const long long *__restrict__ csum, const uint8_t *__restrict__ rstate,
-             double inv_qscale, float2 *__restrict__ KR, const int *__restrict__ cnt)
+             double inv_qscale, float2 *__restrict__ KR, const int *__restrict__ cnt, unsigned long long *__restrict__ ts)
 {
+    stamp_begin(ts);
     if (cnt) {
         nlist = *cnt;
         if ((int)blockIdx.y * KP_S >= nlist) return;
@@ -143,6 +150,7 @@ k_dual_kprod(const int32_t *__restrict__ K, int64_t Nx, int N, const int32_t *__
 #pragma unroll
         for (int c = 0; c < 4; ++c) o[c] = df_mul(df_from_ll(acc[a][c] - cs[c]), iq);
     }
+    stamp_end(ts, true);
 }
 
 __device__ __forceinline__ int64_t dvo(int64_t b, int v, int part, int NV, int64_t Nx)
@@ -178,9 +186,10 @@ __global__ void __launch_bounds__(256)
 k_dual_grad(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, int64_t Nx, int NV, int ring,
             float2 l2, const int32_t *__restrict__ rq, float2 iq, const float2 *__restrict__ KR,
             float2 *__restrict__ dv, double *__restrict__ acc, double *__restrict__ amax,
-            const int *__restrict__ cnt)
+            const int *__restrict__ cnt, unsigned long long *__restrict__ ts)
 {
     if (cnt && (int)blockIdx.y >= *cnt) return;
+    stamp_begin(ts);
     const int b = list[blockIdx.y];
     const DualCtl &S = ctl[b];
     if (S.phase == DC_STOP) return;
@@ -275,6 +284,7 @@ k_dual_grad(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
         if (mg > 0.f) atomic_max_nonneg(amax + 2 * b, (double)mg);
         if (mx > 0.f) atomic_max_nonneg(amax + 2 * b + 1, (double)mx);
     }
+    stamp_end(ts, blockIdx.x == gridDim.x - 1);
 }
 
 // J-part dots of the live history pairs (and the pair the last accept
@@ -301,9 +311,11 @@ constexpr int DOT_MAX_K = MAXHIST + 1;            // the live history and the pu
 
 __global__ void __launch_bounds__(DOT_THREADS, 4)
 k_dual_dots(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, int64_t Nx, int NV, int ring,
-            int newg, const float2 *__restrict__ dv, double *__restrict__ dots, const int *__restrict__ cnt)
+            int newg, const float2 *__restrict__ dv, double *__restrict__ dots, const int *__restrict__ cnt,
+            unsigned long long *__restrict__ ts)
 {
     if (cnt && (int)blockIdx.y >= *cnt) return;
+    stamp_begin(ts);
     const int b = list[blockIdx.y];
     const DualCtl &S = ctl[b];
     if (S.phase == DC_STOP) return;
@@ -342,6 +354,7 @@ k_dual_dots(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
         if (lane == 0 && (sum.x != 0.f || sum.y != 0.f))
             atomicAdd(dots + (int64_t)b * 4 * MAXHIST + (isy ? DOT_Y : 0) + pos, df_to_d(sum));
     }
+    stamp_end(ts, blockIdx.x == gridDim.x - 1);
 }
 
 // A step trial of one sequence with a large step (|t| >= 30), from its
@@ -442,9 +455,13 @@ __global__ void __launch_bounds__(DIR_THREADS, 5)
 k_dual_direction(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, int64_t Nx, int N, int NV,
                  int ring, float2 *__restrict__ dv, float *__restrict__ P0, const float *__restrict__ w,
                  const uint8_t *__restrict__ rstate, float *__restrict__ ud, double *__restrict__ dacc,
-                 const int *__restrict__ cnt)
+                 const int *__restrict__ cnt, unsigned long long *__restrict__ ts,
+                 unsigned long long *__restrict__ ts_clear)
 {
+    // (the stamps of the replay before have been copied: zero for the next)
+    if (ts_clear && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < TS_WORDS) ts_clear[threadIdx.x] = 0ull;
     if (cnt && (int)blockIdx.y >= *cnt) return;
+    stamp_begin(ts);
     const int b = list[blockIdx.y];
     const DualCtl &S = ctl[b];
     if (S.phase == DC_STOP) return;
@@ -556,6 +573,7 @@ k_dual_direction(const DualCtl *__restrict__ ctl, const int32_t *__restrict__ li
     float2 v[4] = {gd, dd, xd, dg0};
     const int idx[4] = {DA_GD, DA_DDJ, DA_XDJ, DA_DG0};
     block_sum_df<4>(v, dacc + (int64_t)b * NDACC, idx);
+    stamp_end(ts, blockIdx.x == gridDim.x - 1);
 }
 
 // FP32 copy of a vector's a part (the current gradient, or x) as the R rows
@@ -818,9 +836,11 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
                   double lambda_J, double lambda_h, const double *__restrict__ dacc, float2 *__restrict__ dv,
                   float4 *__restrict__ ud,
                   const uint8_t *__restrict__ rstate, const float *__restrict__ w, const float4 *__restrict__ P0,
-                  float4 *__restrict__ R, double *__restrict__ acc, const int *__restrict__ cnt)
+                  float4 *__restrict__ R, double *__restrict__ acc, const int *__restrict__ cnt,
+                  unsigned long long *__restrict__ ts)
 {
     if (cnt && (int)blockIdx.x >= *cnt) return;
+    stamp_begin(ts);
     const int b = list[blockIdx.x];
     DualCtl &S = ctl[b];
     if (S.phase != DC_STEP) return;   // (the same for the whole block)
@@ -1033,6 +1053,7 @@ k_dual_linesearch(DualCtl *__restrict__ ctl, const int32_t *__restrict__ list, i
             }
         }
     }
+    stamp_end(ts, true);
 }
 
 constexpr int CTL_WORDS = (int)(sizeof(DualCtl) / 8);
@@ -1121,9 +1142,11 @@ __device__ __forceinline__ bool warp_compact_coeffs(int k, const double *R, cons
 __global__ void __launch_bounds__(32)
 k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32_t *__restrict__ list, int m,
                int max_iterations, double gtol, double lambda_J, double lambda_h, const double *__restrict__ acc,
-               const double *__restrict__ amax, const double *__restrict__ dots, const int *__restrict__ cnt)
+               const double *__restrict__ amax, const double *__restrict__ dots, const int *__restrict__ cnt,
+               unsigned long long *__restrict__ ts)
 {
     if (cnt && (int)blockIdx.x >= *cnt) return;
+    stamp_begin(ts);
     const int b = list[blockIdx.x];
     __shared__ DualCtl S;
     __shared__ double s_eg[Q], s_dt[2 * MAXHIST], s_R[MAXHIST * MAXHIST], s_YY[MAXHIST * MAXHIST];
@@ -1336,6 +1359,7 @@ k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32
         for (int k = threadIdx.x; k < CTL_WORDS; k += 32) dst[k] = src[k];
     }
     if (threadIdx.x == 0) write_summary(S, sum[b]);
+    stamp_end(ts, true);
 }
 
 // After an exact max-norm check (the tensor-core backward X^T a_g with its
@@ -1378,9 +1402,10 @@ __global__ void k_dual_check_apply(DualCtl *__restrict__ ctl, DualSum *__restric
 __global__ void __launch_bounds__(256)
 k_dual_ws_init(const int32_t *__restrict__ list, int64_t Nx, int NV, double c, double inv_qscale,
                const int32_t *__restrict__ rq, const float2 *__restrict__ KR, float2 *__restrict__ dv,
-               const int *__restrict__ cnt)
+               const int *__restrict__ cnt, unsigned long long *__restrict__ ts)
 {
     if (cnt && (int)blockIdx.y >= *cnt) return;
+    stamp_begin(ts);
     const int b = list[blockIdx.y];
     const float2 cd = df_from_d(c), cq = df_from_d(c * inv_qscale);
     float2 *ax = dv + dvo(b, DV_X, 0, NV, Nx), *kx = ax + Nx * 4;
@@ -1390,6 +1415,7 @@ k_dual_ws_init(const int32_t *__restrict__ list, int64_t Nx, int NV, double c, d
         ax[e] = a;
         kx[e] = k;
     }
+    stamp_end(ts, blockIdx.x == gridDim.x - 1);
 }
 
 // The start and final evaluations of the dual form: objective terms, R rows
@@ -1448,40 +1474,44 @@ constexpr int STREAM_PASSES = 8;
 } // namespace
 
 void launch_dual_quant(const Problem &P, const SlotDev *sd, const int32_t *list, int n, const float *R,
-                       const uint8_t *rstate, double qscale, int32_t *rq, long long *csum, cudaStream_t st,
-                       const int *cnt)
+                       const uint8_t *rstate, double qscale, int32_t *rq, long long *csum, __half *Rd, cudaStream_t st,
+                       const int *cnt,
+                       unsigned long long *ts)
 {
     if (n <= 0) return;
     dim3 gq(grid_for(P.Nx, 256 * 4, 64), n);
     k_dual_quant<<<gq, 256, 0, st>>>(sd, list, (int)P.N, P.Nx, reinterpret_cast<const float4 *>(R), rstate,
                                      (float)qscale, reinterpret_cast<int4 *>(rq),
-                                     reinterpret_cast<unsigned long long *>(csum), cnt);
+                                     reinterpret_cast<unsigned long long *>(csum), Rd, cnt, ts);
 }
 
 // K rho on the CUDA cores (64-bit integer multiply-adds): any N
 void launch_dual_kprod(const Problem &P, const int32_t *list, int n, const uint8_t *rstate, const int32_t *K,
                        double qscale, const int32_t *rq, const long long *csum, float2 *KR, cudaStream_t st,
-                       const int *cnt)
+                       const int *cnt,
+                       unsigned long long *ts)
 {
     if (n <= 0) return;
     dim3 gk((unsigned)(P.Nx / KP_M), (unsigned)((n + KP_S - 1) / KP_S));
     k_dual_kprod<<<gk, 256, 0, st>>>(K, P.Nx, (int)P.N, list, n, reinterpret_cast<const int4 *>(rq), csum, rstate,
-                                     1.0 / qscale, KR, cnt);
+                                     1.0 / qscale, KR, cnt, ts);
 }
 
 void launch_dual_grad(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, double qscale,
                       const int32_t *rq, const float2 *KR, float2 *dv, double *acc, double *amax, cudaStream_t st,
-                      const int *cnt)
+                      const int *cnt,
+                       unsigned long long *ts)
 {
     if (n <= 0) return;
     const int NV = DV_S + 2 * P.ring;
     dim3 gg(grid_for(P.Nx * 2, 256 * STREAM_PASSES, 64), n);
     k_dual_grad<<<gg, 256, 0, st>>>(ctl, list, P.Nx, NV, P.ring, df_host(2.0 * P.lambda_J), rq, df_host(1.0 / qscale),
-                                    KR, dv, acc, amax, cnt);
+                                    KR, dv, acc, amax, cnt, ts);
 }
 
 void launch_dual_dots(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, int newg, const float2 *dv,
-                      double *dots, cudaStream_t st, const int *cnt)
+                      double *dots, cudaStream_t st, const int *cnt,
+                       unsigned long long *ts)
 {
     if (n <= 0) return;
     // few slots of few sequences leave the chip idle: share a slot's units out
@@ -1489,17 +1519,18 @@ void launch_dual_dots(const Problem &P, const DualCtl *ctl, const int32_t *list,
     const int64_t blocks = (P.Nx * 4 + DOT_CHUNK - 1) / DOT_CHUNK * n;
     const unsigned z = (unsigned)std::max<int64_t>(1, std::min<int64_t>(10, 8 * 152 / blocks));
     dim3 g((unsigned)((P.Nx * 4 + DOT_CHUNK - 1) / DOT_CHUNK), n, z);
-    k_dual_dots<<<g, DOT_THREADS, 0, st>>>(ctl, list, P.Nx, DV_S + 2 * P.ring, P.ring, newg, dv, dots, cnt);
+    k_dual_dots<<<g, DOT_THREADS, 0, st>>>(ctl, list, P.Nx, DV_S + 2 * P.ring, P.ring, newg, dv, dots, cnt, ts);
 }
 
 void launch_dual_direction(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, float2 *dv,
                            float *P0, const float *w, const uint8_t *rstate, float *ud, double *dacc,
-                           cudaStream_t st, const int *cnt)
+                           cudaStream_t st, const int *cnt, unsigned long long *ts,
+                           unsigned long long *ts_clear)
 {
     if (n <= 0) return;
     dim3 g((unsigned)((P.Nx * 2 + DIR_THREADS - 1) / DIR_THREADS), n);
     k_dual_direction<<<g, DIR_THREADS, 0, st>>>(ctl, list, P.Nx, (int)P.N, DV_S + 2 * P.ring, P.ring, dv, P0, w,
-                                                rstate, ud, dacc, cnt);
+                                                rstate, ud, dacc, cnt, ts, ts_clear);
 }
 
 void launch_dual_eval(const Problem &P, const SlotDev *sd, const int32_t *list, int n, const float2 *dv,
@@ -1513,11 +1544,12 @@ void launch_dual_eval(const Problem &P, const SlotDev *sd, const int32_t *list, 
 
 
 void launch_dual_ws_init(const Problem &P, const int32_t *list, int n, double c, double qscale, const int32_t *rq,
-                         const float2 *KR, float2 *dv, cudaStream_t st, const int *cnt)
+                         const float2 *KR, float2 *dv, cudaStream_t st, const int *cnt,
+                       unsigned long long *ts)
 {
     if (n <= 0) return;
     dim3 g(grid_for(P.Nx * 4, 256 * 4, 64), n);
-    k_dual_ws_init<<<g, 256, 0, st>>>(list, P.Nx, DV_S + 2 * P.ring, c, 1.0 / qscale, rq, KR, dv, cnt);
+    k_dual_ws_init<<<g, 256, 0, st>>>(list, P.Nx, DV_S + 2 * P.ring, c, 1.0 / qscale, rq, KR, dv, cnt, ts);
 }
 
 void launch_dual_to_r(const Problem &P, const DualCtl *ctl, const int32_t *list, int n, int which,
@@ -1573,7 +1605,8 @@ void launch_dual_to_wa(const Problem &P, const SlotDev *sd, const int32_t *list,
 
 void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list, int n, const double *dacc,
                             float2 *dv, float *ud, const uint8_t *rstate,
-                            const float *w, const float *P0, float *R, double *acc, cudaStream_t st, const int *cnt)
+                            const float *w, const float *P0, float *R, double *acc, cudaStream_t st, const int *cnt,
+                       unsigned long long *ts)
 {
     if (n <= 0) return;
     // Few slots: larger blocks, while every SM still holds its slots' blocks
@@ -1590,7 +1623,7 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
     k_dual_linesearch<T><<<n, T + 32, 0, st>>>(ctl, list, (int)P.N, P.Nx, DV_S + 2 * P.ring, P.lambda_J, P.lambda_h,   \
                                           dacc, dv, reinterpret_cast<float4 *>(ud), rstate, w,                    \
                                           reinterpret_cast<const float4 *>(P0), reinterpret_cast<float4 *>(R), acc, \
-                                          cnt)
+                                          cnt, ts)
     if (threads == 64) SDCA_LS_LAUNCH(64);
     else if (threads == 256) SDCA_LS_LAUNCH(256);
     else SDCA_LS_LAUNCH(128);
@@ -1599,11 +1632,12 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
 
 void launch_dual_control(const Problem &P, DualCtl *ctl, DualSum *sum, const int32_t *list, int n,
                          int max_iterations, double gtol, const double *acc, const double *amax, const double *dots,
-                         cudaStream_t st, const int *cnt)
+                         cudaStream_t st, const int *cnt,
+                       unsigned long long *ts)
 {
     if (n <= 0) return;
     k_dual_control<<<n, 32, 0, st>>>(ctl, sum, list, P.m, max_iterations, gtol, P.lambda_J, P.lambda_h, acc, amax,
-                                     dots, cnt);
+                                     dots, cnt, ts);
 }
 
 void launch_dual_check_apply(DualCtl *ctl, DualSum *sum, const int32_t *list, int n, double gtol, const double *acc,

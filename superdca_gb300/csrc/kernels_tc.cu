@@ -39,6 +39,7 @@
 
 #include "df.cuh"
 #include "engine.h"
+#include "kdig.cuh"
 #include "kernels_common.cuh"
 #include "tcgen05.cuh"
 
@@ -611,15 +612,9 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
 // single CTAs of 13 slots), tensor pipe 63 % active; 64 slots of 1000 x 4001:
 // 23 us (26).
 
-constexpr int KD_BM = 128, KD_BK = 64;
-constexpr int KD_KDIG = 3, KD_RDIG = 3;
-constexpr int KD_S = 17;                     // slots per tile
-constexpr int KD_C = 3;                      // product columns per slot (the fourth follows)
+constexpr int KD_BM = 128, KD_BK = 64;   // (the digits' layout: kdig.cuh)
 constexpr int KD_COLS = KD_S * KD_C;         // 51 live columns per plane
-constexpr int KD_PS = 52;                    // rows (accumulator columns) from one plane to the next
-constexpr int KD_NB = 160;                   // rho rows of a tile: accumulator columns per K digit
 constexpr int KD_SEG = 24;                   // k-steps per segment: 1536 sequences
-constexpr int KD_RBASE = 640, KD_RHALF = 320;
 constexpr int KD_A_BYTES = KD_BM * KD_BK * 2;             // one K digit plane tile, 16 KB
 constexpr int KD_B_BYTES = KD_NB / 2 * KD_BK * 2;         // this CTA's half of the rho rows, 10 KB
 constexpr int KD_STAGE = KD_KDIG * KD_A_BYTES + KD_B_BYTES;
@@ -664,6 +659,7 @@ struct KdArgs {
     float2 *KR;                  // K rho / qscale in double-float
     int *err;
     const int *ncount;           // list length in device memory (the grid covers the most slots), or null
+    unsigned long long *ts;      // time stamps, or null
 };
 
 struct KdEpilogue {
@@ -776,6 +772,7 @@ k_kdig(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensor
     const int tiles = m_pairs * ((nlist + KD_S - 1) / KD_S);
     const int tile0 = blockIdx.x >> 1, tstep = gridDim.x >> 1;
     if (tile0 >= tiles) return;   // (both CTAs of the pair, before any barrier or TMEM allocation)
+    stamp_begin(args.ts);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < KD_STG; ++s) {
@@ -870,6 +867,7 @@ k_kdig(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensor
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(KD_TMEM_COLS)
                      : "memory");
     }
+    stamp_end(args.ts, true);
 }
 
 // K (int32, Nx x Nx) less c -> three fp16 planes of balanced base-64 digits,
@@ -887,38 +885,6 @@ __global__ void k_kdig_split_k(const int32_t *__restrict__ K, int64_t Nx, int N,
         Kd[t] = __int2half_rn(d0);
         Kd[(int64_t)nk_rows * Nx + t] = __int2half_rn(d1);
         Kd[2 * (int64_t)nk_rows * Nx + t] = __int2half_rn((v - d1) >> 6);
-    }
-}
-
-// rho_q of list position P (slot list[P]), its first three columns -> fp16
-// balanced base-640 digits: plane p of column c in row 52 p + 3 (P % 17) + c
-// of tile P / 17
-__global__ void k_kdig_split_r(const int32_t *__restrict__ list, int64_t Nx, const int4 *__restrict__ rq,
-                               __half *__restrict__ Rd, const int *__restrict__ cnt)
-{
-    if (cnt && (int)blockIdx.y >= *cnt) return;
-    const int P = blockIdx.y, b = list[P];
-    const int64_t row0 = (int64_t)(P / KD_S) * KD_NB + (P % KD_S) * KD_C;
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < Nx; j += (int64_t)gridDim.x * blockDim.x) {
-        const int4 q = rq[(int64_t)b * Nx + j];
-        const int qq[KD_C] = {q.x, q.y, q.z};
-#pragma unroll
-        for (int c = 0; c < KD_C; ++c) {
-            int v = qq[c];
-#pragma unroll
-            for (int p = 0; p < KD_RDIG; ++p) {
-                int d = v;
-                if (p < KD_RDIG - 1) {
-                    // |v| < 2^28: shifted by a multiple of the base to be positive
-                    constexpr int UP = (1 << 28) / KD_RBASE;
-                    const unsigned t = (unsigned)(v + KD_RHALF) + (unsigned)(UP * KD_RBASE);
-                    const unsigned qt = t / KD_RBASE;
-                    d = (int)(t - qt * KD_RBASE) - KD_RHALF;
-                    v = (int)qt - UP;
-                }
-                Rd[(row0 + p * KD_PS + c) * Nx + j] = __int2half_rn(d);
-            }
-        }
     }
 }
 
@@ -1169,15 +1135,11 @@ void tc_kdig_fill_k(const KdPlan *pl, const Problem &P, const int32_t *K, __half
         K, P.Nx, (int)P.N, kd_center(P), pl->nk_rows, Kd);
 }
 
-cudaError_t tc_launch_kdig(const KdPlan *pl, const Problem &P, const int32_t *list, int n, const int32_t *rq,
-                           const uint8_t *rstate, const long long *csum, double inv_qscale, __half *Rd, float2 *KR,
-                           int *err, cudaStream_t st, const int *cnt)
+cudaError_t tc_launch_kdig(const KdPlan *pl, const Problem &P, const int32_t *list, int n, const uint8_t *rstate,
+                           const long long *csum, double inv_qscale, float2 *KR, int *err, cudaStream_t st, const int *cnt,
+                           unsigned long long *ts)
 {
     if (n <= 0) return cudaSuccess;
-    {
-        dim3 g((unsigned)std::min<int64_t>((P.Nx + 255) / 256, 64), (unsigned)n);
-        tc::k_kdig_split_r<<<g, 256, 0, st>>>(list, P.Nx, reinterpret_cast<const int4 *>(rq), Rd, cnt);
-    }
     tc::KdArgs a{};
     a.kt_total = (int)(P.Nx / tc::KD_BK);
     a.nk_rows = pl->nk_rows;
@@ -1192,6 +1154,7 @@ cudaError_t tc_launch_kdig(const KdPlan *pl, const Problem &P, const int32_t *li
     a.KR = KR;
     a.err = err;
     a.ncount = cnt;
+    a.ts = ts;
     // persistent: at most one CTA pair per two of the 152 SMs
     const int64_t tiles = (int64_t)(pl->nk_rows / (2 * tc::KD_BM)) * ((n + tc::KD_S - 1) / tc::KD_S);
     const unsigned pairs = (unsigned)std::min<int64_t>(tiles, 76);

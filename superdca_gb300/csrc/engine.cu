@@ -142,6 +142,7 @@ struct sdca_handle {
     double *lbase = nullptr, *acc = nullptr, *dots = nullptr, *partial64 = nullptr;
     SlotDev *sd = nullptr;
     int32_t *list = nullptr;
+    int32_t *begin = nullptr;       // slots that loci enter and the loci
     int *flag = nullptr;
     // pinned host mirrors
     SlotDev *sd_h = nullptr;       // host-side slot parameters (edited freely)
@@ -624,10 +625,8 @@ int run_forward(sdca_handle *h, const std::vector<int32_t> &lst, const float *ve
     return SDCA_OK;
 }
 
-// begin a locus in slot b: zero or given start point, logits at the start point
-int dual_ctl_begin(sdca_handle *h, int b);
-
-int slot_begin(sdca_handle *h, int b, int64_t k, int32_t locus, const float *x0_engine)
+// A locus enters slot b: the host's part (slots_begin has the device's)
+void slot_begin(sdca_handle *h, int b, int64_t k, int32_t locus)
 {
     SlotHost &S = h->slots[b];
     S = SlotHost();
@@ -635,29 +634,29 @@ int slot_begin(sdca_handle *h, int b, int64_t k, int32_t locus, const float *x0_
     S.k = k;
     S.locus = locus;
     S.gcur = 0;
-    const Problem &P = h->P;
-    float *wab = h->wa + (int64_t)b * P.Dp;
-    if (x0_engine) {
-        CK(cudaMemcpyAsync(wab, x0_engine, sizeof(float) * P.Dp, cudaMemcpyHostToDevice, h->stream));
-        for (int64_t e = 0; e < P.Dp; ++e) S.xmax = std::max(S.xmax, (double)std::fabs(x0_engine[e]));
-    }
-    else
-        CK(cudaMemsetAsync(wab, 0, sizeof(float) * P.Dp, h->stream));
-    if (h->d) CK(cudaMemsetAsync(h->d + (int64_t)b * P.Dp, 0, sizeof(float) * P.Dp, h->stream));
-    CK(cudaMemcpyAsync(h->rstate + (int64_t)b * P.Nx, (h->scan ? h->TT : h->XT) + (int64_t)locus * P.Nx, P.Nx,
-                       cudaMemcpyDeviceToDevice, h->stream));
-    if (!x0_engine)
-        CK(cudaMemsetAsync(h->lbase + (int64_t)b * P.Nx * 4, 0, sizeof(double) * P.Nx * 4, h->stream));
-    if (h->form == SDCA_FORM_DUAL) {
-        const size_t NV = DV_S + 2 * (size_t)P.ring;
-        CK(cudaMemsetAsync(h->dv + (size_t)b * NV * 2 * P.Nx * 4, 0, sizeof(double) * NV * 2 * P.Nx * 4, h->stream));
-        const int rc = dual_ctl_begin(h, b);
-        if (rc) return rc;
-    }
     S.stp = 0.0;
     S.use_u = false;
     S.push = false;
     S.ring_new = -1;
+}
+
+// Slots `bs` start at zero: parameters, logits, the dual form's vectors and
+// solver state, and the target columns' states.
+int slots_begin(sdca_handle *h, const std::vector<int32_t> &bs)
+{
+    if (bs.empty()) return SDCA_OK;
+    const Problem &P = h->P;
+    std::vector<int32_t> who(2 * bs.size());
+    for (size_t j = 0; j < bs.size(); ++j) {
+        who[2 * j] = bs[j];
+        who[2 * j + 1] = h->slots[bs[j]].locus;
+    }
+    int rc = staged_h2d(h, h->begin, who.data(), sizeof(int32_t) * who.size());
+    if (rc) return rc;
+    const size_t NV = DV_S + 2 * (size_t)P.ring;
+    launch_slots_begin(P, reinterpret_cast<const int2 *>(h->begin), (int)bs.size(), h->scan ? h->TT : h->XT, h->rstate,
+                       h->wa, h->d, h->lbase, h->dv, (int64_t)(NV * 2 * P.Nx * 4), h->ctl, h->stream);
+    CKL();
     return SDCA_OK;
 }
 
@@ -844,24 +843,28 @@ int64_t take(Queue &Qu)
 
 int refill(sdca_handle *h, Queue &Qu)
 {
-    std::vector<int32_t> warm, learned;
+    std::vector<int32_t> fresh, warm, learned;
     for (int b = 0; b < h->P.Bmax; ++b) {
         if (h->slots[b].phase != PH_EMPTY) continue;
         const int64_t k = take(Qu);
         if (k < 0) break;
-        const float *x0 = nullptr;
         if (Qu.x_init && h->form == SDCA_FORM_DUAL)
             return fail(h, SDCA_E_UNSUPPORTED,
                         "the dual form takes no arbitrary start point (x_init): it starts from zero or learned");
-        if (Qu.x_init) {
-            const double *xr = Qu.x_init + k * (QQ * h->P.L + Q);
-            ref_to_engine(h->P, h->scan ? -1 : (int64_t)Qu.loci[k], xr, Qu.xbuf.data());
-            x0 = Qu.xbuf.data();
-        }
-        int rc = slot_begin(h, b, k, (int32_t)Qu.loci[k], x0);
-        if (rc) return rc;
+        slot_begin(h, b, k, (int32_t)Qu.loci[k]);
+        fresh.push_back(b);
         if (h->form == SDCA_FORM_DUAL && h->ws_dual) h->slots[b].phase = PH_WARM;
-        if (x0) {
+    }
+    const int rcb = slots_begin(h, fresh);
+    if (rcb) return rcb;
+    for (int b : fresh) {
+        SlotHost &S = h->slots[b];
+        if (Qu.x_init) {
+            const double *xr = Qu.x_init + S.k * (QQ * h->P.L + Q);
+            ref_to_engine(h->P, h->scan ? -1 : (int64_t)S.locus, xr, Qu.xbuf.data());
+            CK(cudaMemcpyAsync(h->wa + (int64_t)b * h->P.Dp, Qu.xbuf.data(), sizeof(float) * h->P.Dp,
+                               cudaMemcpyHostToDevice, h->stream));
+            for (int64_t e = 0; e < h->P.Dp; ++e) S.xmax = std::max(S.xmax, (double)std::fabs(Qu.xbuf[e]));
             // the copy reads the staging buffer: finish it before the next slot reuses it
             { const int r_ = stream_sync(h); if (r_) return r_; }
             warm.push_back(b);
@@ -1367,16 +1370,6 @@ int phase_step(sdca_handle *h)
 double dot4h(const double *a, const double *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3]; }
 
 // A new locus in slot b: the device state of its solver.
-int dual_ctl_begin(sdca_handle *h, int b)
-{
-    DualCtl c;
-    std::memset(&c, 0, sizeof(c));
-    c.phase = DC_EVAL0;
-    c.ring_new = -1;
-    c.last_check = -1000;
-    return staged_h2d(h, h->ctl + b, &c, sizeof(c));
-}
-
 // Stopped slots of the dual form: x in the engine layout (J = Phi^T a_x,
 // J_rr = 0, h = eta_x), then the final evaluation.  J is formed exactly:
 // the logits K a_x are O(1) while sum_j |K_ij a_j| is hundreds, so a
@@ -2152,7 +2145,7 @@ static int create_lane(const sdca_config *cfg, const sdca_handle *owner, sdca_ha
         (rc = dalloc(h, &h->partial64, (size_t)P.Cg * B * P.Nx * 4)) ||
         (rc = dalloc(h, &h->rows, B * P.L)) || (!dual && (rc = dalloc(h, &h->acc, B * NACC))) ||
         (!dual && (rc = dalloc(h, &h->dots, B * 4 * MAXHIST))) || (rc = dalloc(h, &h->sd, B)) ||
-        (rc = dalloc(h, &h->list, B)) || (rc = dalloc(h, &h->flag, 4)) ||
+        (rc = dalloc(h, &h->list, B)) || (rc = dalloc(h, &h->begin, 2 * B)) || (rc = dalloc(h, &h->flag, 4)) ||
         (rc = dalloc(h, reinterpret_cast<uint8_t **>(&h->Spool), hist_bytes)) ||
         (rc = dalloc(h, reinterpret_cast<uint8_t **>(&h->Ypool), hist_bytes)) ||
         (rc = halloc(h, &h->sd_h, B)) || (rc = halloc(h, &h->list_h, B)) ||

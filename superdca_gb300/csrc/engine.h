@@ -224,6 +224,8 @@ void launch_bwd_gather(const Problem &P, const uint8_t *XT, const SlotDev *sd,
 void launch_hpart(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
                   const float *wa, float *gpool, void *Ypool, const void *Spool, int hist_bf16,
                   double *acc, cudaStream_t st);
+void launch_slots_begin(const Problem &P, const int2 *who, int n, const uint8_t *states, uint8_t *rstate, float *wa,
+                        float *d, double *lbase, float2 *dv, int64_t dv_slot, DualCtl *ctl, cudaStream_t st);
 void launch_search(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
                    const double *lbase, const float *u, const uint8_t *rstate, const double *w,
                    float *R, double *acc, cudaStream_t st);

@@ -220,6 +220,40 @@ k_search(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N
     }
 }
 
+// Loci enter slots (who: slot, locus), starting from zero.  One launch for
+// all of them: as five memsets, a copy and an upload per slot it was the
+// host's time between two rounds, some 16 us per locus.
+__device__ __forceinline__ void zero_span(void *p, int64_t bytes)
+{
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < bytes / 16; k += (int64_t)gridDim.x * blockDim.x)
+        reinterpret_cast<uint4 *>(p)[k] = make_uint4(0, 0, 0, 0);
+}
+
+__global__ void __launch_bounds__(256)
+k_slots_begin(const int2 *__restrict__ who, int64_t Nx, int64_t Dp, const uint8_t *__restrict__ states,
+              uint8_t *__restrict__ rstate, float *__restrict__ wa, float *__restrict__ d, double *__restrict__ lbase,
+              float2 *__restrict__ dv, int64_t dv_slot, DualCtl *__restrict__ ctl)
+{
+    const int64_t b = who[blockIdx.y].x, r = who[blockIdx.y].y;
+    zero_span(wa + b * Dp, Dp * 4);
+    if (d) zero_span(d + b * Dp, Dp * 4);
+    zero_span(lbase + b * Nx * 4, Nx * 32);
+    if (dv) zero_span(dv + b * dv_slot, dv_slot * 8);
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < Nx / 16; k += (int64_t)gridDim.x * blockDim.x)
+        reinterpret_cast<uint4 *>(rstate + b * Nx)[k] = reinterpret_cast<const uint4 *>(states + r * Nx)[k];
+    if (ctl && blockIdx.x == 0) {
+        static_assert(sizeof(DualCtl) % 8 == 0, "zeroed in words");
+        for (unsigned k = threadIdx.x; k < sizeof(DualCtl) / 8; k += blockDim.x)
+            reinterpret_cast<unsigned long long *>(ctl + b)[k] = 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            ctl[b].phase = DC_EVAL0;
+            ctl[b].ring_new = -1;
+            ctl[b].last_check = -1000;
+        }
+    }
+}
+
 // x <- x + stp d; with a history push, s = x_new - x_old goes to ring_new.
 __global__ void k_accept(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list,
                          int64_t Dp, int m, float *__restrict__ wa, const float *__restrict__ d,
@@ -527,6 +561,16 @@ unsigned dgrid(int64_t Dp, int threads, int64_t cap = 256)
 }
 
 } // namespace
+
+void launch_slots_begin(const Problem &P, const int2 *who, int n, const uint8_t *states, uint8_t *rstate, float *wa,
+                        float *d, double *lbase, float2 *dv, int64_t dv_slot, DualCtl *ctl, cudaStream_t st)
+{
+    if (n <= 0) return;
+    // (Nx, Dp and the vectors are multiples of 64 elements)
+    const int64_t words = (std::max(P.Dp * 4, dv ? dv_slot * 8 : 0) / 16 + 255) / 256;
+    k_slots_begin<<<dim3((unsigned)std::min<int64_t>(words, 64), (unsigned)n), 256, 0, st>>>(
+        who, P.Nx, P.Dp, states, rstate, wa, d, lbase, dv, dv_slot, ctl);
+}
 
 // One cluster per slot, its blocks sharing the slot's sequences: as many as
 // there are SMs for, while each evaluating thread still has a sequence.  Two

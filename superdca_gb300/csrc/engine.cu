@@ -191,6 +191,7 @@ struct sdca_handle {
     int32_t *dlist = nullptr;      // the round's slot lists: [evaluations | searching | gradient pass + starts |
                                    // starts], then their lengths (DualCounts)
     cudaEvent_t ev_round = nullptr;   // end of a round's control kernel
+    cudaEvent_t ev_rows = nullptr;    // the retired slots' score rows have reached rows_h
     // the iteration core of a round as two alternating CUDA graphs (DualGraph)
     DualGraph dgraph[2];
     int dgraph_next = 0;
@@ -1431,7 +1432,7 @@ int dual_convert(sdca_handle *h, bool force)
 }
 
 // Score rows of retired slots travel to the host without a wait: copied into
-// the caller's array after the next round's event (or at the end).
+// the caller's array while the next round runs (or at the end).
 int dual_flush_rows(sdca_handle *h, Queue &Qu)
 {
     const Problem &P = h->P;
@@ -1455,6 +1456,7 @@ int dual_retire(sdca_handle *h, Queue &Qu, const std::vector<int32_t> &done)
         CKL();
         CK(cudaMemcpyAsync(h->rows_h, h->rows, sizeof(float) * P.L * done.size(), cudaMemcpyDeviceToHost,
                            h->stream));
+        CK(cudaEventRecord(h->ev_rows, h->stream));
         h->prof.d2h_bytes += (int64_t)sizeof(float) * P.L * done.size();
         for (int b : done) h->rows_pending.push_back(h->slots[b].k);
     }
@@ -1776,6 +1778,10 @@ int dual_round(sdca_handle *h, Queue &Qu)
         }
     }
     if (h->dgraph_off && (rc = dual_core(h, counts, false, h->ev_round, nullptr))) return rc;
+    if (!h->rows_pending.empty()) {
+        CK(cudaEventSynchronize(h->ev_rows));
+        dual_flush_rows(h, Qu);
+    }
     CK(cudaEventSynchronize(ev_sum));
     // the previous round's replay has completed: its timings can be read
     if (other) dual_graph_collect(h, *other);
@@ -1785,7 +1791,6 @@ int dual_round(sdca_handle *h, Queue &Qu)
         return fail(h, SDCA_E_CUDA, "tensor-core pipeline wait timed out (kernel abandoned its tile)");
     if (!W.empty() && h->errs_h[1])
         return fail(h, SDCA_E_CUDA, "warm start: a tensor-core pipeline wait gave up");
-    if (Qu.scores) dual_flush_rows(h, Qu);
 
     std::vector<int32_t> done, chk;
     for (int b : W) h->slots[b].phase = PH_INIT;   // start evaluation next round
@@ -1854,6 +1859,7 @@ int solve_lane(sdca_handle *h, Queue &Qu, cudaEvent_t t0_common)
     if (!t0 || !t1) return fail(h, SDCA_E_CUDA, "cudaEventCreate failed");
     if (!t0_common) CK(cudaEventRecord(t0, h->stream));
     for (auto &S : h->slots) S.phase = PH_EMPTY;
+    h->rows_pending.clear();   // (of a solve that failed)
     // the solver sums over whole vectors: the gradient buffers that
     // sdca_eval may have used get their zero padding back
     if (const int64_t used = QQ * h->P.L + Q; h->P.Dp > used)
@@ -2175,7 +2181,8 @@ static int create_lane(const sdca_config *cfg, const sdca_handle *owner, sdca_ha
         return fail(nullptr, rc, msg);
     }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess ||
-        (dual && cudaEventCreateWithFlags(&h->ev_round, cudaEventDisableTiming) != cudaSuccess)) {
+        (dual && (cudaEventCreateWithFlags(&h->ev_round, cudaEventDisableTiming) != cudaSuccess ||
+                  cudaEventCreateWithFlags(&h->ev_rows, cudaEventDisableTiming) != cudaSuccess))) {
         free_all(h);
         if (h->own_stream) cudaStreamDestroy(h->stream);
         delete h;
@@ -2628,6 +2635,7 @@ int sdca_destroy(sdca_handle *h)
     if (h->ev_lanes) cudaEventDestroy(h->ev_lanes);
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->ev_round) cudaEventDestroy(h->ev_round);
+    if (h->ev_rows) cudaEventDestroy(h->ev_rows);
     dual_graph_free(h);
     for (auto e : h->ev_pool) cudaEventDestroy(e);
     if (h->tc) tc_plan_destroy(h->tc);

@@ -11,6 +11,8 @@
 // (one 16-byte shared load or 16 FMAs per (sequence, locus, slot)).
 #include <algorithm>
 
+#include <cuda_pipeline_primitives.h>
+
 #include "engine.h"
 #include "kernels_common.cuh"
 
@@ -238,63 +240,92 @@ __global__ void k_reduce_partial(const float4 *__restrict__ partial, int C, int 
     }
 }
 
-constexpr int BWD_THREADS = 128;  // loci per CTA
-constexpr int BWD_G = 4;          // slots per CTA
+constexpr int BWD_THREADS = 128;  // loci per CTA (one slot)
+constexpr int BG_THREADS = 64;    // loci per CTA (k_bwd_gather)
+constexpr int BWD_G = 2;          // slots per CTA (k_bwd_gather)
 constexpr int BWD_SUB = 64;       // sequences per shared-memory sub-tile
 
-__global__ void __launch_bounds__(BWD_THREADS)
+// a[s][.] += r for the state s of one sequence, as 16 multiply-adds by 0 or 1
+// in pairs: one FFMA2 does two of them in one issue slot
+__device__ __forceinline__ void add_by_state(int s, float4 r, float2 (&a)[QQ / 2])
+{
+    const float2 lo = make_float2(r.x, r.y), hi = make_float2(r.z, r.w);
+#pragma unroll
+    for (int t = 0; t < Q; ++t) {
+        const float m = s == t ? 1.f : 0.f;
+        a[2 * t] = __ffma2_rn(make_float2(m, m), lo, a[2 * t]);
+        a[2 * t + 1] = __ffma2_rn(make_float2(m, m), hi, a[2 * t + 1]);
+    }
+}
+
+__device__ __forceinline__ void unpack(const float2 (&a)[QQ / 2], float (&c)[QQ])
+{
+#pragma unroll
+    for (int k = 0; k < QQ / 2; ++k) {
+        c[2 * k] = a[k].x;
+        c[2 * k + 1] = a[k].y;
+    }
+}
+
+// Bound by FP32 multiply-adds: 16 per (sequence, locus, slot), 0.11 ms for 64
+// slots of 1000 x 4001 at two clocks per pair and warp.  0.18 ms: that pipe
+// is busy 60 % of the time.  Single multiply-adds, four slots a thread and
+// blocks of 128 loci (110 registers, three or four blocks per SM) took 0.30,
+// the same in pairs 0.21; two slots a thread leave room for twice the warps,
+// and the next sub-tile's residuals are on their way while one is summed.
+__global__ void __launch_bounds__(BG_THREADS, 14)
 k_bwd_gather(const uint8_t *__restrict__ XT, int64_t Nx, int N, int L,
              const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int nlist,
              const float4 *__restrict__ R, const float *__restrict__ wa, float *__restrict__ gpool,
              void *__restrict__ Ypool, const void *__restrict__ Spool, int hist_bf16, int m,
              int64_t Dp, double lambda_J, double *__restrict__ acc)
 {
-    __shared__ float4 sR[BWD_G][BWD_SUB];
-    const int n = blockIdx.x * BWD_THREADS + threadIdx.x;
+    __shared__ float4 sR[2][BWD_G][BWD_SUB];
+    const int n = blockIdx.x * BG_THREADS + threadIdx.x;
     int slot[BWD_G];
 #pragma unroll
     for (int g = 0; g < BWD_G; ++g) {
         const int k = blockIdx.y * BWD_G + g;
         slot[g] = k < nlist ? list[k] : -1;
     }
-    float a[BWD_G][QQ];
+    float2 a2[BWD_G][QQ / 2];
 #pragma unroll
     for (int g = 0; g < BWD_G; ++g)
 #pragma unroll
-        for (int k = 0; k < QQ; ++k) a[g][k] = 0.f;
+        for (int k = 0; k < QQ / 2; ++k) a2[g][k] = make_float2(0.f, 0.f);
 
-    for (int i0 = 0; i0 < N; i0 += BWD_SUB) {
-        for (int k = threadIdx.x; k < BWD_G * BWD_SUB; k += BWD_THREADS) {
-            const int g = k / BWD_SUB, ii = k % BWD_SUB;
-            const int i = i0 + ii;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (slot[g] >= 0 && i < N) v = R[(int64_t)slot[g] * Nx + i];
-            sR[g][ii] = v;
+    static_assert(BG_THREADS == BWD_SUB, "a thread stages one sequence per slot");
+    auto stage = [&](int i0, int buf) {
+        const int i = i0 + threadIdx.x;
+#pragma unroll
+        for (int g = 0; g < BWD_G; ++g) {
+            const bool ok = slot[g] >= 0 && i < N;   // (else zeros)
+            __pipeline_memcpy_async(&sR[buf][g][threadIdx.x], ok ? R + (int64_t)slot[g] * Nx + i : R, 16, ok ? 0 : 16);
         }
+        __pipeline_commit();
+    };
+    stage(0, 0);
+    for (int i0 = 0, buf = 0; i0 < N; i0 += BWD_SUB, buf ^= 1) {
+        if (i0 + BWD_SUB < N) stage(i0 + BWD_SUB, buf ^ 1);
+        else __pipeline_commit();
+        uint4 xw[BWD_SUB / 16];
+        if (n < L)
+#pragma unroll
+            for (int q4 = 0; q4 < BWD_SUB / 16; ++q4) xw[q4] = reinterpret_cast<const uint4 *>(XT + (int64_t)n * Nx + i0)[q4];
+        __pipeline_wait_prior(1);
         __syncthreads();
         if (n < L) {
-            const uint4 *xp = reinterpret_cast<const uint4 *>(XT + (int64_t)n * Nx + i0);
 #pragma unroll
             for (int q4 = 0; q4 < BWD_SUB / 16; ++q4) {
-                const uint4 w = xp[q4];
-                const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+                const uint32_t words[4] = {xw[q4].x, xw[q4].y, xw[q4].z, xw[q4].w};
 #pragma unroll
-                for (int wd = 0; wd < 4; ++wd) {
+                for (int wd = 0; wd < 4; ++wd)
 #pragma unroll
                     for (int bt = 0; bt < 4; ++bt) {
-                        const int ii = q4 * 16 + wd * 4 + bt;
                         const int s = (words[wd] >> (8 * bt)) & 0x3;
-                        const float m0 = s == 0, m1 = s == 1, m2 = s == 2, m3 = s == 3;
 #pragma unroll
-                        for (int g = 0; g < BWD_G; ++g) {
-                            const float4 r = sR[g][ii];
-                            a[g][0] += m0 * r.x; a[g][1] += m0 * r.y; a[g][2] += m0 * r.z; a[g][3] += m0 * r.w;
-                            a[g][4] += m1 * r.x; a[g][5] += m1 * r.y; a[g][6] += m1 * r.z; a[g][7] += m1 * r.w;
-                            a[g][8] += m2 * r.x; a[g][9] += m2 * r.y; a[g][10] += m2 * r.z; a[g][11] += m2 * r.w;
-                            a[g][12] += m3 * r.x; a[g][13] += m3 * r.y; a[g][14] += m3 * r.z; a[g][15] += m3 * r.w;
-                        }
+                        for (int g = 0; g < BWD_G; ++g) add_by_state(s, sR[buf][g][q4 * 16 + wd * 4 + bt], a2[g]);
                     }
-                }
             }
         }
         __syncthreads();
@@ -307,7 +338,9 @@ k_bwd_gather(const uint8_t *__restrict__ XT, int64_t Nx, int N, int L,
         if (slot[g] < 0) continue;  // uniform across the block
         const int b = slot[g];
         GradRed red;
-        if (n < L) grad_locus(sd[b], b, n, a[g], wa, gpool, Ypool, Spool, hist_bf16, m, Dp, l2, red);
+        float a[QQ];
+        unpack(a2[g], a);
+        if (n < L) grad_locus(sd[b], b, n, a, wa, gpool, Ypool, Spool, hist_bf16, m, Dp, l2, red);
         double v[5] = {red.g2, red.x2, red.sy, red.yy, red.ss};
         const int idx[5] = {ACC_G2, ACC_X2J, ACC_SY, ACC_YY, ACC_SS};
         block_sum_atomic<5>(v, acc + (int64_t)b * NACC, idx);
@@ -350,7 +383,7 @@ k_grad_finalize(int L, const SlotDev *__restrict__ sd, const int32_t *__restrict
 // times the work for one, and the point and the gradient were converted on
 // the host between the reference's layout and this one, in 64-bit steps over
 // 16 L values each way: 4.7 ms at 3000 x 94,000, where the passes here take
-// 0.5 ms (0.22 logits, 0.25 gradient) and the call 0.9.
+// 0.44 ms (0.22 logits, 0.19 gradient) and the call 0.8.
 
 // the point from the reference's layout (double) into the engine's (FP32,
 // J_rr = 0, padding 0); the sums start at zero
@@ -493,9 +526,9 @@ k_eval_bwd(const uint8_t *__restrict__ XT, int64_t Nx, int N, int L, int64_t r, 
 {
     __shared__ float4 sR[BWD_SUB];
     const int n = blockIdx.x * BWD_THREADS + threadIdx.x;
-    float a[QQ];
+    float2 a2[QQ / 2];
 #pragma unroll
-    for (int k = 0; k < QQ; ++k) a[k] = 0.f;
+    for (int k = 0; k < QQ / 2; ++k) a2[k] = make_float2(0.f, 0.f);
     for (int i0 = 0; i0 < N; i0 += BWD_SUB) {
         __syncthreads();
         if (threadIdx.x < BWD_SUB) sR[threadIdx.x] = i0 + threadIdx.x < N ? R[i0 + threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -513,16 +546,13 @@ k_eval_bwd(const uint8_t *__restrict__ XT, int64_t Nx, int N, int L, int64_t r, 
 #pragma unroll
                     for (int bt = 0; bt < 4; ++bt) {
                         const int s = (words[wd] >> (8 * bt)) & 0x3;
-                        const float4 v = sR[q4 * 16 + wd * 4 + bt];
-                        const float m0 = s == 0, m1 = s == 1, m2 = s == 2, m3 = s == 3;
-                        a[0] += m0 * v.x; a[1] += m0 * v.y; a[2] += m0 * v.z; a[3] += m0 * v.w;
-                        a[4] += m1 * v.x; a[5] += m1 * v.y; a[6] += m1 * v.z; a[7] += m1 * v.w;
-                        a[8] += m2 * v.x; a[9] += m2 * v.y; a[10] += m2 * v.z; a[11] += m2 * v.w;
-                        a[12] += m3 * v.x; a[13] += m3 * v.y; a[14] += m3 * v.z; a[15] += m3 * v.w;
+                        add_by_state(s, sR[q4 * 16 + wd * 4 + bt], a2);
                     }
             }
         }
     }
+    float a[QQ];
+    unpack(a2, a);
     const float l2 = (float)(2.0 * lambda_J);
     float x2 = 0.f;
     if (n < L) {
@@ -630,8 +660,8 @@ void launch_bwd_gather(const Problem &P, const uint8_t *XT, const SlotDev *sd,
                        double *acc, cudaStream_t st)
 {
     if (n <= 0) return;
-    dim3 grid((unsigned)((P.L + BWD_THREADS - 1) / BWD_THREADS), (unsigned)((n + BWD_G - 1) / BWD_G));
-    k_bwd_gather<<<grid, BWD_THREADS, 0, st>>>(XT, P.Nx, (int)P.N, (int)P.L, sd, list, n,
+    dim3 grid((unsigned)((P.L + BG_THREADS - 1) / BG_THREADS), (unsigned)((n + BWD_G - 1) / BWD_G));
+    k_bwd_gather<<<grid, BG_THREADS, 0, st>>>(XT, P.Nx, (int)P.N, (int)P.L, sd, list, n,
                                                reinterpret_cast<const float4 *>(R), wa, gpool, Ypool,
                                                Spool, hist_bf16, P.ring, P.Dp, P.lambda_J, acc);
 }

@@ -115,7 +115,6 @@ enum { DC_T = 0, DC_G = 1, DC_GW = 2, DC_W = 3, DC_N = 4 };
 
 struct DualGraph {
     cudaGraphExec_t exec = nullptr;
-    cudaEvent_t ev_round = nullptr;     // recorded after the summary copy (the host waits on it)
     std::vector<GraphRec> recs;
     bool pending = false;               // replayed, its timings not collected yet
     int64_t counts[DC_N] = {};          // the list lengths of that replay
@@ -190,7 +189,9 @@ struct sdca_handle {
     std::vector<int32_t> dlist_sent;   // the lists as the device has them
     int32_t *dlist = nullptr;      // the round's slot lists: [evaluations | searching | gradient pass + starts |
                                    // starts], then their lengths (DualCounts)
-    cudaEvent_t ev_round = nullptr;   // end of a round's control kernel
+    cudaEvent_t ev_round = nullptr;   // end of a round's control kernel (rounds without a graph)
+    uint32_t *pub = nullptr, *pub_h = nullptr;   // DualPub::done; DualPub::seq (pinned)
+    uint32_t rounds = 0;              // replays launched
     cudaEvent_t ev_rows = nullptr;    // the retired slots' score rows have reached rows_h
     // the iteration core of a round as two alternating CUDA graphs (DualGraph)
     DualGraph dgraph[2];
@@ -368,6 +369,7 @@ int dual_blocks(sdca_handle *h)
     h->errs_h = reinterpret_cast<int *>(h->out_h + sum + acc);
     h->ts = reinterpret_cast<unsigned long long *>(h->out + sum + acc + errs);
     h->ts_h = reinterpret_cast<unsigned long long *>(h->out_h + sum + acc + errs);
+    if ((rc = dalloc(h, &h->pub, 2)) || (rc = halloc(h, &h->pub_h, 1))) return rc;
     h->zero_bytes = sizeof(double) * B * (CSUM + 2 + 4 * MAXHIST + NDACC);
     if ((rc = dalloc(h, &h->zero, h->zero_bytes))) return rc;
     h->csum = reinterpret_cast<long long *>(h->zero);
@@ -404,6 +406,8 @@ void free_all(sdca_handle *h)
         h->acc_h = nullptr;
         h->sum_h = nullptr;
     }
+    if (h->pub_h) cudaFreeHost(h->pub_h);
+    h->pub_h = nullptr;
     if (h->acc_h) cudaFreeHost(h->acc_h);
     if (h->dots_h) cudaFreeHost(h->dots_h);
     if (h->rows_h) cudaFreeHost(h->rows_h);
@@ -1538,14 +1542,14 @@ int dual_ws_rows(sdca_handle *h, int nW, const int32_t *l_W)
 // The iteration core of a round (dual_round has written the lists and their
 // lengths): the line search of the searching slots, the K rho pass over
 // the gradient pass and the learned starts, the starts themselves, the
-// accept and gradient, history-dot and control kernels, the summary
-// copy and the event `ev`, then the directions.  dev: every grid covers
-// Bmax slots and the kernels read the list lengths from device memory -- the
-// form captured in a CUDA graph and replayed every round, its kernels timed
-// by their own stamps (sixteen event nodes took 46 us of a replay); otherwise
-// the grids are the host's list lengths
-// and the classes are timed as usual.
-int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev, DualGraph *g)
+// accept and gradient, history-dot and control kernels, then the directions.
+// dev: every grid covers Bmax slots and the kernels read the list lengths from
+// device memory -- the form captured in a CUDA graph and replayed every round,
+// its kernels timed by their own stamps (sixteen event nodes took 46 us of a
+// replay), its control kernel telling the host the round's outcome
+// (DualPub).  Otherwise the grids are the host's list lengths, the classes are
+// timed as usual and the outcome is copied, with an event behind it.
+int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, DualGraph *g)
 {
     const Problem &P = h->P;
     const int B = (int)P.Bmax;
@@ -1556,6 +1560,7 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
     auto dcnt = [&](int i) -> const int * { return dev ? cnt + i : nullptr; };
     unsigned long long *const ts = dev ? h->ts + (g - h->dgraph) * TS_WORDS : nullptr;
     unsigned long long *const ts_other = dev ? h->ts + (1 - (g - h->dgraph)) * TS_WORDS : nullptr;
+    const DualPub pub = dev ? DualPub{h->sum_h, h->acc_h, h->errs_h, h->pub_h, h->pub, h->tc_err} : DualPub{};
     // one kernel of a profile class: timed by events, or by its own stamps
     auto region = [&](int cls, int stamp, int cidx, auto &&fn) -> int {
         if (!dev) {
@@ -1619,14 +1624,15 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
         return rc;
     if ((rc = region(SDCA_K_OTHER, TS_CONTROL, DC_G, [&](unsigned long long *t) {
              launch_dual_control(P, h->ctl, h->sum, l_G, len(DC_G), h->cfg.max_iterations, gtol, h->acc, h->amax,
-                                 h->dots, h->stream, dcnt(DC_G), t);
+                                 h->dots, pub, h->stream, dcnt(DC_G), t);
              return SDCA_OK;
          })))
         return rc;
     CKL();
-    CK(cudaMemcpyAsync(h->out_h, h->out, h->out_bytes, cudaMemcpyDeviceToHost, h->stream));
-    if (dev) CK(cudaEventRecordWithFlags(ev, h->stream, cudaEventRecordExternal));
-    else CK(cudaEventRecord(ev, h->stream));
+    if (!dev) {
+        CK(cudaMemcpyAsync(h->out_h, h->out, h->out_bytes, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaEventRecord(h->ev_round, h->stream));
+    }
     if ((rc = region(SDCA_K_DIRECTION, TS_DIRECTION, DC_G, [&](unsigned long long *t) {
              launch_dual_direction(P, h->ctl, l_G, len(DC_G), h->dv, h->P0, h->wf, h->rstate, h->ud, h->dacc,
                                    h->stream, dcnt(DC_G), t, ts_other);
@@ -1634,6 +1640,11 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
          })))
         return rc;
     CKL();
+    if (dev) {
+        // this replay's stamps (the next one's directions clear them)
+        const size_t at = (size_t)(g - h->dgraph) * TS_WORDS;
+        CK(cudaMemcpyAsync(h->ts_h + at, h->ts + at, sizeof(unsigned long long) * TS_WORDS, cudaMemcpyDeviceToHost, h->stream));
+    }
     return SDCA_OK;
 }
 
@@ -1641,13 +1652,12 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, cudaEvent_t ev
 // this thread's capture mode) and instantiate it.
 int dual_graph_build(sdca_handle *h, DualGraph &g)
 {
-    if (!g.ev_round) CK(cudaEventCreateWithFlags(&g.ev_round, cudaEventDisableTiming));
     CK(cudaMemsetAsync(h->ts + (&g - h->dgraph) * TS_WORDS, 0, sizeof(unsigned long long) * TS_WORDS, h->stream));
     g.recs.clear();
     const int64_t any[DC_N] = {1, 1, 1, 1};
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = dual_core(h, any, true, g.ev_round, &g);
+    const int rc = dual_core(h, any, true, &g);
     const cudaError_t e = cudaStreamEndCapture(h->stream, &graph);
     if (rc || e != cudaSuccess || !graph) {
         if (graph) cudaGraphDestroy(graph);
@@ -1694,12 +1704,18 @@ void dual_graph_reset(sdca_handle *h)
     h->dgraph_next = 0;
 }
 
-void dual_graph_free(sdca_handle *h)
+// Wait until the last replay has published its outcome.  The stream is asked
+// now and then: a round that ended, or failed, without it would never.
+int dual_graph_wait(sdca_handle *h)
 {
-    dual_graph_reset(h);
-    for (DualGraph &g : h->dgraph) {
-        if (g.ev_round) cudaEventDestroy(g.ev_round);
-        g.ev_round = nullptr;
+    for (uint32_t spins = 1;; ++spins) {
+        if (__atomic_load_n(h->pub_h, __ATOMIC_ACQUIRE) == h->rounds) return SDCA_OK;
+        if (spins % 65536) continue;
+        const cudaError_t e = cudaStreamQuery(h->stream);
+        if (e == cudaErrorNotReady) continue;
+        CK(e);
+        if (__atomic_load_n(h->pub_h, __ATOMIC_ACQUIRE) == h->rounds) return SDCA_OK;
+        return fail(h, SDCA_E_CUDA, "a round ended without its summary");
     }
 }
 
@@ -1760,7 +1776,6 @@ int dual_round(sdca_handle *h, Queue &Qu)
     }
     CKL();
     // the iteration core: a replay of this lane's CUDA graph, or the kernels one by one
-    cudaEvent_t ev_sum = h->ev_round;
     DualGraph *other = nullptr;
     if (!h->dgraph_off) {
         DualGraph &g = h->dgraph[h->dgraph_next];
@@ -1770,19 +1785,23 @@ int dual_round(sdca_handle *h, Queue &Qu)
         }
         if (!h->dgraph_off) {
             CK(cudaGraphLaunch(g.exec, h->stream));
+            ++h->rounds;
             std::copy(counts, counts + DC_N, g.counts);
             g.pending = true;
-            ev_sum = g.ev_round;
             other = &h->dgraph[1 - h->dgraph_next];
             h->dgraph_next = 1 - h->dgraph_next;
         }
     }
-    if (h->dgraph_off && (rc = dual_core(h, counts, false, h->ev_round, nullptr))) return rc;
+    if (h->dgraph_off && (rc = dual_core(h, counts, false, nullptr))) return rc;
     if (!h->rows_pending.empty()) {
         CK(cudaEventSynchronize(h->ev_rows));
         dual_flush_rows(h, Qu);
     }
-    CK(cudaEventSynchronize(ev_sum));
+    if (other) {
+        if ((rc = dual_graph_wait(h))) return rc;
+    } else {
+        CK(cudaEventSynchronize(h->ev_round));
+    }
     // the previous round's replay has completed: its timings can be read
     if (other) dual_graph_collect(h, *other);
     // every staged host-to-device copy was queued before the event
@@ -1888,9 +1907,6 @@ int solve_lane(sdca_handle *h, Queue &Qu, cudaEvent_t t0_common)
     CK(cudaEventElapsedTime(&ms, t0, t1));
     h->prof.solve_ms = ms;
     if (h->dgraph[0].pending || h->dgraph[1].pending) {
-        // the last replay's stamps, the directions' included
-        CK(cudaMemcpyAsync(h->ts_h, h->ts, sizeof(unsigned long long) * 2 * TS_WORDS, cudaMemcpyDeviceToHost, h->stream));
-        { const int r_ = stream_sync(h); if (r_) return r_; }
         for (DualGraph &g : h->dgraph) dual_graph_collect(h, g);
     }
     prof_collect(h);
@@ -2636,7 +2652,7 @@ int sdca_destroy(sdca_handle *h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->ev_round) cudaEventDestroy(h->ev_round);
     if (h->ev_rows) cudaEventDestroy(h->ev_rows);
-    dual_graph_free(h);
+    dual_graph_reset(h);
     for (auto e : h->ev_pool) cudaEventDestroy(e);
     if (h->tc) tc_plan_destroy(h->tc);
     if (h->kd) tc_kdig_plan_destroy(h->kd);

@@ -166,6 +166,18 @@ enum DualAcc {
     NDACC = 4
 };
 
+// What a replayed round's control kernel tells the host by itself, in pinned
+// host memory (the same layout as the device's): the slots' summaries, the
+// objective sums, the pipelines' error words and, last, the round's number.
+struct DualPub {
+    DualSum *sum;           // null: nothing is published
+    double *acc;
+    int *errs;
+    volatile uint32_t *seq;
+    uint32_t *done;         // device: blocks that have published, rounds published
+    const int *errs_d;
+};
+
 // class sums of rho_q per slot: [a * 4 + c] the sum of column c over the
 // sequences with state a at the slot's locus (0 in scan mode), then the sums
 // of columns 0..2 over all sequences
@@ -269,7 +281,7 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
                             const float *w, const float *P0, float *R, double *acc, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_control(const Problem &P, DualCtl *ctl, DualSum *sum, const int32_t *list, int n,
                          int max_iterations, double gtol, const double *acc, const double *amax, const double *dots,
-                         cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
+                         const DualPub &pub, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_check_apply(DualCtl *ctl, DualSum *sum, const int32_t *list, int n, double gtol, const double *acc,
                              cudaStream_t st);
 void launch_dual_digits(const Problem &P, const SlotDev *sd, const int32_t *list, int n, int d, const float2 *dv,

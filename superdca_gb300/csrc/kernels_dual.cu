@@ -1139,12 +1139,46 @@ __device__ __forceinline__ bool warp_compact_coeffs(int k, const double *R, cons
 //   Gram matrices S^T Y and Y^T Y from the history dots, the compact-form
 //   coefficients of the next direction and its h part, and the ring
 //   position the next accepted step will fill.
-__global__ void __launch_bounds__(32)
+//
+// In a replayed round the host is told as soon as the stops and wishes stand,
+// by the block's second warp, while the first works out the coefficients and
+// the direction kernel runs: a copy node and an event node behind this kernel
+// took 12 us, and the host's 27 us until the next launch began after them.
+__device__ __forceinline__ void publish(const DualPub &pub, const DualSum *s, int b, const double *acc)
+{
+    const int lane = threadIdx.x & 31;
+    static_assert(sizeof(DualSum) % 8 == 0 && sizeof(DualSum) <= 32 * 8, "one word per lane");
+    if (s && lane < (int)(sizeof(DualSum) / 8))
+        reinterpret_cast<volatile unsigned long long *>(pub.sum + b)[lane] = reinterpret_cast<const unsigned long long *>(s)[lane];
+    const int64_t f = (int64_t)blockIdx.x * NACC + ACC_F;   // (a replay has a block per slot)
+    if (lane == 0) *reinterpret_cast<volatile double *>(pub.acc + f) = acc[f];
+    if (blockIdx.x == 0 && lane < 2) reinterpret_cast<volatile int *>(pub.errs)[lane] = pub.errs_d[lane];
+    __syncwarp();
+    if (lane == 0) {
+        __threadfence_system();
+        if (atomicAdd(pub.done, 1u) == gridDim.x - 1) {
+            pub.done[0] = 0;
+            const uint32_t round = ++pub.done[1];
+            __threadfence_system();
+            *pub.seq = round;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(64)
 k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32_t *__restrict__ list, int m,
                int max_iterations, double gtol, double lambda_J, double lambda_h, const double *__restrict__ acc,
-               const double *__restrict__ amax, const double *__restrict__ dots, const int *__restrict__ cnt,
-               unsigned long long *__restrict__ ts)
+               const double *__restrict__ amax, const double *__restrict__ dots, const DualPub pub,
+               const int *__restrict__ cnt, unsigned long long *__restrict__ ts)
 {
+    __shared__ DualSum s_sum;
+    if (threadIdx.x >= 32) {   // the publishing warp
+        if (!pub.sum) return;
+        const bool mine = !cnt || (int)blockIdx.x < *cnt;
+        if (mine) asm volatile("bar.sync 1, 64;" ::: "memory");
+        publish(pub, mine ? &s_sum : nullptr, mine ? list[blockIdx.x] : 0, acc);
+        return;
+    }
     if (cnt && (int)blockIdx.x >= *cnt) return;
     stamp_begin(ts);
     const int b = list[blockIdx.x];
@@ -1276,6 +1310,14 @@ k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32
         }
     }
     __syncwarp();
+    if (pub.sum) {
+        if (lane == 0) {
+            write_summary(S, s_sum);
+            if (go) s_sum.phase = DC_STEP;
+        }
+        __syncwarp();
+        asm volatile("bar.arrive 1, 64;" ::: "memory");
+    }
     // compact-form coefficients of the next direction, on the warp's lanes
     // (lane j: history pair j)
     if (go) {
@@ -1632,12 +1674,12 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
 
 void launch_dual_control(const Problem &P, DualCtl *ctl, DualSum *sum, const int32_t *list, int n,
                          int max_iterations, double gtol, const double *acc, const double *amax, const double *dots,
-                         cudaStream_t st, const int *cnt,
+                         const DualPub &pub, cudaStream_t st, const int *cnt,
                        unsigned long long *ts)
 {
     if (n <= 0) return;
-    k_dual_control<<<n, 32, 0, st>>>(ctl, sum, list, P.m, max_iterations, gtol, P.lambda_J, P.lambda_h, acc, amax,
-                                     dots, cnt, ts);
+    k_dual_control<<<n, 64, 0, st>>>(ctl, sum, list, P.m, max_iterations, gtol, P.lambda_J, P.lambda_h, acc, amax,
+                                     dots, pub, cnt, ts);
 }
 
 void launch_dual_check_apply(DualCtl *ctl, DualSum *sum, const int32_t *list, int n, double gtol, const double *acc,

@@ -1560,7 +1560,11 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, DualGraph *g)
     auto dcnt = [&](int i) -> const int * { return dev ? cnt + i : nullptr; };
     unsigned long long *const ts = dev ? h->ts + (g - h->dgraph) * TS_WORDS : nullptr;
     unsigned long long *const ts_other = dev ? h->ts + (1 - (g - h->dgraph)) * TS_WORDS : nullptr;
-    const DualPub pub = dev ? DualPub{h->sum_h, h->acc_h, h->errs_h, h->pub_h, h->pub, h->tc_err} : DualPub{};
+    DualPub pub{};
+    if (dev) {
+        const size_t prev = (size_t)(1 - (g - h->dgraph)) * TS_WORDS;
+        pub = {h->sum_h, h->acc_h, h->errs_h, h->pub_h, h->pub, h->tc_err, h->ts_h + prev, h->ts + prev};
+    }
     // one kernel of a profile class: timed by events, or by its own stamps
     auto region = [&](int cls, int stamp, int cidx, auto &&fn) -> int {
         if (!dev) {
@@ -1640,11 +1644,6 @@ int dual_core(sdca_handle *h, const int64_t (&n)[DC_N], bool dev, DualGraph *g)
          })))
         return rc;
     CKL();
-    if (dev) {
-        // this replay's stamps (the next one's directions clear them)
-        const size_t at = (size_t)(g - h->dgraph) * TS_WORDS;
-        CK(cudaMemcpyAsync(h->ts_h + at, h->ts + at, sizeof(unsigned long long) * TS_WORDS, cudaMemcpyDeviceToHost, h->stream));
-    }
     return SDCA_OK;
 }
 
@@ -1769,8 +1768,9 @@ int dual_round(sdca_handle *h, Queue &Qu)
     }
     int rc;
     if (!W.empty() && (rc = dual_ws_rows(h, (int)W.size(), l_W))) return rc;
-    if ((rc = zero_acc(h))) return rc;
     if (!ef.empty()) {
+        // (the sums of a gradient pass are cleared by the control kernel)
+        if ((rc = zero_acc(h))) return rc;
         Timed t(h, SDCA_K_LINESEARCH, 1, (int64_t)ef.size());
         launch_dual_eval(P, h->sd, l_ef, (int)ef.size(), h->dv, h->rstate, h->w, h->R, h->acc, h->stream);
     }
@@ -1906,8 +1906,13 @@ int solve_lane(sdca_handle *h, Queue &Qu, cudaEvent_t t0_common)
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, t0, t1));
     h->prof.solve_ms = ms;
-    if (h->dgraph[0].pending || h->dgraph[1].pending) {
-        for (DualGraph &g : h->dgraph) dual_graph_collect(h, g);
+    for (DualGraph &g : h->dgraph) {
+        if (!g.pending) continue;
+        // the last replay's stamps
+        const size_t at = (size_t)(&g - h->dgraph) * TS_WORDS;
+        CK(cudaMemcpyAsync(h->ts_h + at, h->ts + at, sizeof(unsigned long long) * TS_WORDS, cudaMemcpyDeviceToHost, h->stream));
+        { const int r_ = stream_sync(h); if (r_) return r_; }
+        dual_graph_collect(h, g);
     }
     prof_collect(h);
     return SDCA_OK;

@@ -176,6 +176,8 @@ struct DualPub {
     volatile uint32_t *seq;
     uint32_t *done;         // device: blocks that have published, rounds published
     const int *errs_d;
+    unsigned long long *ts;         // the round before's stamps, complete by now
+    const unsigned long long *ts_d;
 };
 
 // class sums of rho_q per slot: [a * 4 + c] the sum of column c over the
@@ -280,7 +282,7 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
                             float2 *dv, float *ud, const uint8_t *rstate,
                             const float *w, const float *P0, float *R, double *acc, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_control(const Problem &P, DualCtl *ctl, DualSum *sum, const int32_t *list, int n,
-                         int max_iterations, double gtol, const double *acc, const double *amax, const double *dots,
+                         int max_iterations, double gtol, double *acc, const double *amax, const double *dots,
                          const DualPub &pub, cudaStream_t st, const int *cnt = nullptr, unsigned long long *ts = nullptr);
 void launch_dual_check_apply(DualCtl *ctl, DualSum *sum, const int32_t *list, int n, double gtol, const double *acc,
                              cudaStream_t st);

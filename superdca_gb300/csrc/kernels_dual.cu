@@ -1152,7 +1152,11 @@ __device__ __forceinline__ void publish(const DualPub &pub, const DualSum *s, in
         reinterpret_cast<volatile unsigned long long *>(pub.sum + b)[lane] = reinterpret_cast<const unsigned long long *>(s)[lane];
     const int64_t f = (int64_t)blockIdx.x * NACC + ACC_F;   // (a replay has a block per slot)
     if (lane == 0) *reinterpret_cast<volatile double *>(pub.acc + f) = acc[f];
-    if (blockIdx.x == 0 && lane < 2) reinterpret_cast<volatile int *>(pub.errs)[lane] = pub.errs_d[lane];
+    if (blockIdx.x == 0) {
+        static_assert(TS_WORDS <= 32, "one word per lane");
+        if (lane < 2) reinterpret_cast<volatile int *>(pub.errs)[lane] = pub.errs_d[lane];
+        if (lane < TS_WORDS) reinterpret_cast<volatile unsigned long long *>(pub.ts)[lane] = pub.ts_d[lane];
+    }
     __syncwarp();
     if (lane == 0) {
         __threadfence_system();
@@ -1167,7 +1171,7 @@ __device__ __forceinline__ void publish(const DualPub &pub, const DualSum *s, in
 
 __global__ void __launch_bounds__(64)
 k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32_t *__restrict__ list, int m,
-               int max_iterations, double gtol, double lambda_J, double lambda_h, const double *__restrict__ acc,
+               int max_iterations, double gtol, double lambda_J, double lambda_h, double *__restrict__ acc,
                const double *__restrict__ amax, const double *__restrict__ dots, const DualPub pub,
                const int *__restrict__ cnt, unsigned long long *__restrict__ ts)
 {
@@ -1393,6 +1397,8 @@ k_dual_control(DualCtl *__restrict__ ctl, DualSum *__restrict__ sum, const int32
             S.phase = DC_STEP;
         }
     }
+    // the gradient pass of the next round adds to these
+    if (lane < 5) acc[(int64_t)b * NACC + (lane == 0 ? ACC_G2 : lane == 1 ? ACC_X2J : lane == 2 ? ACC_SY : lane == 3 ? ACC_YY : ACC_SS)] = 0.0;
     __syncwarp();
     {
         unsigned long long *dst = reinterpret_cast<unsigned long long *>(ctl + b);
@@ -1673,7 +1679,7 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
 }
 
 void launch_dual_control(const Problem &P, DualCtl *ctl, DualSum *sum, const int32_t *list, int n,
-                         int max_iterations, double gtol, const double *acc, const double *amax, const double *dots,
+                         int max_iterations, double gtol, double *acc, const double *amax, const double *dots,
                          const DualPub &pub, cudaStream_t st, const int *cnt,
                        unsigned long long *ts)
 {

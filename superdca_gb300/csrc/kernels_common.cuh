@@ -34,25 +34,6 @@ __device__ __forceinline__ float warp_sum_f(float v)
     return v;
 }
 
-// Eight sums over the warp by halving what each lane keeps (4, 2 and 1 values)
-// and two plain steps, 9 additions instead of 40: lane 4 k returns value k
-// (bits of k: lane bits 16, 8, 4).
-__device__ __forceinline__ double warp_sum8(double (&v)[8])
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int s = 0, h = 4; s < 3; ++s, h >>= 1) {
-        const int bit = 16 >> s;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const double give = lane & bit ? v[k] : v[k + h], keep = lane & bit ? v[k + h] : v[k];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
-        }
-    }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
 // Sum K per-thread values over the block; thread 0 adds them to dst[idx[k]].
 // Warp sums run in FP32 (each thread's value is itself an FP32 partial over
 // a stretch of one vector), the cross-warp sum in FP64.
@@ -168,31 +149,6 @@ __device__ __forceinline__ void stamp_end(unsigned long long *ts, bool mine)
 
 struct GradRed {
     float gmax = 0.f, g2 = 0.f, x2 = 0.f, sy = 0.f, yy = 0.f, ss = 0.f;
-
-    // Four gradient entries (c the contraction's), zero in the J_rr block;
-    // with a push y = g - g_old to the ring at hoff.
-    __device__ __forceinline__ float4 entries(float4 c, float4 xv, float l2, bool zero, bool push, const float4 *go,
-                                              void *Ypool, const void *Spool, int64_t hoff, int hist_bf16)
-    {
-        float4 gv;
-        gv.x = zero ? 0.f : c.x + l2 * xv.x;
-        gv.y = zero ? 0.f : c.y + l2 * xv.y;
-        gv.z = zero ? 0.f : c.z + l2 * xv.z;
-        gv.w = zero ? 0.f : c.w + l2 * xv.w;
-        gmax = fmaxf(gmax, fmaxf(fmaxf(fabsf(gv.x), fabsf(gv.y)), fmaxf(fabsf(gv.z), fabsf(gv.w))));
-        g2 += dot4(gv, gv);
-        x2 += dot4(xv, xv);
-        if (push) {
-            const float4 ov = *go;
-            float4 yv = make_float4(gv.x - ov.x, gv.y - ov.y, gv.z - ov.z, gv.w - ov.w);
-            yv = store_hist4(Ypool, hoff, yv, hist_bf16);
-            const float4 sv = load_hist4(Spool, hoff, hist_bf16);
-            sy += dot4(sv, yv);
-            yy += dot4(yv, yv);
-            ss += dot4(sv, sv);
-        }
-        return gv;
-    }
 };
 
 // Gradient of the 16 J entries of locus n for one slot: g = c + 2 lambda_J x
@@ -212,11 +168,27 @@ __device__ __forceinline__ void grad_locus(const SlotT &S, int b, int64_t n, con
     const bool push = (S.flags & 2) && S.ring_new >= 0;
     const int64_t hoff = ((int64_t)b * ring + (push ? S.ring_new : 0)) * Dp + n * 16;
 #pragma unroll
-    for (int k4 = 0; k4 < 4; ++k4)
-        reinterpret_cast<float4 *>(gn)[k4] =
-            red.entries(make_float4(c[4 * k4], c[4 * k4 + 1], c[4 * k4 + 2], c[4 * k4 + 3]),
-                        reinterpret_cast<const float4 *>(x)[k4], l2, zero, push, reinterpret_cast<const float4 *>(go) + k4,
-                        Ypool, Spool, hoff + 4 * k4, hist_bf16);
+    for (int k4 = 0; k4 < 4; ++k4) {
+        const float4 xv = reinterpret_cast<const float4 *>(x)[k4];
+        float4 gv;
+        gv.x = zero ? 0.f : c[4 * k4 + 0] + l2 * xv.x;
+        gv.y = zero ? 0.f : c[4 * k4 + 1] + l2 * xv.y;
+        gv.z = zero ? 0.f : c[4 * k4 + 2] + l2 * xv.z;
+        gv.w = zero ? 0.f : c[4 * k4 + 3] + l2 * xv.w;
+        reinterpret_cast<float4 *>(gn)[k4] = gv;
+        red.gmax = fmaxf(red.gmax, fmaxf(fmaxf(fabsf(gv.x), fabsf(gv.y)), fmaxf(fabsf(gv.z), fabsf(gv.w))));
+        red.g2 += dot4(gv, gv);
+        red.x2 += dot4(xv, xv);
+        if (push) {
+            const float4 ov = reinterpret_cast<const float4 *>(go)[k4];
+            float4 yv = make_float4(gv.x - ov.x, gv.y - ov.y, gv.z - ov.z, gv.w - ov.w);
+            yv = store_hist4(Ypool, hoff + 4 * k4, yv, hist_bf16);
+            const float4 sv = load_hist4(Spool, hoff + 4 * k4, hist_bf16);
+            red.sy += dot4(sv, yv);
+            red.yy += dot4(yv, yv);
+            red.ss += dot4(sv, sv);
+        }
+    }
 }
 
 } // namespace sdca

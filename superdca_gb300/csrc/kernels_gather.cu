@@ -203,28 +203,16 @@ __global__ void k_reduce_partial(const float4 *__restrict__ partial, int C, int 
         // every thread of the block takes part in the reduction
         double ru = 0.0;
         if (i < N) {
-            // the sum of C + 1 singles, rounded once: FP32 with the additions'
-            // own errors summed beside (Knuth's two-sum), which leaves some
-            // C^2 2^-48 of it; in FP64 the additions were most of the kernel
-            // (53 us for 64 slots of 3000 sequences and 12 slices, now 12)
-            float t[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+            double t[4] = {0, 0, 0, 0};
             if (add_h) {
                 const float *h = vecs + (int64_t)b * Dp + hoff;
                 t[0] = h[0]; t[1] = h[1]; t[2] = h[2]; t[3] = h[3];
             }
             for (int c = 0; c < C; ++c) {
-                const float4 p4 = partial[((int64_t)c * Bmax + b) * Nx + i];
-                const float p[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-                for (int a = 0; a < 4; ++a) {
-                    const float s = __fadd_rn(t[a], p[a]), bb = __fsub_rn(s, t[a]);
-                    lo[a] += __fadd_rn(__fsub_rn(t[a], __fsub_rn(s, bb)), __fsub_rn(p[a], bb));
-                    t[a] = s;
-                }
+                const float4 p = partial[((int64_t)c * Bmax + b) * Nx + i];
+                t[0] += p.x; t[1] += p.y; t[2] += p.z; t[3] += p.w;
             }
-#pragma unroll
-            for (int a = 0; a < 4; ++a) t[a] += lo[a] == lo[a] ? lo[a] : 0.f;   // (no error beside an infinite sum)
-            const float4 uf = make_float4(t[0], t[1], t[2], t[3]);
+            const float4 uf = make_float4((float)t[0], (float)t[1], (float)t[2], (float)t[3]);
             out_f[(int64_t)b * Nx + i] = uf;
             const float4 r = R[(int64_t)b * Nx + i];
             ru = (double)r.x * uf.x + (double)r.y * uf.y + (double)r.z * uf.z + (double)r.w * uf.w;
@@ -362,45 +350,32 @@ k_bwd_gather(const uint8_t *__restrict__ XT, int64_t Nx, int N, int L,
 }
 
 // The tensor-core backward leaves X^T R (scaled back) in the new-gradient
-// buffer; this adds the L2 part and does the same bookkeeping, 16 bytes of
-// each vector a thread and step.  Bound by memory: x, the old gradient, s and
-// the contraction read, the gradient and y written.  A locus per thread, in
-// blocks of 128 loci that each reduced five FP64 sums, took 98 us for 64 slots
-// of 3000 x 10,000 (0.25 GB, FP32 history); now 47.
-constexpr int GF_THREADS = 256;
-
-__global__ void __launch_bounds__(GF_THREADS)
-k_grad_finalize(int64_t L, const SlotDev *__restrict__ sd, const int32_t *__restrict__ list,
+// buffer; this adds the L2 part and does the same bookkeeping.
+__global__ void __launch_bounds__(BWD_THREADS)
+k_grad_finalize(int L, const SlotDev *__restrict__ sd, const int32_t *__restrict__ list,
                 const float *__restrict__ wa, float *__restrict__ gpool, void *__restrict__ Ypool,
                 const void *__restrict__ Spool, int hist_bf16, int m, int64_t Dp, double lambda_J,
                 double *__restrict__ acc)
 {
-    __shared__ double part[GF_THREADS / 32][8];
     const int b = list[blockIdx.y];
     const SlotDev &S = sd[b];
     const float l2 = (float)(2.0 * lambda_J);
-    const bool push = (S.flags & SLOT_F_PUSH) && S.ring_new >= 0;
-    const int64_t hoff = ((int64_t)b * m + (push ? S.ring_new : 0)) * Dp;
-    const float4 *x = reinterpret_cast<const float4 *>(wa + (int64_t)b * Dp);
-    float4 *gn = reinterpret_cast<float4 *>(gpool + (int64_t)(2 * b + 1 - S.gcur) * Dp);
-    const float4 *go = reinterpret_cast<const float4 *>(gpool + (int64_t)(2 * b + S.gcur) * Dp);
     GradRed red;
-    for (int64_t e = (int64_t)blockIdx.x * GF_THREADS + threadIdx.x; e < 4 * L; e += (int64_t)gridDim.x * GF_THREADS)
-        gn[e] = red.entries(gn[e], x[e], l2, e / 4 == S.locus, push, go + e, Ypool, Spool, hoff + 4 * e, hist_bf16);
-    double v[8] = {red.g2, red.x2, red.sy, red.yy, red.ss, 0.0, 0.0, 0.0};
-    const double t = warp_sum8(v);
-    const int lane = threadIdx.x & 31;
-    if ((lane & 3) == 0) part[threadIdx.x >> 5][lane >> 2] = t;
-    __syncthreads();
-    if (threadIdx.x < 5) {
-        const int idx[5] = {ACC_G2, ACC_X2J, ACC_SY, ACC_YY, ACC_SS};
-        double s = 0.0;
+    for (int64_t n = (int64_t)blockIdx.x * BWD_THREADS + threadIdx.x; n < L; n += (int64_t)gridDim.x * BWD_THREADS) {
+        const float4 *gr = reinterpret_cast<const float4 *>(gpool + (int64_t)(2 * b + 1 - S.gcur) * Dp + n * QQ);
+        float c[16];
 #pragma unroll
-        for (int k = 0; k < GF_THREADS / 32; ++k) s += part[k][threadIdx.x];
-        if (s != 0.0) atomicAdd(acc + (int64_t)b * NACC + idx[threadIdx.x], s);
+        for (int k4 = 0; k4 < 4; ++k4) {
+            const float4 v = gr[k4];
+            c[4 * k4] = v.x; c[4 * k4 + 1] = v.y; c[4 * k4 + 2] = v.z; c[4 * k4 + 3] = v.w;
+        }
+        grad_locus(S, b, n, c, wa, gpool, Ypool, Spool, hist_bf16, m, Dp, l2, red);
     }
+    double v[5] = {red.g2, red.x2, red.sy, red.yy, red.ss};
+    const int idx[5] = {ACC_G2, ACC_X2J, ACC_SY, ACC_YY, ACC_SS};
+    block_sum_atomic<5>(v, acc + (int64_t)b * NACC, idx);
     const float wm = warp_max(red.gmax);
-    if (lane == 0 && wm > 0.f) atomic_max_nonneg(acc + (int64_t)b * NACC + ACC_GMAX, (double)wm);
+    if ((threadIdx.x & 31) == 0 && wm > 0.f) atomic_max_nonneg(acc + (int64_t)b * NACC + ACC_GMAX, (double)wm);
 }
 
 // ---- one evaluation (sdca_eval): the same sums as the batch kernels above and
@@ -673,11 +648,10 @@ void launch_grad_finalize(const Problem &P, const SlotDev *sd, const int32_t *li
                           double *acc, cudaStream_t st)
 {
     if (n <= 0) return;
-    // about eight blocks per SM in all, each thread some steps long
-    const int64_t need = (4 * P.L + GF_THREADS - 1) / GF_THREADS, per_slot = std::max<int64_t>(1, (8 * 152 + n - 1) / n);
-    dim3 grid((unsigned)std::min(need, per_slot), (unsigned)n);
-    k_grad_finalize<<<grid, GF_THREADS, 0, st>>>(P.L, sd, list, wa, gpool, Ypool, Spool, hist_bf16,
-                                                  P.ring, P.Dp, P.lambda_J, acc);
+    const int64_t need = (P.L + BWD_THREADS - 1) / BWD_THREADS;
+    dim3 grid((unsigned)(need < 512 ? need : 512), (unsigned)n);
+    k_grad_finalize<<<grid, BWD_THREADS, 0, st>>>((int)P.L, sd, list, wa, gpool, Ypool, Spool, hist_bf16,
+                                                   P.ring, P.Dp, P.lambda_J, acc);
 }
 
 void launch_bwd_gather(const Problem &P, const uint8_t *XT, const SlotDev *sd,

@@ -156,8 +156,21 @@ k_search(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N
                 v[2] += r[0]; v[3] += r[1]; v[4] += r[2]; v[5] += r[3];
                 R[o0 + i] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
             }
-            const double t = warp_sum8(v);
-            if ((lane & 3) == 0) warp_part[wid][lane >> 2] = t;
+            // six sums over the warp by halving what each lane keeps: 4, 2 and
+            // 1 values, then two plain steps; lane 4 k holds value k (bits
+            // of k: lane bits 16, 8, 4)
+#pragma unroll
+            for (int s = 0, h = 4; s < 3; ++s, h >>= 1) {
+                const int bit = 16 >> s;
+#pragma unroll
+                for (int k = 0; k < h; ++k) {
+                    const double give = lane & bit ? v[k] : v[k + h], keep = lane & bit ? v[k + h] : v[k];
+                    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            }
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+            if ((lane & 3) == 0) warp_part[wid][lane >> 2] = v[0];
         }
         __syncthreads();
         const int k8 = lane & 7, g8 = lane >> 3;   // the searcher's lane: value, and one of four groups of rows

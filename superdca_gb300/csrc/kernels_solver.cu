@@ -343,215 +343,138 @@ __global__ void k_hpart(const SlotDev *__restrict__ sd, const int32_t *__restric
 }
 
 constexpr int DOT_THREADS = 256;
-constexpr int DOT_E = 16;   // entries per thread and tile: 16-byte loads of four (FP32) or eight (BF16) each
-constexpr int DOT_BLOCKS = 2 * 152;   // resident blocks
+constexpr int DOT_U = 4;  // float4 groups per thread per tile: 16 KB runs per stream per block
 
-// A thread's entries of a tile: load u covers the E entries from
-// E (t0 + u DOT_THREADS), E = 4 or 8 by the history's type
-template <bool BF16> struct Tile {
-    static constexpr int E = BF16 ? 8 : 4, U = DOT_E / E;
-    int64_t t0, n;   // in loads
-    __device__ Tile(int64_t tile, int64_t Dp) : t0(tile * (DOT_THREADS * U) + threadIdx.x), n(Dp / E) {}
-    __device__ __forceinline__ bool has(int u) const { return t0 + u * DOT_THREADS < n; }
-    __device__ __forceinline__ int64_t entry(int u) const { return (t0 + u * DOT_THREADS) * E; }
-    // FP32 vector
-    __device__ __forceinline__ void load_f(const float *v, float (&x)[DOT_E]) const
-    {
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int q = 0; q < E / 4; ++q) {
-                const float4 f = has(u) ? reinterpret_cast<const float4 *>(v + entry(u))[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-                x[u * E + 4 * q] = f.x; x[u * E + 4 * q + 1] = f.y; x[u * E + 4 * q + 2] = f.z; x[u * E + 4 * q + 3] = f.w;
-            }
-    }
-    // history vector at offset off: the loads, and their values
-    __device__ __forceinline__ void load_h(const void *v, int64_t off, uint4 (&raw)[U]) const
-    {
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            raw[u] = has(u) ? *reinterpret_cast<const uint4 *>(reinterpret_cast<const char *>(v) + (off + entry(u)) * (BF16 ? 2 : 4))
-                            : make_uint4(0, 0, 0, 0);
-    }
-    static __device__ __forceinline__ void values(const uint4 (&raw)[U], float (&x)[DOT_E])
-    {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if constexpr (BF16) {
-                    x[u * 8 + 2 * q] = __uint_as_float(w[q] << 16);
-                    x[u * 8 + 2 * q + 1] = __uint_as_float(w[q] & 0xFFFF0000u);
-                } else {
-                    x[u * 4 + q] = __uint_as_float(w[q]);
-                }
-            }
-        }
-    }
-};
-
-__device__ __forceinline__ float dot_e(const float (&a)[DOT_E], const float (&b)[DOT_E])
-{
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < DOT_E; ++k) t = fmaf(a[k], b[k], t);
-    return t;
-}
-
-// dots[b] = [S_j.g | Y_j.g | S_j.y_new | Y_j.y_new], j over the history; a
-// block takes the s or the y vectors (blockIdx.z) of a stretch of tiles: g and
-// y_new stay in registers while the vectors stream through, one on its way
-// while one is summed.
-//
-// Bound by memory: 20 history vectors, g and y_new.  Both kinds of vectors in
-// one block (128 registers, 40 sums reduced by five shuffles each and a chain
-// of FP64 additions per sum) and grids of 10 blocks per slot whatever they left
-// of a wave took 205 us for 64 slots of 3000 x 10,000 (FP32 history, 0.9 GB)
-// and 111 for 1000 x 4001 (BF16, 0.2 GB); now 165 and 54.
-template <bool BF16>
-__global__ void __launch_bounds__(DOT_THREADS, 2)
+// dots[b] = [S_j.g | Y_j.g | S_j.y_new | Y_j.y_new], j over the history.
+// Blocks walk tiles of DOT_THREADS x DOT_U float4 groups; within a tile g and
+// y_new stay in registers while the history vectors stream through one at a
+// time, so every stream is read in long contiguous runs.
+__global__ void __launch_bounds__(DOT_THREADS)
 k_hist_dots(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int64_t Dp, int m,
             const float *__restrict__ gpool, const void *__restrict__ Spool,
-            const void *__restrict__ Ypool, double *__restrict__ dots)
+            const void *__restrict__ Ypool, int hist_bf16, double *__restrict__ dots)
 {
-    using T = Tile<BF16>;
-    constexpr int AHEAD = BF16 ? 4 : 2;   // vectors on their way
-    __shared__ float part[DOT_THREADS / 32][32];
     const int b = list[blockIdx.y];
     const SlotDev &S = sd[b];
     const int nh = S.nhist;
-    const bool isy = blockIdx.z;
-    const float *g = gpool + (int64_t)(2 * b + S.gcur) * Dp;
+    const float4 *g4 = reinterpret_cast<const float4 *>(gpool + (int64_t)(2 * b + S.gcur) * Dp);
     const bool has_new = S.ring_new >= 0;
     const int64_t ybase = ((int64_t)b * m + (has_new ? S.ring_new : 0)) * Dp;
-    const void *pool = isy ? Ypool : Spool;
-    const int64_t tiles = (Dp + DOT_THREADS * DOT_E - 1) / (DOT_THREADS * DOT_E);
-    float v[32];   // [0, MAXHIST) with g, [MAXHIST, 2 MAXHIST) with y_new
+    const int64_t nv4 = Dp / 4, tile = (int64_t)DOT_THREADS * DOT_U;
+    float aSg[MAXHIST], aYg[MAXHIST], aSy[MAXHIST], aYy[MAXHIST];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) v[k] = 0.f;
-    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const T t(tile, Dp);
-        float gv[DOT_E], yn[DOT_E];
-        uint4 next[AHEAD][T::U];
+    for (int j = 0; j < MAXHIST; ++j) aSg[j] = aYg[j] = aSy[j] = aYy[j] = 0.f;
+    for (int64_t tb = (int64_t)blockIdx.x * tile; tb < nv4; tb += (int64_t)gridDim.x * tile) {
+        float4 gv[DOT_U], yn[DOT_U];
 #pragma unroll
-        for (int j = 0; j < AHEAD; ++j)
-            if (j < nh) t.load_h(pool, ((int64_t)b * m + S.ring[j]) * Dp, next[j]);
-        t.load_f(g, gv);
-        if (has_new) {
-            uint4 raw[T::U];
-            t.load_h(Ypool, ybase, raw);
-            T::values(raw, yn);
-        } else {
-#pragma unroll
-            for (int k = 0; k < DOT_E; ++k) yn[k] = 0.f;
+        for (int u = 0; u < DOT_U; ++u) {
+            const int64_t v = tb + u * DOT_THREADS + threadIdx.x;
+            const bool ok = v < nv4;
+            gv[u] = ok ? g4[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+            yn[u] = (ok && has_new) ? load_hist4(Ypool, ybase + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int j = 0; j < MAXHIST; ++j) {
             if (j < nh) {
-                float x[DOT_E];
-                T::values(next[j % AHEAD], x);
-                if (j + AHEAD < nh) t.load_h(pool, ((int64_t)b * m + S.ring[j + AHEAD]) * Dp, next[j % AHEAD]);
-                v[j] += dot_e(x, gv);
-                v[MAXHIST + j] += dot_e(x, yn);
+                const int64_t base = ((int64_t)b * m + S.ring[j]) * Dp;
+                float4 sv[DOT_U], yv[DOT_U];
+#pragma unroll
+                for (int u = 0; u < DOT_U; ++u) {
+                    const int64_t v = tb + u * DOT_THREADS + threadIdx.x;
+                    const bool ok = v < nv4;
+                    sv[u] = ok ? load_hist4(Spool, base + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    yv[u] = ok ? load_hist4(Ypool, base + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int u = 0; u < DOT_U; ++u) {
+                    aSg[j] += dot4(sv[u], gv[u]);
+                    aYg[j] += dot4(yv[u], gv[u]);
+                    aSy[j] += dot4(sv[u], yn[u]);
+                    aYy[j] += dot4(yv[u], yn[u]);
+                }
             }
         }
     }
-    // sums over the warp by halving what each lane keeps: lane k holds value k
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float v[4 * MAXHIST];
+    int idx[4 * MAXHIST];
 #pragma unroll
-    for (int s = 0, h = 16; s < 5; ++s, h >>= 1) {
-        const bool up = lane & h;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const float give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
-        }
+    for (int j = 0; j < MAXHIST; ++j) {
+        v[j] = aSg[j];
+        v[MAXHIST + j] = aYg[j];
+        v[2 * MAXHIST + j] = aSy[j];
+        v[3 * MAXHIST + j] = aYy[j];
     }
-    part[wid][lane] = v[0];
-    __syncthreads();
-    if (threadIdx.x < 2 * MAXHIST) {
-        const int k = threadIdx.x, j = k % MAXHIST, q = k / MAXHIST;
-        double t = 0.0;
 #pragma unroll
-        for (int w = 0; w < DOT_THREADS / 32; ++w) t += part[w][k];
-        if (j < nh && t != 0.0) atomicAdd(dots + (int64_t)b * 4 * MAXHIST + (2 * q + isy) * MAXHIST + j, t);
-    }
+    for (int k = 0; k < 4 * MAXHIST; ++k) idx[k] = k;
+    block_sum_atomic_f<4 * MAXHIST>(v, dots + (int64_t)b * 4 * MAXHIST, idx);
 }
 
 // d = coef_g g + sum_j (coefS_j s_j + coefY_j y_j), J_rr block zero;
 // reductions g.d, d.d and x.d split into the J and h parts, and max|d|.
-// Same tiling as k_hist_dots, s and y of a pair together: d and g of a tile
-// stay in registers while the history streams through.  (8-byte loads of a
-// BF16 history and 10 blocks per slot: 185 us at 64 slots of 3000 x 10,000, 74
-// at 1000 x 4001; now 155 and 46.)
-template <bool BF16>
-__global__ void __launch_bounds__(DOT_THREADS, 2)
+// Same tiling as k_hist_dots: d and g of a tile stay in registers while the
+// history streams through.
+__global__ void __launch_bounds__(DOT_THREADS)
 k_direction(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int64_t L,
             int64_t Dp, int m, const float *__restrict__ gpool, const void *__restrict__ Spool,
-            const void *__restrict__ Ypool, const float *__restrict__ wa,
+            const void *__restrict__ Ypool, int hist_bf16, const float *__restrict__ wa,
             float *__restrict__ d, double *__restrict__ acc)
 {
-    using T = Tile<BF16>;
-    constexpr int AHEAD = BF16 ? 2 : 1;   // pairs on their way
     const int b = list[blockIdx.y];
     const SlotDev &S = sd[b];
     const int nh = S.nhist;
-    const float *g = gpool + (int64_t)(2 * b + S.gcur) * Dp, *x = wa + (int64_t)b * Dp;
+    const float4 *g4 = reinterpret_cast<const float4 *>(gpool + (int64_t)(2 * b + S.gcur) * Dp);
+    const float4 *x4 = reinterpret_cast<const float4 *>(wa + (int64_t)b * Dp);
+    float4 *d4 = reinterpret_cast<float4 *>(d + (int64_t)b * Dp);
     const float cg = (float)S.coef_g;
-    const int64_t hoff = QQ * L, rlo = (int64_t)S.locus * QQ, rhi = rlo + QQ;
-    const int64_t tiles = (Dp + DOT_THREADS * DOT_E - 1) / (DOT_THREADS * DOT_E);
+    const int64_t hoff4 = QQ * L / 4;
+    const int64_t rlo4 = (int64_t)S.locus * QQ / 4, rhi4 = rlo4 + QQ / 4;
+    const int64_t nv4 = Dp / 4, tile = (int64_t)DOT_THREADS * DOT_U;
     float gd = 0.f, ddJ = 0.f, ddH = 0.f, xdJ = 0.f, xdH = 0.f, dmax = 0.f;
-    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const T t(tile, Dp);
-        uint4 sn[AHEAD][T::U], yn[AHEAD][T::U];
+    for (int64_t tb = (int64_t)blockIdx.x * tile; tb < nv4; tb += (int64_t)gridDim.x * tile) {
+        float4 gv[DOT_U], dv[DOT_U];
 #pragma unroll
-        for (int j = 0; j < AHEAD; ++j)
-            if (j < nh) {
-                const int64_t base = ((int64_t)b * m + S.ring[j]) * Dp;
-                t.load_h(Spool, base, sn[j]);
-                t.load_h(Ypool, base, yn[j]);
-            }
-        float gv[DOT_E], dv[DOT_E];
-        t.load_f(g, gv);
-#pragma unroll
-        for (int k = 0; k < DOT_E; ++k) dv[k] = cg * gv[k];
+        for (int u = 0; u < DOT_U; ++u) {
+            const int64_t v = tb + u * DOT_THREADS + threadIdx.x;
+            gv[u] = v < nv4 ? g4[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+            dv[u] = make_float4(cg * gv[u].x, cg * gv[u].y, cg * gv[u].z, cg * gv[u].w);
+        }
 #pragma unroll
         for (int j = 0; j < MAXHIST; ++j) {
             if (j < nh) {
+                const int64_t base = ((int64_t)b * m + S.ring[j]) * Dp;
                 const float cs = (float)S.coefS[j], cy = (float)S.coefY[j];
-                float sv[DOT_E], yv[DOT_E];
-                T::values(sn[j % AHEAD], sv);
-                T::values(yn[j % AHEAD], yv);
-                if (j + AHEAD < nh) {
-                    const int64_t base = ((int64_t)b * m + S.ring[j + AHEAD]) * Dp;
-                    t.load_h(Spool, base, sn[j % AHEAD]);
-                    t.load_h(Ypool, base, yn[j % AHEAD]);
+                float4 sv[DOT_U], yv[DOT_U];
+#pragma unroll
+                for (int u = 0; u < DOT_U; ++u) {
+                    const int64_t v = tb + u * DOT_THREADS + threadIdx.x;
+                    const bool ok = v < nv4;
+                    sv[u] = ok ? load_hist4(Spool, base + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    yv[u] = ok ? load_hist4(Ypool, base + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
-                for (int k = 0; k < DOT_E; ++k) dv[k] += cs * sv[k] + cy * yv[k];
+                for (int u = 0; u < DOT_U; ++u) {
+                    dv[u].x += cs * sv[u].x + cy * yv[u].x;
+                    dv[u].y += cs * sv[u].y + cy * yv[u].y;
+                    dv[u].z += cs * sv[u].z + cy * yv[u].z;
+                    dv[u].w += cs * sv[u].w + cy * yv[u].w;
+                }
             }
         }
 #pragma unroll
-        for (int u = 0; u < T::U; ++u) {
-            if (!t.has(u)) continue;
-#pragma unroll
-            for (int q = 0; q < T::E / 4; ++q) {
-                const int64_t e = t.entry(u) + 4 * q;
-                const int k = u * T::E + 4 * q;
-                float4 D = make_float4(dv[k], dv[k + 1], dv[k + 2], dv[k + 3]);
-                if (e >= rlo && e < rhi) D = make_float4(0.f, 0.f, 0.f, 0.f);
-                *reinterpret_cast<float4 *>(d + (int64_t)b * Dp + e) = D;
-                const float4 X = *reinterpret_cast<const float4 *>(x + e);
-                gd += dot4(make_float4(gv[k], gv[k + 1], gv[k + 2], gv[k + 3]), D);
-                dmax = fmaxf(dmax, fmaxf(fmaxf(fabsf(D.x), fabsf(D.y)), fmaxf(fabsf(D.z), fabsf(D.w))));
-                if (e < hoff) {
-                    ddJ += dot4(D, D);
-                    xdJ += dot4(X, D);
-                } else {
-                    ddH += dot4(D, D);
-                    xdH += dot4(X, D);
-                }
+        for (int u = 0; u < DOT_U; ++u) {
+            const int64_t v = tb + u * DOT_THREADS + threadIdx.x;
+            if (v >= nv4) continue;
+            if (v >= rlo4 && v < rhi4) dv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            d4[v] = dv[u];
+            const float4 xv = x4[v];
+            gd += dot4(gv[u], dv[u]);
+            dmax = fmaxf(dmax, fmaxf(fmaxf(fabsf(dv[u].x), fabsf(dv[u].y)), fmaxf(fabsf(dv[u].z), fabsf(dv[u].w))));
+            if (v < hoff4) {
+                ddJ += dot4(dv[u], dv[u]);
+                xdJ += dot4(xv, dv[u]);
+            } else {
+                ddH += dot4(dv[u], dv[u]);
+                xdH += dot4(xv, dv[u]);
             }
         }
     }
@@ -637,25 +560,6 @@ unsigned dgrid(int64_t Dp, int threads, int64_t cap = 256)
     return (unsigned)(need < cap ? need : cap);
 }
 
-int64_t Dp_tiles(int64_t Dp) { return (Dp + DOT_THREADS * DOT_E - 1) / (DOT_THREADS * DOT_E); }
-
-// blocks per slot for a pass over `tiles` tiles of each of n slots: the
-// fewest, up to four waves, whose waves of resident blocks take the least tiles in a row (a
-// block's reduction counted as half a tile)
-unsigned tile_blocks(int64_t tiles, int64_t n)
-{
-    int64_t best = 1;
-    double least = 1e300;
-    for (int64_t c = 1; c <= std::min<int64_t>(tiles, std::max<int64_t>(1, 4 * DOT_BLOCKS / n)); ++c) {
-        const double t = (double)((n * c + DOT_BLOCKS - 1) / DOT_BLOCKS) * ((double)((tiles + c - 1) / c) + 0.5);
-        if (t < least) {
-            least = t;
-            best = c;
-        }
-    }
-    return (unsigned)best;
-}
-
 } // namespace
 
 void launch_slots_begin(const Problem &P, const int2 *who, int n, const uint8_t *states, uint8_t *rstate, float *wa,
@@ -725,9 +629,12 @@ void launch_hist_dots(const Problem &P, const SlotDev *sd, const int32_t *list, 
                       double *dots, cudaStream_t st)
 {
     if (n <= 0) return;
-    dim3 grid(tile_blocks(Dp_tiles(P.Dp), 2 * n), (unsigned)n, 2);
-    if (hist_bf16) k_hist_dots<true><<<grid, DOT_THREADS, 0, st>>>(sd, list, P.Dp, P.ring, gpool, Spool, Ypool, dots);
-    else k_hist_dots<false><<<grid, DOT_THREADS, 0, st>>>(sd, list, P.Dp, P.ring, gpool, Spool, Ypool, dots);
+    // enough blocks for about two waves in total, each thread streaming
+    // hundreds of float4 before the block reduction
+    const int64_t per_slot = std::max<int64_t>(4, std::min<int64_t>(64, (4 * 152 + n - 1) / n));
+    dim3 grid(dgrid(P.Dp, DOT_THREADS * DOT_U, per_slot), (unsigned)n);
+    k_hist_dots<<<grid, DOT_THREADS, 0, st>>>(sd, list, P.Dp, P.ring, gpool, Spool, Ypool, hist_bf16,
+                                              dots);
 }
 
 void launch_direction(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
@@ -735,9 +642,10 @@ void launch_direction(const Problem &P, const SlotDev *sd, const int32_t *list, 
                       const float *wa, float *d, double *acc, cudaStream_t st)
 {
     if (n <= 0) return;
-    dim3 grid(tile_blocks(Dp_tiles(P.Dp), n), (unsigned)n);
-    if (hist_bf16) k_direction<true><<<grid, DOT_THREADS, 0, st>>>(sd, list, P.L, P.Dp, P.ring, gpool, Spool, Ypool, wa, d, acc);
-    else k_direction<false><<<grid, DOT_THREADS, 0, st>>>(sd, list, P.L, P.Dp, P.ring, gpool, Spool, Ypool, wa, d, acc);
+    const int64_t per_slot = std::max<int64_t>(4, std::min<int64_t>(128, (4 * 152 + n - 1) / n));
+    dim3 grid(dgrid(P.Dp, DOT_THREADS * DOT_U, per_slot), (unsigned)n);
+    k_direction<<<grid, DOT_THREADS, 0, st>>>(sd, list, P.L, P.Dp, P.ring, gpool, Spool, Ypool,
+                                              hist_bf16, wa, d, acc);
 }
 
 void launch_score(const Problem &P, const SlotDev *sd, const int32_t *list, int n,

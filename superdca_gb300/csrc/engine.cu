@@ -44,7 +44,8 @@ std::string g_create_err;
 enum Phase {
     PH_EMPTY = 0,
     PH_INIT,        // needs the evaluation at its start point
-    PH_LS,          // a direction is ready: needs its line search
+    PH_LS,          // line search: needs a trial at ls.stp
+    PH_FINAL_EVAL,  // search ended without a trial at its step: evaluate there
     PH_READY_INIT,  // start point evaluated, waiting for the gradient pass
     PH_READY_STEP,  // step accepted, waiting for the gradient pass
     PH_FINALIZE,    // converged: logits refreshed, needs the final evaluation
@@ -89,7 +90,7 @@ struct SlotHost {
     // lives on the device): h part of x, max |a| of the gradient and of x
     double eta_x[Q] = {0, 0, 0, 0};
     double amax_g = 0.0, amax_x = 0.0;
-    double alpha = 0.0;      // first trial step of the next search
+    MoreThuente ls;
 };
 
 struct ProfRec {
@@ -536,8 +537,6 @@ int upload_list(sdca_handle *h, const std::vector<int32_t> &lst)
     return staged_h2d(h, h->list, lst.data(), sizeof(int32_t) * lst.size());
 }
 
-LineL2 line_l2(const SlotHost &S) { return {S.x2J, S.x2H, S.xdJ, S.xdH, S.ddJ, S.ddH}; }
-
 // copy the host slot parameters of `lst` into the device mirror
 int upload_slots(sdca_handle *h, const std::vector<int32_t> &lst)
 {
@@ -549,11 +548,8 @@ int upload_slots(sdca_handle *h, const std::vector<int32_t> &lst)
         D.ring_new = S.ring_new;
         D.nhist = (int)S.hist.size();
         for (int j = 0; j < D.nhist; ++j) D.ring[j] = S.hist[j];
-        D.flags = (S.use_u ? SLOT_F_USE_U : 0) | (S.push ? SLOT_F_PUSH : 0) | (S.phase == PH_LS ? SLOT_F_SEARCH : 0);
+        D.flags = (S.use_u ? SLOT_F_USE_U : 0) | (S.push ? SLOT_F_PUSH : 0);
         D.stp = S.stp;
-        D.f0 = S.f;
-        D.alpha = S.alpha;
-        D.l2 = line_l2(S);
         for (int a = 0; a < Q; ++a) D.rs[a] = S.rs[a];
     }
     // the mirror is small; copy it whole
@@ -942,7 +938,19 @@ int retire(sdca_handle *h, Queue &Qu, const std::vector<int32_t> &done)
     return SDCA_OK;
 }
 
-// phase A: the line searches, and single evaluations, until no slot needs one
+double l2_along(const Problem &P, const SlotHost &S, double stp)
+{
+    const double j2 = S.x2J + 2.0 * stp * S.xdJ + stp * stp * S.ddJ;
+    const double h2 = S.x2H + 2.0 * stp * S.xdH + stp * stp * S.ddH;
+    return P.lambda_J * j2 + P.lambda_h * h2;
+}
+
+double dl2_along(const Problem &P, const SlotHost &S, double stp)
+{
+    return 2.0 * P.lambda_J * (S.xdJ + stp * S.ddJ) + 2.0 * P.lambda_h * (S.xdH + stp * S.ddH);
+}
+
+// phase A: line-search rounds until no slot needs a trial
 int phase_trials(sdca_handle *h, Queue &Qu)
 {
     const Problem &P = h->P;
@@ -950,16 +958,18 @@ int phase_trials(sdca_handle *h, Queue &Qu)
         std::vector<int32_t> lst;
         for (int b = 0; b < P.Bmax; ++b) {
             const int ph = h->slots[b].phase;
-            if (ph == PH_INIT || ph == PH_LS || ph == PH_FINALIZE || ph == PH_REFRESH) lst.push_back(b);
+            if (ph == PH_INIT || ph == PH_LS || ph == PH_FINAL_EVAL || ph == PH_FINALIZE || ph == PH_REFRESH)
+                lst.push_back(b);
         }
         if (lst.empty()) return SDCA_OK;
         int rc = upload_slots(h, lst);
         if (rc) return rc;
+        rc = zero_acc(h);
+        if (rc) return rc;
         {
-            // (the slopes at 0 that the forward left in acc start the searches)
             Timed t(h, SDCA_K_LINESEARCH, 1, (int64_t)lst.size());
-            launch_search(P, h->sd, h->list, (int)lst.size(), h->lbase, h->u, h->rstate, h->w, h->R, h->acc,
-                          h->stream);
+            launch_trial(P, h->sd, h->list, (int)lst.size(), h->lbase, h->u, h->rstate, h->w, h->R, h->acc,
+                         h->stream);
         }
         CKL();
         rc = fetch_acc(h);
@@ -978,21 +988,27 @@ int phase_trials(sdca_handle *h, Queue &Qu)
             } else if (S.phase == PH_FINALIZE) {
                 S.f_final = fdata + P.lambda_J * S.x2J + P.lambda_h * S.x2H;
                 done.push_back(b);
-            } else {  // PH_LS: the accepted point is the last trial
-                S.stp = acc_get(h, b, ACC_STP);
-                S.f = fdata + line_l2(S).value(P.lambda_J, P.lambda_h, S.stp);
-                S.trials = (int)acc_get(h, b, ACC_TRIALS);
+            } else if (S.phase == PH_FINAL_EVAL) {
+                S.f = fdata + l2_along(P, S, S.stp);
                 S.phase = PH_READY_STEP;
-                const int outcome = (int)acc_get(h, b, ACC_LS);
-                if (outcome == LS_NO_DESCENT) {
-                    // not downhill along this line: stay, and restart from
-                    // steepest descent at the next iteration
-                    if (S.hist.empty()) S.stalled = true;
-                    else S.force_restart = true;
-                    S.weak++;
-                } else if (outcome != LS_NOT_FINITE) {
-                    if (outcome != LS_MET) S.weak++;
+            } else {  // PH_LS
+                const double f = fdata + l2_along(P, S, S.stp);
+                const double dg = acc_get(h, b, ACC_DG) + dl2_along(P, S, S.stp);
+                S.trials++;
+                if (!std::isfinite(f) || !std::isfinite(dg)) {
+                    S.f = f;
+                    S.phase = PH_READY_STEP;
+                    continue;
+                }
+                const double stp_eval = S.stp;
+                if (S.ls.feed(f, dg) == MoreThuente::DONE) {
+                    S.stp = stp_eval;  // the accepted point is the last trial
+                    S.f = f;
+                    S.phase = PH_READY_STEP;
+                    if (S.ls.info != 1) S.weak++;
                     S.max_trials = std::max(S.max_trials, S.trials);
+                } else {
+                    S.stp = S.ls.stp;
                 }
             }
         }
@@ -1075,10 +1091,12 @@ int phase_step(sdca_handle *h)
             }
             rc = upload_slots(h, fresh);
             if (rc) return rc;
+            rc = zero_acc(h);
+            if (rc) return rc;
             {
                 Timed t(h, SDCA_K_LINESEARCH, 1, (int64_t)fresh.size());
-                launch_search(P, h->sd, h->list, (int)fresh.size(), h->lbase, h->u, h->rstate, h->w, h->R,
-                              h->acc, h->stream);
+                launch_trial(P, h->sd, h->list, (int)fresh.size(), h->lbase, h->u, h->rstate, h->w, h->R,
+                             h->acc, h->stream);
             }
             CKL();
             rc = fetch_acc(h);
@@ -1351,14 +1369,28 @@ int phase_step(sdca_handle *h)
     if (rc) return rc;
     rc = run_forward(h, cont, h->d, false);
     if (rc) return rc;
+    rc = fetch_acc(h);
+    if (rc) return rc;
     for (int b : cont) {
         SlotHost &S = h->slots[b];
-        S.alpha = restarted[b] ? 1.0 : 1.0 / std::sqrt(S.g2);
-        S.stp = 0.0;
+        const double alpha_init = restarted[b] ? 1.0 : 1.0 / std::sqrt(S.g2);
         S.trials = 0;
         S.use_u = true;
         S.push = false;
-        S.phase = PH_LS;
+        // slope of the search line at 0 from the numbers the trials use
+        const double dg0 = acc_get(h, b, ACC_DG0) + dl2_along(P, S, 0.0);
+        if (S.ls.start(S.f, dg0, alpha_init) == MoreThuente::NEED_EVAL) {
+            S.stp = S.ls.stp;
+            S.phase = PH_LS;
+        } else {
+            // not downhill along this line: stay, and restart from steepest
+            // descent at the next iteration
+            S.stp = 0.0;
+            S.phase = PH_FINAL_EVAL;
+            if (S.hist.empty()) S.stalled = true;
+            else S.force_restart = true;
+            S.weak++;
+        }
     }
     return SDCA_OK;
 }

@@ -18,7 +18,6 @@
 #include <cuda_runtime.h>
 
 #include "../../include/superdca_gb300.h"
-#include "linesearch.h"
 
 namespace sdca {
 
@@ -53,9 +52,9 @@ constexpr int MLP_ALPHA = 2;      // version 2: the shrinkage of the predicted r
 
 // per-slot accumulators (doubles), zeroed by the host before each use
 enum Acc {
-    ACC_F = 0,      // sum_i w_i (lse_i - l_i[s_i(r)])             (search)
-    ACC_DG,         // sum_i R_i . u_i                              (search)
-    ACC_RS0,        // sum_i R_i[a], a = 0..3                       (search)
+    ACC_F = 0,      // sum_i w_i (lse_i - l_i[s_i(r)])             (trial)
+    ACC_DG,         // sum_i R_i . u_i                              (trial)
+    ACC_RS0,        // sum_i R_i[a], a = 0..3                       (trial)
     ACC_RS1, ACC_RS2, ACC_RS3,
     ACC_G2,         // ||g||^2                                      (gradient)
     ACC_X2J,        // ||x_J||^2                                    (gradient)
@@ -71,16 +70,8 @@ enum Acc {
     ACC_DMAX,       // max |d| (bits of a non-negative double, atomicMax) (direction)
     ACC_DG0,        // sum_i R_i . u_i at the current point: slope of the search line at 0 (forward)
     ACC_SS,         // s_k . s_k                                    (gradient)
-    ACC_STP,        // step of the last trial                       (search)
-    ACC_TRIALS,     // trials taken                                 (search)
-    ACC_LS,         // LineOutcome                                  (search)
-    NACC = 24
+    NACC = 20
 };
-
-// how a line search ended: a step that meets both conditions; the last trial
-// of a search that ended otherwise; not downhill (the point itself was
-// evaluated); a value that is not finite
-enum LineOutcome { LS_MET = 0, LS_ENDED, LS_NO_DESCENT, LS_NOT_FINITE };
 
 // Per-slot parameters the kernels read; mirrored from the host before launches.
 struct SlotDev {
@@ -99,8 +90,6 @@ struct SlotDev {
     double tc_scale;        // power of two applied to d before the fp16 hi/lo split
     double tc_inv_scale;
     double eta[Q];          // dual form: h part of the direction (trial logits) or of x (final layout)
-    double f0, alpha;       // a search: the objective at step 0, the first trial step
-    LineL2 l2;              // a search: the L2 part along the line
 };
 
 // dual form: per slot, vectors (a, k = K a) of N x 4 doubles each:
@@ -193,7 +182,6 @@ constexpr int TS_WORDS = 2 * TS_KERNELS;
 enum SlotFlags {
     SLOT_F_USE_U = 1,       // trial logits use lbase + stp u (else lbase)
     SLOT_F_PUSH = 2,        // accept pushes an (s, y) pair into the history
-    SLOT_F_SEARCH = 4,      // search along d (else one evaluation at stp)
 };
 
 struct DevBuf {
@@ -240,9 +228,9 @@ void launch_hpart(const Problem &P, const SlotDev *sd, const int32_t *list, int 
                   double *acc, cudaStream_t st);
 void launch_slots_begin(const Problem &P, const int2 *who, int n, const uint8_t *states, uint8_t *rstate, float *wa,
                         float *d, double *lbase, float2 *dv, int64_t dv_slot, DualCtl *ctl, cudaStream_t st);
-void launch_search(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
-                   const double *lbase, const float *u, const uint8_t *rstate, const double *w,
-                   float *R, double *acc, cudaStream_t st);
+void launch_trial(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
+                  const double *lbase, const float *u, const uint8_t *rstate, const double *w,
+                  float *R, double *acc, cudaStream_t st);
 void launch_accept(const Problem &P, const SlotDev *sd, const int32_t *list, int n, float *wa,
                    const float *d, void *Spool, int hist_bf16, cudaStream_t st);
 void launch_lbase_update(const Problem &P, const SlotDev *sd, const int32_t *list, int n,

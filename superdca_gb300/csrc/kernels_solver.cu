@@ -7,21 +7,25 @@
 // u_i = X_i . d_J + d_h, so a trial needs O(N q) work per slot.  This is
 // exactly SuperDCA's objective along the search line (plmDCA_objective.hpp:
 // 126-151 for the pseudo-likelihood part; the L2 part is a quadratic in stp
-// from x.d and d.d).
+// that the host evaluates from x.d and d.d).
 #include <algorithm>
-#include <new>
 
-#include <cooperative_groups.h>
-
+#include "df.cuh"
 #include "engine.h"
-#include "exp_log64.h"
 #include "kernels_common.cuh"
 
 namespace sdca {
 
 namespace {
 
-// base logits (FP64)
+constexpr int TRIAL_THREADS = 256;
+
+// the direction's logits u and the base logits: float4 / FP64
+__device__ __forceinline__ double4 load4(const float4 *u, int64_t o)
+{
+    const float4 v = u[o];
+    return make_double4(v.x, v.y, v.z, v.w);
+}
 __device__ __forceinline__ double4 load4(const double *v, int64_t o)
 {
     const double2 a = reinterpret_cast<const double2 *>(v + o * 4)[0];
@@ -29,195 +33,44 @@ __device__ __forceinline__ double4 load4(const double *v, int64_t o)
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
-constexpr int SEARCH_WARPS = 15, SEARCH_THREADS = 32 * SEARCH_WARPS;   // evaluating; one more searches
-constexpr int SEARCH_CLUSTER = 8;
-constexpr int SEARCH_K = 6;   // sums of a trial: f, slope, R per state
-
-// order of doubles as 64-bit integers (comparisons are FP64 work too)
-__device__ __forceinline__ bool above_eq(double a, double b)
+template <typename UT, typename LT>
+__global__ void __launch_bounds__(TRIAL_THREADS)
+k_trial(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N, int64_t Nx,
+        const LT *__restrict__ lbase, const UT *__restrict__ u,
+        const uint8_t *__restrict__ rstate, const double *__restrict__ w, float4 *__restrict__ R,
+        double *__restrict__ acc)
 {
-    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-    const long long kx = x ^ ((x >> 63) & 0x7fffffffffffffffll), ky = y ^ ((y >> 63) & 0x7fffffffffffffffll);
-    return kx >= ky;
-}
-
-// One sequence at logits l, state sr, weight w: adds w (lse - l[sr]) to f and
-// gives the residuals w (p - [a = sr]).  The largest logit's exponential is 1,
-// so three are left.
-__device__ __forceinline__ void belief(const double (&l)[4], int sr, double w, const ExpTab *E, const LogTab *G,
-                                       double &f, double (&r)[4])
-{
-    const bool a = above_eq(l[0], l[1]), b = above_eq(l[2], l[3]);
-    const double M0 = a ? l[0] : l[1], M1 = b ? l[2] : l[3];
-    const bool c = above_eq(M0, M1);
-    const double mx = c ? M0 : M1;
-    const double dn0 = (a ? l[1] : l[0]) - mx, dn1 = (b ? l[3] : l[2]) - mx, dm = (c ? M1 : M0) - mx;
-    const double en0 = exp64(dn0, E), en1 = exp64(dn1, E), em = exp64(dm, E);
-    // (an infinite largest logit leaves no belief)
-    const double one = (__double2hiint(mx) & 0x7ff00000) == 0x7ff00000 ? __longlong_as_double(0x7ff8000000000000ll) : 1.0;
-    const double z = (one + em) + (en0 + en1);
-    const double dM0 = c ? 0.0 : dm, dM1 = c ? dm : 0.0;
-    const double d[4] = {a ? dM0 : dn0, a ? dn0 : dM0, b ? dM1 : dn1, b ? dn1 : dM1};
-    const double ds = sr & 2 ? (sr & 1 ? d[3] : d[2]) : (sr & 1 ? d[1] : d[0]);
-    f = fma(w, log64(z, G) - ds, f);
-    const double rz = w * rcp64(z);
-    const double pm = em * rz, pn0 = en0 * rz, pn1 = en1 * rz;
-    const double pM0 = c ? rz : pm, pM1 = c ? pm : rz;
-    r[0] = a ? pM0 : pn0;
-    r[1] = a ? pn0 : pM0;
-    r[2] = b ? pM1 : pn1;
-    r[3] = b ? pn1 : pM1;
-    const double rs = (sr & 2 ? (sr & 1 ? r[3] : r[2]) : (sr & 1 ? r[1] : r[0])) - w;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) r[k] = k == sr ? rs : r[k];
-}
-
-// Line searches, one per cluster: every trial evaluates the slot's sequences
-// at lbase + stp u (FP64), the blocks exchange their sums through distributed
-// shared memory, and each block's last warp runs the same search step on the
-// same numbers, so that one cluster barrier per trial is enough.  While a
-// trial runs that warp works out what the step needs besides its values (L2
-// part, reciprocal).  Without SLOT_F_SEARCH one evaluation at S.stp.  The R,
-// sums and step left behind are the last trial's.
-//
-// Bound by FP64 issue: 84 instructions per sequence and trial at one in 64
-// clocks per quarter of an SM (95 % of that while all slots search), and by
-// the serial part of a trial, some 9 us, for the last slots.  64 slots of
-// 3000 sequences: 46 us for one evaluation (83 with CUDA's exp, log and
-// divisions), 43 per trial, 18 for a lone slot's; a launch, a copy back and a
-// search step on the host per trial took another 35 each.  Solves of 64 loci:
-// 3000 x 10,000 376 -> 257 ms (tensor-core form), 1000 x 4001 115 -> 94 (plain).
-__global__ void __launch_bounds__(SEARCH_THREADS + 32, 2)
-k_search(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N, int64_t Nx, double lambda_J,
-         double lambda_h, const double *__restrict__ lbase, const float4 *__restrict__ u,
-         const uint8_t *__restrict__ rstate, const double *__restrict__ w, float4 *__restrict__ R,
-         double *__restrict__ acc)
-{
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    __shared__ ExpTab sE[EXP_N];
-    __shared__ LogTab sG[LOG_N];
-    __shared__ double warp_part[SEARCH_WARPS + 1][8];   // (a zero row)
-    __shared__ double parts[2][SEARCH_CLUSTER][8];   // the blocks' sums, by parity of the trial
-    __shared__ __align__(16) unsigned char mt_raw[sizeof(MoreThuente)];
-    __shared__ double s_stp;
-    __shared__ int s_more;
-    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const bool searcher = wid == SEARCH_WARPS;
-    for (int k = tid; k < EXP_N; k += blockDim.x) sE[k] = kExpTab[k];
-    for (int k = tid; k < LOG_N; k += blockDim.x) sG[k] = kLogTab[k];
-    const int b = list[blockIdx.x / C];
+    const int b = list[blockIdx.y];
     const SlotDev &S = sd[b];
+    const double stp = S.stp;
     const bool use_u = S.flags & SLOT_F_USE_U;
-    double *A = acc + (int64_t)b * NACC;
-    MoreThuente &mt = *reinterpret_cast<MoreThuente *>(mt_raw);   // the searcher's lane 0
-    bool search = S.flags & SLOT_F_SEARCH;
-    int outcome = LS_MET, trials = 0;
-    if (searcher && lane == 0) {
-        double stp = S.stp;
-        if (search) {
-            new (mt_raw) MoreThuente();
-            // slope of the search line at 0 from the numbers the trials use
-            const double dg0 = A[ACC_DG0] + S.l2.slope(lambda_J, lambda_h, 0.0);
-            if (mt.start(S.f0, dg0, S.alpha) == MoreThuente::NEED_EVAL) {
-                stp = mt.stp;
-            } else {
-                outcome = LS_NO_DESCENT;
-                search = false;
-                stp = 0.0;
-            }
+    double f = 0, dg = 0, rs0 = 0, rs1 = 0, rs2 = 0, rs3 = 0;
+    for (int i = blockIdx.x * TRIAL_THREADS + threadIdx.x; i < N; i += gridDim.x * TRIAL_THREADS) {
+        const int64_t o = (int64_t)b * Nx + i;
+        const double4 lb = load4(lbase, o);
+        const double4 uu = use_u ? load4(u, o) : make_double4(0.0, 0.0, 0.0, 0.0);
+        double l[4] = {lb.x + stp * uu.x, lb.y + stp * uu.y, lb.z + stp * uu.z, lb.w + stp * uu.w};
+        const double mx = fmax(fmax(l[0], l[1]), fmax(l[2], l[3]));
+        double e[4], z = 0;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            e[a] = exp(l[a] - mx);
+            z += e[a];
         }
-        s_stp = stp;
+        const double lse = mx + log(z);
+        const int sr = rstate[o];
+        const double wi = w[i];
+        f += wi * (lse - l[sr]);
+        double r[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) r[a] = wi * (e[a] / z) - (a == sr ? wi : 0.0);
+        dg += r[0] * uu.x + r[1] * uu.y + r[2] * uu.z + r[3] * uu.w;
+        rs0 += r[0]; rs1 += r[1]; rs2 += r[2]; rs3 += r[3];
+        R[o] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
     }
-    if (searcher && lane < 8) warp_part[SEARCH_WARPS][lane] = 0;
-    const int64_t o0 = (int64_t)b * Nx;
-    cl.sync();   // (every block runs before its shared memory is written)
-    for (int par = 0;; par ^= 1) {
-        const double stp = s_stp;
-        double l2f = 0, l2g = 0;
-        if (searcher) {
-            if (lane == 0 && search) {
-                mt.ahead();
-                l2f = S.l2.value(lambda_J, lambda_h, stp);
-                l2g = S.l2.slope(lambda_J, lambda_h, stp);
-            }
-        } else {
-            double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int i = rank * SEARCH_THREADS + tid; i < N; i += C * SEARCH_THREADS) {
-                const double4 lb = load4(lbase, o0 + i);
-                const float4 uf = use_u ? u[o0 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
-                const double4 uu = make_double4(uf.x, uf.y, uf.z, uf.w);
-                const double l[4] = {fma(stp, uu.x, lb.x), fma(stp, uu.y, lb.y), fma(stp, uu.z, lb.z),
-                                     fma(stp, uu.w, lb.w)};
-                double r[4];
-                belief(l, rstate[o0 + i], w[i], sE, sG, v[0], r);
-                v[1] += r[0] * uu.x + r[1] * uu.y + r[2] * uu.z + r[3] * uu.w;
-                v[2] += r[0]; v[3] += r[1]; v[4] += r[2]; v[5] += r[3];
-                R[o0 + i] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
-            }
-            // six sums over the warp by halving what each lane keeps: 4, 2 and
-            // 1 values, then two plain steps; lane 4 k holds value k (bits
-            // of k: lane bits 16, 8, 4)
-#pragma unroll
-            for (int s = 0, h = 4; s < 3; ++s, h >>= 1) {
-                const int bit = 16 >> s;
-#pragma unroll
-                for (int k = 0; k < h; ++k) {
-                    const double give = lane & bit ? v[k] : v[k + h], keep = lane & bit ? v[k + h] : v[k];
-                    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
-                }
-            }
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-            if ((lane & 3) == 0) warp_part[wid][lane >> 2] = v[0];
-        }
-        __syncthreads();
-        const int k8 = lane & 7, g8 = lane >> 3;   // the searcher's lane: value, and one of four groups of rows
-        auto groups = [](double t) {
-            t += __shfl_xor_sync(0xffffffffu, t, 8);
-            return t + __shfl_xor_sync(0xffffffffu, t, 16);
-        };
-        if (searcher) {
-            double t = warp_part[g8][k8];
-#pragma unroll
-            for (int k = 4; k < SEARCH_WARPS + 1; k += 4) t += warp_part[g8 + k][k8];
-            t = groups(t);
-            for (int k = g8; k < C; k += 4) cl.map_shared_rank(&parts[par][rank][0], k)[k8] = t;
-        }
-        cl.sync();
-        if (searcher) {
-            double t = 0;
-            for (int k = g8; k < C; k += 4) t += parts[par][k][k8];
-            t = groups(t);
-            const double fd = __shfl_sync(0xffffffffu, t, 0), dd = __shfl_sync(0xffffffffu, t, 1);
-            int more = 0;
-            if (lane == 0 && search) {
-                ++trials;
-                const double f = fd + l2f, dg = dd + l2g;
-                if (!isfinite(f) || !isfinite(dg)) {
-                    outcome = LS_NOT_FINITE;
-                } else if (mt.feed(f, dg) == MoreThuente::DONE) {
-                    outcome = mt.info == 1 ? LS_MET : LS_ENDED;
-                } else {
-                    more = 1;
-                    s_stp = mt.stp;
-                }
-            }
-            if (lane == 0) s_more = more;
-            more = __shfl_sync(0xffffffffu, more, 0);
-            if (!more && rank == 0) {
-                if (lane < SEARCH_K) A[ACC_F + lane] = t;
-                if (lane == 0) {
-                    A[ACC_STP] = stp;
-                    A[ACC_TRIALS] = trials;
-                    A[ACC_LS] = outcome;
-                }
-            }
-        }
-        __syncthreads();
-        if (!s_more) return;
-    }
+    double v[6] = {f, dg, rs0, rs1, rs2, rs3};
+    const int idx[6] = {ACC_F, ACC_DG, ACC_RS0, ACC_RS1, ACC_RS2, ACC_RS3};
+    block_sum_atomic<6>(v, acc + (int64_t)b * NACC, idx);
 }
 
 // Loci enter slots (who: slot, locus), starting from zero.  One launch for
@@ -572,30 +425,17 @@ void launch_slots_begin(const Problem &P, const int2 *who, int n, const uint8_t 
         who, P.Nx, P.Dp, states, rstate, wa, d, lbase, dv, dv_slot, ctl);
 }
 
-// One cluster per slot, its blocks sharing the slot's sequences: as many as
-// there are SMs for, while each evaluating thread still has a sequence.  Two
-// blocks per SM, which would let a slot that ends early leave its SM to the
-// other, took longer (54 us for 46 above: the blocks do not spread evenly; with
-// clusters of eight and blocks of 256 threads some SMs stay empty, 57).
-void launch_search(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
-                   const double *lbase, const float *u, const uint8_t *rstate, const double *w,
-                   float *R, double *acc, cudaStream_t st)
+void launch_trial(const Problem &P, const SlotDev *sd, const int32_t *list, int n,
+                  const double *lbase, const float *u, const uint8_t *rstate, const double *w,
+                  float *R, double *acc, cudaStream_t st)
 {
     if (n <= 0) return;
-    int c = 1;
-    while (c < SEARCH_CLUSTER && (int64_t)c * SEARCH_THREADS < P.N && (int64_t)2 * c * n <= 152) c *= 2;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)c * n);
-    cfg.blockDim = dim3(SEARCH_THREADS + 32);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)c;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_search, sd, list, (int)P.N, P.Nx, P.lambda_J, P.lambda_h, lbase,
-                       reinterpret_cast<const float4 *>(u), rstate, w, reinterpret_cast<float4 *>(R), acc);
+    int gx = (int)((P.N + TRIAL_THREADS - 1) / TRIAL_THREADS);
+    if (gx > 32) gx = 32;
+    dim3 grid((unsigned)gx, (unsigned)n);
+    k_trial<float4, double><<<grid, TRIAL_THREADS, 0, st>>>(sd, list, (int)P.N, P.Nx, lbase,
+                                                    reinterpret_cast<const float4 *>(u), rstate, w,
+                                                    reinterpret_cast<float4 *>(R), acc);
 }
 
 void launch_accept(const Problem &P, const SlotDev *sd, const int32_t *list, int n, float *wa,

@@ -1,4 +1,4 @@
-// linesearch.h -- resumable More-Thuente line search (host and device, FP64).
+// linesearch.h -- resumable More-Thuente line search (host, FP64).
 //
 // SuperDCA minimises each locus with CppNumericalSolvers' LbfgsSolver, whose
 // line search is More & Thuente's (ACM TOMS 20(3), 1994; MINPACK cvsrch /
@@ -11,9 +11,9 @@
 // The search is written as a state machine so that every slot of a batch can
 // hold its own search: start() gives the first trial step, each feed() takes
 // f and g.s at the last trial and either asks for another step or finishes.
-// The accepted point is always the last trial evaluated.  It runs on the
-// device: one search per thread block in the dual form's line-search kernel,
-// one per cluster in the other forms'.
+// The accepted point is always the last trial evaluated.  The same code runs
+// on the host (tensor-core and plain forms) and on the device (the dual
+// form's line-search kernel, one search per thread block).
 #pragma once
 
 #include <math.h>
@@ -57,22 +57,6 @@ SDCA_HD inline double mt_gamma(double theta, double a, double b, bool clip)
     const double t = theta * inv, r = t * t - (a * inv) * (b * inv);
     return s * sqrt(clip ? mt_max(0.0, r) : r);
 }
-
-// The L2 part along x + stp d, a quadratic in the step: squared norms and
-// products of the J and h parts of x and d.
-struct LineL2 {
-    double x2J = 0, x2H = 0, xdJ = 0, xdH = 0, ddJ = 0, ddH = 0;
-    SDCA_HD double value(double lambda_J, double lambda_h, double stp) const
-    {
-        const double j2 = x2J + 2.0 * stp * xdJ + stp * stp * ddJ;
-        const double h2 = x2H + 2.0 * stp * xdH + stp * stp * ddH;
-        return lambda_J * j2 + lambda_h * h2;
-    }
-    SDCA_HD double slope(double lambda_J, double lambda_h, double stp) const
-    {
-        return 2.0 * lambda_J * (xdJ + stp * ddJ) + 2.0 * lambda_h * (xdH + stp * ddH);
-    }
-};
 
 class MoreThuente {
 public:

@@ -17,8 +17,6 @@
 #pragma once
 
 #include <math.h>
-#include <stdint.h>
-#include <string.h>
 
 #ifdef __CUDACC__
 #define SDCA_HD __host__ __device__
@@ -33,29 +31,28 @@ namespace sdca {
 SDCA_HD inline double mt_min(double a, double b) { return (b < a) ? b : a; }
 SDCA_HD inline double mt_max(double a, double b) { return (a < b) ? b : a; }
 
-// The power of two at or below s (s >= 0), and its reciprocal: scaling by it
-// is exact and needs no division (GB300's FP64 divisions are long serial
-// chains, and one thread runs this search between two trials).
-SDCA_HD inline double mt_pow2(double s, double &inv)
-{
-    uint64_t b;
-    memcpy(&b, &s, sizeof(b));
-    b &= 0x7ff0000000000000ull;
-    const uint64_t i = b >= 0x7fe0000000000000ull ? 0ull : 0x7fe0000000000000ull - b;
-    double p;
-    memcpy(&p, &b, sizeof(p));
-    memcpy(&inv, &i, sizeof(inv));
-    return p;
-}
-
-// s sqrt((theta / s)^2 - (a / s)(b / s)) (not below zero if `clip`), with s the
-// power of two of the largest magnitude, so that no square overflows
+// The cubic's gamma = s sqrt((theta / s)^2 - (a / s)(b / s)) (not below zero
+// if `clip`), s the largest magnitude, so that no square overflows.  On the
+// device s is the power of two at or below that: scaling by it is exact and
+// needs no division (GB300's FP64 divisions are long serial chains, and one
+// thread runs this search between two trials).  On the host, where they cost
+// nothing beside a trial, as published: a search's steps decide which iterate
+// below the threshold a locus stops at, and the forms that search on the host
+// are reproducible for few sequences.
 SDCA_HD inline double mt_gamma(double theta, double a, double b, bool clip)
 {
-    double inv;
-    const double s = mt_pow2(mt_max(fabs(theta), mt_max(fabs(a), fabs(b))), inv);
+#ifdef __CUDA_ARCH__
+    const double m = mt_max(fabs(theta), mt_max(fabs(a), fabs(b)));
+    const unsigned long long e = (unsigned long long)__double_as_longlong(m) & 0x7ff0000000000000ull;
+    const double s = __longlong_as_double((long long)e);
+    const double inv = __longlong_as_double((long long)(e >= 0x7fe0000000000000ull ? 0ull : 0x7fe0000000000000ull - e));
     const double t = theta * inv, r = t * t - (a * inv) * (b * inv);
     return s * sqrt(clip ? mt_max(0.0, r) : r);
+#else
+    const double s = mt_max(fabs(theta), mt_max(fabs(a), fabs(b)));
+    const double r = (theta / s) * (theta / s) - (a / s) * (b / s);
+    return s * sqrt(clip ? mt_max(0.0, r) : r);
+#endif
 }
 
 class MoreThuente {
@@ -171,12 +168,18 @@ private:
             return;
         bool bound = false;
         const double sgnd = dx > 0.0 ? dp : -dp;   // (dx is not zero here)
+#ifdef __CUDA_ARCH__
         const double slope = (fxv - fp) * rinv;     // (fx - f) / (st - sx)
+        const double three = 3.0 * slope;
+#else
+        const double slope = (fxv - fp) / (st - sx);
+        const double three = 3.0 * (fxv - fp) / (st - sx);
+#endif
         double stpf, stpc, stpq;
         if (fp > fxv) {
             infoc = 1;
             bound = true;
-            const double theta = 3.0 * slope + dx + dp;
+            const double theta = three + dx + dp;
             double gamma = mt_gamma(theta, dx, dp, false);
             if (st < sx) gamma = -gamma;
             const double p = (gamma - dx) + theta, q = ((gamma - dx) + gamma) + dp;
@@ -186,7 +189,7 @@ private:
             brackt = true;
         } else if (sgnd < 0.0) {
             infoc = 2;
-            const double theta = 3.0 * slope + dx + dp;
+            const double theta = three + dx + dp;
             double gamma = mt_gamma(theta, dx, dp, false);
             if (st > sx) gamma = -gamma;
             const double p = (gamma - dp) + theta, q = ((gamma - dp) + gamma) + dx;
@@ -197,7 +200,7 @@ private:
         } else if (fabs(dp) < fabs(dx)) {
             infoc = 3;
             bound = true;
-            const double theta = 3.0 * slope + dx + dp;
+            const double theta = three + dx + dp;
             double gamma = mt_gamma(theta, dx, dp, true);
             if (st > sx) gamma = -gamma;
             const double p = (gamma - dp) + theta, q = (gamma + (dx - dp)) + gamma;

@@ -9,6 +9,7 @@
 // 126-151 for the pseudo-likelihood part; the L2 part is a quadratic in stp
 // that the host evaluates from x.d and d.d).
 #include <algorithm>
+#include <type_traits>
 
 #include "df.cuh"
 #include "engine.h"
@@ -33,6 +34,9 @@ __device__ __forceinline__ double4 load4(const double *v, int64_t o)
     return make_double4(a.x, a.y, b.x, b.y);
 }
 
+// Bound by FP64 issue (one instruction per 64 clocks and quarter of an SM).
+// Three exponentials instead of four and four quotients from one reciprocal,
+// the same bits: 80 -> 70 us for 64 slots of 3000 sequences, 31 -> 26 of 1000.
 template <typename UT, typename LT>
 __global__ void __launch_bounds__(TRIAL_THREADS)
 k_trial(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N, int64_t Nx,
@@ -51,19 +55,31 @@ k_trial(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N,
         const double4 uu = use_u ? load4(u, o) : make_double4(0.0, 0.0, 0.0, 0.0);
         double l[4] = {lb.x + stp * uu.x, lb.y + stp * uu.y, lb.z + stp * uu.z, lb.w + stp * uu.w};
         const double mx = fmax(fmax(l[0], l[1]), fmax(l[2], l[3]));
-        double e[4], z = 0;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            e[a] = exp(l[a] - mx);
-            z += e[a];
-        }
+        // the largest logit's exponential is 1 (k: its state, 0 with a NaN among
+        // them, whose exponential is then not skipped): three are left
+        const double t[4] = {l[0] - mx, l[1] - mx, l[2] - mx, l[3] - mx};
+        auto zero = [](double v) { return __double_as_longlong(v) == 0ll; };
+        const int k = zero(t[0]) ? 0 : zero(t[1]) ? 1 : zero(t[2]) ? 2 : 3;
+        const double x0 = exp(k == 0 ? t[1] : t[0]), x1 = exp(k <= 1 ? t[2] : t[1]), x2 = exp(k <= 2 ? t[3] : t[2]);
+        const double xk = zero(k == 0 ? t[0] : k == 1 ? t[1] : k == 2 ? t[2] : t[3]) ? 1.0 : __longlong_as_double(0x7ff8000000000000ll);
+        const double e[4] = {k == 0 ? xk : x0, k == 1 ? xk : k == 0 ? x0 : x1, k == 2 ? xk : k < 2 ? x1 : x2, k == 3 ? xk : x2};
+        const double z = ((e[0] + e[1]) + e[2]) + e[3];
         const double lse = mx + log(z);
         const int sr = rstate[o];
         const double wi = w[i];
         f += wi * (lse - l[sr]);
+        // e / z, rounded correctly, from the reciprocal (Markstein, IBM J. Res.
+        // Dev. 34(1), 1990): a quotient within a unit and its exact remainder
+        const double rz = __drcp_rn(z);
+        auto quotient = [&](double v) {
+            const double q = v * rz;
+            return fma(fma(-q, z, v), rz, q);
+        };
+        const double q0 = quotient(x0), q1 = quotient(x1), q2 = quotient(x2);
+        const double p[4] = {k == 0 ? rz : q0, k == 1 ? rz : k == 0 ? q0 : q1, k == 2 ? rz : k < 2 ? q1 : q2, k == 3 ? rz : q2};
         double r[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) r[a] = wi * (e[a] / z) - (a == sr ? wi : 0.0);
+        for (int a = 0; a < 4; ++a) r[a] = wi * p[a] - (a == sr ? wi : 0.0);
         dg += r[0] * uu.x + r[1] * uu.y + r[2] * uu.z + r[3] * uu.w;
         rs0 += r[0]; rs1 += r[1]; rs2 += r[2]; rs3 += r[3];
         R[o] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
@@ -196,70 +212,121 @@ __global__ void k_hpart(const SlotDev *__restrict__ sd, const int32_t *__restric
 }
 
 constexpr int DOT_THREADS = 256;
-constexpr int DOT_U = 4;  // float4 groups per thread per tile: 16 KB runs per stream per block
+constexpr int DOT_U = 4;  // float4 groups per thread per tile
 
-// dots[b] = [S_j.g | Y_j.g | S_j.y_new | Y_j.y_new], j over the history.
-// Blocks walk tiles of DOT_THREADS x DOT_U float4 groups; within a tile g and
-// y_new stay in registers while the history vectors stream through one at a
-// time, so every stream is read in long contiguous runs.
-__global__ void __launch_bounds__(DOT_THREADS)
+// A thread's four groups of four entries of a tile (the same groups, in the
+// same order, for every vector: the order of the sums decides their last bits
+// and, through them, the iterate a locus stops at)
+template <bool BF16> struct Tile {
+    using Raw = typename std::conditional<BF16, uint2, uint4>::type;
+    int64_t t0, n;
+    __device__ Tile(int64_t tile, int64_t Dp) : t0(tile * (DOT_THREADS * DOT_U) + threadIdx.x), n(Dp / 4) {}
+    __device__ __forceinline__ bool has(int u) const { return t0 + u * DOT_THREADS < n; }
+    __device__ __forceinline__ int64_t group(int u) const { return t0 + u * DOT_THREADS; }
+    // FP32 vector
+    __device__ __forceinline__ void load_f(const float *v, float4 (&x)[DOT_U]) const
+    {
+#pragma unroll
+        for (int u = 0; u < DOT_U; ++u)
+            x[u] = has(u) ? reinterpret_cast<const float4 *>(v)[group(u)] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // history vector at offset off: the loads, and their values
+    __device__ __forceinline__ void load_h(const void *v, int64_t off, Raw (&raw)[DOT_U]) const
+    {
+#pragma unroll
+        for (int u = 0; u < DOT_U; ++u) raw[u] = has(u) ? reinterpret_cast<const Raw *>(v)[off / 4 + group(u)] : Raw{};
+    }
+    static __device__ __forceinline__ float4 value(const Raw &r)
+    {
+        if constexpr (BF16)
+            return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u),
+                               __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xFFFF0000u));
+        else
+            return make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w));
+    }
+};
+
+// dots[b] = [S_j.g | Y_j.g | S_j.y_new | Y_j.y_new], j over the history; a
+// block takes the s or the y vectors (blockIdx.z) of a stretch of tiles: g and
+// y_new stay in registers while the vectors stream through, one on its way
+// while one is summed.
+//
+// Bound by memory: 20 history vectors, g and y_new.  Both kinds of vectors in
+// one block (128 registers, 40 sums reduced by five shuffles each and a chain
+// of FP64 additions per sum) took 205 us for 64 slots of 3000 x 10,000 (FP32
+// history, 0.9 GB) and 111 for 1000 x 4001 (BF16, 0.2 GB); now 170 and 48,
+// every bit of the sums as before (a thread's groups, their order and the
+// blocks of a slot are the same).
+template <bool BF16>
+__global__ void __launch_bounds__(DOT_THREADS, 2)
 k_hist_dots(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int64_t Dp, int m,
             const float *__restrict__ gpool, const void *__restrict__ Spool,
-            const void *__restrict__ Ypool, int hist_bf16, double *__restrict__ dots)
+            const void *__restrict__ Ypool, double *__restrict__ dots)
 {
+    using T = Tile<BF16>;
+    constexpr int AHEAD = BF16 ? 4 : 2;   // vectors on their way
+    __shared__ float part[DOT_THREADS / 32][32];
     const int b = list[blockIdx.y];
     const SlotDev &S = sd[b];
     const int nh = S.nhist;
-    const float4 *g4 = reinterpret_cast<const float4 *>(gpool + (int64_t)(2 * b + S.gcur) * Dp);
+    const bool isy = blockIdx.z;
+    const float *g = gpool + (int64_t)(2 * b + S.gcur) * Dp;
     const bool has_new = S.ring_new >= 0;
     const int64_t ybase = ((int64_t)b * m + (has_new ? S.ring_new : 0)) * Dp;
-    const int64_t nv4 = Dp / 4, tile = (int64_t)DOT_THREADS * DOT_U;
-    float aSg[MAXHIST], aYg[MAXHIST], aSy[MAXHIST], aYy[MAXHIST];
+    const void *pool = isy ? Ypool : Spool;
+    const int64_t tiles = (Dp / 4 + DOT_THREADS * DOT_U - 1) / (DOT_THREADS * DOT_U);
+    float v[32];   // [0, MAXHIST) with g, [MAXHIST, 2 MAXHIST) with y_new
 #pragma unroll
-    for (int j = 0; j < MAXHIST; ++j) aSg[j] = aYg[j] = aSy[j] = aYy[j] = 0.f;
-    for (int64_t tb = (int64_t)blockIdx.x * tile; tb < nv4; tb += (int64_t)gridDim.x * tile) {
+    for (int k = 0; k < 32; ++k) v[k] = 0.f;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const T t(tile, Dp);
         float4 gv[DOT_U], yn[DOT_U];
+        typename T::Raw next[AHEAD][DOT_U];
 #pragma unroll
-        for (int u = 0; u < DOT_U; ++u) {
-            const int64_t v = tb + u * DOT_THREADS + threadIdx.x;
-            const bool ok = v < nv4;
-            gv[u] = ok ? g4[v] : make_float4(0.f, 0.f, 0.f, 0.f);
-            yn[u] = (ok && has_new) ? load_hist4(Ypool, ybase + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < AHEAD; ++j)
+            if (j < nh) t.load_h(pool, ((int64_t)b * m + S.ring[j]) * Dp, next[j]);
+        t.load_f(g, gv);
+        {
+            typename T::Raw raw[DOT_U] = {};
+            if (has_new) t.load_h(Ypool, ybase, raw);
+#pragma unroll
+            for (int u = 0; u < DOT_U; ++u) yn[u] = T::value(raw[u]);
         }
 #pragma unroll
         for (int j = 0; j < MAXHIST; ++j) {
             if (j < nh) {
-                const int64_t base = ((int64_t)b * m + S.ring[j]) * Dp;
-                float4 sv[DOT_U], yv[DOT_U];
+                float4 x[DOT_U];
+#pragma unroll
+                for (int u = 0; u < DOT_U; ++u) x[u] = T::value(next[j % AHEAD][u]);
+                if (j + AHEAD < nh) t.load_h(pool, ((int64_t)b * m + S.ring[j + AHEAD]) * Dp, next[j % AHEAD]);
 #pragma unroll
                 for (int u = 0; u < DOT_U; ++u) {
-                    const int64_t v = tb + u * DOT_THREADS + threadIdx.x;
-                    const bool ok = v < nv4;
-                    sv[u] = ok ? load_hist4(Spool, base + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    yv[u] = ok ? load_hist4(Ypool, base + 4 * v, hist_bf16) : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-#pragma unroll
-                for (int u = 0; u < DOT_U; ++u) {
-                    aSg[j] += dot4(sv[u], gv[u]);
-                    aYg[j] += dot4(yv[u], gv[u]);
-                    aSy[j] += dot4(sv[u], yn[u]);
-                    aYy[j] += dot4(yv[u], yn[u]);
+                    v[j] += dot4(x[u], gv[u]);
+                    v[MAXHIST + j] += dot4(x[u], yn[u]);
                 }
             }
         }
     }
-    float v[4 * MAXHIST];
-    int idx[4 * MAXHIST];
+    // sums over the warp by halving what each lane keeps: lane k holds value k
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int j = 0; j < MAXHIST; ++j) {
-        v[j] = aSg[j];
-        v[MAXHIST + j] = aYg[j];
-        v[2 * MAXHIST + j] = aSy[j];
-        v[3 * MAXHIST + j] = aYy[j];
+    for (int s = 0, h = 16; s < 5; ++s, h >>= 1) {
+        const bool up = lane & h;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const float give = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        }
     }
+    part[wid][lane] = v[0];
+    __syncthreads();
+    if (threadIdx.x < 2 * MAXHIST) {
+        const int k = threadIdx.x, j = k % MAXHIST, q = k / MAXHIST;
+        double t = 0.0;
 #pragma unroll
-    for (int k = 0; k < 4 * MAXHIST; ++k) idx[k] = k;
-    block_sum_atomic_f<4 * MAXHIST>(v, dots + (int64_t)b * 4 * MAXHIST, idx);
+        for (int w = 0; w < DOT_THREADS / 32; ++w) t += part[w][k];
+        if (j < nh && t != 0.0) atomicAdd(dots + (int64_t)b * 4 * MAXHIST + (2 * q + isy) * MAXHIST + j, t);
+    }
 }
 
 // d = coef_g g + sum_j (coefS_j s_j + coefY_j y_j), J_rr block zero;
@@ -473,8 +540,9 @@ void launch_hist_dots(const Problem &P, const SlotDev *sd, const int32_t *list, 
     // hundreds of float4 before the block reduction
     const int64_t per_slot = std::max<int64_t>(4, std::min<int64_t>(64, (4 * 152 + n - 1) / n));
     dim3 grid(dgrid(P.Dp, DOT_THREADS * DOT_U, per_slot), (unsigned)n);
-    k_hist_dots<<<grid, DOT_THREADS, 0, st>>>(sd, list, P.Dp, P.ring, gpool, Spool, Ypool, hist_bf16,
-                                              dots);
+    grid.z = 2;   // (s and y)
+    if (hist_bf16) k_hist_dots<true><<<grid, DOT_THREADS, 0, st>>>(sd, list, P.Dp, P.ring, gpool, Spool, Ypool, dots);
+    else k_hist_dots<false><<<grid, DOT_THREADS, 0, st>>>(sd, list, P.Dp, P.ring, gpool, Spool, Ypool, dots);
 }
 
 void launch_direction(const Problem &P, const SlotDev *sd, const int32_t *list, int n,

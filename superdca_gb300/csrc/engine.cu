@@ -514,9 +514,8 @@ int stream_sync(sdca_handle *h)
     return SDCA_OK;
 }
 
-// Copy `bytes` from src to device dst through a staging region that no copy
-// still queued on the stream reads.
-int staged_h2d(sdca_handle *h, void *dst, const void *src, size_t bytes)
+// A staging region that no copy still queued on the stream reads.
+int stage(sdca_handle *h, size_t bytes, uint8_t **p)
 {
     const size_t need = (bytes + 255) & ~(size_t)255;
     if (need > h->stage_cap) return fail(h, SDCA_E_ARG, "staging arena too small");
@@ -524,8 +523,17 @@ int staged_h2d(sdca_handle *h, void *dst, const void *src, size_t bytes)
         int rc = stream_sync(h);
         if (rc) return rc;
     }
-    uint8_t *p = h->stage + h->stage_off;
+    *p = h->stage + h->stage_off;
     h->stage_off += need;
+    return SDCA_OK;
+}
+
+// Copy `bytes` from src to device dst through a staging region.
+int staged_h2d(sdca_handle *h, void *dst, const void *src, size_t bytes)
+{
+    uint8_t *p = nullptr;
+    const int rc = stage(h, bytes, &p);
+    if (rc) return rc;
     std::memcpy(p, src, bytes);
     CK(cudaMemcpyAsync(dst, p, bytes, cudaMemcpyHostToDevice, h->stream));
     return SDCA_OK;
@@ -535,6 +543,22 @@ int upload_list(sdca_handle *h, const std::vector<int32_t> &lst)
 {
     if (lst.empty()) return SDCA_OK;
     return staged_h2d(h, h->list, lst.data(), sizeof(int32_t) * lst.size());
+}
+
+// The mirror (small: whole) and the list behind it in one copy.  Two copies
+// here and a separate one of the error word in fetch_acc were a good part of
+// what stands between two trials of the plain and tensor-core forms (solves of
+// 64 loci: 1000 x 4001 98 -> 91 ms, 3000 x 10,000 337 -> 302).
+int upload_mirror(sdca_handle *h, const std::vector<int32_t> &lst)
+{
+    const size_t sd = sizeof(SlotDev) * h->P.Bmax, bytes = sd + sizeof(int32_t) * lst.size();
+    uint8_t *p = nullptr;
+    const int rc = stage(h, bytes, &p);
+    if (rc) return rc;
+    std::memcpy(p, h->sd_h, sd);
+    if (!lst.empty()) std::memcpy(p + sd, lst.data(), bytes - sd);
+    CK(cudaMemcpyAsync(h->sd, p, bytes, cudaMemcpyHostToDevice, h->stream));
+    return SDCA_OK;
 }
 
 // copy the host slot parameters of `lst` into the device mirror
@@ -552,10 +576,7 @@ int upload_slots(sdca_handle *h, const std::vector<int32_t> &lst)
         D.stp = S.stp;
         for (int a = 0; a < Q; ++a) D.rs[a] = S.rs[a];
     }
-    // the mirror is small; copy it whole
-    int rc = staged_h2d(h, h->sd, h->sd_h, sizeof(SlotDev) * h->P.Bmax);
-    if (rc) return rc;
-    return upload_list(h, lst);
+    return upload_mirror(h, lst);
 }
 
 int zero_acc(sdca_handle *h)
@@ -566,13 +587,14 @@ int zero_acc(sdca_handle *h)
 
 int fetch_acc(sdca_handle *h)
 {
-    CK(cudaMemcpyAsync(h->acc_h, h->acc, sizeof(double) * NACC * h->P.Bmax, cudaMemcpyDeviceToHost,
-                       h->stream));
-    if (h->tc_err) CK(cudaMemcpyAsync(h->flag_h + 1, h->tc_err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    // (the pipelines' error word lies behind the sums)
+    const size_t n = (size_t)NACC * h->P.Bmax;
+    CK(cudaMemcpyAsync(h->acc_h, h->acc, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, h->stream));
     int rc = stream_sync(h);
     if (rc) return rc;
-    if (h->tc_err && h->flag_h[1])
-        return fail(h, SDCA_E_CUDA, "tensor-core pipeline wait timed out (kernel abandoned its tile)");
+    int err;
+    std::memcpy(&err, h->acc_h + n, sizeof(err));
+    if (err) return fail(h, SDCA_E_CUDA, "tensor-core pipeline wait timed out (kernel abandoned its tile)");
     return SDCA_OK;
 }
 
@@ -1309,9 +1331,7 @@ int phase_step(sdca_handle *h)
             D.nhist = (int)S.hist.size();
             for (int j = 0; j < D.nhist; ++j) D.ring[j] = S.hist[j];
         }
-        int r2 = staged_h2d(h, h->sd, h->sd_h, sizeof(SlotDev) * P.Bmax);
-        if (r2) return r2;
-        r2 = upload_list(h, lst);
+        int r2 = upload_mirror(h, lst);
         if (r2) return r2;
         r2 = zero_acc(h);
         if (r2) return r2;
@@ -2202,13 +2222,13 @@ static int create_lane(const sdca_config *cfg, const sdca_handle *owner, sdca_ha
         (rc = dalloc(h, &h->R, B * P.Nx * 4)) || (rc = dalloc(h, &h->lbase, B * P.Nx * 4)) ||
         (rc = dalloc(h, &h->partial, (size_t)P.C * B * P.Nx * 4)) ||
         (rc = dalloc(h, &h->partial64, (size_t)P.Cg * B * P.Nx * 4)) ||
-        (rc = dalloc(h, &h->rows, B * P.L)) || (!dual && (rc = dalloc(h, &h->acc, B * NACC))) ||
-        (!dual && (rc = dalloc(h, &h->dots, B * 4 * MAXHIST))) || (rc = dalloc(h, &h->sd, B)) ||
-        (rc = dalloc(h, &h->list, B)) || (rc = dalloc(h, &h->begin, 2 * B)) || (rc = dalloc(h, &h->flag, 4)) ||
+        (rc = dalloc(h, &h->rows, B * P.L)) || (!dual && (rc = dalloc(h, &h->acc, B * NACC + 1))) ||
+        (!dual && (rc = dalloc(h, &h->dots, B * 4 * MAXHIST))) || (rc = dalloc(h, &h->sd, B + (4 * B + sizeof(SlotDev) - 1) / sizeof(SlotDev))) ||
+        (rc = dalloc(h, &h->begin, 2 * B)) || (rc = dalloc(h, &h->flag, 4)) ||
         (rc = dalloc(h, reinterpret_cast<uint8_t **>(&h->Spool), hist_bytes)) ||
         (rc = dalloc(h, reinterpret_cast<uint8_t **>(&h->Ypool), hist_bytes)) ||
         (rc = halloc(h, &h->sd_h, B)) || (rc = halloc(h, &h->list_h, B)) ||
-        (!dual && (rc = halloc(h, &h->acc_h, B * NACC))) || (rc = halloc(h, &h->dots_h, B * 4 * MAXHIST)) ||
+        (!dual && (rc = halloc(h, &h->acc_h, B * NACC + 1))) || (rc = halloc(h, &h->dots_h, B * 4 * MAXHIST)) ||
         (rc = halloc(h, &h->rows_h, B * P.L)) || (rc = halloc(h, &h->flag_h, 4)) ||
         (rc = halloc(h, &h->stage, (h->stage_cap = 64 * (((sizeof(SlotDev) + 4) * B + 1024 + 255) & ~(size_t)255)))) ||
         (dual && ((rc = halloc(h, &h->amax_h, 2 * B)) || (rc = dual_blocks(h)) ||
@@ -2225,14 +2245,15 @@ static int create_lane(const sdca_config *cfg, const sdca_handle *owner, sdca_ha
         (tcres &&
          ((!dual && (rc = dalloc(h, &h->Dhi, 4 * B * (size_t)round_up(4 * P.L, 64)))) ||
           (!dual && (rc = dalloc(h, &h->Dlo, 4 * B * (size_t)round_up(4 * P.L, 64)))) ||
-          (rc = dalloc(h, &h->Rhi, 4 * B * (size_t)P.Nx)) || (rc = dalloc(h, &h->Rlo, 4 * B * (size_t)P.Nx)) ||
-          (!dual && (rc = dalloc(h, &h->tc_err, 4)))))) {
+          (rc = dalloc(h, &h->Rhi, 4 * B * (size_t)P.Nx)) || (rc = dalloc(h, &h->Rlo, 4 * B * (size_t)P.Nx))))) {
         std::string msg = h->err;
         free_all(h);
         if (h->own_stream) cudaStreamDestroy(h->stream);
         delete h;
         return fail(nullptr, rc, msg);
     }
+    h->list = reinterpret_cast<int32_t *>(h->sd + B);
+    if (!dual && tcres) h->tc_err = reinterpret_cast<int *>(h->acc + B * NACC);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess ||
         (dual && (cudaEventCreateWithFlags(&h->ev_round, cudaEventDisableTiming) != cudaSuccess ||
                   cudaEventCreateWithFlags(&h->ev_rows, cudaEventDisableTiming) != cudaSuccess))) {

@@ -444,6 +444,8 @@ k_gemm(const __grid_constant__ CUtensorMap tmRaw, const __grid_constant__ CUtens
                     failed = true;
                     break;
                 }
+                // (A in TMEM: the stores below follow the MMAs whose completion was waited for)
+                if (AT) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t st = sbase + (uint32_t)s * SB;
 #pragma unroll
                 for (int ms2 = 0; ms2 < MSUB; ms2 += 2) {

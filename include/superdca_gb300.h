@@ -294,8 +294,10 @@ const char *sdca_mlp_last_error(void);
  * f (one double).  lambda_h and lambda_J are absolute strengths (as
  * sdca_get_lambdas reports them).  Work is queued on `stream` (a cudaStream_t
  * or NULL) of the current device and is complete when that stream is.
- * Intermediate values live in g (until its values are written) and in one
- * fixed __device__ array of the library
+ * g may be x (an evaluation in place) or overlap weights, whose values the call
+ * then overwrites; it must not overlap states.  f is written last.
+ * Intermediate values live in g (until its values are written; not when g
+ * overlaps x or weights) and in one fixed __device__ array of the library
  * (about 2.1 MB, held by every GPU that loads the library until exit), so
  * n_seqs <= SDCA_NOALLOC_MAX_SEQS and n_loci <= SDCA_NOALLOC_MAX_LOCI, else
  * SDCA_E_ARG before any work is queued.  All calls share that array: calls

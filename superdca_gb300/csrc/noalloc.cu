@@ -10,7 +10,8 @@
 // values (per-sequence node beliefs, per-block partial sums and an error
 // word) live in one file-scope __device__ array of fixed size, SCRATCH_BYTES
 // below, which every GPU that loads this library holds until the process
-// exits; the caller's g holds partial logits until the gradient is written.
+// exits; the caller's g holds partial logits until the gradient is written,
+// unless it overlaps x or the weights (an evaluation in place).
 //
 // The array is shared by every call: two calls whose kernels overlap on the
 // GPU (different streams, or different host threads) race on it.  Each call
@@ -225,9 +226,9 @@ k_na_logits(const uint8_t *__restrict__ states, int64_t N, int64_t L, int64_t r,
 }
 
 // pass 2, one warp per sequence: the logits from their partial sums,
-// objective term and node beliefs (plmDCA_objective.hpp:126-151).  With one
-// slice part may be nb itself: a warp reads its sequence's logits before it
-// writes the beliefs to the same place.
+// objective term and node beliefs (plmDCA_objective.hpp:126-151).  part may be
+// nb itself: a warp reads its sequence's logits, of which the first slice's
+// lie where it writes the beliefs afterwards.
 __global__ void __launch_bounds__(NA_THREADS)
 k_na_beliefs(const uint8_t *__restrict__ states, int64_t N, int64_t L, int64_t r, const double *__restrict__ w,
              const double *__restrict__ x, int slices, const double *part, double *nb,
@@ -282,8 +283,8 @@ constexpr int NG_LOCI = 1, NG_SEQS = 32, NG_SETS = NG_SEQS / 8;
 
 __global__ void __launch_bounds__(NG_THREADS)
 k_na_gradient(const uint8_t *__restrict__ states, int64_t N, int64_t L, int64_t r, double lambda_J,
-              const double *__restrict__ x, double *__restrict__ g, double *__restrict__ part,
-              const double *__restrict__ nb, double *__restrict__ scratch)
+              const double *x, double *g, double *__restrict__ part, const double *__restrict__ nb,
+              double *__restrict__ scratch)
 {
     __shared__ __align__(16) double2 set[NG_SETS][256][2];
     __shared__ __align__(16) double2 half[2 * NG_SETS][16][2];
@@ -350,6 +351,14 @@ k_na_gradient(const uint8_t *__restrict__ states, int64_t N, int64_t L, int64_t 
     for (int q = 0; q < NG_LOCI; ++q) {
         const int64_t n = n0 + (int64_t)q * NG_THREADS;
         if (n >= L) continue;
+        // (g may be x: this thread's entries are read before it writes any)
+        double xv[4][4] = {};
+        if (!part && n != r) {
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int a = 0; a < 4; ++a) xv[s][a] = x[na_index(L, n, s, a)];
+        }
 #pragma unroll
         for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -360,8 +369,8 @@ k_na_gradient(const uint8_t *__restrict__ states, int64_t N, int64_t L, int64_t 
                 } else if (n == r) {
                     g[o] = 0.0;
                 } else {
-                    g[o] = c[q][s][a] + 2.0 * lambda_J * x[o];
-                    v[0] += lambda_J * x[o] * x[o];
+                    g[o] = c[q][s][a] + 2.0 * lambda_J * xv[s][a];
+                    v[0] += lambda_J * xv[s][a] * xv[s][a];
                 }
             }
     }
@@ -373,19 +382,20 @@ k_na_gradient(const uint8_t *__restrict__ states, int64_t N, int64_t L, int64_t 
 // the gradient from its shares, and the L2 part of the objective
 __global__ void __launch_bounds__(NA_THREADS)
 k_na_gradient_sum(int64_t L, int64_t r, double lambda_J, int shares, const double *__restrict__ part,
-                  const double *__restrict__ x, double *__restrict__ g, double *__restrict__ scratch)
+                  const double *x, double *g, double *__restrict__ scratch)
 {
     double v[1] = {0.0};
     for (int64_t e = (int64_t)blockIdx.x * NA_THREADS + threadIdx.x; e < 16 * L; e += (int64_t)gridDim.x * NA_THREADS) {
         // the locus of entry e: 16-locus blocks, [s][locus][a] inside
         const int64_t b = e / 256, width = b < L / 16 ? 16 : L % 16, n = b * 16 + (e - b * 256) / 4 % width;
+        const double xv = x[e];   // (g may be x)
         double u = 0.0;
         for (int k = 0; k < shares; ++k) u += part[(int64_t)k * 16 * L + e];
         if (n == r) {
             g[e] = 0.0;
         } else {
-            g[e] = u + 2.0 * lambda_J * x[e];
-            v[0] += lambda_J * x[e] * x[e];
+            g[e] = u + 2.0 * lambda_J * xv;
+            v[0] += lambda_J * xv * xv;
         }
     }
     na_block_sum<1>(v);
@@ -395,8 +405,8 @@ k_na_gradient_sum(int64_t L, int64_t r, double lambda_J, int shares, const doubl
 // pass 4, one block: totals, h gradient and the h part of the objective.
 // A state code >= 4 seen by pass 1 makes f and the h gradient NaN; the
 // error word is returned to zero for the next call.
-__global__ void k_na_total(int64_t L, int nb1, int nb2, double lambda_h, const double *__restrict__ x,
-                           double *__restrict__ f, double *__restrict__ g, double *__restrict__ scratch)
+__global__ void k_na_total(int64_t L, int nb1, int nb2, double lambda_h, const double *x, double *f, double *g,
+                           double *__restrict__ scratch)
 {
     const double *p1 = scratch + NA_MAX_SEQS * 4;
     const double *p2 = p1 + (size_t)NA_MAX_BLOCKS * 8;
@@ -409,11 +419,11 @@ __global__ void k_na_total(int64_t L, int nb1, int nb2, double lambda_h, const d
         unsigned long long *err = reinterpret_cast<unsigned long long *>(scratch + NA_ERR_OFFSET);
         const bool bad = *err != 0ull;
         *err = 0ull;
-        const double *h = x + 16 * L;
         double fv = v[0] + v[5];
         for (int a = 0; a < 4; ++a) {
-            fv += lambda_h * h[a] * h[a];
-            g[16 * L + a] = bad ? nan("") : v[1 + a] + 2.0 * lambda_h * h[a];
+            const double h = x[16 * L + a];   // (g may be x)
+            fv += lambda_h * h * h;
+            g[16 * L + a] = bad ? nan("") : v[1 + a] + 2.0 * lambda_h * h;
         }
         *f = bad ? nan("") : fv;
     }
@@ -457,12 +467,21 @@ extern "C" int sdca_eval_noalloc(const uint8_t *states, int64_t n_seqs, int64_t 
     // Logits: slices of the loci x blocks of up to 1024 sequences, three blocks
     // per SM.  The slices' sums (4 n_seqs doubles each) go to g, whose values
     // overwrite them afterwards; where g has no room for two, one slice goes
-    // to the beliefs' own place.
+    // to the beliefs' own place.  A g that overlaps x or the weights must not
+    // be written before these have been read: then as many slices as the
+    // scratch array holds, the first in the beliefs' place.
+    const auto apart = [](const double *a, int64_t na, const double *b, int64_t nb_) {
+        const uintptr_t a0 = reinterpret_cast<uintptr_t>(a), b0 = reinterpret_cast<uintptr_t>(b);
+        return a0 + 8 * (uintptr_t)na <= b0 || b0 + 8 * (uintptr_t)nb_ <= a0;
+    };
+    const int64_t params = 16 * n_loci + 4;
+    const bool in_g = apart(g, params, x, params) && apart(g, params, weights, n_seqs);
     const int spt = (int)std::min<int64_t>(NA_MAX_SPT, (n_seqs + NA_THREADS - 1) / NA_THREADS);
     const int64_t seq_blocks = (n_seqs + (int64_t)NA_THREADS * spt - 1) / ((int64_t)NA_THREADS * spt);
     const int64_t steps = (n_loci + NA_STEP - 1) / NA_STEP;
-    int64_t slices = std::min({std::max<int64_t>(1, 456 / seq_blocks), steps, (16 * n_loci + 4) / (4 * n_seqs)});
-    double *part = g;
+    const int64_t fit = in_g ? params / (4 * n_seqs) : NA_MAX_SEQS / n_seqs;
+    int64_t slices = std::min({std::max<int64_t>(1, 456 / seq_blocks), steps, fit});
+    double *part = in_g ? g : nb;
     if (slices < 2) {
         slices = 1;
         part = nb;

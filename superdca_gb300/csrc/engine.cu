@@ -804,8 +804,8 @@ int ws_begin(sdca_handle *h, const std::vector<int32_t> &bs)
             const int64_t M = (int64_t)G * P.L, rows = std::min<int64_t>(WS_ROWS, WS_G * P.L);
             Timed t(h, SDCA_K_OTHER, (int)((M + rows - 1) / rows + 1), G);
             for (int64_t r0 = 0; r0 < M; r0 += rows)
-                mlp_infer(h->ws_params, h->ws_wb, h->ws_feats + r0 * MLP_IN, std::min(rows, M - r0),
-                          h->ws_out + r0 * MLP_OUT, h->ws_err, h->stream);
+                CK(mlp_infer(h->ws_params, h->ws_wb, h->ws_feats + r0 * MLP_IN, std::min(rows, M - r0),
+                             h->ws_out + r0 * MLP_OUT, h->ws_err, h->stream));
             launch_ws_scatter((int)P.L, P.Dp, h->ws_idx, h->ws_idx + WS_G, G, h->ws_out, h->ws_params,
                               P.b_eff / (2.0 * P.lambda_J), h->wa, h->ws_xmax, h->stream);
         }
@@ -1584,7 +1584,7 @@ int dual_ws_rows(sdca_handle *h, int nW, const int32_t *l_W)
         const int n = std::min(h->dws_cap, nW - c0);
         launch_dual_ws_feats(h->rstate, l_W + c0, n, (int)P.N, P.Nx, (int)P.L, h->w, h->knn, h->knn_d, h->dws_feats,
                              h->stream);
-        mlp_infer(h->ws_params, h->ws_wb, h->dws_feats, (int64_t)n * P.Nx, h->dws_out, h->ws_err, h->stream);
+        CK(mlp_infer(h->ws_params, h->ws_wb, h->dws_feats, (int64_t)n * P.Nx, h->dws_out, h->ws_err, h->stream));
         launch_dual_ws_r(l_W + c0, n, (int)P.N, P.Nx, h->dws_out, h->ws_params, h->ws_alpha, h->wf, h->R, h->stream);
     }
     CKL();

@@ -293,8 +293,8 @@ void launch_dual_to_wa(const Problem &P, const SlotDev *sd, const int32_t *list,
 // outputs (M x MLP_OUT) in the blob's output units; *err is set when a wait
 // of the kernel gives up
 void mlp_pack(const float *p_dev, void *wb, cudaStream_t st);
-void mlp_infer(const float *p_dev, const void *wb, const float *X, int64_t M, float *out, int *err,
-               cudaStream_t st);
+cudaError_t mlp_infer(const float *p_dev, const void *wb, const float *X, int64_t M, float *out, int *err,
+                      cudaStream_t st);
 int64_t packed_words(int64_t L);   // 64-bit words per sequence of the packed states (distances, weights)
 void launch_distances(const uint8_t *X, int64_t ld, int N, int L, uint64_t *packed, int32_t *dist,
                       cudaStream_t st);

@@ -20,7 +20,6 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
-#include <mutex>
 #include <random>
 #include <string>
 #include <vector>
@@ -606,19 +605,22 @@ int bwd_blocks(int64_t M)
     return (int)std::min<int64_t>(152, (M + r - 1) / r);
 }
 
-cudaError_t bwd_configure()
+// A kernel's limit of dynamic shared memory, which belongs to the current
+// device: raised by every call that launches it (a host call of about a
+// microsecond), so that each device of a process has it and every call that
+// cannot raise it says so.
+template <typename Kernel> cudaError_t allow_smem(Kernel *k, int bytes)
 {
-    static std::once_flag once;
-    static cudaError_t e = cudaSuccess;
-    std::call_once(once, [] { e = cudaFuncSetAttribute(k_mlp_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, BW_SMEM); });
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) cudaGetLastError();   // (reported by the call, not left pending)
     return e;
 }
 
-// the gradient's partial sums (bwd_blocks(M) x MLP_NPAR) and the loss
+// the gradient's partial sums (bwd_blocks(M) x MLP_NPAR) and the loss (after
+// allow_smem)
 void backward(cudaStream_t st, const float *p, const int32_t *idx, const float *X, const float *T, int64_t M,
               const Scratch &s, float *part, double *loss)
 {
-    if (bwd_configure() != cudaSuccess) return;   // the caller's launch check reports it
     k_mlp_bwd<<<bwd_blocks(M), BW_THREADS, BW_SMEM, st>>>(M, bwd_tile_rows(M), idx, X, T, p, s.out, s.h1, s.h2, part, loss);
 }
 
@@ -654,20 +656,12 @@ void mlp_pack(const float *p_dev, void *wb, cudaStream_t st)
 
 namespace {
 
-cudaError_t mt_configure()
-{
-    static std::once_flag once;
-    static cudaError_t e = cudaSuccess;
-    std::call_once(once, [] { e = cudaFuncSetAttribute(k_mlp_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM); });
-    return e;
-}
-
-// the fused forward over M rows: outputs, and the FP32 activations when h1, h2 are given
+// the fused forward over M rows (after allow_smem): outputs, and the FP32
+// activations when h1, h2 are given
 void mt_forward(const float *p_dev, const void *wb, const int32_t *idx, const float *X, int64_t M, float *out,
                 float *h1, float *h2, int *err, cudaStream_t st)
 {
     if (M <= 0) return;
-    if (mt_configure() != cudaSuccess) return;   // the caller's launch check reports it
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 152;
@@ -679,9 +673,12 @@ void mt_forward(const float *p_dev, const void *wb, const int32_t *idx, const fl
 
 } // namespace
 
-void mlp_infer(const float *p_dev, const void *wb, const float *X, int64_t M, float *out, int *err, cudaStream_t st)
+cudaError_t mlp_infer(const float *p_dev, const void *wb, const float *X, int64_t M, float *out, int *err,
+                      cudaStream_t st)
 {
-    mt_forward(p_dev, wb, nullptr, X, M, out, nullptr, nullptr, err, st);
+    const cudaError_t e = allow_smem(k_mlp_tc, MT_SMEM);
+    if (e == cudaSuccess) mt_forward(p_dev, wb, nullptr, X, M, out, nullptr, nullptr, err, st);
+    return e;
 }
 
 } // namespace sdca
@@ -703,6 +700,7 @@ int sdca_mlp_grad(const float *params, const float *X, const float *T, int64_t M
     float *part = d.alloc<float>((size_t)bwd_blocks(M) * MLP_NPAR);
     double *l = d.alloc<double>(1);
     if (!d.ok) return mfail("device allocation failed"), SDCA_E_NOMEM;
+    MK(allow_smem(k_mlp_bwd, BW_SMEM));
     MK(cudaMemcpy(p, params, sizeof(float) * MLP_BLOB_SIZE, cudaMemcpyHostToDevice));
     MK(cudaMemcpy(x, X, sizeof(float) * M * MLP_IN, cudaMemcpyHostToDevice));
     MK(cudaMemcpy(t, T, sizeof(float) * M * MLP_OUT, cudaMemcpyHostToDevice));
@@ -732,7 +730,7 @@ int sdca_mlp_predict(const float *params, const float *X, int64_t M, float *out)
     MK(cudaMemcpy(x, X, sizeof(float) * M * MLP_IN, cudaMemcpyHostToDevice));
     MK(cudaMemset(err, 0, sizeof(int)));
     mlp_pack(p, wb, 0);
-    mlp_infer(p, wb, x, M, o, err, 0);
+    MK(mlp_infer(p, wb, x, M, o, err, 0));
     MK(cudaGetLastError());
     int e = 0;
     MK(cudaMemcpy(&e, err, sizeof(int), cudaMemcpyDeviceToHost));
@@ -757,6 +755,8 @@ int sdca_mlp_train(float *params, const float *X, const float *T, int64_t M, int
     __nv_bfloat16 *wb = d.alloc<__nv_bfloat16>(MT_WB_ELEMS);
     int *err = d.alloc<int>(1);
     if (!d.ok) return mfail("device allocation failed"), SDCA_E_NOMEM;
+    MK(allow_smem(k_mlp_tc, MT_SMEM));
+    MK(allow_smem(k_mlp_bwd, BW_SMEM));
     MK(cudaMemset(err, 0, sizeof(int)));
     MK(cudaMemcpy(p, params, sizeof(float) * MLP_BLOB_SIZE, cudaMemcpyHostToDevice));
     MK(cudaMemcpy(x, X, sizeof(float) * M * MLP_IN, cudaMemcpyHostToDevice));

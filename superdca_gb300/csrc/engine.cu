@@ -2564,7 +2564,10 @@ int sdca_set_targets(sdca_handle *h, const uint8_t *targets, int64_t n_target_lo
     }
     int rc = SDCA_OK;
     do {
+        // (k_transpose reads whole rows: the padding past the last locus is zero)
         if (cudaMemsetAsync(h->TT, 0, (size_t)n_target_loci * P.Nx, h->stream) != cudaSuccess ||
+            (LTx > n_target_loci && cudaMemset2DAsync(tmp + n_target_loci, LTx, 0, LTx - n_target_loci, P.N,
+                                                      h->stream) != cudaSuccess) ||
             cudaMemcpy2DAsync(tmp, LTx, targets, n_target_loci, n_target_loci, P.N, cudaMemcpyHostToDevice,
                               h->stream) != cudaSuccess ||
             cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream) != cudaSuccess) {

@@ -2,75 +2,12 @@
 need more dynamic shared memory than a launch gets by default, and the raised
 limit belongs to one device: every device needs it, and a call that cannot
 raise it has to say so each time, not only the first.  The library runs here
-on a stand-in for the CUDA runtime (preloaded: host memory, two devices, no
-kernel runs) that refuses what the runtime refuses.  No GPU."""
+on the stand-in for the CUDA runtime (cuda_standin.py).  No GPU."""
 import json
-import os
-import shutil
-import subprocess
-import sys
 
 import pytest
 
-ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-
-RUNTIME = r"""
-#include <cstdlib>
-#include <cstring>
-#include <map>
-#include <utility>
-
-struct Dim3 { unsigned x, y, z; };
-struct Config { Dim3 grid, block; size_t smem; void *stream; };
-static int device = 0, refuse_limit = 0, pending = 0, launches = 0;
-static std::map<std::pair<int, const void *>, int> limit;
-static Config config;
-
-extern "C" {
-void standin_device(int d) { device = d; }
-void standin_refuse_limit(int r) { refuse_limit = r; }
-int standin_launches() { const int n = launches; launches = 0; return n; }
-
-int cudaGetDevice(int *d) { *d = device; return 0; }
-int cudaDeviceGetAttribute(int *v, int, int) { *v = 152; return 0; }
-int cudaMalloc(void **p, size_t n) { *p = std::calloc(1, n); return *p ? 0 : 2; }
-int cudaFree(void *p) { std::free(p); return 0; }
-int cudaMemcpy(void *d, const void *s, size_t n, int) { std::memcpy(d, s, n); return 0; }
-int cudaMemset(void *d, int v, size_t n) { std::memset(d, v, n); return 0; }
-int cudaGetLastError() { const int e = pending; pending = 0; return e; }
-int cudaPeekAtLastError() { return pending; }
-const char *cudaGetErrorString(int) { return "refused"; }
-int cudaFuncSetAttribute(const void *f, int, int value)
-{
-    if (refuse_limit) return pending = 1;
-    limit[{device, f}] = value;
-    return 0;
-}
-unsigned __cudaPushCallConfiguration(Dim3 g, Dim3 b, size_t smem, void *st)
-{
-    config = {g, b, smem, st};
-    return 0;
-}
-int __cudaPopCallConfiguration(Dim3 *g, Dim3 *b, size_t *smem, void *st)
-{
-    *g = config.grid;
-    *b = config.block;
-    *smem = config.smem;
-    *static_cast<void **>(st) = config.stream;
-    return 0;
-}
-int __cudaGetKernel(const void **k, const void *f) { *k = f; return 0; }
-static int launch(const void *f, size_t smem)
-{
-    const auto it = limit.find({device, f});
-    if (smem > 48 * 1024 && (it == limit.end() || (size_t)it->second < smem)) return pending = 1;
-    ++launches;
-    return 0;
-}
-int __cudaLaunchKernel(const void *k, Dim3, Dim3, void **, size_t smem, void *) { return launch(k, smem); }
-int cudaLaunchKernel(const void *k, Dim3, Dim3, void **, size_t smem, void *) { return launch(k, smem); }
-}
-"""
+import cuda_standin
 
 CHILD = r"""
 import ctypes as C, json, sys
@@ -103,21 +40,8 @@ print(json.dumps(res))
 def run(tmp_path_factory, engine_lib):
     from superdca_gb300 import _lib
 
-    cxx = shutil.which("g++") or shutil.which("c++")
-    if not cxx:
-        pytest.skip("no host C++ compiler")
-    d = tmp_path_factory.mktemp("runtime")
-    (d / "standin.cpp").write_text(RUNTIME)
-    so = str(d / "standin.so")
-    subprocess.run([cxx, "-O1", "-std=c++17", "-shared", "-fPIC", str(d / "standin.cpp"), "-o", so], check=True)
-
-    def call(steps):
-        out = subprocess.run([sys.executable, "-c", CHILD, _lib.LIB_PATH, so, json.dumps(steps)], capture_output=True,
-                             text=True, env=dict(os.environ, LD_PRELOAD=so), timeout=120)
-        assert out.returncode == 0, out.stderr[-2000:]
-        return json.loads(out.stdout.strip().splitlines()[-1])
-
-    return call
+    so = cuda_standin.build(tmp_path_factory.mktemp("runtime"))
+    return lambda steps: json.loads(cuda_standin.run(so, CHILD, _lib.LIB_PATH, so, json.dumps(steps)))
 
 
 def test_every_device_gets_the_limit(run):

@@ -28,6 +28,7 @@
 #include "kdig.cuh"
 #include "kernels_common.cuh"
 #include "linesearch.h"
+#include "quotient.h"
 
 namespace sdca {
 namespace {
@@ -1086,9 +1087,8 @@ __device__ void write_summary(const DualCtl &S, DualSum &o)
 // working alone waits for the FP64 pipe's latency some 200 times at k = 10:
 // the control kernel took 42 us whatever the number of slots (64 slots of
 // 1000 x 4001, 512 of 3000 x 94,000), most of it here; with the warp's lanes
-// the kernel takes 21 us.  Divisions by the diagonal are a multiplication by
-// its reciprocal and one residual correction (the quotient to the last bit
-// or two).  R, YY, sg, yg: shared memory, as there.  False (on every lane)
+// the kernel takes 21 us.  Divisions by the diagonal go by its reciprocal
+// (quotient_by: Markstein's correction).  R, YY, sg, yg: shared memory, as there.  False (on every lane)
 // if R is singular; else lane a < k holds coefS[a], coefY[a].
 __device__ __forceinline__ bool warp_compact_coeffs(int k, const double *R, const double *YY, const double *sg,
                                                     const double *yg, double gamma, double &coefS, double &coefY)
@@ -1097,14 +1097,10 @@ __device__ __forceinline__ bool warp_compact_coeffs(int k, const double *R, cons
     const double diag = R[a * k + a];
     if (__any_sync(0xffffffffu, !(diag != 0.0))) return false;
     const double inv = 1.0 / diag;
-    auto quotient = [&](double v) {
-        const double q = v * inv;
-        return fma(fma(-q, diag, v), inv, q);
-    };
     // t = R^-1 sg (back substitution)
     double v = sg[a], t = 0.0;
     for (int j = k - 1; j >= 0; --j) {
-        const double tj = __shfl_sync(0xffffffffu, quotient(v), j);
+        const double tj = __shfl_sync(0xffffffffu, quotient_by(v, diag, inv), j);
         if (lane == j) t = tj;
         if (lane < j) v = fma(-R[a * k + j], tj, v);
     }
@@ -1120,7 +1116,7 @@ __device__ __forceinline__ bool warp_compact_coeffs(int k, const double *R, cons
     // p = R^-T w (forward substitution)
     double p = 0.0;
     for (j = 0; j < k; ++j) {
-        const double pj = __shfl_sync(0xffffffffu, quotient(v), j);
+        const double pj = __shfl_sync(0xffffffffu, quotient_by(v, diag, inv), j);
         if (lane == j) p = pj;
         if (lane > j && lane < k) v = fma(-R[j * k + a], pj, v);
     }

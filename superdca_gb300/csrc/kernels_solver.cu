@@ -14,6 +14,7 @@
 #include "df.cuh"
 #include "engine.h"
 #include "kernels_common.cuh"
+#include "quotient.h"
 
 namespace sdca {
 
@@ -35,8 +36,8 @@ __device__ __forceinline__ double4 load4(const double *v, int64_t o)
 }
 
 // Bound by FP64 issue (one instruction per 64 clocks and quarter of an SM).
-// Three exponentials instead of four and four quotients from one reciprocal,
-// the same bits: 80 -> 70 us for 64 slots of 3000 sequences, 31 -> 26 of 1000.
+// Three exponentials instead of four (the same bits) and four quotients from
+// one reciprocal (the same bits down to 2^-960, quotient.h): 80 -> 70 us for 64 slots of 3000 sequences, 31 -> 26 of 1000.
 template <typename UT, typename LT>
 __global__ void __launch_bounds__(TRIAL_THREADS)
 k_trial(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N, int64_t Nx,
@@ -68,14 +69,9 @@ k_trial(const SlotDev *__restrict__ sd, const int32_t *__restrict__ list, int N,
         const int sr = rstate[o];
         const double wi = w[i];
         f += wi * (lse - l[sr]);
-        // e / z, rounded correctly, from the reciprocal (Markstein, IBM J. Res.
-        // Dev. 34(1), 1990): a quotient within a unit and its exact remainder
+        // e / z (z in [1, 4])
         const double rz = __drcp_rn(z);
-        auto quotient = [&](double v) {
-            const double q = v * rz;
-            return fma(fma(-q, z, v), rz, q);
-        };
-        const double q0 = quotient(x0), q1 = quotient(x1), q2 = quotient(x2);
+        const double q0 = quotient_by(x0, z, rz), q1 = quotient_by(x1, z, rz), q2 = quotient_by(x2, z, rz);
         const double p[4] = {k == 0 ? rz : q0, k == 1 ? rz : k == 0 ? q0 : q1, k == 2 ? rz : k < 2 ? q1 : q2, k == 3 ? rz : q2};
         double r[4];
 #pragma unroll

@@ -591,7 +591,8 @@ def engine_arm(args):
     Dp = ((16 * L + 4 + 63) // 64) * 64
     iso = None
     if args.form == "dual" and lanes > 1:
-        # Launches of different lanes overlap, so their event durations
+        # Launches of different lanes overlap, so their durations (the kernels'
+        # own time stamps in replayed rounds, launch and drain outside)
         # include the GPU share the other lanes take.  One untimed step on a
         # single lane (after the timed region) gives the isolated durations:
         # the class that dominates there is the one the roofline reports.

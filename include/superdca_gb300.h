@@ -89,7 +89,9 @@ typedef struct {
 
 typedef struct {
     double solve_ms;           /* device time of the last sdca_solve* call (CUDA events) */
-    double kernel_ms[8];       /* device time per kernel class (see SDCA_K_*) */
+    double kernel_ms[8];       /* device time per kernel class (see SDCA_K_*): CUDA events, or, for the dual
+                                  form's replayed rounds, the kernels' own time stamps, which leave out
+                                  launch and drain (about 1 % of a 1 ms kernel) */
     int64_t kernel_launches[8];/* kernels launched per class */
     int64_t kernel_units[8];   /* slot-passes per class: one unit = one target locus
                                   through one launch of that class */
@@ -128,7 +130,10 @@ int sdca_set_alignment(sdca_handle *h, const uint8_t *states, const double *weig
 /* Sequence reweighting on the GPU: weights of SuperDCA's calculate_weights
  * (plmDCA_optimizer_parameters.hpp:39-98) with identity = (L - d_ij)/L, d_ij
  * the number of loci whose codes differ.  mult: per-sequence multiplicities
- * or NULL. */
+ * or NULL.  Its device workspace, shared with the dual form's sdca_set_alignment
+ * and the learned starts, stays with the handle: the states packed two bits a
+ * locus and two doubles a sequence (70 MB at 3000 x 94,000, 1.1 GB at 16,383 x
+ * 262,144). */
 int sdca_compute_weights(sdca_handle *h, const uint8_t *states, const double *mult,
                          double threshold, double *weights_out);
 

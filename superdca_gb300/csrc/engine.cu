@@ -547,8 +547,11 @@ int upload_list(sdca_handle *h, const std::vector<int32_t> &lst)
 
 // The mirror (small: whole) and the list behind it in one copy.  Two copies
 // here and a separate one of the error word in fetch_acc were a good part of
-// what stands between two trials of the plain and tensor-core forms (solves of
-// 64 loci: 1000 x 4001 98 -> 91 ms, 3000 x 10,000 337 -> 302).
+// what stands between two trials of the plain and tensor-core forms: medians of
+// repeated solves of 64 loci went from 98 to 91 ms in the plain form at 1000 x
+// 4001.  In the tensor-core form at 3000 x 10,000 a solve takes 249 to 366 ms,
+// by the number of rounds its slowest locus happens to need, and the medians
+// (337 and 302) lie within that.
 int upload_mirror(sdca_handle *h, const std::vector<int32_t> &lst)
 {
     const size_t sd = sizeof(SlotDev) * h->P.Bmax, bytes = sd + sizeof(int32_t) * lst.size();
@@ -1419,14 +1422,14 @@ int phase_step(sdca_handle *h)
 // runs on the device (k_dual_linesearch: restart test, More-Thuente search
 // and its trials; K rho; k_dual_grad: the accept and the gradient; k_dual_control:
 // history, tests and the next direction's coefficients; k_dual_direction).
-// The host, once per round, reads a summary of every slot (one stream
-// event, taken before the direction kernel so that the host's work overlaps
-// it), batches the exact max-norm checks, forms the solutions of stopped
+// The host, once per round, reads a summary of every slot (published to
+// pinned memory by the control kernel, whose sequence number the host polls,
+// or copied, with an event, where rounds are not replayed; either way before
+// the direction kernel, so that the host's work overlaps it), batches the exact max-norm checks, forms the solutions of stopped
 // slots, retires finished loci and admits new ones.
 
 double dot4h(const double *a, const double *b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3]; }
 
-// A new locus in slot b: the device state of its solver.
 // Stopped slots of the dual form: x in the engine layout (J = Phi^T a_x,
 // J_rr = 0, h = eta_x), then the final evaluation.  J is formed exactly:
 // the logits K a_x are O(1) while sum_j |K_ij a_j| is hundreds, so a

@@ -97,12 +97,12 @@ struct SlotDev {
 constexpr int DV_X = 0, DV_D = 1, DV_G = 2, DV_S = 4;
 constexpr int DOT_Y = 2 * MAXHIST;  // dual-form dots by ring position: s at [p], y at [DOT_Y + p]
 
-// Dual form: the solver state of one slot, owned by the device while the
-// slot iterates.  The host writes it once when a locus enters the slot and
-// reads the DualSum summary after each round; the line-search kernel, the
+// Dual form: the solver state of one slot, owned by the device.
+// k_slots_begin writes it when a locus enters the slot, and the host reads
+// the DualSum summary after each round; the line-search kernel, the
 // accept and gradient kernels and the control kernel advance it.
 enum DualPhase {
-    DC_EVAL0 = 0,   // start point evaluated by k_trial_dual: the next gradient pass is the first
+    DC_EVAL0 = 0,   // start point evaluated by k_dual_eval: the next gradient pass is the first
     DC_STEP = 1,    // a direction is ready: line search, accept, gradient pass
     DC_STOP = 2,    // stopped (status set): the host forms the solution
 };

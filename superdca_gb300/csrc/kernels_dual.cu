@@ -1087,7 +1087,7 @@ __device__ void write_summary(const DualCtl &S, DualSum &o)
 // working alone waits for the FP64 pipe's latency some 200 times at k = 10:
 // the control kernel took 42 us whatever the number of slots (64 slots of
 // 1000 x 4001, 512 of 3000 x 94,000), most of it here; with the warp's lanes
-// the kernel takes 21 us.  Divisions by the diagonal go by its reciprocal
+// here and in the bookkeeping it takes 12 (64 slots).  Divisions by the diagonal go by its reciprocal
 // (quotient_by: Markstein's correction).  R, YY, sg, yg: shared memory, as there.  False (on every lane)
 // if R is singular; else lane a < k holds coefS[a], coefY[a].
 __device__ __forceinline__ bool warp_compact_coeffs(int k, const double *R, const double *YY, const double *sg,
@@ -1653,10 +1653,17 @@ void launch_dual_linesearch(const Problem &P, DualCtl *ctl, const int32_t *list,
                        unsigned long long *ts)
 {
     if (n <= 0) return;
-    // Few slots: larger blocks, while every SM still holds its slots' blocks
-    // at once.  64 slots of 1000 x 4001: 51, 39 and 36 us
-    // with 64, 128 and 256 threads; 233 slots of 200 x 500: 44, 42 and 43.
-    // SDCA_LS_THREADS overrides the rule.
+    // Few slots: larger blocks, which shorten a search's passes over its
+    // sequences.  The line lies at one block per SM (152 slots), below which
+    // the larger block won at every size measured (above it for 1000 sequences
+    // and more, not for 616 at 304 slots); us a launch with 64, 128 and 256
+    // threads (trees of N sequences, a mean over whole solves):
+    //   N      64 slots      152           200           304
+    //   616    42 34 32      44 35 35      43 36 34      45 36 37
+    //   1000   54 41 38      53 39 36      56 44 41      55 42 40
+    //   3000   126 79 62     123 76 62     143 87 68     134 88 70
+    // and 233 slots of 200 x 500: 44, 42 and 43.  SDCA_LS_THREADS overrides the
+    // rule.
     static const int forced = [] {
         const char *e = std::getenv("SDCA_LS_THREADS");
         const int v = e ? std::atoi(e) : 0;

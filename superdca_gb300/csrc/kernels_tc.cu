@@ -16,8 +16,8 @@
 //     128-byte-swizzled K-major layout the MMA reads (the one-hot matrix never
 //     exists in HBM: 1 byte per locus is read instead of 8), fence to the async
 //     proxy, arrive on full_a[s];
-//   * warp 1, one thread: tcgen05.mma kind::f16 (M128 N128 K16, FP32
-//     accumulators in TMEM): A x B_hi and then A x B_lo into the same
+//   * warp 1, uniformly, its elected lane issuing: tcgen05.mma kind::f16 (M128
+//     K16, N fitted to the live columns, FP32 accumulators in TMEM): A x B_hi and then A x B_lo into the same
 //     accumulator (or, with exact fp16 operands, a second N tile in the lo
 //     slot); tcgen05.commit frees the stage;
 //   * warps 11-14: tcgen05.ld the accumulator and store it, scaled back
